@@ -132,7 +132,8 @@ def tune(quick=False, out: Path = TABLE, log=print, sizes=None, precisions=None)
                         rule = [code, unit, n, dims, threads, slots, dp, cluster, per_sm]
                         arr = _rules_array([rule])
                         lib.hdb_set_tuning(arr.ctypes.data_as(ctypes.c_void_p), 1)
-                        plan = Plan(offsets, dims, min_cluster_size=5, min_samples=ms, precision=precision)
+                        plan = Plan(offsets, dims, min_cluster_size=5, min_samples=ms, precision=precision,
+                                    test_flags=_lib.HDB_FLAG_NO_SPARSE)
                         desc = json.loads(plan.describe())["classes"][0]
                         if (desc["threads"], desc["vertices_per_thread"], desc["register_dims"],
                                 desc["cluster"], desc["per_sm"]) != (threads, slots, dp, cluster, per_sm):

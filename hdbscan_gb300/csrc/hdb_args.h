@@ -56,6 +56,10 @@ struct ForwardArgs {
     // broadcast, so every CTA's first wait runs out (nothing is in flight then).
     int64_t wait_limit_ns;
     int stall_first_ticket;
+    // General path behind the sparse one: only windows with a non-zero flag are
+    // done (null = all; only[n_only] = 0: none is).
+    const int32_t* only;
+    int n_only;
 };
 
 struct DistanceArgs {
@@ -68,6 +72,8 @@ struct DistanceArgs {
     void* dist;                  // packed blocks
     const int64_t* dist_offsets; // [B]
     int32_t* status;
+    const int32_t* only;         // as ForwardArgs::only
+    int n_only;
 };
 
 struct CoreArgs {
@@ -82,7 +88,67 @@ struct CoreArgs {
     void* core;                  // [T]
     int32_t* core_nbr;           // [T] or null
     int32_t* status;
+    const int32_t* only;         // as ForwardArgs::only
+    int n_only;
 };
+
+// Sparse path (hdb_sparse.cuh): one launch group covers the `n_windows` windows
+// of `queue` (descending sizes, at most nmax points each).  Per-point arrays
+// are indexed by packed point row, per-window ones by window.
+struct SparseArgs {
+    const void* X;
+    const int64_t* offsets;
+    const int32_t* queue;
+    int n_windows;
+    int nmax;
+    int64_t T;                   // points of the whole batch (stride of the per-level arrays)
+    int D;
+    int ms;
+    int unit_core;
+    int32_t* flags;              // [B+1] 1 = the window takes the general path; [B] = any window does
+    int n_flags;                 // B
+    float* y;                    // [T, D] float64 input rounded to float32 around each window's first point
+    uint32_t* range;             // [B] float bits of max |x - x0| (float64)
+    void* dist;                  // distance blocks (float32 values, see sparse_block)
+    const int64_t* dist_offsets;
+    uint16_t* knn_idx;           // [T, list] nearest neighbours by (distance, index), self included
+    float* knn_d;                // [T, list]
+    int list;                    // row stride of the lists (8, 16, 32 or 64)
+    int keep;                    // valid entries of each list (<= list)
+    void* core;                  // [T] Real
+    int32_t* core_nbr;           // [T]
+    float* core_up;              // [T] core distance rounded up (float32: core itself)
+    float* core_down;            // [T] core distance rounded down (float32: core itself)
+    uint16_t* part;              // [T] component number after the list rounds
+    int32_t* parts;              // [B] their count
+    unsigned long long* edges;   // [T] tree edges found so far
+    unsigned long long* table;   // least edge between each two components, parts^2 per window
+    const int64_t* table_offsets;  // [B]
+    uint16_t* level_comp;        // [kSparseLevels, T] component (its representative vertex) after each merge round
+    float* level_max_v;          // [kSparseLevels, T] by vertex: largest tree edge on the way up
+    uint16_t* level_end_v;       // [kSparseLevels, T] by vertex: end of the component's leaf interval
+    uint16_t* perm;              // [T] leaf order -> vertex
+    float* level_max;            // the same in leaf order
+    uint16_t* level_end;
+    int32_t* levels;             // [B] merge rounds
+    uint16_t* pos;               // [T] vertex -> leaf position
+    int32_t* light_count;        // [B] light edges other than star edges
+    uint32_t* light_uv;          // [T * light_cap] u | v << 16
+    void* light_w;               // [T * light_cap] Real
+    int light_cap;               // kept per point
+    int32_t* star_count;         // [B] star edges the order needs
+    uint32_t* star_uv;           // [T * star_cap] x | u << 16, of weight core_x
+    unsigned long long* star_mask;  // [T] list positions of each point's star
+    int star_cap;
+    uint16_t* edge_rank;         // [T * (light_cap + star_cap)]
+    uint32_t* adj;               // [T * (light_cap + star_cap) * 2] adjacency that shared memory does not hold
+};
+// Components that the list rounds may leave.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int sparse_parts_cap(int n) { return n < 256 ? 32 : n / 8; }
+constexpr int kSparseLevels = 12;  // every merge round at least halves the components: 2^12 points
 
 constexpr int kBackwardWarps = 8;  // backward kernel: warps (32 linkage rows each) per CTA
 

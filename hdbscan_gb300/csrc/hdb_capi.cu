@@ -26,6 +26,7 @@
 #include "../../include/hdbscan_gb300.h"
 #include "hdb_args.h"
 #include "hdb_registry.h"
+#include "hdb_sparse.h"
 
 namespace {
 
@@ -52,8 +53,17 @@ struct CoreLaunch {
     size_t select_smem = 0;
 };
 
+// Windows of the sparse path that are launched together (hdb_sparse.cuh).
+struct SparseGroup {
+    std::vector<int> windows;  // descending n
+    int nmax = 0;
+    size_t queue_off = 0;
+    int priority = 0;
+};
+
 struct WindowClass {
     const hdb::ForwardVariant* fv = nullptr;
+    bool general = false;      // does the sparse path's flagged windows, after all else
     int x_in_smem = 0;
     int n_arenas = 1;
     hdb::ForwardLayout layout{};
@@ -86,6 +96,14 @@ struct hdb_plan {
     std::vector<int64_t> offsets;
     const hdb::PrecisionKernels* k = nullptr;
     std::vector<WindowClass> classes;
+    std::vector<SparseGroup> groups;        // windows on the sparse path
+    int list = 0, keep = 0;                 // neighbour list stride and length
+    int light_cap = 0, star_cap = 0;        // light and star edges per point
+    std::vector<int64_t> table_offsets;     // per window (entries) of the component tables
+    size_t t_table = 0, t_flags = 0, t_range = 0, t_light_count = 0, t_star_count = 0;
+    size_t w_y = 0, w_knn_idx = 0, w_knn_d = 0, w_core_up = 0, w_core_down = 0, w_part = 0, w_parts = 0, w_edges = 0, w_table = 0, w_level_comp = 0, w_level_max_v = 0,
+           w_level_end_v = 0, w_perm = 0, w_pos = 0, w_level_max = 0, w_level_end = 0, w_levels = 0, w_light_uv = 0, w_light_w = 0,
+           w_star_uv = 0, w_star_mask = 0, w_edge_rank = 0, w_adj = 0;
     std::vector<int32_t> tiles;             // (window, ti, tj), grouped by class
     std::vector<int64_t> dist_offsets;      // per window (elements), -1 if not materialized
     int64_t dist_elems = 0;
@@ -136,6 +154,16 @@ int real_bytes(int precision) { return precision == HDB_F32 ? 4 : 8; }
 constexpr size_t kChunks = 4;     // pipeline depth for large matrix-variant classes
 constexpr size_t kMinChunk = 8;   // windows per chunk at least
 constexpr int kTile128MinN = 384;  // float32 matrix classes from this size use 128x128 distance tiles
+
+// Windows of fewer points stay on the general path (their dense loop is short).
+constexpr int kSparseMinN = 16;
+constexpr unsigned kNoSparseFlags =
+    HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
+constexpr unsigned kGeneralGrid = 152 * 8;  // CTAs of a general-path launch that may find nothing to do
+
+// Windows of one bin share their launches; shared memory, threads and grids
+// are sized by the largest.
+int sparse_bin(int n) { return n <= 128 ? 0 : (n <= 512 ? 1 : (n <= 1024 ? 2 : (n <= 2048 ? 3 : 4))); }
 
 cudaError_t raise_smem_limit(const void* func, size_t bytes) { return hdb::raise_dynamic_smem(func, bytes); }
 
@@ -295,24 +323,50 @@ int build_plan(hdb_plan* p) {
         ctas -= chosen[w]->cluster - 1;
         chosen[w] = single;
     }
+    // The sparse path: float64 windows that the table gives one CTA.  All of
+    // them share one general class, which does the windows it flags.
+    std::vector<char> sparse(p->B, 0);
+    int sparse_nmax = 0;
+    p->list = hdb::sparse_list(p->precision, p->ms);
+    if (p->precision == HDB_F64 && p->list && !(p->flags & kNoSparseFlags)) {
+        for (int w : order) sparse[w] = size_of(w) >= kSparseMinN && chosen[w]->cluster == 1;
+        for (int w : order)
+            if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
+        bool fits = true;
+        if (sparse_nmax) HDB_CUDA(hdb::sparse_prepare(p->precision, sparse_nmax, (size_t)optin, &fits));
+        if (!fits) {
+            std::fill(sparse.begin(), sparse.end(), 0);
+            sparse_nmax = 0;
+        }
+    }
     for (int w : order) {
         const int n = size_of(w);
+        if (sparse[w]) {
+            // Descending sizes: a group ends where the next size bin begins.
+            if (p->groups.empty() || sparse_bin(n) != sparse_bin(p->groups.back().nmax)) p->groups.emplace_back();
+            p->groups.back().windows.push_back(w);
+            p->groups.back().nmax = std::max(p->groups.back().nmax, n);
+            chosen[w] = choose_variant(k, p->precision, sparse_nmax, p->D, unit, true);
+            if (!chosen[w]) return fail(HDB_E_INVALID, "no matrix variant for a window of " + std::to_string(n) + " points");
+        }
         const hdb::ForwardVariant* fv = chosen[w];
         size_t budget = 0;
         int rc = smem_budget(fv, optin, per_sm_smem, &budget);
         if (rc) return rc;
         hdb::ForwardLayout layout{};
-        if (!fv->layout(n, unit, budget, &layout))
+        if (!fv->layout(sparse[w] ? sparse_nmax : n, unit, budget, &layout))
             return fail(HDB_E_INVALID, "window of " + std::to_string(n) + " points exceeds shared memory");
         WindowClass* cls = nullptr;
         for (auto& c : p->classes)
-            if (c.fv == fv && c.x_in_smem == layout.x_in_smem && c.n_arenas == layout.n_arenas) { cls = &c; break; }
+            if (c.fv == fv && c.x_in_smem == layout.x_in_smem && c.n_arenas == layout.n_arenas &&
+                c.general == (sparse[w] != 0)) { cls = &c; break; }
         if (!cls) {
             p->classes.emplace_back();
             cls = &p->classes.back();
             cls->fv = fv;
             cls->x_in_smem = layout.x_in_smem;
             cls->n_arenas = layout.n_arenas;
+            cls->general = sparse[w] != 0;
         }
         cls->windows.push_back(w);
         cls->nmax = std::max(cls->nmax, n);
@@ -324,7 +378,7 @@ int build_plan(hdb_plan* p) {
         std::vector<WindowClass> chunked;
         for (auto& c : p->classes) {
             const size_t W = c.windows.size();
-            const size_t parts = (c.fv->dp == 0 && W >= 2 * kMinChunk) ? std::min<size_t>(kChunks, W / kMinChunk) : 1;
+            const size_t parts = (c.fv->dp == 0 && !c.general && W >= 2 * kMinChunk) ? std::min<size_t>(kChunks, W / kMinChunk) : 1;
             for (size_t part = 0; part < parts; ++part) {
                 WindowClass piece = c;
                 const size_t lo = W * part / parts, hi = W * (part + 1) / parts;
@@ -335,9 +389,24 @@ int build_plan(hdb_plan* p) {
             }
         }
         p->classes.swap(chunked);
+        // Sparse groups of larger windows likewise: one chunk's Prim and
+        // hierarchy run while the next one's distances are computed.
+        std::vector<SparseGroup> groups;
+        for (auto& g : p->groups) {
+            const size_t W = g.windows.size();
+            const size_t parts = (g.nmax > 512 && W >= 2 * kMinChunk) ? std::min<size_t>(kChunks, W / kMinChunk) : 1;
+            for (size_t part = 0; part < parts; ++part) {
+                SparseGroup piece;
+                piece.windows.assign(g.windows.begin() + W * part / parts, g.windows.begin() + W * (part + 1) / parts);
+                for (int w : piece.windows) piece.nmax = std::max(piece.nmax, size_of(w));
+                groups.push_back(std::move(piece));
+            }
+        }
+        p->groups.swap(groups);
     }
-    std::stable_sort(p->classes.begin(), p->classes.end(),
-                     [](const WindowClass& a, const WindowClass& b) { return a.nmax > b.nmax; });
+    std::stable_sort(p->classes.begin(), p->classes.end(), [](const WindowClass& a, const WindowClass& b) {
+        return a.general != b.general ? b.general : a.nmax > b.nmax;
+    });
 
     // ---- distance blocks and tiles for matrix-variant windows --------------
     p->dist_offsets.assign(p->B, -1);
@@ -441,7 +510,26 @@ int build_plan(hdb_plan* p) {
         c.ticket = (int)i;
         queue.insert(queue.end(), c.windows.begin(), c.windows.end());
     }
+    for (auto& g : p->groups) {
+        g.queue_off = queue.size();
+        queue.insert(queue.end(), g.windows.begin(), g.windows.end());
+    }
     p->t_queue = put(image, cursor, queue);
+    if (!p->groups.empty()) {
+        const std::vector<int32_t> zeros((size_t)p->B + 1, 0);
+        p->table_offsets.assign(p->B + 1, 0);
+        for (auto& g : p->groups)
+            for (int w : g.windows) {
+                const int64_t c = hdb::sparse_parts_cap(size_of(w));
+                p->table_offsets[w] = p->table_offsets[p->B];
+                p->table_offsets[p->B] += c * c;
+            }
+        p->t_table = put(image, cursor, p->table_offsets);
+        p->t_flags = put(image, cursor, zeros);
+        p->t_range = put(image, cursor, zeros);
+        p->t_light_count = put(image, cursor, zeros);
+        p->t_star_count = put(image, cursor, zeros);
+    }
     p->t_tickets = put(image, cursor, tickets);
     p->t_tiles = put(image, cursor, p->tiles);
     for (auto& cls : p->classes)
@@ -467,23 +555,64 @@ int build_plan(hdb_plan* p) {
     ws += (size_t)p->dist_elems * rb;
     p->w_prep = ws = align_up(ws, 256);
     if (p->prepared) ws += (size_t)p->T * (size_t)p->D * rb;
+    if (!p->groups.empty()) {
+        p->keep = unit ? 8 : std::min(p->list, std::max(p->ms + 3, 8));
+        // About one to three of each per point in ordinary data; more send a window to the general path.
+        p->light_cap = 12;
+        p->star_cap = unit ? 0 : 8;
+        const size_t per_point = (size_t)(p->light_cap + p->star_cap);
+        const size_t T = (size_t)p->T, L = hdb::kSparseLevels;
+        auto take = [&](size_t bytes) {
+            const size_t at = align_up(ws, 256);
+            ws = at + bytes;
+            return at;
+        };
+        if (p->precision == HDB_F64) {
+            p->w_y = take(T * (size_t)p->D * sizeof(float));
+            p->w_core_up = take(T * sizeof(float));
+            p->w_core_down = take(T * sizeof(float));
+        }
+        p->w_knn_idx = take(T * (size_t)p->list * sizeof(uint16_t));
+        p->w_knn_d = take(T * (size_t)p->list * sizeof(float));
+        p->w_part = take(T * sizeof(uint16_t));
+        p->w_parts = take((size_t)p->B * sizeof(int32_t));
+        p->w_edges = take(T * sizeof(unsigned long long));
+        p->w_table = take((size_t)p->table_offsets[p->B] * sizeof(unsigned long long));
+        p->w_level_comp = take(T * L * sizeof(uint16_t));
+        p->w_level_max_v = take(T * L * sizeof(float));
+        p->w_level_end_v = take(T * L * sizeof(uint16_t));
+        p->w_perm = take(T * sizeof(uint16_t));
+        p->w_level_max = take(T * L * sizeof(float));
+        p->w_level_end = take(T * L * sizeof(uint16_t));
+        p->w_levels = take((size_t)p->B * sizeof(int32_t));
+        p->w_pos = take(T * sizeof(uint16_t));
+        p->w_light_uv = take(T * (size_t)p->light_cap * sizeof(uint32_t));
+        p->w_light_w = take(T * (size_t)p->light_cap * rb);
+        p->w_star_uv = take(T * (size_t)p->star_cap * sizeof(uint32_t));
+        p->w_star_mask = take(unit ? 0 : T * sizeof(unsigned long long));
+        p->w_edge_rank = take(T * per_point * sizeof(uint16_t));
+        p->w_adj = take(2 * T * per_point * sizeof(uint32_t));
+    }
     p->ws_bytes = align_up(std::max<size_t>(ws, 256), 256);
 
     HDB_CUDA(cudaEventCreateWithFlags(&p->uploaded, cudaEventDisableTiming));
 
     // ---- streams for concurrent classes ------------------------------------
-    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && p->classes.size() > 1;
+    const size_t forks = p->classes.size() + p->groups.size();
+    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && forks > (p->groups.empty() ? 1 : 2);
     if (fork) {
         int least = 0, greatest = 0;  // numerically: greatest <= least
         HDB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        for (size_t i = 0; i < p->classes.size(); ++i) {
+        for (size_t i = 0; i < forks; ++i) {
             cudaStream_t s;
-            const int priority = std::min(least, greatest + (int)i);
-            p->classes[i].priority = priority;
+            const size_t g = i < p->groups.size() ? i : i - p->groups.size();
+            const int priority = std::min(least, greatest + (int)g);
+            if (i < p->groups.size()) p->groups[i].priority = priority;
+            else p->classes[g].priority = priority;
             HDB_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
             p->aux.push_back(s);
         }
-        for (size_t i = 0; i < 2 * p->classes.size(); ++i) {
+        for (size_t i = 0; i < 2 * forks; ++i) {
             cudaEvent_t e;
             HDB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
             p->events.push_back(e);
@@ -574,64 +703,14 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         return fail(HDB_E_INVALID, "cl_parent needs cl_birth, cl_stability, cl_selected, point_parent, n_clusters");
 
     const bool fork = !p->aux.empty() && !spans;
-    for (size_t i = 0; i < p->classes.size(); ++i) {
-        const WindowClass& c = p->classes[i];
-        // 1. distance blocks of this class's matrix-variant windows (caller's stream)
-        if (c.n_tiles) {
-            hdb::DistanceArgs a{};
-            a.X = X;
-            a.offsets = d_offsets;
-            a.tiles = reinterpret_cast<const int32_t*>(ws + p->t_tiles) + 3 * c.tiles_first;
-            a.n_tiles = (int)c.n_tiles;
-            a.tile = c.tile;
-            a.D = p->D;
-            a.dist = dist;
-            a.dist_offsets = d_dist_off;
-            a.status = status;
-            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_DISTANCE, stream));
-            HDB_CUDA(k.launch_distance(a, a.n_tiles, stream, c.priority));
-            if (spans) HDB_CUDA(spans->end(stream));
-        }
-        // 2. core distances of its windows (caller's stream)
-        for (const auto& cl : c.cores) {
-            hdb::CoreArgs a{};
-            a.X = X;
-            a.offsets = d_offsets;
-            a.items = reinterpret_cast<const int32_t*>(ws + cl.items_off);
-            a.n_items = (int)(cl.items.size() / 2);
-            a.D = p->D;
-            a.ms = p->ms;
-            a.dist = cl.matrix ? dist : nullptr;
-            a.dist_offsets = d_dist_off;
-            a.core = core;
-            a.core_nbr = core_nbr;
-            a.status = status;
-            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_CORE, stream));
-            if (cl.cv) HDB_CUDA(cl.cv->launch(a, a.n_items, stream, c.priority));
-            else HDB_CUDA(k.launch_select(a, a.n_items, cl.select_smem, stream, c.priority));
-            if (spans) HDB_CUDA(spans->end(stream));
-        }
-        cudaStream_t s = stream;
-        if (fork) {
-            s = p->aux[i];
-            HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
-            HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * i], 0));
-        }
-        // 3. the persistent forward over its queue
+    const int32_t* only = p->groups.empty() ? nullptr : reinterpret_cast<const int32_t*>(ws + p->t_flags);
+    auto forward_args = [&]() {
         hdb::ForwardArgs a{};
         a.X = X;
         a.offsets = d_offsets;
-        a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
-        a.queue_len = (int)c.windows.size();
-        a.ticket = reinterpret_cast<int32_t*>(ws + p->t_tickets) + c.ticket;
         a.D = p->D;
         a.mcs = p->mcs;
         a.unit_core = unit ? 1 : 0;
-        a.x_in_smem = c.x_in_smem;
-        a.n_arenas = c.layout.n_arenas;
-        a.arena_stride = (int)c.layout.arena_stride;
-        a.x_off = (int)c.layout.x_off;
-        a.core_off = (int)c.layout.core_off;
         a.eps = p->eps;
         a.core = unit ? nullptr : core;
         a.dist = dist;
@@ -654,20 +733,176 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.probabilities = ex->probabilities;
         a.cl_size = ex->cl_size;
         a.point_lambda = ex->point_lambda;
+        a.method = (p->flags & HDB_FLAG_LEAF) ? 1 : 0;
+        a.allow_single = (p->flags & HDB_FLAG_ALLOW_SINGLE) ? 1 : 0;
+        return a;
+    };
+    // ---- sparse path: distances, lists and cores on the caller's stream, the
+    // rest of each group on its own ---------------------------------------------
+    for (size_t i = 0; i < p->groups.size(); ++i) {
+        const SparseGroup& g = p->groups[i];
+        hdb::SparseArgs a{};
+        a.X = X;
+        a.offsets = d_offsets;
+        a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + g.queue_off;
+        a.n_windows = (int)g.windows.size();
+        a.nmax = g.nmax;
+        a.T = p->T;
+        a.D = p->D;
+        a.ms = p->ms;
+        a.unit_core = unit ? 1 : 0;
+        a.flags = reinterpret_cast<int32_t*>(ws + p->t_flags);
+        a.n_flags = p->B;
+        a.y = reinterpret_cast<float*>(ws + p->w_y);
+        a.range = reinterpret_cast<uint32_t*>(ws + p->t_range);
+        a.dist = dist;
+        a.dist_offsets = d_dist_off;
+        a.knn_idx = reinterpret_cast<uint16_t*>(ws + p->w_knn_idx);
+        a.knn_d = reinterpret_cast<float*>(ws + p->w_knn_d);
+        a.list = p->list;
+        a.keep = p->keep;
+        a.core = core;
+        a.core_nbr = core_nbr;
+        a.core_up = p->precision == HDB_F64 ? reinterpret_cast<float*>(ws + p->w_core_up) : static_cast<float*>(core);
+        a.core_down = p->precision == HDB_F64 ? reinterpret_cast<float*>(ws + p->w_core_down) : static_cast<float*>(core);
+        a.part = reinterpret_cast<uint16_t*>(ws + p->w_part);
+        a.parts = reinterpret_cast<int32_t*>(ws + p->w_parts);
+        a.edges = reinterpret_cast<unsigned long long*>(ws + p->w_edges);
+        a.table = reinterpret_cast<unsigned long long*>(ws + p->w_table);
+        a.table_offsets = reinterpret_cast<const int64_t*>(ws + p->t_table);
+        a.level_comp = reinterpret_cast<uint16_t*>(ws + p->w_level_comp);
+        a.level_max_v = reinterpret_cast<float*>(ws + p->w_level_max_v);
+        a.level_end_v = reinterpret_cast<uint16_t*>(ws + p->w_level_end_v);
+        a.perm = reinterpret_cast<uint16_t*>(ws + p->w_perm);
+        a.level_max = reinterpret_cast<float*>(ws + p->w_level_max);
+        a.level_end = reinterpret_cast<uint16_t*>(ws + p->w_level_end);
+        a.levels = reinterpret_cast<int32_t*>(ws + p->w_levels);
+        a.pos = reinterpret_cast<uint16_t*>(ws + p->w_pos);
+        a.light_count = reinterpret_cast<int32_t*>(ws + p->t_light_count);
+        a.light_uv = reinterpret_cast<uint32_t*>(ws + p->w_light_uv);
+        a.light_w = ws + p->w_light_w;
+        a.light_cap = p->light_cap;
+        a.star_count = reinterpret_cast<int32_t*>(ws + p->t_star_count);
+        a.star_uv = reinterpret_cast<uint32_t*>(ws + p->w_star_uv);
+        a.star_mask = reinterpret_cast<unsigned long long*>(ws + p->w_star_mask);
+        a.star_cap = p->star_cap;
+        a.edge_rank = reinterpret_cast<uint16_t*>(ws + p->w_edge_rank);
+        a.adj = reinterpret_cast<uint32_t*>(ws + p->w_adj);
+        const hdb::ForwardArgs fa = forward_args();
+        auto stage = [&](hdb::SparseStage st, int phase, cudaStream_t s) -> int {
+            if (spans) HDB_CUDA(spans->begin(phase, s));
+            HDB_CUDA(hdb::sparse_launch(p->precision, st, a, &fa, s, g.priority));
+            if (spans) HDB_CUDA(spans->end(s));
+            return HDB_OK;
+        };
+        const bool wide = p->precision == HDB_F64;
+        int rc = HDB_OK;
+        if (wide) rc = stage(hdb::SparseStage::kNarrow, HDB_PHASE_PREPARE, stream);
+        if (!rc && wide) rc = stage(hdb::SparseStage::kTiles, HDB_PHASE_DISTANCE, stream);
+        if (!rc) rc = stage(hdb::SparseStage::kRows, HDB_PHASE_CORE, stream);
+        if (!rc && wide && !unit) rc = stage(hdb::SparseStage::kCore, HDB_PHASE_CORE, stream);
+        if (rc) return rc;
+        cudaStream_t s = stream;
+        if (fork) {
+            s = p->aux[i];
+            HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
+            HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * i], 0));
+        }
+        rc = stage(hdb::SparseStage::kForest, HDB_PHASE_FORWARD, s);
+        if (!rc) rc = stage(hdb::SparseStage::kBetween, HDB_PHASE_FORWARD, s);
+        if (!rc) rc = stage(hdb::SparseStage::kTree, HDB_PHASE_FORWARD, s);
+        if (!rc) rc = stage(hdb::SparseStage::kLight, HDB_PHASE_FORWARD, s);
+        if (!rc && !unit) rc = stage(hdb::SparseStage::kStar, HDB_PHASE_FORWARD, s);
+        if (!rc && wide) rc = stage(hdb::SparseStage::kWeights, HDB_PHASE_FORWARD, s);
+        if (!rc) rc = stage(hdb::SparseStage::kPrim, HDB_PHASE_FORWARD, s);
+        if (rc) return rc;
+        if (fork) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], s));
+    }
+    auto join = [&](size_t first, size_t last) -> int {
+        if (fork)
+            for (size_t i = first; i < last; ++i) HDB_CUDA(cudaStreamWaitEvent(stream, p->events[2 * i + 1], 0));
+        return HDB_OK;
+    };
+    const size_t n_groups = p->groups.size();
+    size_t joined = 0;
+    for (size_t i = 0; i < p->classes.size(); ++i) {
+        const WindowClass& c = p->classes[i];
+        // The general class (the last one) starts when everything else is done.
+        if (c.general) {
+            int rc = join(0, n_groups + i);
+            if (rc) return rc;
+            joined = n_groups + i;
+        }
+        const unsigned grid_limit = c.general ? kGeneralGrid : 0xffffffffu;
+        // 1. distance blocks of this class's matrix-variant windows (caller's stream)
+        if (c.n_tiles) {
+            hdb::DistanceArgs a{};
+            a.X = X;
+            a.offsets = d_offsets;
+            a.tiles = reinterpret_cast<const int32_t*>(ws + p->t_tiles) + 3 * c.tiles_first;
+            a.n_tiles = (int)c.n_tiles;
+            a.tile = c.tile;
+            a.D = p->D;
+            a.dist = dist;
+            a.dist_offsets = d_dist_off;
+            a.status = status;
+            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_DISTANCE, stream));
+            a.only = c.general ? only : nullptr;
+            a.n_only = p->B;
+            HDB_CUDA(k.launch_distance(a, (int)std::min<unsigned>((unsigned)a.n_tiles, grid_limit), stream, c.priority));
+            if (spans) HDB_CUDA(spans->end(stream));
+        }
+        // 2. core distances of its windows (caller's stream)
+        for (const auto& cl : c.cores) {
+            hdb::CoreArgs a{};
+            a.X = X;
+            a.offsets = d_offsets;
+            a.items = reinterpret_cast<const int32_t*>(ws + cl.items_off);
+            a.n_items = (int)(cl.items.size() / 2);
+            a.D = p->D;
+            a.ms = p->ms;
+            a.dist = cl.matrix ? dist : nullptr;
+            a.dist_offsets = d_dist_off;
+            a.core = core;
+            a.core_nbr = core_nbr;
+            a.status = status;
+            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_CORE, stream));
+            a.only = c.general ? only : nullptr;
+            a.n_only = p->B;
+            if (cl.cv) HDB_CUDA(cl.cv->launch(a, (int)std::min<unsigned>((unsigned)a.n_items, grid_limit), stream, c.priority));
+            else HDB_CUDA(k.launch_select(a, a.n_items, cl.select_smem, stream, c.priority));
+            if (spans) HDB_CUDA(spans->end(stream));
+        }
+        cudaStream_t s = stream;
+        const size_t f = n_groups + i;
+        const bool forked = fork && !c.general;
+        if (forked) {
+            s = p->aux[f];
+            HDB_CUDA(cudaEventRecord(p->events[2 * f], stream));
+            HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * f], 0));
+        }
+        // 3. the persistent forward over its queue
+        hdb::ForwardArgs a = forward_args();
+        a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
+        a.queue_len = (int)c.windows.size();
+        a.ticket = reinterpret_cast<int32_t*>(ws + p->t_tickets) + c.ticket;
+        a.x_in_smem = c.x_in_smem;
+        a.n_arenas = c.layout.n_arenas;
+        a.arena_stride = (int)c.layout.arena_stride;
+        a.x_off = (int)c.layout.x_off;
+        a.core_off = (int)c.layout.core_off;
+        a.only = c.general ? only : nullptr;
+        a.n_only = p->B;
         if (p->flags & HDB_FLAG_TEST_STALL) {
             a.stall_first_ticket = 1;
             a.wait_limit_ns = 1000000;  // 1 ms
         }
-        a.method = (p->flags & HDB_FLAG_LEAF) ? 1 : 0;
-        a.allow_single = (p->flags & HDB_FLAG_ALLOW_SINGLE) ? 1 : 0;
         if (spans) HDB_CUDA(spans->begin(HDB_PHASE_FORWARD, s));
         HDB_CUDA(c.fv->launch(a, c.grid, c.smem, s, c.priority));
         if (spans) HDB_CUDA(spans->end(s));
-        if (fork) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], s));
+        if (forked) HDB_CUDA(cudaEventRecord(p->events[2 * f + 1], s));
     }
-    if (fork)
-        for (size_t i = 0; i < p->classes.size(); ++i) HDB_CUDA(cudaStreamWaitEvent(stream, p->events[2 * i + 1], 0));
-    return HDB_OK;
+    return join(joined, n_groups + p->classes.size() - (p->groups.empty() ? 0 : 1));
 }
 
 // ---- plan cache of the dense seam -----------------------------------------
@@ -861,25 +1096,35 @@ int hdb_plan_destroy(hdb_plan_t* p) {
 
 size_t hdb_plan_workspace_bytes(const hdb_plan_t* p) { return p ? p->ws_bytes : 0; }
 
-// Sum over a class's windows of n (power 1) or n^2 (power 2).
-static int64_t class_points(const hdb_plan* p, const WindowClass& c, int power) {
-    int64_t total = 0;
-    for (int w : c.windows) {
-        const int64_t n = p->offsets[w + 1] - p->offsets[w];
-        total += power == 2 ? n * n : n;
-    }
-    return total;
-}
-
 int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
     if (!p || !buffer || !size) return fail(HDB_E_INVALID, "describe needs a plan and a buffer");
     std::string s = "{\"precision\":\"" + std::string(p->precision == HDB_F32 ? "float32" : "float64") +
                     "\",\"windows\":" + std::to_string(p->B) + ",\"points\":" + std::to_string(p->T) +
                     ",\"dims\":" + std::to_string(p->D) + ",\"workspace_bytes\":" + std::to_string(p->ws_bytes) +
-                    ",\"distance_tiles\":" + std::to_string(p->tiles.size() / 3) + ",\"classes\":[";
+                    ",\"distance_tiles\":" + std::to_string(p->tiles.size() / 3) +
+                    // int32 [windows] in the workspace after a forward: 1 = the window left the sparse path.
+                    ",\"general_flags_offset\":" + std::to_string(p->groups.empty() ? -1 : (int64_t)p->t_flags) +
+                    ",\"classes\":[";
+    bool first_class = true;
+    auto points = [&](const std::vector<int>& windows, int power) {
+        int64_t total = 0;
+        for (int w : windows) {
+            const int64_t n = p->offsets[w + 1] - p->offsets[w];
+            total += power == 2 ? n * n : n;
+        }
+        return std::to_string(total);
+    };
+    for (const auto& g : p->groups) {
+        s += (first_class ? "" : ",") + std::string("{\"variant\":\"sparse\",\"cluster\":1,\"list\":") +
+             std::to_string(p->list) + ",\"light_edges_per_point\":" + std::to_string(p->light_cap) + ",\"priority\":" +
+             std::to_string(g.priority) + ",\"windows\":" + std::to_string(g.windows.size()) + ",\"points\":" +
+             points(g.windows, 1) + ",\"sum_n2\":" + points(g.windows, 2) + ",\"nmax\":" + std::to_string(g.nmax) + "}";
+        first_class = false;
+    }
     for (size_t i = 0; i < p->classes.size(); ++i) {
         const auto& c = p->classes[i];
-        s += (i ? "," : "") + std::string("{\"threads\":") + std::to_string(c.fv->threads) +
+        if (c.general) continue;
+        s += (first_class ? "" : ",") + std::string("{\"threads\":") + std::to_string(c.fv->threads) +
              ",\"vertices_per_thread\":" + std::to_string(c.fv->v) + ",\"register_dims\":" +
              std::to_string(c.fv->dp) + ",\"cluster\":" + std::to_string(c.fv->cluster) +
              ",\"per_sm\":" + std::to_string(c.fv->per_sm) +
@@ -888,14 +1133,16 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
              ",\"distance_tiles\":" + std::to_string(c.n_tiles) + ",\"tile\":" + std::to_string(c.tile) +
              ",\"priority\":" + std::to_string(c.priority) +
              ",\"windows\":" + std::to_string(c.windows.size()) + ",\"points\":" +
-             std::to_string(class_points(p, c, 1)) + ",\"sum_n2\":" + std::to_string(class_points(p, c, 2)) +
+             points(c.windows, 1) + ",\"sum_n2\":" + points(c.windows, 2) +
              ",\"nmax\":" + std::to_string(c.nmax) + ",\"smem\":" +
              std::to_string(c.smem) + ",\"grid\":" + std::to_string(c.grid) + "}";
+        first_class = false;
     }
     s += "],\"core\":[";
     bool first = true;
     for (const auto& cls : p->classes)
         for (const auto& c : cls.cores) {
+            if (cls.general) continue;
             s += (first ? "" : ",") + std::string("{\"kernel\":\"") +
                  (c.cv ? (c.matrix ? "core_matrix" : "core_points") : "core_select") + "\",\"k\":" +
                  std::to_string(c.cv ? c.cv->k : 0) + ",\"register_dims\":" + std::to_string(c.cv ? c.cv->dp : 0) +

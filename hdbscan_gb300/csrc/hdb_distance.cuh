@@ -59,14 +59,13 @@ template <> struct DistVec<double> {
 // float64: 64 registers, 4 CTAs per SM (the integer-pipe arithmetic is
 // latency-bound at 3 CTAs; 5 would spill).
 template <typename Real>
-__global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_kernel(const DistanceArgs args) {
+__device__ __forceinline__ void distance_tile(const DistanceArgs& args, int tile) {
     using T = RealTraits<Real>;
     constexpr int KC = DistVec<Real>::KC;
     __shared__ __align__(16) Real s_i[KC][kDistTile];
     __shared__ __align__(16) Real s_j[KC][kDistTile];
-    const int tile = blockIdx.x;
-    if (tile >= args.n_tiles) return;
     const int w = args.tiles[3 * tile], ti = args.tiles[3 * tile + 1], tj = args.tiles[3 * tile + 2];
+    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const int D = args.D;
@@ -209,6 +208,14 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_k
         }
     }
     if (__syncthreads_or(overflow) && tid == 0) atomic_status(args.status, kOverflow);
+}
+
+// One CTA a tile, or (behind the sparse path, where most launches find no
+// flagged window) a fixed grid over all tiles.
+template <typename Real>
+__global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_kernel(const DistanceArgs args) {
+    if (args.only && !args.only[args.n_only]) return;
+    for (int tile = blockIdx.x; tile < args.n_tiles; tile += gridDim.x) distance_tile<Real>(args, tile);
 }
 
 // Float32 blocks of larger windows: 128x128 tiles, 256 threads, 8x8 pairs per
@@ -489,16 +496,15 @@ __device__ __forceinline__ Key key_select(bool c, Key a, Key b) {
 }
 
 template <typename Real, int K>
-__global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_core_rows_kernel(const CoreArgs args) {
+__device__ __forceinline__ void core_rows_item(const CoreArgs& args, int item) {
     static_assert(K <= 64, "at most two list entries per lane");
     using T = RealTraits<Real>;
     using Key = typename T::Bits;
     constexpr int E = (K + 31) / 32;     // list entries per lane
     constexpr Key kNone = (Key)~(Key)0;  // above every distance key (and +inf's)
     constexpr int U = 8;                 // row chunks per group of loads
-    const int item = blockIdx.x;
-    if (item >= args.n_items) return;
     const int w = args.items[2 * item], r0 = args.items[2 * item + 1];
+    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const Real* __restrict__ Dw = static_cast<const Real*>(args.dist) + args.dist_offsets[w];
@@ -579,6 +585,13 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_core_rows_kernel(cons
             }
         }
     }
+}
+
+// One CTA an item, or a fixed grid over all items behind the sparse path.
+template <typename Real, int K>
+__global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_core_rows_kernel(const CoreArgs args) {
+    if (args.only && !args.only[args.n_only]) return;
+    for (int item = blockIdx.x; item < args.n_items; item += gridDim.x) core_rows_item<Real, K>(args, item);
 }
 
 // Any ms: one CTA (256 threads) per row; the row is computed (or read) into

@@ -428,6 +428,18 @@ __device__ __noinline__ void tree_window(const ForwardArgs& args, unsigned char*
     if (args.stage_ns && lane == 0) args.stage_ns[8 * w + 7] = global_ns();
 }
 
+// Next window of the queue for this CTA (queue_len = none left).  Behind the
+// sparse path only flagged windows are taken.
+__device__ __forceinline__ int next_ticket(const ForwardArgs& args) {
+    if (!args.only) return atomicAdd(args.ticket, 1);
+    if (!args.only[args.n_only]) return args.queue_len;
+    int item;
+    do {
+        item = atomicAdd(args.ticket, 1);
+    } while (item < args.queue_len && !args.only[args.queue[item]]);
+    return item;
+}
+
 struct WindowMeta {
     int w;      // window index, -1 = queue exhausted
     int n;
@@ -495,7 +507,7 @@ __global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid
     Real* s_core = reinterpret_cast<Real*>(smem + args.core_off);
 
     if constexpr (kJoinSort) {
-        if (tid == 0) s_item = atomicAdd(args.ticket, 1);
+        if (tid == 0) s_item = next_ticket(args);
     }
     for (int k = 0; k < (1 << 30); ++k) {
         const int b = nb == 2 ? (k & 1) : 0;
@@ -503,7 +515,7 @@ __global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid
         if constexpr (kJoinSort) {
             if (tid == 0) s_flags[par] = 0;  // the ticket was taken before the last hand-off
         } else {
-            if (tid == 0) { s_item = atomicAdd(args.ticket, 1); s_flags[par] = 0; }
+            if (tid == 0) { s_item = next_ticket(args); s_flags[par] = 0; }
         }
         bar_sync(kBarStart, PT);
         const int item = s_item;
@@ -574,7 +586,7 @@ __global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid
         if constexpr (kJoinSort) {
             // The next window's ticket, taken before the hand-off so that the
             // CTA's last window is known as such.
-            if (tid == 0) s_item = atomicAdd(args.ticket, 1);
+            if (tid == 0) s_item = next_ticket(args);
         }
         bar_sync(kBarStart, PT);
         const int flags = s_flags[par];

@@ -1,0 +1,1354 @@
+// Sparse path: the exact minimum spanning tree without a dense Prim loop.
+//
+// Prim over the dense graph is a serial chain of n-1 row reads and block-wide
+// argmins (matrix variant, float32: 1.0 us a step at 2048 points, 1.4 us at
+// 4096), and float64 distances are bound by the FP64 pipe.  Both go away once
+// the few edges that can matter are known:
+//   1. a spanning tree T', minimal up to roundings, is built from each point's
+//      nearest neighbours by rounds of component merging (Boruvka), and from one
+//      pass over the distances between the components whose lists are used up;
+//   2. an edge heavier than the largest edge on the T' path between its ends
+//      lies in no minimum spanning tree (the filter of Karger, Klein and
+//      Tarjan 1995), so one pass over all pairs keeps only the light ones.  The
+//      path maximum comes from the merge rounds alone: the tree whose nodes are
+//      the components of every round, with the edge each component chose as the
+//      weight to its parent, has the same path maxima as T' (King 1997);
+//   3. Prim's vertex order follows from the light edges: every edge of minimal
+//      weight across any cut is light, so each step sees the same minimum and
+//      the same lowest vertex of that weight as over the dense graph.  A
+//      vertex's source (strict '<' keeps the older one) is then the first
+//      visited end of its light edges of that weight.
+//
+// Most light edges are ties: max(core_x, core_u, d) = core_x for every point u
+// among x's ms nearest with a smaller core (x's star).  They need no distance,
+// they are in the neighbour lists, and one of them for each component that the
+// star touches below core_x is enough for the order (hdb_sparse_star_kernel).
+//
+// float64: the pass over all pairs and the neighbour lists use float32
+// distances with a proven bound (sparse_bound); every comparison that decides
+// something takes the safe side, and all weights, core distances and ties come
+// from exact float64 arithmetic on the few pairs that remain.  float32: the
+// distance blocks are the exact ones and the bounds are zero.
+//
+// A window that does not fit (more light edges than the workspace holds, as
+// with many equal distances; neighbours that the bound cannot tell apart;
+// values outside the range of the bound; infinite distances) sets its flag and
+// takes the general path, whose kernels look at the flags.
+#pragma once
+#include "hdb_common.cuh"
+#include "hdb_distance.cuh"
+#include "hdb_forward.cuh"
+
+namespace hdb {
+
+constexpr int kSparseRowsCta = 32;   // rows per CTA of the neighbour kernel
+constexpr int kLightRows = 16;       // rows per CTA of the light-edge kernel
+
+__device__ __forceinline__ void sparse_flag(const SparseArgs& a, int w) {
+    a.flags[w] = 1;
+    a.flags[a.n_flags] = 1;
+}
+
+// The window's float32 distance block: its own block (float32), or the first
+// half of the float64 block's place (the general path overwrites it later).
+template <typename Real>
+__device__ __forceinline__ float* sparse_block(const SparseArgs& a, int w) {
+    return reinterpret_cast<float*>(static_cast<Real*>(a.dist) + a.dist_offsets[w]);
+}
+
+// Bound between a float32 distance d~ and the float64 one, d:
+// |d~ - d| <= shift + d~ * scale.  Inputs are y = RN32(x - x0), R >= |x - x0|
+// for every coordinate of the window:
+//   * each coordinate difference is off by at most 2^-23 R from the two
+//     roundings of y, so the difference vector is off by sqrt(D) 2^-23 R;
+//   * the float32 difference, its square, the D-term sum (any order, fused or
+//     not) and the root add a relative (D/2 + 3) 2^-24 to first order.
+// Both are taken 5% larger (plus some units) than that, which covers second
+// order terms, the float64 arithmetic's own rounding and the evaluation of the
+// bound itself.
+struct SparseBound {
+    float shift, scale;
+    __device__ __forceinline__ float up(float d) const {
+        return __fmaf_ru(d, __fadd_ru(1.0f, scale), shift);
+    }
+    __device__ __forceinline__ float down(float d) const {
+        return __fmaf_rd(d, __fadd_rd(1.0f, -scale), -shift);
+    }
+};
+template <typename Real>
+__device__ __forceinline__ SparseBound sparse_bound(const SparseArgs& a, int w) {
+    if constexpr (sizeof(Real) == 4) return SparseBound{0.0f, 0.0f};
+    const float R = __uint_as_float(a.range[w]);
+    return SparseBound{1.05f * sqrtf((float)a.D) * 1.1920929e-7f * R, 1.05f * (0.5f * (float)a.D + 8.0f) * 5.9604645e-8f};
+}
+
+// Exact distance of two rows in the reference's order (k-ordered sum).
+template <typename Real>
+__device__ __forceinline__ Real sparse_exact(const Real* __restrict__ xa, const Real* __restrict__ xb, int D) {
+    using T = RealTraits<Real>;
+    Real acc = Real(0);
+    int k = 0;
+    for (; k + 8 <= D; k += 8) {
+        Real p[8], q[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { p[j] = xa[k + j]; q[j] = xb[k + j]; }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const Real delta = T::sub(p[j], q[j]);
+            acc = T::add(acc, T::mul(delta, delta));
+        }
+    }
+    for (; k < D; ++k) {
+        const Real delta = T::sub(xa[k], xb[k]);
+        acc = T::add(acc, T::mul(delta, delta));
+    }
+    return T::sqrt_rn(acc);
+}
+
+// ---------------------------------------------------------------------------
+// float64 input -> float32 around the window's first point, with the window's
+// range.  One CTA per 64 rows; non-finite values and ranges outside
+// [2^-40, 2^40] (the bound assumes no overflow or underflow in float32) flag
+// the window.
+// ---------------------------------------------------------------------------
+constexpr int kNarrowRows = 64;
+
+__global__ void __launch_bounds__(256) hdb_sparse_narrow_kernel(const SparseArgs a) {
+    const int per = (a.nmax + kNarrowRows - 1) / kNarrowRows;
+    const int item = blockIdx.x / per, r0 = (blockIdx.x - item * per) * kNarrowRows;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (r0 >= n) return;
+    const int D = a.D;
+    const int rows = min(kNarrowRows, n - r0);
+    const double* __restrict__ X = static_cast<const double*>(a.X) + base * D;
+    float* __restrict__ y = a.y + (base + r0) * D;
+    const double* __restrict__ x = X + (int64_t)r0 * D;
+    uint32_t top = 0;
+    bool bad = false;
+    for (int i = threadIdx.x; i < rows * D; i += 256) {
+        const double v = x[i];
+        const double c = v - X[i % D];
+        const uint32_t mag = __float_as_uint(__double2float_ru(fabs(c)));  // NaN and infinity rank highest
+        bad |= ((uint32_t)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
+        top = max(top, mag & 0x7fffffffu);
+        y[i] = (float)c;
+    }
+    top = __reduce_max_sync(0xffffffffu, top);
+    const float R = __uint_as_float(top);
+    if (bad || !(R <= 1.0995e12f)) sparse_flag(a, w);  // also tests NaN
+    if ((threadIdx.x & 31) == 0) atomicMax(a.range + w, top);
+}
+
+// ---------------------------------------------------------------------------
+// float32 distance blocks of the narrowed input: 128x128 tiles of the upper
+// triangle, 8x8 pairs a thread, differences and fused squares in packed f32x2
+// instructions (one instruction a pair and coordinate, half of the exact
+// kernel's), mirrored like the exact blocks.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseArgs a) {
+    constexpr int KC = 32;
+    constexpr int TS = 128;
+    __shared__ __align__(16) float s_i[KC][TS];
+    __shared__ __align__(16) float s_j[KC][TS];
+    const int tmax = (a.nmax + TS - 1) / TS;
+    const int per = tmax * (tmax + 1) / 2;
+    const int item = blockIdx.x / per;
+    int t = blockIdx.x - item * per;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    // Tile t of the lower triangle row by row: (row tj, column ti <= tj).
+    int tj = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (tj * (tj + 1) / 2 > t) --tj;
+    while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
+    const int ti = t - tj * (tj + 1) / 2;
+    if (tj * TS >= n || a.flags[w]) return;
+    const int D = a.D;
+    const float* __restrict__ Y = a.y + base * D;
+    float* __restrict__ Dw = sparse_block<double>(a, w);
+    const int64_t ld = dist_ld(n);
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+    const int i0 = ti * TS, j0 = tj * TS;
+    float2 acc[8][4];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) acc[p][q] = make_float2(0.0f, 0.0f);
+    for (int k0 = 0; k0 < D; k0 += KC) {
+        {
+            const int r = tid & (TS - 1), kq = tid >> 7;
+            const int gi = i0 + r, gj = j0 + r;
+#pragma unroll
+            for (int kk = 0; kk < KC / 2; ++kk) {
+                const int k = kq * (KC / 2) + kk, gk = k0 + k;
+                s_i[k][r] = (gi < n && gk < D) ? Y[(int64_t)gi * D + gk] : 0.0f;
+                s_j[k][r] = (gj < n && gk < D) ? Y[(int64_t)gj * D + gk] : 0.0f;
+            }
+        }
+        __syncthreads();
+        const int kend = min(KC, D - k0);
+        auto step = [&](int k) {
+            float xi[8];
+            float2 xj[4];
+            DistVec<float>::load4(&s_i[k][ty * 4], xi);
+            DistVec<float>::load4(&s_i[k][64 + ty * 4], xi + 4);
+            const float4 u = *reinterpret_cast<const float4*>(&s_j[k][tx * 4]);
+            const float4 v = *reinterpret_cast<const float4*>(&s_j[k][64 + tx * 4]);
+            xj[0] = make_float2(u.x, u.y); xj[1] = make_float2(u.z, u.w);
+            xj[2] = make_float2(v.x, v.y); xj[3] = make_float2(v.z, v.w);
+#pragma unroll
+            for (int p = 0; p < 8; ++p) {
+                const float2 xa = make_float2(xi[p], xi[p]);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const float2 d = __ffma2_rn(xj[q], make_float2(-1.0f, -1.0f), xa);
+                    acc[p][q] = __ffma2_rn(d, d, acc[p][q]);
+                }
+            }
+        };
+        if (kend == KC) {
+#pragma unroll 4
+            for (int k = 0; k < KC; ++k) step(k);
+        } else {
+            for (int k = 0; k < kend; ++k) step(k);
+        }
+        __syncthreads();
+    }
+    float out[8][8];
+#pragma unroll
+    for (int p = 0; p < 8; ++p)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            out[p][2 * q] = __fsqrt_rn(acc[p][q].x);
+            out[p][2 * q + 1] = __fsqrt_rn(acc[p][q].y);
+        }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int cj = j0 + h * 64 + tx * 4;
+        if (cj < ld) {
+#pragma unroll
+            for (int p = 0; p < 8; ++p) {
+                const int gi = i0 + (p < 4 ? ty * 4 + p : 64 + ty * 4 + p - 4);
+                if (gi < n)
+                    DistVec<float>::store4(Dw + gi * ld + cj, out[p][4 * h], out[p][4 * h + 1], out[p][4 * h + 2],
+                                           out[p][4 * h + 3]);
+            }
+        }
+        if (ti != tj) {
+            const int ci = i0 + h * 64 + ty * 4;
+            if (ci < ld) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    const int gj = j0 + (q < 4 ? tx * 4 + q : 64 + tx * 4 + q - 4);
+                    if (gj < n)
+                        DistVec<float>::store4(Dw + gj * ld + ci, out[4 * h][q], out[4 * h + 1][q], out[4 * h + 2][q],
+                                               out[4 * h + 3][q]);
+                }
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Nearest-neighbour lists of every row, one warp a row, as hdb_core_rows_kernel
+// builds them (the K smallest (distance, index), ascending, position p in lane
+// p % 32).  float32 with core distances: position ms - 1 is the core distance.
+// float64: the rank ms - 1 is certain except among the entries whose bounds
+// overlap the entry at position ms - 1; their positions [c, e) go to core_nbr
+// for hdb_sparse_core_kernel.  A list that ends inside that range, or a
+// distance that is not finite, flags the window.
+// ---------------------------------------------------------------------------
+template <typename Real, int K>
+__global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(const SparseArgs a) {
+    static_assert(K <= 64, "at most two list entries per lane");
+    constexpr int E = (K + 31) / 32;
+    constexpr uint32_t kNone = 0xffffffffu;
+    constexpr int U = 8;
+    const int per = (a.nmax + kSparseRowsCta - 1) / kSparseRowsCta;
+    const int item = blockIdx.x / per, r0 = (blockIdx.x - item * per) * kSparseRowsCta;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    // float32 core distances also serve the general path of a flagged window.
+    if (r0 >= n || (sizeof(Real) == 8 && a.flags[w])) return;
+    const float* __restrict__ Dw = sparse_block<Real>(a, w);
+    const int64_t ld = dist_ld(n);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int keep = a.keep;
+    const int last = keep - 1;
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    for (int r = warp; r < kSparseRowsCta; r += kCoreRowsWarps) {
+        const int i = r0 + r;
+        if (i >= n) break;  // warp-uniform
+        const float* __restrict__ row = Dw + (int64_t)i * ld;
+        uint32_t lk[E], biggest = 0;
+        int li[E];
+        lk[0] = lane < n ? RealTraits<float>::key(__ldcg(row + lane)) : kNone;
+        biggest = lane < n ? lk[0] : 0u;
+        li[0] = lane;
+        if constexpr (E > 1) { lk[1] = kNone; li[1] = 32 + lane; }
+#pragma unroll
+        for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                const uint32_t pk = __shfl_xor_sync(0xffffffffu, lk[0], j);
+                const int pi = __shfl_xor_sync(0xffffffffu, li[0], j);
+                const bool partner_less = pk < lk[0] || (pk == lk[0] && pi < li[0]);
+                const bool keep_min = ((lane & k) == 0) == ((lane & j) == 0);
+                const bool take = keep_min ? partner_less : !partner_less;
+                lk[0] = take ? pk : lk[0];
+                li[0] = take ? pi : li[0];
+            }
+        }
+        auto at = [&](int p) {
+            const uint32_t lo = __shfl_sync(0xffffffffu, lk[0], p & 31);
+            if constexpr (E > 1) {
+                const uint32_t hi = __shfl_sync(0xffffffffu, lk[1], p & 31);
+                return p < 32 ? lo : hi;
+            }
+            return lo;
+        };
+        uint32_t tau = at(last);
+        for (int j0 = 32; j0 < n; j0 += 32 * U) {
+            uint32_t v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int j = j0 + 32 * u + lane;
+                v[u] = j < n ? RealTraits<float>::key(__ldcg(row + j)) : kNone;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (v[u] != kNone) biggest = max(biggest, v[u]);
+                unsigned bal = __ballot_sync(0xffffffffu, v[u] < tau);
+                while (bal) {
+                    const int src = __ffs(bal) - 1;
+                    bal &= bal - 1;
+                    const uint32_t ck = __shfl_sync(0xffffffffu, v[u], src);
+                    if (ck < tau) {  // warp-uniform; tau only decreases
+                        const int cj = j0 + 32 * u + src;
+                        uint32_t pk[E];
+                        int pi[E];
+                        pk[0] = __shfl_up_sync(0xffffffffu, lk[0], 1);
+                        pi[0] = __shfl_up_sync(0xffffffffu, li[0], 1);
+                        if constexpr (E > 1) {
+                            const uint32_t upk = __shfl_up_sync(0xffffffffu, lk[1], 1);
+                            const int upi = __shfl_up_sync(0xffffffffu, li[1], 1);
+                            const uint32_t endk = __shfl_sync(0xffffffffu, lk[0], 31);
+                            const int endi = __shfl_sync(0xffffffffu, li[0], 31);
+                            pk[1] = lane == 0 ? endk : upk;
+                            pi[1] = lane == 0 ? endi : upi;
+                        }
+#pragma unroll
+                        for (int h = 0; h < E; ++h) {
+                            const bool shift = (h > 0 || lane > 0) && ck < pk[h];
+                            const bool place = !shift && ck < lk[h];
+                            lk[h] = shift ? pk[h] : (place ? ck : lk[h]);
+                            li[h] = shift ? pi[h] : (place ? cj : li[h]);
+                        }
+                        tau = at(last);
+                    }
+                }
+            }
+        }
+        const bool wild = __any_sync(0xffffffffu, biggest >= 0x7f800000u);
+        const int64_t row_at = base + i;
+#pragma unroll
+        for (int h = 0; h < E; ++h) {
+            const int p = lane + 32 * h;
+            if (p < keep) {
+                a.knn_idx[row_at * a.list + p] = (uint16_t)(p < n ? li[h] : i);
+                a.knn_d[row_at * a.list + p] = __uint_as_float(p < n ? lk[h] : 0x7f800000u);
+            }
+        }
+        bool unsure = wild;
+        if (!a.unit_core) {
+            const int pos = a.ms - 1;
+            if constexpr (sizeof(Real) == 4) {
+#pragma unroll
+                for (int h = 0; h < E; ++h)
+                    if (pos == lane + 32 * h) {
+                        static_cast<float*>(a.core)[row_at] = __uint_as_float(lk[h]);
+                        a.core_nbr[row_at] = li[h];
+                    }
+                // Points as far as the core distance may follow the list's end.
+                if (at(last) <= at(pos) && keep < n) unsure = true;
+            } else {
+                const float mid = __uint_as_float(at(pos));
+                const float least = bound.down(mid), most = bound.up(mid);
+                int c = 0, e = 0;
+#pragma unroll
+                for (int h = 0; h < E; ++h) {
+                    const float d = __uint_as_float(lk[h]);
+                    const bool in = lane + 32 * h < min(keep, n);
+                    c += __popc(__ballot_sync(0xffffffffu, in && bound.up(d) < least));
+                    e += __popc(__ballot_sync(0xffffffffu, in && bound.down(d) <= most));
+                }
+                if (e >= keep && keep < n) unsure = true;  // the range may go on beyond the list
+                if (lane == 0) a.core_nbr[row_at] = c | (e << 8);
+            }
+        }
+        if (unsure && lane == 0) sparse_flag(a, w);
+    }
+}
+
+// float64 core distances: the exact distances of each row's uncertain range
+// (nearly always one entry), the right one by (distance, index).
+__global__ void __launch_bounds__(128) hdb_sparse_core_kernel(const SparseArgs a) {
+    const int per = (a.nmax + 127) / 128;
+    const int item = blockIdx.x / per, i = (blockIdx.x - item * per) * 128 + threadIdx.x;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (i >= n || a.flags[w]) return;
+    const int D = a.D;
+    const double* __restrict__ X = static_cast<const double*>(a.X) + base * D;
+    const double* __restrict__ xi = X + (int64_t)i * D;
+    const int64_t row = base + i;
+    const uint16_t* __restrict__ list = a.knn_idx + row * a.list;
+    const int range = a.core_nbr[row];
+    const int c = range & 0xff, e = range >> 8;
+    double value = 0;
+    int index = -1;
+    if (e - c == 1) {
+        index = list[c];
+        value = sparse_exact<double>(xi, X + (int64_t)index * D, D);
+    } else {
+        // The (ms - 1 - c)-th smallest of the range: repeated minimum above the last one taken.
+        double d_last = -1.0;
+        int j_last = -1;
+        for (int t = c; t <= a.ms - 1; ++t) {
+            double d_best = 0;
+            int j_best = -1;
+            for (int s = c; s < e; ++s) {
+                const int j = list[s];
+                const double d = sparse_exact<double>(xi, X + (int64_t)j * D, D);
+                const bool above = d > d_last || (d == d_last && j > j_last);
+                if (above && (j_best < 0 || d < d_best || (d == d_best && j < j_best))) { d_best = d; j_best = j; }
+            }
+            d_last = d_best;
+            j_last = j_best;
+        }
+        value = d_last;
+        index = j_last;
+    }
+    static_cast<double*>(a.core)[row] = value;
+    a.core_nbr[row] = index;
+    a.core_up[row] = __double2float_ru(value);
+    a.core_down[row] = __double2float_rd(value);
+}
+
+// ---------------------------------------------------------------------------
+// The spanning tree T' and its merge rounds, in three kernels.  Edges are
+// ordered by (weight rounded up, smaller end, larger end), so all minima below
+// are unique; T' is the minimum spanning tree of those weights, up to edges
+// taken in forced rounds.
+//
+// hdb_sparse_forest_kernel (one CTA a window): rounds in which every component
+// takes its least edge among the neighbour lists, as long as no edge outside
+// the lists can be shorter (a list ends at a known distance).  What is left,
+// typically a few percent of the points, are components whose least outgoing
+// edge is longer than some member's list reaches.
+//
+// hdb_sparse_between_kernel (all rows): the least edge between each two of
+// those components, into a table.
+//
+// hdb_sparse_tree_kernel (one CTA a window): the remaining rounds on the table;
+// then the merge rounds (Boruvka over the n-1 edges of T') and the leaf order in
+// which every component of every round is an interval.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ unsigned long long sparse_key(float wgt, int u, int v) {
+    const uint32_t lo = (uint32_t)min(u, v), hi = (uint32_t)max(u, v);
+    return ((unsigned long long)__float_as_uint(wgt) << 32) | (lo << 12) | hi;
+}
+__device__ __forceinline__ uint32_t key_weight(unsigned long long key) { return (uint32_t)(key >> 32); }
+__device__ __forceinline__ int key_low(unsigned long long key) { return (int)((uint32_t)key >> 12) & 0xfff; }
+__device__ __forceinline__ int key_high(unsigned long long key) { return (int)key & 0xfff; }
+
+__host__ __device__ inline int sparse_round(int n) { return (n + 15) & ~15; }
+__host__ __device__ inline size_t sparse_forest_smem(int n) {
+    return (size_t)sparse_round(n) * (8 + 4 + 4 + 4 + 2 + 2 + 1) + 64;
+}
+__host__ __device__ inline size_t sparse_between_smem(int n) {
+    return (size_t)sparse_round(n) * (2 + 4) + (size_t)sparse_parts_cap(n) * 8 + 64;
+}
+__host__ __device__ inline size_t sparse_tree_smem(int n) {
+    return (size_t)sparse_round(n) * (8 + 8 + 4 + 2 + 2) + 64;
+}
+
+constexpr unsigned long long kNoChoice = ~0ull;
+
+// Root (in `up`) that component r's chosen edge leads to.  Both ends choosing
+// the same edge is the only cycle: the smaller id stays the root.
+__device__ __forceinline__ int sparse_target(const unsigned long long* choice, const uint16_t* comp, int r) {
+    const unsigned long long key = choice[r];
+    if (key == kNoChoice) return r;
+    const int lo = comp[key_low(key)], hi = comp[key_high(key)];
+    const int to = lo == r ? hi : lo;
+    return (choice[to] == key && r < to) ? r : to;
+}
+__device__ __forceinline__ int sparse_root(const uint16_t* up, int r, int n) {
+    for (int guard = 0; guard < n && up[r] != r; ++guard) r = up[r];
+    return r;
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(512) hdb_sparse_forest_kernel(const SparseArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_edges;   // tree edges found
+    __shared__ int s_parts;   // components
+    __shared__ int s_next;
+    const int w = a.queue[blockIdx.x];
+    if (a.flags[w]) return;
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int cap = sparse_round(n);
+    unsigned long long* choice = reinterpret_cast<unsigned long long*>(smem);
+    float* core = reinterpret_cast<float*>(choice + cap);   // core distances rounded up
+    uint32_t* reach_v = reinterpret_cast<uint32_t*>(core + cap);  // float bits: shortest edge a point's list can miss
+    uint32_t* reach = reach_v + cap;                        // the same over a component
+    uint16_t* comp = reinterpret_cast<uint16_t*>(reach + cap);
+    uint16_t* up = comp + cap;
+    uint8_t* at = reinterpret_cast<uint8_t*>(up + cap);
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    if constexpr (sizeof(Real) == 8) {
+        // A range below 2^-40 (other than identical points) is outside the bound's domain.
+        const float R = __uint_as_float(a.range[w]);
+        if (R != 0.0f && R < 9.1e-13f) {
+            if (tid == 0) sparse_flag(a, w);
+            return;
+        }
+    }
+    const float* core_g = a.core_up;
+    const int keep = min(a.keep, n);
+    for (int u = tid; u < n; u += nt) {
+        const float c = a.unit_core ? 0.0f : core_g[base + u];
+        comp[u] = (uint16_t)u;
+        core[u] = c;
+        at[u] = 0;
+        const float end = bound.up(a.knn_d[(base + u) * a.list + keep - 1]);
+        reach_v[u] = keep == n ? 0x7f800000u : __float_as_uint(fmaxf(c, end));
+    }
+    if (tid == 0) s_edges = 0;
+    unsigned long long* edges = a.edges + base;
+    int parts = n;
+    bool forced = false;
+    for (int round = 0; round < 2 * kSparseLevels; ++round) {
+        __syncthreads();
+        for (int u = tid; u < n; u += nt) { choice[u] = kNoChoice; reach[u] = 0x7f800000u; }
+        __syncthreads();
+        for (int u = tid; u < n; u += nt) {
+            const uint16_t* __restrict__ idx = a.knn_idx + (base + u) * a.list;
+            const float* __restrict__ dd = a.knn_d + (base + u) * a.list;
+            const int cu = comp[u];
+            const float core_u = core[u];
+            unsigned long long best = kNoChoice;
+            int bv = 0;
+            bool lead = true;
+            int first = at[u];
+            for (int t = first; t < keep; ++t) {
+                const int v = idx[t];
+                if (comp[v] == cu) {  // the point itself, or already joined: never looked at again
+                    if (lead) first = t + 1;
+                    continue;
+                }
+                lead = false;
+                const float d = bound.up(dd[t]);
+                if (__float_as_uint(d) > key_weight(best)) break;
+                const unsigned long long key = sparse_key(fmaxf(fmaxf(core_u, core[v]), d), u, v);
+                if (key < best) { best = key; bv = v; }
+            }
+            at[u] = (uint8_t)first;
+            if (reach_v[u] < reach[cu]) atomicMin(&reach[cu], reach_v[u]);
+            if (best != kNoChoice) {
+                if (best < choice[cu]) atomicMin(&choice[cu], best);
+                const int cv = comp[bv];
+                if (best < choice[cv]) atomicMin(&choice[cv], best);
+            }
+        }
+        __syncthreads();
+        // An edge that the lists may have missed could be shorter: not chosen.
+        if (!forced) {
+            for (int r = tid; r < n; r += nt)
+                if (comp[r] == r && key_weight(choice[r]) > reach[r]) choice[r] = kNoChoice;
+            __syncthreads();
+        }
+        for (int r = tid; r < n; r += nt) {
+            if (comp[r] != r) continue;
+            const int to = sparse_target(choice, comp, r);
+            up[r] = (uint16_t)to;
+            if (to != r) edges[min(atomicAdd(&s_edges, 1), n - 1)] = choice[r];
+        }
+        __syncthreads();
+        for (int u = tid; u < n; u += nt) comp[u] = (uint16_t)sparse_root(up, comp[u], n);
+        const int now = n - s_edges;
+        if (now == 1) { parts = now; break; }
+        if (now == parts) {  // stalled: few enough components for the table, or joined whatever their lists say
+            if (now <= sparse_parts_cap(n)) break;
+            if (forced) break;
+            forced = true;
+        } else if (forced && now <= sparse_parts_cap(n)) {
+            parts = now;
+            break;
+        }
+        parts = now;
+    }
+    __syncthreads();
+    const int parts_cap = sparse_parts_cap(n);
+    if (parts > parts_cap) {  // unreachable: components that hold all their points' lists have 8 points or more
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    // ---- components numbered, rows sorted by them, table cleared --------------
+    uint32_t* number = reinterpret_cast<uint32_t*>(choice);
+    uint32_t* count = number + cap;
+    if (tid == 0) { s_parts = 0; s_next = 0; }
+    for (int u = tid; u < n; u += nt) count[u] = 0;
+    __syncthreads();
+    for (int u = tid; u < n; u += nt) {
+        atomicAdd(&count[comp[u]], 1u);
+        if (comp[u] == u) number[u] = (uint32_t)atomicAdd(&s_parts, 1);
+    }
+    __syncthreads();
+    for (int u = tid; u < n; u += nt)
+        if (comp[u] == u) count[u] = (uint32_t)atomicAdd(&s_next, (int)count[u]);
+    __syncthreads();
+    for (int u = tid; u < n; u += nt) {
+        const int r = comp[u];
+        a.part[base + u] = (uint16_t)number[r];
+        a.perm[base + atomicAdd(&count[r], 1u)] = (uint16_t)u;
+    }
+    unsigned long long* table = a.table + a.table_offsets[w];
+    if (parts > 1)
+        for (int e = tid; e < parts * parts; e += nt) table[e] = kNoChoice;
+    if (tid == 0) a.parts[w] = parts;
+}
+
+// The least edge between each two components: every row against all columns of
+// higher-numbered components.  A CTA takes kBetweenRows rows in component order
+// and keeps the table row of the current component in shared memory.
+constexpr int kBetweenRows = 32;
+
+template <typename Real>
+__global__ void __launch_bounds__(256) hdb_sparse_between_kernel(const SparseArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int per = (a.nmax + kBetweenRows - 1) / kBetweenRows;
+    const int item = blockIdx.x / per, p0 = (blockIdx.x - item * per) * kBetweenRows;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (p0 >= n || a.flags[w]) return;
+    const int parts = a.parts[w];
+    if (parts <= 1) return;
+    const int tid = threadIdx.x;
+    const int cap = sparse_round(n);
+    unsigned long long* least = reinterpret_cast<unsigned long long*>(smem);
+    float* core = reinterpret_cast<float*>(least + sparse_parts_cap(n));
+    uint16_t* part = reinterpret_cast<uint16_t*>(core + cap);
+    const uint32_t* least_w = reinterpret_cast<const uint32_t*>(least) + 1;  // high words: weights
+    const float* core_g = a.core_up;
+    for (int u = tid; u < n; u += 256) {
+        core[u] = a.unit_core ? 0.0f : core_g[base + u];
+        part[u] = a.part[base + u];
+    }
+    const float* __restrict__ Dw = sparse_block<Real>(a, w);
+    const int64_t ld = dist_ld(n);
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    unsigned long long* table = a.table + a.table_offsets[w];
+    const int pend = min(p0 + kBetweenRows, n);
+    int mine = -1;
+    auto flush = [&]() {
+        __syncthreads();
+        if (mine >= 0)
+            for (int c = mine + 1 + tid; c < parts; c += 256)
+                if (least[c] < table[(int64_t)mine * parts + c]) atomicMin(&table[(int64_t)mine * parts + c], least[c]);
+    };
+    __syncthreads();
+    for (int p = p0; p < pend; ++p) {
+        const int u = a.perm[base + p];
+        const int cu = part[u];
+        if (cu == parts - 1) continue;
+        if (cu != mine) {
+            flush();
+            mine = cu;
+            __syncthreads();
+            for (int c = mine + 1 + tid; c < parts; c += 256) least[c] = table[(int64_t)mine * parts + c];
+            __syncthreads();
+        }
+        const float* __restrict__ row = Dw + (int64_t)u * ld;
+        const float core_u = core[u];
+        constexpr int U = 8;
+        for (int v0 = tid; v0 < n; v0 += 256 * U) {
+            float d[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) d[q] = v0 + 256 * q < n ? __ldcg(row + v0 + 256 * q) : 0.0f;
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int v = v0 + 256 * q;
+                if (v >= n) break;
+                const int cv = part[v];
+                if (cv <= cu) continue;
+                const float wgt = fmaxf(fmaxf(core_u, core[v]), bound.up(d[q]));
+                if (__float_as_uint(wgt) > least_w[2 * cv]) continue;
+                atomicMin(&least[cv], sparse_key(wgt, u, v));
+            }
+        }
+    }
+    flush();
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(512) hdb_sparse_tree_kernel(const SparseArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_edges;   // tree edges found
+    __shared__ int s_parts;   // components
+    const int w = a.queue[blockIdx.x];
+    if (a.flags[w]) return;
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const int cap = sparse_round(n);
+    unsigned long long* choice = reinterpret_cast<unsigned long long*>(smem);
+    unsigned long long* edge = choice + cap;
+    float* top = reinterpret_cast<float*>(edge + cap);     // largest edge from the leaf up
+    uint16_t* comp = reinterpret_cast<uint16_t*>(top + cap);
+    uint16_t* up = comp + cap;
+    // ---- the remaining rounds, on the table ------------------------------------
+    const int parts = a.parts[w];
+    const unsigned long long* __restrict__ table = a.table + a.table_offsets[w];
+    for (int e = tid; e < n - parts; e += nt) edge[e] = a.edges[base + e];
+    if (tid == 0) s_edges = n - parts;
+    uint16_t* owner = reinterpret_cast<uint16_t*>(top);     // component of each table row, by number
+    for (int c = tid; c < parts; c += nt) owner[c] = (uint16_t)c;
+    // In these rounds component numbers stand for the points: comp maps a point
+    // to its number's current root.
+    uint16_t* part = up;
+    for (int u = tid; u < n; u += nt) part[u] = a.part[base + u];
+    uint16_t* next = comp;  // next[c]: root that number c's component joins
+    __syncthreads();
+    for (int round = 0; round < kSparseLevels && s_edges < n - 1; ++round) {
+        for (int c = tid; c < parts; c += nt) choice[c] = kNoChoice;
+        __syncthreads();
+        for (int i = tid; i < parts * parts; i += nt) {
+            const int r = i / parts, c = i - r * parts;
+            if (c <= r) continue;
+            const int cr = owner[r], cc = owner[c];
+            if (cr == cc) continue;
+            const unsigned long long key = table[i];
+            if (key < choice[cr]) atomicMin(&choice[cr], key);
+            if (key < choice[cc]) atomicMin(&choice[cc], key);
+        }
+        __syncthreads();
+        for (int r = tid; r < parts; r += nt) {
+            if (owner[r] != r) continue;
+            const unsigned long long key = choice[r];
+            int to = r;
+            if (key != kNoChoice) {
+                const int lo = owner[part[key_low(key)]], hi = owner[part[key_high(key)]];
+                to = lo == r ? hi : lo;
+                if (choice[to] == key && r < to) to = r;
+                if (to != r) edge[min(atomicAdd(&s_edges, 1), n - 1)] = key;
+            }
+            next[r] = (uint16_t)to;
+        }
+        __syncthreads();
+        for (int c = tid; c < parts; c += nt) owner[c] = (uint16_t)sparse_root(next, owner[c], parts);
+        __syncthreads();
+    }
+    if (s_edges != n - 1) {  // unreachable: each round at least halves the components, 2^kSparseLevels points
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    // ---- merge rounds of T' ---------------------------------------------------
+    __syncthreads();
+    for (int u = tid; u < n; u += nt) { comp[u] = (uint16_t)u; top[u] = 0.0f; }
+    int level = 0;
+    for (; level < kSparseLevels; ++level) {
+        for (int u = tid; u < n; u += nt) choice[u] = kNoChoice;
+        if (tid == 0) s_parts = 0;
+        __syncthreads();
+        for (int e = tid; e < n - 1; e += nt) {
+            const unsigned long long key = edge[e];
+            const int lo = comp[key_low(key)], hi = comp[key_high(key)];
+            if (lo == hi) continue;
+            if (key < choice[lo]) atomicMin(&choice[lo], key);
+            if (key < choice[hi]) atomicMin(&choice[hi], key);
+        }
+        __syncthreads();
+        for (int r = tid; r < n; r += nt)
+            if (comp[r] == r) up[r] = (uint16_t)sparse_target(choice, comp, r);
+        __syncthreads();
+        for (int u = tid; u < n; u += nt) {
+            const unsigned long long key = choice[comp[u]];
+            if (key != kNoChoice) top[u] = fmaxf(top[u], __uint_as_float(key_weight(key)));
+            const int r = sparse_root(up, comp[u], n);
+            a.level_comp[(int64_t)level * a.T + base + u] = (uint16_t)r;
+            a.level_max_v[(int64_t)level * a.T + base + u] = top[u];
+            if (u == r) atomicAdd(&s_parts, 1);
+        }
+        __syncthreads();
+        for (int u = tid; u < n; u += nt) comp[u] = a.level_comp[(int64_t)level * a.T + base + u];
+        const int left = s_parts;
+        __syncthreads();
+        if (left == 1) { ++level; break; }
+    }
+    if (s_parts != 1) {  // unreachable, as above
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    // ---- leaf order: intervals handed down the rounds ------------------------
+    uint32_t* cursor = reinterpret_cast<uint32_t*>(choice);  // next free leaf of each component
+    uint32_t* place = cursor + cap;                          // first leaf of each component one round down
+    uint32_t* size = reinterpret_cast<uint32_t*>(top);
+    for (int u = tid; u < n; u += nt) cursor[u] = 0;
+    __syncthreads();
+    for (int l = level; l >= 1; --l) {
+        const uint16_t* parent = a.level_comp + (int64_t)(l - 1) * a.T + base;  // component after l rounds
+        const uint16_t* child = l >= 2 ? a.level_comp + (int64_t)(l - 2) * a.T + base : nullptr;
+        if (child) {
+            for (int u = tid; u < n; u += nt) size[u] = 0;
+            __syncthreads();
+            for (int u = tid; u < n; u += nt) atomicAdd(&size[child[u]], 1u);
+            __syncthreads();
+        }
+        for (int r = tid; r < n; r += nt)
+            if (!child || child[r] == r) place[r] = atomicAdd(&cursor[parent[r]], child ? size[r] : 1u);
+        __syncthreads();
+        if (child) {
+            for (int r = tid; r < n; r += nt)
+                if (child[r] == r) cursor[r] = place[r];
+            for (int u = tid; u < n; u += nt)
+                a.level_end_v[(int64_t)(l - 2) * a.T + base + u] = (uint16_t)(place[child[u]] + size[child[u]]);
+            __syncthreads();
+        }
+    }
+    for (int u = tid; u < n; u += nt) {
+        const uint32_t p = place[u];
+        a.perm[base + p] = (uint16_t)u;
+        a.pos[base + u] = (uint16_t)p;
+        for (int l = 0; l < level; ++l) {
+            a.level_max[(int64_t)l * a.T + base + p] = a.level_max_v[(int64_t)l * a.T + base + u];
+            a.level_end[(int64_t)l * a.T + base + p] =
+                l + 1 < level ? a.level_end_v[(int64_t)l * a.T + base + u] : (uint16_t)n;
+        }
+    }
+    if (tid == 0) a.levels[w] = level;
+}
+
+// ---------------------------------------------------------------------------
+// Light edges: all pairs (p < q in leaf order) whose distance is at most the
+// path maximum max(top_l(p), top_l(q)), l the first round that joins them.  Core
+// distances need no test: both ends' maxima are at least their own cores.
+// Pairs whose weight is certainly a core distance are star edges and left to
+// hdb_sparse_star_kernel.  One CTA per kLightRows rows; a row is staged in
+// shared memory and read in leaf order.
+// ---------------------------------------------------------------------------
+template <typename Real>
+__global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ int s_end[kSparseLevels];
+    __shared__ float s_top[kSparseLevels];
+    float* row = reinterpret_cast<float*>(smem);
+    const int per = (a.nmax + kLightRows - 1) / kLightRows;
+    const int item = blockIdx.x / per, p0 = (blockIdx.x - item * per) * kLightRows;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (p0 >= n || a.flags[w]) return;
+    const int levels = a.levels[w];
+    const float* __restrict__ Dw = sparse_block<Real>(a, w);
+    const int64_t ld = dist_ld(n);
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    const uint16_t* __restrict__ perm = a.perm + base;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int limit = n * a.light_cap;
+    uint32_t* light_uv = a.light_uv + base * a.light_cap;
+    Real* light_w = static_cast<Real*>(a.light_w) + base * a.light_cap;
+    const int pend = min(p0 + kLightRows, n - 1);
+    for (int p = p0; p < pend; ++p) {
+        const int u = perm[p];
+        const float* __restrict__ src = Dw + (int64_t)u * ld;
+        __syncthreads();
+        for (int j = 4 * tid; j < n; j += 4 * 256)
+            *reinterpret_cast<float4*>(row + j) = __ldcg(reinterpret_cast<const float4*>(src + j));
+        if (tid < levels) {
+            s_end[tid] = a.level_end[(int64_t)tid * a.T + base + p];
+            s_top[tid] = a.level_max[(int64_t)tid * a.T + base + p];
+        }
+        __syncthreads();
+        const float core_u = a.unit_core ? -1.0f : a.core_down[base + u];
+        int l = 0;
+        for (int q0 = p + 1; q0 < n; q0 += 256) {
+            const int q = q0 + tid;
+            bool light = false;
+            int v = 0;
+            float d = 0.0f;
+            if (q < n) {
+                while (l + 1 < levels && q >= s_end[l]) ++l;
+                v = perm[q];
+                d = row[v];
+                light = bound.down(d) <= fmaxf(s_top[l], a.level_max[(int64_t)l * a.T + base + q]);
+                if (light && !a.unit_core) light = !(bound.up(d) <= fmaxf(core_u, a.core_down[base + v]));
+            }
+            const unsigned bal = __ballot_sync(0xffffffffu, light);
+            if (!bal) continue;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(a.light_count + w, __popc(bal));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
+            if (light) {
+                if (at >= limit) {
+                    sparse_flag(a, w);
+                } else {
+                    light_uv[at] = (uint32_t)u | ((uint32_t)v << 16);
+                    if constexpr (sizeof(Real) == 4) light_w[at] = d;  // above both cores
+                }
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Stars: of each point x, the list entries u whose edge weighs core_x
+// (d <= core_x, and u's core smaller, or equal with u < x so that the edge has
+// one owner).  All are kept as a mask over the list, for the sources.  The order
+// needs one edge per component below core_x: x is alone below core_x, and a
+// component that Prim has entered is finished before an edge of core_x is
+// taken; entering from x, the lowest vertex comes first.  So of entries that T'
+// joins below core_x (neighbours in leaf order, a sufficient test) only the
+// lowest vertex is emitted.  One warp a point.
+// ---------------------------------------------------------------------------
+template <typename Real>
+__global__ void __launch_bounds__(256) hdb_sparse_star_kernel(const SparseArgs a) {
+    const int per = (a.nmax + kSparseRowsCta - 1) / kSparseRowsCta;
+    const int item = blockIdx.x / per, r0 = (blockIdx.x - item * per) * kSparseRowsCta;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (r0 >= n || a.flags[w]) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int levels = a.levels[w];
+    const int keep = min(a.keep, n);
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    const Real* __restrict__ core = static_cast<const Real*>(a.core) + base;
+    const int limit = n * a.star_cap;
+    for (int r = warp; r < kSparseRowsCta; r += 8) {
+        const int x = r0 + r;
+        if (x >= n) break;  // warp-uniform
+        const Real core_x = core[x];
+        const float down_x = a.core_down[base + x];
+        unsigned long long members = 0;
+        for (int h = 0; h < keep; h += 32) {
+            const int t = h + lane;
+            uint32_t key = 0xffffffffu;
+            if (t < keep) {
+                const int u = a.knn_idx[(base + x) * a.list + t];
+                if (u != x && bound.up(a.knn_d[(base + x) * a.list + t]) <= down_x) {
+                    const Real core_u = core[u];
+                    if (core_u < core_x || (core_u == core_x && u < x))
+                        key = ((uint32_t)a.pos[base + u] << 12) | (uint32_t)u;
+                }
+            }
+            const unsigned in = __ballot_sync(0xffffffffu, key != 0xffffffffu);
+            members |= (unsigned long long)in << h;
+            if (!in) continue;
+            // Entries in leaf order.
+#pragma unroll
+            for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    const uint32_t other = __shfl_xor_sync(0xffffffffu, key, j);
+                    const bool keep_min = ((lane & k) == 0) == ((lane & j) == 0);
+                    key = keep_min ? min(key, other) : max(key, other);
+                }
+            }
+            const uint32_t before = __shfl_up_sync(0xffffffffu, key, 1);
+            const bool valid = key != 0xffffffffu;
+            bool joined = false;  // to the entry before, below core_x
+            if (valid && lane > 0) {
+                const int p = (int)(before >> 12), q = (int)(key >> 12);
+                int l = 0;
+                while (l + 1 < levels && q >= a.level_end[(int64_t)l * a.T + base + p]) ++l;
+                joined = fmaxf(a.level_max[(int64_t)l * a.T + base + p], a.level_max[(int64_t)l * a.T + base + q]) < down_x;
+            }
+            // Lowest vertex of each run of joined entries.
+            uint32_t low = key & 0xfffu;
+            const unsigned heads = __ballot_sync(0xffffffffu, valid && !joined);
+            const int head = 31 - __clz(heads & ((2u << lane) - 1u));  // lane 0 is a head whenever any lane is valid
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, low, o);
+                if (lane - o >= head) low = min(low, y);
+            }
+            const unsigned valid_mask = __ballot_sync(0xffffffffu, valid);
+            const bool last = valid && (lane == 31 || !((valid_mask >> (lane + 1)) & 1u) || ((heads >> (lane + 1)) & 1u));
+            const unsigned emit = __ballot_sync(0xffffffffu, last);
+            int at = 0;
+            if (lane == 0) at = atomicAdd(a.star_count + w, __popc(emit));
+            at = __shfl_sync(0xffffffffu, at, 0) + __popc(emit & lanemask_lt());
+            if (last) {
+                if (at >= limit) sparse_flag(a, w);
+                else a.star_uv[base * a.star_cap + at] = (uint32_t)x | (low << 16);
+            }
+        }
+        if (lane == 0) a.star_mask[base + x] = members;
+    }
+}
+
+// Exact weights of the light edges (float64).
+constexpr int kWeightsPerWindow = 8;  // CTAs of 128 threads sharing a window's edges
+
+__global__ void __launch_bounds__(128) hdb_sparse_weights_kernel(const SparseArgs a) {
+    using T = RealTraits<double>;
+    const int item = blockIdx.x / kWeightsPerWindow, part = blockIdx.x - item * kWeightsPerWindow;
+    const int w = a.queue[item];
+    if (a.flags[w]) return;
+    const int64_t base = a.offsets[w];
+    const int D = a.D;
+    const int count = a.light_count[w];
+    const double* __restrict__ X = static_cast<const double*>(a.X) + base * D;
+    const double* core = static_cast<const double*>(a.core);
+    double* light_w = static_cast<double*>(a.light_w) + base * a.light_cap;
+    for (int e = part * 128 + threadIdx.x; e < count; e += 128 * kWeightsPerWindow) {
+        const uint32_t uv = a.light_uv[base * a.light_cap + e];
+        const int u = uv & 0xffff, v = uv >> 16;
+        double d = sparse_exact<double>(X + (int64_t)u * D, X + (int64_t)v * D, D);
+        if (!a.unit_core) d = T::vmax(T::vmax(core[base + u], core[base + v]), d);
+        light_w[e] = d;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Prim and the hierarchy: one CTA a window.
+//  1. Boruvka over the light and star edges gives the weights of the minimum
+//     spanning trees; sorted, they turn weights into ranks.  An edge whose
+//     weight is none of them lies in no minimum spanning tree and is dropped.
+//  2. The rest become adjacency rows of packed (rank, vertex) words in shared
+//     memory (in the workspace when they do not fit).
+//  3. One warp runs Prim.  Vertices are split over the lanes in 32 blocks of
+//     2^shift; a lane keeps its block's least word (rank << 12 | vertex).  An
+//     update only lowers it; when the block loses its least vertex to the tree
+//     the warp rescans the block.  A step is one redux over the lanes and three
+//     dependent shared-memory loads (row start, row, best of the neighbours).
+//  4. Sources, then the hierarchy stages as in the dense form (the sort on all
+//     warps).
+// Shared memory: the arena (r0 weights, r1 sorted weights, s0 ranks then
+// sources, s1 order; row starts and best words in r2, and s2/s3 for float32;
+// adjacency behind them to the arena's end and on).
+// ---------------------------------------------------------------------------
+template <typename Real> struct SparsePrimLayout {
+    // Adjacency words per point that prim_smem provides.
+    static constexpr int kAdj = 5;
+    __host__ __device__ static size_t adj_offset(int n) {
+        const size_t cap = (size_t)Arena<Real>::round_cap(n);
+        return 3 * cap * sizeof(Real) + cap * 2 * (sizeof(Real) == 4 ? 4 : 2);
+    }
+    __host__ __device__ static size_t bytes(int n) {
+        const size_t need = adj_offset(n) + (size_t)n * kAdj * sizeof(uint32_t);
+        return need > Arena<Real>::bytes(n) ? need : Arena<Real>::bytes(n);
+    }
+};
+
+constexpr uint32_t kWordIn = 0xffffffffu;         // in the tree
+constexpr uint32_t kWordUnreached = 0x7fffffffu;  // above every (rank, vertex) word
+
+__device__ __forceinline__ bool sparse_prim_warp(int n, const uint32_t* start, uint32_t* best, const uint32_t* adj,
+                                                 int16_t* order, int16_t* rank) {
+    const int lane = threadIdx.x & 31;
+    const int shift = n <= 1024 ? 5 : (n <= 2048 ? 6 : 7);
+    const int block = 1 << shift;
+    uint32_t least = (lane << shift) < n ? kWordUnreached : kWordIn;
+    int cur = 0;
+    if (lane == 0) best[0] = kWordIn;
+    __syncwarp();
+    for (int it = 0; it < n - 1; ++it) {
+        const uint32_t row = start[cur];  // first word << 12 | count
+        const int count = (int)(row & 0xfffu);
+        const uint32_t* words = adj + (row >> 12);
+        uint32_t word = lane < count ? words[lane] : kWordIn;
+        // The block that cur left.
+        const int own = cur >> shift;
+        uint32_t rest = kWordIn;
+        for (int j = lane; j < block; j += 32) {
+            const int v = (own << shift) + j;
+            if (v < n) rest = min(rest, best[v]);
+        }
+        rest = __reduce_min_sync(0xffffffffu, rest);
+        if (lane == own) least = rest;
+        for (int e = 0; e < count; e += 32) {
+            if (e) word = e + lane < count ? words[e + lane] : kWordIn;
+            bool lower = false;
+            if (word != kWordIn) {
+                const int v = (int)(word & 0xfffu);
+                const uint32_t b = best[v];
+                lower = b != kWordIn && word < b;
+                if (lower) best[v] = word;
+            }
+            unsigned bal = __ballot_sync(0xffffffffu, lower);
+            while (bal) {
+                const int s = __ffs(bal) - 1;
+                bal &= bal - 1;
+                const uint32_t x = __shfl_sync(0xffffffffu, word, s);
+                if ((int)((x & 0xfffu) >> shift) == lane) least = min(least, x);
+            }
+        }
+        const uint32_t next = __reduce_min_sync(0xffffffffu, least);
+        if (next >= kWordUnreached) return false;  // not connected
+        cur = (int)(next & 0xfffu);
+        if (lane == 0) {
+            order[it] = (int16_t)cur;
+            rank[it] = (int16_t)(next >> 12);
+            best[cur] = kWordIn;
+        }
+        __syncwarp();
+    }
+    return true;
+}
+
+// Ascending bitonic sort of k[0..P) (P a power of two) by the CTA.
+template <typename Key>
+__device__ __forceinline__ void bitonic_cta(Key* k, int P) {
+    for (int size = 2; size <= P; size <<= 1) {
+        for (int j = size >> 1; j > 0; j >>= 1) {
+            for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
+                const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
+                const Key x = k[lo], y = k[hi];
+                if (key_lt(y, x) == ((lo & size) == 0)) { k[lo] = y; k[hi] = x; }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a, const __grid_constant__ ForwardArgs f) {
+    using T = RealTraits<Real>;
+    using Key = typename T::Bits;
+    constexpr bool kWide = sizeof(Real) == 8;
+    constexpr Key kNoKey = (Key)~(Key)0;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_scan[32];
+    __shared__ int s_ctr[4];
+    __shared__ int s_edges;
+    __shared__ int s_ok;
+    const int w = a.queue[blockIdx.x];
+    if (a.flags[w]) return;
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    Arena<Real> ar = Arena<Real>::carve(smem, n);
+    const int cap = Arena<Real>::round_cap(n);
+    if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 0] = f.stage_ns[8 * w + 1] = global_ns();
+    const int n_light = a.light_count[w], n_star = a.unit_core ? 0 : a.star_count[w];
+    const int m = n_light + n_star;
+    const uint32_t* __restrict__ light_uv = a.light_uv + base * a.light_cap;
+    const Real* __restrict__ light_w = static_cast<const Real*>(a.light_w) + base * a.light_cap;
+    const uint32_t* __restrict__ star_uv = a.star_uv + base * a.star_cap;
+    const Real* __restrict__ core = static_cast<const Real*>(a.core) + base;
+    uint16_t* edge_rank = a.edge_rank + base * (a.light_cap + a.star_cap);
+    auto edge = [&](int e, int& u, int& v, Key& key) {
+        const uint32_t uv = e < n_light ? light_uv[e] : star_uv[e - n_light];
+        u = (int)(uv & 0xffff);
+        v = (int)(uv >> 16);
+        key = T::key(e < n_light ? light_w[e] : core[u]);
+    };
+    // ---- 1. minimum spanning tree weights ---------------------------------------
+    // Choice of a component: its least (weight, ends); float32 in one 64-bit word.
+    unsigned long long* choice = reinterpret_cast<unsigned long long*>(ar.r1);
+    uint32_t* choice_uv = reinterpret_cast<uint32_t*>(ar.r2);  // float64 only
+    uint16_t* comp = reinterpret_cast<uint16_t*>(ar.s2);
+    uint16_t* up = reinterpret_cast<uint16_t*>(ar.s3);
+    for (int v = tid; v < n; v += nt) comp[v] = (uint16_t)v;
+    if (tid == 0) s_edges = 0;
+    for (int round = 0; round < kSparseLevels; ++round) {
+        for (int v = tid; v < n; v += nt) {
+            choice[v] = kNoChoice;
+            if (kWide) choice_uv[v] = 0xffffffffu;
+        }
+        __syncthreads();
+        for (int e = tid; e < m; e += nt) {
+            int u, v;
+            Key key;
+            edge(e, u, v, key);
+            const int cu = comp[u], cv = comp[v];
+            if (cu == cv) continue;
+            unsigned long long word = key;
+            if (!kWide) word = (word << 32) | ((uint32_t)min(u, v) << 12) | (uint32_t)max(u, v);
+            if (word < choice[cu]) atomicMin(&choice[cu], word);
+            if (word < choice[cv]) atomicMin(&choice[cv], word);
+        }
+        __syncthreads();
+        if (kWide) {
+            for (int e = tid; e < m; e += nt) {
+                int u, v;
+                Key key;
+                edge(e, u, v, key);
+                const int cu = comp[u], cv = comp[v];
+                if (cu == cv) continue;
+                const uint32_t ends = ((uint32_t)min(u, v) << 12) | (uint32_t)max(u, v);
+                if (choice[cu] == (unsigned long long)key) atomicMin(&choice_uv[cu], ends);
+                if (choice[cv] == (unsigned long long)key) atomicMin(&choice_uv[cv], ends);
+            }
+            __syncthreads();
+        }
+        for (int r = tid; r < n; r += nt) {
+            if (comp[r] != r) continue;
+            const unsigned long long word = choice[r];
+            int to = r;
+            if (word != kNoChoice) {
+                const uint32_t ends = kWide ? choice_uv[r] : (uint32_t)word;
+                const int lo = comp[(ends >> 12) & 0xfff], hi = comp[ends & 0xfff];
+                to = lo == r ? hi : lo;
+                if (choice[to] == word && (!kWide || choice_uv[to] == ends) && r < to) to = r;
+                if (to != r) ar.r0[min(atomicAdd(&s_edges, 1), n - 1)] = T::from_key((Key)(kWide ? word : word >> 32));
+            }
+            up[r] = (uint16_t)to;
+        }
+        __syncthreads();
+        for (int v = tid; v < n; v += nt) comp[v] = (uint16_t)sparse_root(up, comp[v], n);
+        const int found = s_edges;
+        __syncthreads();
+        if (found >= n - 1) break;
+    }
+    if (s_edges != n - 1) {  // the light and star edges hold a spanning tree: unreachable
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    Key* sorted = reinterpret_cast<Key*>(ar.r1);  // over r1 and r2 while sorting
+    int P = 1;
+    while (P < n - 1) P <<= 1;
+    __syncthreads();
+    for (int i = tid; i < P; i += nt) sorted[i] = i < n - 1 ? T::key(ar.r0[i]) : kNoKey;
+    __syncthreads();
+    bitonic_cta<Key>(sorted, P);
+    // ---- 2. adjacency -----------------------------------------------------------
+    uint32_t* start = reinterpret_cast<uint32_t*>(ar.r2);
+    uint32_t* best = kWide ? start + cap : reinterpret_cast<uint32_t*>(ar.s2);
+    uint32_t* adj = reinterpret_cast<uint32_t*>(smem + SparsePrimLayout<Real>::adj_offset(n));
+    for (int v = tid; v < n; v += nt) best[v] = 0;  // degrees
+    __syncthreads();
+    for (int e = tid; e < m; e += nt) {
+        int u, v;
+        Key key;
+        edge(e, u, v, key);
+        int lo = 0, hi = n - 1;  // first sorted weight not below this edge's
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (key_lt(sorted[mid], key)) lo = mid + 1; else hi = mid;
+        }
+        const bool in = lo < n - 1 && key_eq(sorted[lo], key);
+        edge_rank[e] = in ? (uint16_t)lo : (uint16_t)0xffff;
+        if (in) {
+            atomicAdd(&best[u], 1u);
+            atomicAdd(&best[v], 1u);
+        }
+    }
+    __syncthreads();
+    // Exclusive scan of the degrees: a contiguous run of vertices a thread.
+    const int run = (n + nt - 1) / nt;
+    uint32_t sum = 0;
+    for (int v = tid * run; v < min(n, (tid + 1) * run); ++v) sum += best[v];
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (int j = 0; j < (nt >> 5); ++j) {
+        if (j < warp) before += s_scan[j];
+        total += s_scan[j];
+    }
+    before += incl - sum;
+    for (int v = tid * run; v < min(n, (tid + 1) * run); ++v) {
+        const uint32_t d = best[v];
+        start[v] = (before << 12) | d;
+        best[v] = before;  // next free word
+        before += d;
+    }
+    const bool on_chip = total <= (uint32_t)(n * SparsePrimLayout<Real>::kAdj);
+    uint32_t* adj_off = a.adj + 2 * base * (a.light_cap + a.star_cap);
+    __syncthreads();
+    for (int e = tid; e < m; e += nt) {
+        const uint32_t r = edge_rank[e];
+        if (r == 0xffffu) continue;
+        const uint32_t uv = e < n_light ? light_uv[e] : star_uv[e - n_light];
+        const uint32_t u = uv & 0xffff, v = uv >> 16;
+        const uint32_t at_u = atomicAdd(&best[u], 1u), at_v = atomicAdd(&best[v], 1u);
+        if (on_chip) {
+            adj[at_u] = (r << 12) | v;
+            adj[at_v] = (r << 12) | u;
+        } else {
+            adj_off[at_u] = (r << 12) | v;
+            adj_off[at_v] = (r << 12) | u;
+        }
+    }
+    __syncthreads();
+    for (int v = tid; v < n; v += nt) best[v] = kWordUnreached;
+    __syncthreads();
+    // ---- 3. order ---------------------------------------------------------------
+    if (warp == 0) {
+        const bool ok = on_chip ? sparse_prim_warp(n, start, best, adj, ar.s1, ar.s0)
+                                : sparse_prim_warp(n, start, best, adj_off, ar.s1, ar.s0);
+        if (lane == 0) s_ok = ok;
+    }
+    __syncthreads();
+    if (!s_ok) {  // unreachable, as above
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    // ---- 4. sources: the first visited end of an edge of the vertex's weight --------
+    uint32_t* place = best;     // position << 12 | rank of each vertex's edge
+    uint32_t* source = start;   // position of its source
+    for (int v = tid; v < n; v += nt) source[v] = 0xffffu;
+    if (tid == 0) place[0] = 0xfffu;  // the start has no edge
+    for (int i = tid; i < n - 1; i += nt)
+        place[ar.s1[i]] = ((uint32_t)(i + 1) << 12) | (uint32_t)(uint16_t)ar.s0[i];
+    __syncthreads();
+    for (int e = tid; e < n_light; e += nt) {
+        const uint32_t r = edge_rank[e];
+        if (r == 0xffffu) continue;
+        const uint32_t uv = light_uv[e];
+        const uint32_t u = uv & 0xffff, v = uv >> 16;
+        const uint32_t pu = place[u], pv = place[v];
+        const bool forward = pu < pv;
+        if (((forward ? pv : pu) & 0xfffu) == r) atomicMin(&source[forward ? v : u], (forward ? pu : pv) >> 12);
+    }
+    if (!a.unit_core) {
+        for (int x = tid; x < n; x += nt) {
+            unsigned long long members = a.star_mask[base + x];
+            const Key key = T::key(core[x]);
+            const uint32_t px = place[x];
+            while (members) {
+                const int t = __ffsll((long long)members) - 1;
+                members &= members - 1;
+                const int u = a.knn_idx[(base + x) * a.list + t];
+                const uint32_t pu = place[u];
+                const bool forward = px < pu;  // x first: it may be u's source
+                const uint32_t r = (forward ? pu : px) & 0xfffu;
+                if (r != 0xfffu && key_eq(sorted[r], key)) atomicMin(&source[forward ? u : x], (forward ? px : pu) >> 12);
+            }
+        }
+    }
+    __syncthreads();
+    bool lost = false;
+    for (int i = tid; i < n - 1; i += nt) {
+        const uint32_t p = source[ar.s1[i]];
+        lost |= p > (uint32_t)i;
+        ar.r0[i] = T::from_key(sorted[ar.s0[i]]);
+        ar.s0[i] = p == 0 || p > (uint32_t)i ? (int16_t)0 : ar.s1[p - 1];
+    }
+    if (__syncthreads_or(lost)) {  // unreachable: every vertex has a source
+        if (tid == 0) sparse_flag(a, w);
+        return;
+    }
+    if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 2] = global_ns();
+    const bool help = !a.unit_core && n - 1 >= kHelpMinEdges;
+    if (warp == 0) tree_window<Real>(f, smem, w, n, help ? s_ctr : nullptr);
+    else if (help) sort_edges_cta<Real>(ar, n - 1, nt, kBarHelp, s_ctr);
+}
+
+}  // namespace hdb

@@ -1,0 +1,24 @@
+// Host interface of the sparse path (hdb_sparse.cu): one launcher per stage.
+#pragma once
+#include <cuda_runtime.h>
+
+#include "hdb_args.h"
+
+namespace hdb {
+
+enum class SparseStage { kNarrow, kTiles, kRows, kCore, kForest, kBetween, kTree, kLight, kStar, kWeights, kPrim };
+
+// Launches `stage` for the windows of `a`; `f` is the forward's argument block
+// (kPrim only).  precision: 0 float32, 1 float64 (kNarrow, kTiles, kCore and
+// kWeights exist for float64 only).
+cudaError_t sparse_launch(int precision, SparseStage stage, const SparseArgs& a, const ForwardArgs* f,
+                          cudaStream_t stream, int priority);
+
+// Raises the dynamic shared-memory limits for windows of up to n points; false
+// in *fits when a window of that size does not fit in `budget` bytes.
+cudaError_t sparse_prepare(int precision, int n, size_t budget, bool* fits);
+
+// Row stride of the neighbour lists for min_samples ms (0: not supported).
+int sparse_list(int precision, int ms);
+
+}  // namespace hdb

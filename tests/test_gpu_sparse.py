@@ -1,0 +1,141 @@
+"""The sparse path (light edges + sparse Prim) against the CPU oracle, bit for bit on every exported stage.
+
+Sizes sit at the edges of its bins, blocks and tiles; the data include what
+its float32 bound cannot separate (duplicates, lattices, tiny or huge values,
+small clusters far from the origin), where windows fall back to the general
+path.  Nothing here has a tolerance: integers and bit patterns are equal.
+"""
+
+import json
+
+import numpy as np
+import pytest
+
+from oracle import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _mixture(rng, n, d):
+    centres = rng.uniform(-4, 4, (6, d))
+    x = centres[rng.integers(0, 6, n)] + rng.normal(0, 0.4, (n, d))
+    x[rng.random(n) < 0.08] += rng.uniform(-6, 6, d)
+    return x
+
+
+def _uniform(rng, n, d):
+    return rng.uniform(-1, 1, (n, d))
+
+
+def _line(rng, n, d):  # neighbours in a row: long merge chains
+    x = np.zeros((n, d))
+    x[:, 0] = np.cumsum(1.0 + 0.3 * rng.random(n))
+    return x[rng.permutation(n)]
+
+
+def _nested(rng, n, d):  # growing gaps: deep dendrogram, one component swallows the rest
+    x = np.zeros((n, d))
+    x[:, 0] = np.cumsum(1.0 + 0.01 * np.arange(n)) + 1e-3 * rng.random(n)
+    return x
+
+
+def _far(rng, n, d):  # small clusters far from the origin and from each other
+    return 1e6 + 1e3 * rng.integers(0, 3, (n, 1)) + rng.normal(0, 1e-3, (n, d))
+
+
+def _duplicates(rng, n, d):
+    return np.repeat(rng.normal(size=(n // 3 + 1, d)), 3, axis=0)[:n][rng.permutation(n)]
+
+
+def _lattice(rng, n, d):
+    return rng.integers(-3, 4, (n, d)) / 2.0
+
+
+def _tiny(rng, n, d):
+    return _mixture(rng, n, d) * 1e-30
+
+
+def _huge(rng, n, d):
+    return _mixture(rng, n, d) * 1e15
+
+
+MAKERS = {f.__name__[1:]: f for f in (_mixture, _uniform, _line, _nested, _far, _duplicates, _lattice, _tiny, _huge)}
+
+
+def _run(windows, mcs, ms, eps, precision):
+    import torch
+
+    from hdbscan_gb300._cuda import Plan, pack
+
+    packed, offsets = pack(windows, precision)
+    plan = Plan(offsets, packed.shape[1], min_cluster_size=mcs, min_samples=ms, cluster_selection_epsilon=eps,
+                precision=precision)
+    workspace = plan.workspace()
+    buffers = plan.export_buffers(hierarchy=True, gradients=True, probabilities=True)
+    labels, status = plan.forward(packed, workspace=workspace, exports=buffers)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    host = {k: v.cpu().numpy() for k, v in buffers.items()}
+    host["labels"] = labels.cpu().numpy()
+    describe = json.loads(plan.describe())
+    at = describe["general_flags_offset"]
+    flags = None
+    if at >= 0:
+        flags = workspace[at:at + 4 * plan.windows].cpu().numpy().view(np.int32)
+    return host, offsets, describe, flags
+
+
+def _check(windows, mcs, ms, eps, precision):
+    dtype = np.float32 if precision == "float32" else np.float64
+    windows = [np.asarray(x, dtype) for x in windows]
+    host, offsets, describe, flags = _run(windows, mcs, ms, eps, precision)
+    for w, x in enumerate(windows):
+        o = oracle.cluster(x, mcs, ms, eps, precision)
+        lo, hi = offsets[w], offsets[w + 1]
+        e0, e1 = lo - w, hi - w - 1
+        ctx = f"window {w} n={len(x)} d={x.shape[1]} mcs={mcs} ms={ms} {precision}"
+        for name, part in (("edges_uv", slice(e0, e1)), ("edge_w", slice(e0, e1)), ("order", slice(e0, e1)),
+                           ("link_lr", slice(e0, e1)), ("link_w", slice(e0, e1)), ("link_size", slice(e0, e1)),
+                           ("labels", slice(lo, hi)), ("point_parent", slice(lo, hi))) + (
+                               (("core", slice(lo, hi)),) if ms > 2 else ()):
+            got, want = np.ascontiguousarray(host[name][part]), np.ascontiguousarray(o[name])
+            np.testing.assert_array_equal(got.view(np.uint8), want.astype(got.dtype).view(np.uint8),
+                                          err_msg=f"{ctx}: {name}")
+    return describe, flags
+
+
+@pytest.mark.parametrize("ms", [1, 2, 3, 5, 6, 7, 14, 15, 16])
+@pytest.mark.parametrize("maker", sorted(MAKERS))
+def test_sizes_and_data_float64(cuda, maker, ms):
+    rng = np.random.default_rng(zlib_seed(maker, ms))
+    sizes = [15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 257, 511, 512, 513]
+    d = int(rng.integers(1, 20))
+    describe, flags = _check([MAKERS[maker](rng, max(n, ms), d) for n in sizes], 4, ms, 0.05, "float64")
+    assert any(c["variant"] == "sparse" for c in describe["classes"])
+    if maker in ("mixture", "uniform"):
+        assert not flags.any(), "ordinary data stays on the sparse path"
+
+
+def zlib_seed(name, ms):
+    import zlib
+
+    return zlib.crc32(f"{name}/{ms}".encode())
+
+
+@pytest.mark.parametrize("dims", [1, 2, 31, 32, 33, 64, 65, 129, 300])
+def test_dimensions_float64(cuda, dims):
+    rng = np.random.default_rng(dims)
+    _check([_mixture(rng, n, dims) for n in (100, 260, 700)], 5, 5, 0.0, "float64")
+
+
+@pytest.mark.parametrize("ms", [2, 16])
+@pytest.mark.parametrize("n", [1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096])
+def test_large_windows_float64(cuda, n, ms):
+    rng = np.random.default_rng(n + ms)
+    _check([_mixture(rng, n, 9), _uniform(rng, n, 9)], 8, ms, 0.0, "float64")
+
+
+@pytest.mark.parametrize("ms", [30, 31, 62, 63])
+def test_long_lists_float64(cuda, ms):
+    rng = np.random.default_rng(ms)
+    _check([_mixture(rng, n, 7) for n in (ms, ms + 1, 200, 900)], 10, ms, 0.0, "float64")
