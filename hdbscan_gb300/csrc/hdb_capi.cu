@@ -323,13 +323,16 @@ int build_plan(hdb_plan* p) {
         ctas -= chosen[w]->cluster - 1;
         chosen[w] = single;
     }
-    // The sparse path: float64 windows that the table gives one CTA.  All of
-    // them share one general class, which does the windows it flags.
+    // The sparse path: float64 windows and float32 windows of the matrix
+    // variant that the table gives one CTA.  All of them share one general
+    // class, which does the windows it flags.
     std::vector<char> sparse(p->B, 0);
     int sparse_nmax = 0;
     p->list = hdb::sparse_list(p->precision, p->ms);
-    if (p->precision == HDB_F64 && p->list && !(p->flags & kNoSparseFlags)) {
-        for (int w : order) sparse[w] = size_of(w) >= kSparseMinN && chosen[w]->cluster == 1;
+    if (p->list && !(p->flags & kNoSparseFlags)) {
+        for (int w : order)
+            sparse[w] = size_of(w) >= kSparseMinN && chosen[w]->cluster == 1 &&
+                        (p->precision == HDB_F64 || chosen[w]->dp == 0);
         for (int w : order)
             if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
         bool fits = true;
@@ -416,12 +419,13 @@ int build_plan(hdb_plan* p) {
         if (c.fv->dp != 0) continue;
         // Float32 classes of larger windows take the 128x128 tile kernel.
         c.tile = (p->precision == HDB_F32 && c.nmax >= kTile128MinN) ? 128 : 64;
+        const bool tiles = !(c.general && p->precision == HDB_F32);  // those come from the sparse path
         for (int w : c.windows) {
             const int n = size_of(w);
             const int64_t ld = (n + 3) & ~3;
             p->dist_offsets[w] = p->dist_elems;
             p->dist_elems += align_up((size_t)(n * ld), 64);
-            const int t = (n + c.tile - 1) / c.tile;
+            const int t = tiles ? (n + c.tile - 1) / c.tile : 0;
             for (int ti = 0; ti < t; ++ti)
                 for (int tj = ti; tj < t; ++tj) {
                     p->tiles.push_back(w);
@@ -436,6 +440,7 @@ int build_plan(hdb_plan* p) {
     if (!unit) {
         for (auto& c : p->classes) {
             const bool matrix = c.fv->dp == 0;
+            if (c.general && p->precision == HDB_F32) continue;  // the sparse path leaves exact core distances
             CoreLaunch launch;
             launch.matrix = matrix;
             launch.cv = choose_core(k, p->precision, p->ms, p->D, matrix);
@@ -798,7 +803,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         const bool wide = p->precision == HDB_F64;
         int rc = HDB_OK;
         if (wide) rc = stage(hdb::SparseStage::kNarrow, HDB_PHASE_PREPARE, stream);
-        if (!rc && wide) rc = stage(hdb::SparseStage::kTiles, HDB_PHASE_DISTANCE, stream);
+        if (!rc) rc = stage(hdb::SparseStage::kTiles, HDB_PHASE_DISTANCE, stream);
         if (!rc) rc = stage(hdb::SparseStage::kRows, HDB_PHASE_CORE, stream);
         if (!rc && wide && !unit) rc = stage(hdb::SparseStage::kCore, HDB_PHASE_CORE, stream);
         if (rc) return rc;
@@ -834,8 +839,10 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             joined = n_groups + i;
         }
         const unsigned grid_limit = c.general ? kGeneralGrid : 0xffffffffu;
+        // float32: the sparse path left the exact distances and core distances.
+        const bool have_rows = c.general && p->precision == HDB_F32;
         // 1. distance blocks of this class's matrix-variant windows (caller's stream)
-        if (c.n_tiles) {
+        if (c.n_tiles && !have_rows) {
             hdb::DistanceArgs a{};
             a.X = X;
             a.offsets = d_offsets;
@@ -854,6 +861,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         }
         // 2. core distances of its windows (caller's stream)
         for (const auto& cl : c.cores) {
+            if (have_rows) break;
             hdb::CoreArgs a{};
             a.X = X;
             a.offsets = d_offsets;

@@ -33,6 +33,10 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
     switch (stage) {
         case SparseStage::kRows:
             return launch_rows<Real>(a, s, priority);
+        case SparseStage::kTiles: {
+            const unsigned t = blocks(a.nmax, 128);
+            return launch_ex(hdb_sparse_tiles_kernel<Real>, W * (t * (t + 1) / 2), 256, 0, s, priority, 1, a);
+        }
         case SparseStage::kForest:
             return launch_ex(hdb_sparse_forest_kernel<Real>, W, (unsigned)window_threads(a.nmax),
                              sparse_forest_smem(a.nmax), s, priority, 1, a);
@@ -54,12 +58,9 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
             break;
     }
     if constexpr (sizeof(Real) == 8) {
-        const unsigned t = blocks(a.nmax, 128);
         switch (stage) {
             case SparseStage::kNarrow:
                 return launch_ex(hdb_sparse_narrow_kernel, W * blocks(a.nmax, kNarrowRows), 256, 0, s, priority, 1, a);
-            case SparseStage::kTiles:
-                return launch_ex(hdb_sparse_tiles_kernel, W * (t * (t + 1) / 2), 256, 0, s, priority, 1, a);
             case SparseStage::kCore:
                 return launch_ex(hdb_sparse_core_kernel, W * blocks(a.nmax, 128), 128, 0, s, priority, 1, a);
             case SparseStage::kWeights:

@@ -142,12 +142,15 @@ __global__ void __launch_bounds__(256) hdb_sparse_narrow_kernel(const SparseArgs
 }
 
 // ---------------------------------------------------------------------------
-// float32 distance blocks of the narrowed input: 128x128 tiles of the upper
-// triangle, 8x8 pairs a thread, differences and fused squares in packed f32x2
-// instructions (one instruction a pair and coordinate, half of the exact
-// kernel's), mirrored like the exact blocks.
+// float32 distance blocks: 128x128 tiles of the upper triangle, 8x8 pairs a
+// thread, mirrored, differences in packed f32x2 instructions.  float32 windows:
+// the exact arithmetic of hdb_distance128_kernel (packed squares, scalar
+// k-ordered sums).  float64 windows: the narrowed input, squares fused into the
+// sums (one instruction a pair and coordinate, half of the exact form's).
 // ---------------------------------------------------------------------------
+template <typename Real>
 __global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseArgs a) {
+    constexpr bool kExact = sizeof(Real) == 4;
     constexpr int KC = 32;
     constexpr int TS = 128;
     __shared__ __align__(16) float s_i[KC][TS];
@@ -166,8 +169,8 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseAr
     const int ti = t - tj * (tj + 1) / 2;
     if (tj * TS >= n || a.flags[w]) return;
     const int D = a.D;
-    const float* __restrict__ Y = a.y + base * D;
-    float* __restrict__ Dw = sparse_block<double>(a, w);
+    const float* __restrict__ Y = (kExact ? static_cast<const float*>(a.X) : a.y) + base * D;
+    float* __restrict__ Dw = sparse_block<Real>(a, w);
     const int64_t ld = dist_ld(n);
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
     const int i0 = ti * TS, j0 = tj * TS;
@@ -204,7 +207,13 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseAr
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const float2 d = __ffma2_rn(xj[q], make_float2(-1.0f, -1.0f), xa);
-                    acc[p][q] = __ffma2_rn(d, d, acc[p][q]);
+                    if constexpr (kExact) {
+                        const float2 sq = __fmul2_rn(d, d);
+                        acc[p][q].x = __fadd_rn(acc[p][q].x, sq.x);
+                        acc[p][q].y = __fadd_rn(acc[p][q].y, sq.y);
+                    } else {
+                        acc[p][q] = __ffma2_rn(d, d, acc[p][q]);
+                    }
                 }
             }
         };

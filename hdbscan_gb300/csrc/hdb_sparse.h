@@ -9,7 +9,7 @@ namespace hdb {
 enum class SparseStage { kNarrow, kTiles, kRows, kCore, kForest, kBetween, kTree, kLight, kStar, kWeights, kPrim };
 
 // Launches `stage` for the windows of `a`; `f` is the forward's argument block
-// (kPrim only).  precision: 0 float32, 1 float64 (kNarrow, kTiles, kCore and
+// (kPrim only).  precision: 0 float32, 1 float64 (kNarrow, kCore and
 // kWeights exist for float64 only).
 cudaError_t sparse_launch(int precision, SparseStage stage, const SparseArgs& a, const ForwardArgs* f,
                           cudaStream_t stream, int priority);

@@ -106,11 +106,14 @@ def _check(windows, mcs, ms, eps, precision):
 
 @pytest.mark.parametrize("ms", [1, 2, 3, 5, 6, 7, 14, 15, 16])
 @pytest.mark.parametrize("maker", sorted(MAKERS))
-def test_sizes_and_data_float64(cuda, maker, ms):
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_sizes_and_data(cuda, maker, ms, precision):
     rng = np.random.default_rng(zlib_seed(maker, ms))
     sizes = [15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 128, 129, 255, 257, 511, 512, 513]
-    d = int(rng.integers(1, 20))
-    describe, flags = _check([MAKERS[maker](rng, max(n, ms), d) for n in sizes], 4, ms, 0.05, "float64")
+    d = int(rng.integers(1, 20)) if precision == "float64" else 33  # float32: the matrix variant's dims
+    if precision == "float32" and maker == "huge":
+        pytest.skip("squares overflow float32")
+    describe, flags = _check([MAKERS[maker](rng, max(n, ms), d) for n in sizes], 4, ms, 0.05, precision)
     assert any(c["variant"] == "sparse" for c in describe["classes"])
     if maker in ("mixture", "uniform"):
         assert not flags.any(), "ordinary data stays on the sparse path"
@@ -122,20 +125,25 @@ def zlib_seed(name, ms):
     return zlib.crc32(f"{name}/{ms}".encode())
 
 
+@pytest.mark.parametrize("precision", ["float32", "float64"])
 @pytest.mark.parametrize("dims", [1, 2, 31, 32, 33, 64, 65, 129, 300])
-def test_dimensions_float64(cuda, dims):
+def test_dimensions(cuda, dims, precision):
     rng = np.random.default_rng(dims)
-    _check([_mixture(rng, n, dims) for n in (100, 260, 700)], 5, 5, 0.0, "float64")
+    _check([_mixture(rng, n, dims) for n in (100, 260, 700)], 5, 5, 0.0, precision)
 
 
+@pytest.mark.parametrize("precision", ["float32", "float64"])
 @pytest.mark.parametrize("ms", [2, 16])
 @pytest.mark.parametrize("n", [1023, 1024, 1025, 2047, 2048, 2049, 4095, 4096])
-def test_large_windows_float64(cuda, n, ms):
+def test_large_windows(cuda, n, ms, precision):
     rng = np.random.default_rng(n + ms)
-    _check([_mixture(rng, n, 9), _uniform(rng, n, 9)], 8, ms, 0.0, "float64")
+    d = 9 if precision == "float64" else 40
+    _check([_mixture(rng, n, d), _uniform(rng, n, d)], 8, ms, 0.0, precision)
 
 
-@pytest.mark.parametrize("ms", [30, 31, 62, 63])
-def test_long_lists_float64(cuda, ms):
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+@pytest.mark.parametrize("ms", [30, 31, 62, 63, 64])
+def test_long_lists(cuda, ms, precision):
     rng = np.random.default_rng(ms)
-    _check([_mixture(rng, n, 7) for n in (ms, ms + 1, 200, 900)], 10, ms, 0.0, "float64")
+    d = 7 if precision == "float64" else 70
+    _check([_mixture(rng, n, d) for n in (ms, ms + 1, 200, 900)], 10, ms, 0.0, precision)
