@@ -1035,11 +1035,8 @@ __global__ void __launch_bounds__(128) hdb_sparse_weights_kernel(const SparseArg
 //     weight is none of them lies in no minimum spanning tree and is dropped.
 //  2. The rest become adjacency rows of packed (rank, vertex) words in shared
 //     memory (in the workspace when they do not fit).
-//  3. One warp runs Prim.  Vertices are split over the lanes in 32 blocks of
-//     2^shift; a lane keeps its block's least word (rank << 12 | vertex).  An
-//     update only lowers it; when the block loses its least vertex to the tree
-//     the warp rescans the block.  A step is one redux over the lanes and three
-//     dependent shared-memory loads (row start, row, best of the neighbours).
+//  3. One warp runs Prim over them (sparse_prim_warp): vertices are split over
+//     the lanes in 32 blocks, a lane keeps its block's least word.
 //  4. Sources, then the hierarchy stages as in the dense form (the sort on all
 //     warps).
 // Shared memory: the arena (r0 weights, r1 sorted weights, s0 ranks then
@@ -1059,60 +1056,118 @@ template <typename Real> struct SparsePrimLayout {
     }
 };
 
+// A word is rank << 14 | vertex << 2 (the vertex as a byte offset).  As a
+// signed number kWordIn is below every word (no update passes), as an unsigned
+// one above all (no minimum).
 constexpr uint32_t kWordIn = 0xffffffffu;         // in the tree
-constexpr uint32_t kWordUnreached = 0x7fffffffu;  // above every (rank, vertex) word
+constexpr uint32_t kWordUnreached = 0x7fffffffu;  // above every word
+__device__ __forceinline__ uint32_t prim_word(uint32_t rank, uint32_t vertex) { return (rank << 14) | (vertex << 2); }
+__device__ __forceinline__ uint32_t word_offset(uint32_t word) { return word & 0x3ffcu; }
 
-__device__ __forceinline__ bool sparse_prim_warp(int n, const uint32_t* start, uint32_t* best, const uint32_t* adj,
-                                                 int16_t* order, int16_t* rank) {
-    const int lane = threadIdx.x & 31;
-    const int shift = n <= 1024 ? 5 : (n <= 2048 ? 6 : 7);
-    const int block = 1 << shift;
-    uint32_t least = (lane << shift) < n ? kWordUnreached : kWordIn;
-    int cur = 0;
-    if (lane == 0) best[0] = kWordIn;
-    __syncwarp();
+// Shared-memory accesses in program order, predicated instead of branched
+// around: the warp never diverges inside a step.
+__device__ __forceinline__ uint32_t shared_address(const void* p) {
+    return (uint32_t)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t at) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(at));
+    return v;
+}
+__device__ __forceinline__ uint32_t lds32_if(bool p, uint32_t at, uint32_t other) {
+    uint32_t v = other;
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p ld.shared.u32 %0, [%1]; }" : "+r"(v) : "r"(at), "r"((uint32_t)p));
+    return v;
+}
+__device__ __forceinline__ void sts32_if(bool p, uint32_t at, uint32_t v) {
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p st.shared.u32 [%0], %1; }" ::"r"(at), "r"(v), "r"((uint32_t)p));
+}
+__device__ __forceinline__ void sts16_if(bool p, uint32_t at, uint32_t v) {
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p st.shared.u16 [%0], %1; }" ::"r"(at), "h"((unsigned short)v),
+                 "r"((uint32_t)p));
+}
+__device__ __forceinline__ void reds_min_if(bool p, uint32_t at, uint32_t v) {
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %2, 0; @p red.shared.min.u32 [%0], %1; }" ::"r"(at), "r"(v),
+                 "r"((uint32_t)p));
+}
+
+// A step is bound by its chain: redux -> row start -> words -> best of the
+// neighbours -> redux.  The next vertex is the least of the lanes' block minima
+// and of this step's own updates, so the updates need not reach their blocks
+// within the step: they go to `mail` (32 words, one per block: the least update
+// since the block's last rescan), read in the shadow of the next step's loads,
+// as is the rescan of the block that the last vertex left.  BL: words of a
+// block a lane rescans (a block is 32 * BL vertices).  Measured on synthetic
+// sparse graphs of degree 4: 253 / 261 / 265 cycles a step for BL = 1 / 2 / 4;
+// with the updates handed over by shuffles 633 to 655, by the mailbox within
+// the step 377 to 392.
+template <int BL, bool kOnChip>
+__device__ __forceinline__ bool sparse_prim_warp(int n, uint32_t start, uint32_t best, uint32_t adj,
+                                                 const uint32_t* adj_off, uint32_t order, uint32_t rank, uint32_t mail) {
+    constexpr int kShift = (BL == 1 ? 5 : (BL == 2 ? 6 : 7)) + 2;  // of byte offsets
+    static_assert((32 << kShift) == 4096 * BL, "32 blocks of 32 * BL vertices");
+    const uint32_t lane = threadIdx.x & 31, end = 4u * (uint32_t)n;
+    const uint32_t mine = mail + 4 * lane;
+    uint32_t least = (lane << kShift) < end ? kWordUnreached : kWordIn;
+    sts32_if(true, mine, 0xffffffffu);
+    uint32_t cur = 0;
+    bool ok = true;
+    auto words_at = [&](uint32_t first, uint32_t i, uint32_t count) {
+        if constexpr (kOnChip) return lds32_if(i < count, adj + 4 * (first + i), kWordUnreached);
+        return i < count ? adj_off[first + i] : kWordUnreached;
+    };
     for (int it = 0; it < n - 1; ++it) {
-        const uint32_t row = start[cur];  // first word << 12 | count
-        const int count = (int)(row & 0xfffu);
-        const uint32_t* words = adj + (row >> 12);
-        uint32_t word = lane < count ? words[lane] : kWordIn;
-        // The block that cur left.
-        const int own = cur >> shift;
-        uint32_t rest = kWordIn;
-        for (int j = lane; j < block; j += 32) {
-            const int v = (own << shift) + j;
-            if (v < n) rest = min(rest, best[v]);
+        const uint32_t own = cur >> kShift;
+        const uint32_t row = lds32(start + cur);  // first word << 12 | count
+        sts32_if(lane == 0, best + cur, kWordIn);
+        const uint32_t post = lds32(mine);
+        uint32_t block[BL];
+#pragma unroll
+        for (int j = 0; j < BL; ++j) {
+            const uint32_t v = (own << kShift) + 128 * j + 4 * lane;
+            block[j] = lds32_if(v < end, best + v, kWordIn);
         }
+        const uint32_t count = row & 0xfffu, first = row >> 12;
+        uint32_t word = words_at(first, lane, count);
+        least = min(least, post);
+        uint32_t rest = block[0];
+#pragma unroll
+        for (int j = 1; j < BL; ++j) rest = min(rest, block[j]);
         rest = __reduce_min_sync(0xffffffffu, rest);
+        uint32_t b = lds32_if(lane < count, best + word_offset(word), 0u);
+        sts32_if(lane == own, mine, 0xffffffffu);
         if (lane == own) least = rest;
-        for (int e = 0; e < count; e += 32) {
-            if (e) word = e + lane < count ? words[e + lane] : kWordIn;
-            bool lower = false;
-            if (word != kWordIn) {
-                const int v = (int)(word & 0xfffu);
-                const uint32_t b = best[v];
-                lower = b != kWordIn && word < b;
-                if (lower) best[v] = word;
-            }
-            unsigned bal = __ballot_sync(0xffffffffu, lower);
-            while (bal) {
-                const int s = __ffs(bal) - 1;
-                bal &= bal - 1;
-                const uint32_t x = __shfl_sync(0xffffffffu, word, s);
-                if ((int)((x & 0xfffu) >> shift) == lane) least = min(least, x);
-            }
+        bool lower = (int)word < (int)b;  // strict: an equal older edge stays
+        uint32_t update = lower ? word : 0xffffffffu;
+        sts32_if(lower, best + word_offset(word), word);
+        reds_min_if(lower, mail + 4 * (word_offset(word) >> kShift), word);
+        for (uint32_t e = 32; e < count; e += 32) {
+            word = words_at(first, e + lane, count);
+            b = lds32_if(e + lane < count, best + word_offset(word), 0u);
+            lower = (int)word < (int)b;
+            if (lower) update = min(update, word);
+            sts32_if(lower, best + word_offset(word), word);
+            reds_min_if(lower, mail + 4 * (word_offset(word) >> kShift), word);
         }
-        const uint32_t next = __reduce_min_sync(0xffffffffu, least);
-        if (next >= kWordUnreached) return false;  // not connected
-        cur = (int)(next & 0xfffu);
-        if (lane == 0) {
-            order[it] = (int16_t)cur;
-            rank[it] = (int16_t)(next >> 12);
-            best[cur] = kWordIn;
-        }
-        __syncwarp();
+        const uint32_t next = __reduce_min_sync(0xffffffffu, min(least, update));
+        ok = ok && next < kWordUnreached;  // else not connected: every vertex left is unreached
+        cur = word_offset(next) < end ? word_offset(next) : 0;
+        sts16_if(lane == 0, order + 2 * it, cur >> 2);
+        sts16_if(lane == 0, rank + 2 * it, next >> 14);
     }
-    return true;
+    __syncwarp();
+    return ok;
+}
+
+template <bool kOnChip>
+__device__ __forceinline__ bool sparse_prim(int n, const uint32_t* start, const uint32_t* best, const uint32_t* adj,
+                                            const uint32_t* adj_off, const int16_t* order, const int16_t* rank,
+                                            const uint32_t* mail) {
+    const uint32_t s = shared_address(start), b = shared_address(best), a = shared_address(adj),
+                   o = shared_address(order), r = shared_address(rank), m = shared_address(mail);
+    if (n <= 1024) return sparse_prim_warp<1, kOnChip>(n, s, b, a, adj_off, o, r, m);
+    if (n <= 2048) return sparse_prim_warp<2, kOnChip>(n, s, b, a, adj_off, o, r, m);
+    return sparse_prim_warp<4, kOnChip>(n, s, b, a, adj_off, o, r, m);
 }
 
 // Ascending bitonic sort of k[0..P) (P a power of two) by the CTA.
@@ -1148,7 +1203,7 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
     Arena<Real> ar = Arena<Real>::carve(smem, n);
     const int cap = Arena<Real>::round_cap(n);
-    if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 0] = f.stage_ns[8 * w + 1] = global_ns();
+    if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 0] = global_ns();
     const int n_light = a.light_count[w], n_star = a.unit_core ? 0 : a.star_count[w];
     const int m = n_light + n_star;
     const uint32_t* __restrict__ light_uv = a.light_uv + base * a.light_cap;
@@ -1288,20 +1343,21 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
         const uint32_t u = uv & 0xffff, v = uv >> 16;
         const uint32_t at_u = atomicAdd(&best[u], 1u), at_v = atomicAdd(&best[v], 1u);
         if (on_chip) {
-            adj[at_u] = (r << 12) | v;
-            adj[at_v] = (r << 12) | u;
+            adj[at_u] = prim_word(r, v);
+            adj[at_v] = prim_word(r, u);
         } else {
-            adj_off[at_u] = (r << 12) | v;
-            adj_off[at_v] = (r << 12) | u;
+            adj_off[at_u] = prim_word(r, v);
+            adj_off[at_v] = prim_word(r, u);
         }
     }
     __syncthreads();
     for (int v = tid; v < n; v += nt) best[v] = kWordUnreached;
     __syncthreads();
+    if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 1] = global_ns();
     // ---- 3. order ---------------------------------------------------------------
     if (warp == 0) {
-        const bool ok = on_chip ? sparse_prim_warp(n, start, best, adj, ar.s1, ar.s0)
-                                : sparse_prim_warp(n, start, best, adj_off, ar.s1, ar.s0);
+        const bool ok = on_chip ? sparse_prim<true>(n, start, best, adj, adj_off, ar.s1, ar.s0, s_scan)
+                                : sparse_prim<false>(n, start, best, adj, adj_off, ar.s1, ar.s0, s_scan);
         if (lane == 0) s_ok = ok;
     }
     __syncthreads();
