@@ -66,7 +66,7 @@ cudaError_t launch_select(const CoreArgs& a, int grid, size_t smem, cudaStream_t
 template <typename Real>
 cudaError_t launch_prepare(const void* X, int input_type, void* out, int64_t points, int D, int normalize,
                            cudaStream_t s, int priority) {
-    const unsigned grid = (unsigned)((points + 255) / 256);
+    const unsigned grid = (unsigned)((points + kPreparePoints - 1) / kPreparePoints);
     Real* y = static_cast<Real*>(out);
     if (input_type == kInputBF16)
         return launch_ex(hdb_prepare_kernel<Real, __nv_bfloat16>, grid, 256, 0, s, priority, 1,
