@@ -83,6 +83,7 @@ struct CoreArgs {
     int n_items;
     int D;
     int ms;                      // order statistic k = ms-1 (0-based), self included
+    int rows;                    // select kernel: rows per item
     const void* dist;            // matrix variant only
     const int64_t* dist_offsets;
     void* core;                  // [T]

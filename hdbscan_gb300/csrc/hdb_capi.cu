@@ -51,6 +51,7 @@ struct CoreLaunch {
     std::vector<int32_t> items;             // (window, row) pairs
     size_t items_off = 0;                   // byte offset in tables
     size_t select_smem = 0;
+    int select_rows = 1;                    // rows per item
 };
 
 // Windows of the sparse path that are launched together (hdb_sparse.cuh).
@@ -446,17 +447,18 @@ int build_plan(hdb_plan* p) {
             launch.cv = choose_core(k, p->precision, p->ms, p->D, matrix);
             CoreLaunch select;
             select.matrix = matrix;
+            select.select_rows = hdb::select_rows(c.nmax, real_bytes(p->precision));
             for (int w : c.windows) {
                 const int n = size_of(w);
                 if (launch.cv) {
                     for (int r = 0; r < n; r += launch.cv->rows) { launch.items.push_back(w); launch.items.push_back(r); }
                 } else {
-                    for (int r = 0; r < n; ++r) { select.items.push_back(w); select.items.push_back(r); }
+                    for (int r = 0; r < n; r += select.select_rows) { select.items.push_back(w); select.items.push_back(r); }
                 }
             }
             if (!launch.items.empty()) c.cores.push_back(launch);
             if (!select.items.empty()) {
-                select.select_smem = (size_t)c.nmax * (size_t)real_bytes(p->precision);
+                select.select_smem = (size_t)select.select_rows * (size_t)c.nmax * (size_t)real_bytes(p->precision);
                 c.cores.push_back(select);
             }
         }
@@ -500,7 +502,7 @@ int build_plan(hdb_plan* p) {
     }
     for (auto& cls : p->classes)
         for (auto& c : cls.cores)
-            if (!c.cv && c.select_smem > 48 * 1024) HDB_CUDA(raise_smem_limit(k.select_func, c.select_smem));
+            if (!c.cv) HDB_CUDA(raise_smem_limit(k.select_func, c.select_smem));
 
     // ---- table image --------------------------------------------------------
     std::vector<unsigned char> image;
@@ -869,6 +871,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             a.n_items = (int)(cl.items.size() / 2);
             a.D = p->D;
             a.ms = p->ms;
+            a.rows = cl.select_rows;
             a.dist = cl.matrix ? dist : nullptr;
             a.dist_offsets = d_dist_off;
             a.core = core;

@@ -238,8 +238,9 @@ extern "C" int hdb_cluster_noalloc(int precision, const void* X, int batch, int 
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fv->func, fv->threads + 32, smem);
     if (e != cudaSuccess) return fail(HDB_E_CUDA, std::string("forward kernel set-up: ") + cudaGetErrorString(e));
     if (per_sm < 1) return fail(HDB_E_INVALID, "forward kernel variant cannot be resident");
-    const size_t select_smem = (size_t)n * (precision == HDB_F32 ? 4 : 8);
-    if (!unit && !cv && select_smem > 48 * 1024) {
+    const int select_rows = hdb::select_rows(n, precision == HDB_F32 ? 4 : 8);
+    const size_t select_smem = (size_t)select_rows * (size_t)n * (precision == HDB_F32 ? 4 : 8);
+    if (!unit && !cv) {
         e = hdb::raise_dynamic_smem(k.select_func, select_smem);
         if (e != cudaSuccess) return fail(HDB_E_CUDA, std::string("select kernel set-up: ") + cudaGetErrorString(e));
     }
@@ -250,7 +251,7 @@ extern "C" int hdb_cluster_noalloc(int precision, const void* X, int batch, int 
     int32_t* ticket = reinterpret_cast<int32_t*>(scratch + kOffTicket);
     int32_t* items = reinterpret_cast<int32_t*>(scratch + kOffItems);
     void* core = scratch + kOffCore;
-    const int rows_per_item = unit ? 1 : (cv ? cv->rows : 1);
+    const int rows_per_item = unit ? 1 : (cv ? cv->rows : select_rows);
     const int n_items = unit ? 0 : batch * ((n + rows_per_item - 1) / rows_per_item);
     const int work = (batch + 1 > n_items ? batch + 1 : n_items);
     noalloc_tables_kernel<<<(work + 255) / 256, 256, 0, stream>>>(offsets, queue, ticket, items, batch, n,
@@ -266,6 +267,7 @@ extern "C" int hdb_cluster_noalloc(int precision, const void* X, int batch, int 
         a.n_items = n_items;
         a.D = dims;
         a.ms = min_samples;
+        a.rows = select_rows;
         a.core = core;
         a.status = status;
         if (cv) e = cv->launch(a, n_items, stream, 0);

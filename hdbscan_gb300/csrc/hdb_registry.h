@@ -66,6 +66,14 @@ const PrecisionKernels& kernels_f64();
 const ForwardVariant* cluster_variants_f32(int* count);
 const ForwardVariant* cluster_variants_f64(int* count);
 
+// Rows per CTA of the select kernel (one warp each): their distances share
+// 64 KB of shared memory, so that three CTAs fit an SM.
+inline int select_rows(int nmax, int real_bytes) {
+    int rows = 8;
+    while (rows > 1 && (size_t)rows * (size_t)nmax * (size_t)real_bytes > (64u << 10)) rows >>= 1;
+    return rows;
+}
+
 // Raise (never lower) a kernel's dynamic shared-memory limit; thread-safe.
 cudaError_t raise_dynamic_smem(const void* func, size_t bytes);
 
