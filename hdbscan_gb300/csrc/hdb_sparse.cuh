@@ -38,6 +38,7 @@
 #include "hdb_common.cuh"
 #include "hdb_distance.cuh"
 #include "hdb_forward.cuh"
+#include "hdb_tree_cta.cuh"
 
 namespace hdb {
 
@@ -1170,21 +1171,6 @@ __device__ __forceinline__ bool sparse_prim(int n, const uint32_t* start, const 
     return sparse_prim_warp<4, kOnChip>(n, s, b, a, adj_off, o, r, m);
 }
 
-// Ascending bitonic sort of k[0..P) (P a power of two) by the CTA.
-template <typename Key>
-__device__ __forceinline__ void bitonic_cta(Key* k, int P) {
-    for (int size = 2; size <= P; size <<= 1) {
-        for (int j = size >> 1; j > 0; j >>= 1) {
-            for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-                const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
-                const Key x = k[lo], y = k[hi];
-                if (key_lt(y, x) == ((lo & size) == 0)) { k[lo] = y; k[hi] = x; }
-            }
-            __syncthreads();
-        }
-    }
-}
-
 template <typename Real>
 __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a, const __grid_constant__ ForwardArgs f) {
     using T = RealTraits<Real>;
@@ -1192,7 +1178,7 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
     constexpr bool kWide = sizeof(Real) == 8;
     constexpr Key kNoKey = (Key)~(Key)0;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ uint32_t s_scan[32];
+    __shared__ uint32_t s_scan[33];
     __shared__ int s_ctr[4];
     __shared__ int s_edges;
     __shared__ int s_ok;
@@ -1286,6 +1272,9 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
     for (int i = tid; i < P; i += nt) sorted[i] = i < n - 1 ? T::key(ar.r0[i]) : kNoKey;
     __syncthreads();
     bitonic_cta<Key>(sorted, P);
+    bool twin = false;
+    for (int i = tid; i + 1 < n - 1; i += nt) twin |= key_eq(sorted[i], sorted[i + 1]);
+    const bool distinct = !__syncthreads_or(twin);
     // ---- 2. adjacency -----------------------------------------------------------
     uint32_t* start = reinterpret_cast<uint32_t*>(ar.r2);
     uint32_t* best = kWide ? start + cap : reinterpret_cast<uint32_t*>(ar.s2);
@@ -1403,6 +1392,8 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
     for (int i = tid; i < n - 1; i += nt) {
         const uint32_t p = source[ar.s1[i]];
         lost |= p > (uint32_t)i;
+        if (distinct) ar.s2[ar.s0[i]] = (int16_t)i;
+        else ar.s2[i] = ar.s0[i];
         ar.r0[i] = T::from_key(sorted[ar.s0[i]]);
         ar.s0[i] = p == 0 || p > (uint32_t)i ? (int16_t)0 : ar.s1[p - 1];
     }
@@ -1411,9 +1402,7 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
         return;
     }
     if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 2] = global_ns();
-    const bool help = !a.unit_core && n - 1 >= kHelpMinEdges;
-    if (warp == 0) tree_window<Real>(f, smem, w, n, help ? s_ctr : nullptr);
-    else if (help) sort_edges_cta<Real>(ar, n - 1, nt, kBarHelp, s_ctr);
+    tree_window_cta<Real>(f, smem, w, n, distinct, s_scan, s_ctr, kBarHelp);
 }
 
 }  // namespace hdb

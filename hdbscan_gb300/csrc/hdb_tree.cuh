@@ -48,6 +48,21 @@ namespace hdb {
 template <typename Real> struct SortPair;
 template <> struct __align__(8) SortPair<float> { float w; int32_t idx; };
 template <> struct __align__(16) SortPair<double> { double w; int64_t idx; };
+// Rank of the weight << 16 | index: where ranks are known, one word stands for both.
+struct RankPair { uint32_t v; };
+
+// What the introsort compares and returns of its elements.
+template <typename Pair> struct SortTraits;
+template <typename Real> struct SortTraits<SortPair<Real>> {
+    using Key = Real;
+    __device__ __forceinline__ static Real key(const SortPair<Real>& p) { return p.w; }
+    __device__ __forceinline__ static bool lt(Real a, Real b) { return RealTraits<Real>::lt(a, b); }
+};
+template <> struct SortTraits<RankPair> {
+    using Key = uint32_t;
+    __device__ __forceinline__ static uint32_t key(const RankPair& p) { return p.v >> 16; }
+    __device__ __forceinline__ static bool lt(uint32_t a, uint32_t b) { return a < b; }
+};
 
 // Shared-memory arena for one window of capacity `cap` points (cap >= n).
 //  r0  Real[cap]  Prim edge weights -> weights in sorted order (merge weights)
@@ -98,62 +113,65 @@ __device__ __forceinline__ unsigned lanemask_lt() {
 // ---------------------------------------------------------------------------
 // Introsort (reference: _kernels.py:358-516; NumPy 2.3.5 aquicksort).
 // ---------------------------------------------------------------------------
-template <typename Real>
-__device__ void heap_sort_pairs(SortPair<Real>* p, int lo, int hi) {
+template <typename Pair>
+__device__ void heap_sort_pairs(Pair* p, int lo, int hi) {
+    using S = SortTraits<Pair>;
     const int count = hi - lo + 1;
-    SortPair<Real>* a = p + lo - 1;  // 1-based
+    Pair* a = p + lo - 1;  // 1-based
     for (int root = count / 2; root >= 1; --root) {
-        SortPair<Real> value = a[root];
+        Pair value = a[root];
         int pos = root, child = 2 * root;
         while (child <= count) {
-            if (child < count && RealTraits<Real>::lt(a[child].w, a[child + 1].w)) ++child;
-            if (RealTraits<Real>::lt(value.w, a[child].w)) { a[pos] = a[child]; pos = child; child *= 2; } else break;
+            if (child < count && S::lt(S::key(a[child]), S::key(a[child + 1]))) ++child;
+            if (S::lt(S::key(value), S::key(a[child]))) { a[pos] = a[child]; pos = child; child *= 2; } else break;
         }
         a[pos] = value;
     }
     for (int end = count; end > 1;) {
-        SortPair<Real> value = a[end];
+        Pair value = a[end];
         a[end] = a[1];
         --end;
         int pos = 1, child = 2;
         while (child <= end) {
-            if (child < end && RealTraits<Real>::lt(a[child].w, a[child + 1].w)) ++child;
-            if (RealTraits<Real>::lt(value.w, a[child].w)) { a[pos] = a[child]; pos = child; child *= 2; } else break;
+            if (child < end && S::lt(S::key(a[child]), S::key(a[child + 1]))) ++child;
+            if (S::lt(S::key(value), S::key(a[child]))) { a[pos] = a[child]; pos = child; child *= 2; } else break;
         }
         a[pos] = value;
     }
 }
 
-template <typename Real>
-__device__ void insertion_sort_pairs(SortPair<Real>* p, int lo, int hi) {
+template <typename Pair>
+__device__ void insertion_sort_pairs(Pair* p, int lo, int hi) {
+    using S = SortTraits<Pair>;
     for (int i = lo + 1; i <= hi; ++i) {
-        SortPair<Real> value = p[i];
+        Pair value = p[i];
         int j = i;
-        while (j > lo && RealTraits<Real>::lt(value.w, p[j - 1].w)) { p[j] = p[j - 1]; --j; }
+        while (j > lo && S::lt(S::key(value), S::key(p[j - 1]))) { p[j] = p[j - 1]; --j; }
         p[j] = value;
     }
 }
 
-template <typename Real>
-__device__ __forceinline__ void swap_pairs(SortPair<Real>* p, int i, int j) {
-    SortPair<Real> t = p[i]; p[i] = p[j]; p[j] = t;
+template <typename Pair>
+__device__ __forceinline__ void swap_pairs(Pair* p, int i, int j) {
+    Pair t = p[i]; p[i] = p[j]; p[j] = t;
 }
 
 // One Hoare partition of p[lo..hi] (hi - lo > 15) by one lane: NumPy's
 // median-of-three, pivot parked at hi-1, unguarded i/j scans (p[hi-1] and
 // p[lo] are the sentinels) and the final swap (_kernels.py:444-462).
-template <typename Real>
-__device__ int partition_serial(SortPair<Real>* p, int lo, int hi) {
+template <typename Pair>
+__device__ int partition_serial(Pair* p, int lo, int hi) {
+    using S = SortTraits<Pair>;
     const int mid = lo + ((hi - lo) >> 1);
-    if (RealTraits<Real>::lt(p[mid].w, p[lo].w)) swap_pairs(p, mid, lo);
-    if (RealTraits<Real>::lt(p[hi].w, p[mid].w)) swap_pairs(p, hi, mid);
-    if (RealTraits<Real>::lt(p[mid].w, p[lo].w)) swap_pairs(p, mid, lo);
+    if (S::lt(S::key(p[mid]), S::key(p[lo]))) swap_pairs(p, mid, lo);
+    if (S::lt(S::key(p[hi]), S::key(p[mid]))) swap_pairs(p, hi, mid);
+    if (S::lt(S::key(p[mid]), S::key(p[lo]))) swap_pairs(p, mid, lo);
     swap_pairs(p, mid, hi - 1);
-    const Real pivot = p[hi - 1].w;
+    const auto pivot = S::key(p[hi - 1]);
     int i = lo, j = hi - 1;
     for (;;) {
-        do ++i; while (RealTraits<Real>::lt(p[i].w, pivot));
-        do --j; while (RealTraits<Real>::lt(pivot, p[j].w));
+        do ++i; while (S::lt(S::key(p[i]), pivot));
+        do --j; while (S::lt(pivot, S::key(p[j])));
         if (i >= j) break;
         swap_pairs(p, i, j);
     }
@@ -173,8 +191,8 @@ static_assert((kLaneSortMax >> (kLaneStack - 1)) <= 16, "lane introsort stack to
 // checked: a checked segment with negative depth is heapsorted (the check a
 // popped segment gets); an unchecked one (the smaller side that the loop
 // continues on) is partitioned first (_kernels.py:433-470).
-template <typename Real>
-__device__ void introsort_lane(SortPair<Real>* p, int lo, int hi, int code) {
+template <typename Pair>
+__device__ void introsort_lane(Pair* p, int lo, int hi, int code) {
     int depth = code >> 1;  // arithmetic shift keeps negative depths
     bool checked = code & 1;
     int st_lo[kLaneStack], st_hi[kLaneStack], st_depth[kLaneStack];
@@ -200,27 +218,28 @@ __device__ void introsort_lane(SortPair<Real>* p, int lo, int hi, int code) {
 
 // One Hoare partition of p[lo..hi] (hi - lo > 15) by the whole warp.
 // Returns the pivot's final position (warp-uniform).
-template <typename Real>
-__device__ int partition_warp(SortPair<Real>* p, int lo, int hi, int16_t* list_a, int16_t* list_b) {
+template <typename Pair>
+__device__ int partition_warp(Pair* p, int lo, int hi, int16_t* list_a, int16_t* list_b) {
+    using S = SortTraits<Pair>;
     const int lane = threadIdx.x & 31;
     if (lane == 0) {
         const int mid = lo + ((hi - lo) >> 1);
-        if (RealTraits<Real>::lt(p[mid].w, p[lo].w)) swap_pairs(p, mid, lo);
-        if (RealTraits<Real>::lt(p[hi].w, p[mid].w)) swap_pairs(p, hi, mid);
-        if (RealTraits<Real>::lt(p[mid].w, p[lo].w)) swap_pairs(p, mid, lo);
+        if (S::lt(S::key(p[mid]), S::key(p[lo]))) swap_pairs(p, mid, lo);
+        if (S::lt(S::key(p[hi]), S::key(p[mid]))) swap_pairs(p, hi, mid);
+        if (S::lt(S::key(p[mid]), S::key(p[lo]))) swap_pairs(p, mid, lo);
         swap_pairs(p, mid, hi - 1);
     }
     __syncwarp();
-    const Real pivot = p[hi - 1].w;
+    const auto pivot = S::key(p[hi - 1]);
     // Pass 1: stopper totals.
     int total_a = 0, total_b = 0;
     for (int base = lo; base <= hi - 1; base += 32) {
         const int pos = base + lane;
         bool fa = false, fb = false;
         if (pos <= hi - 1) {
-            const Real w = p[pos].w;
-            fa = pos >= lo + 1 && !RealTraits<Real>::lt(w, pivot);
-            fb = pos <= hi - 2 && !RealTraits<Real>::lt(pivot, w);
+            const auto w = S::key(p[pos]);
+            fa = pos >= lo + 1 && !S::lt(w, pivot);
+            fb = pos <= hi - 2 && !S::lt(pivot, w);
         }
         total_a += __popc(__ballot_sync(0xffffffffu, fa));
         total_b += __popc(__ballot_sync(0xffffffffu, fb));
@@ -232,9 +251,9 @@ __device__ int partition_warp(SortPair<Real>* p, int lo, int hi, int16_t* list_a
         const int pos = base + lane;
         bool fa = false, fb = false;
         if (pos <= hi - 1) {
-            const Real w = p[pos].w;
-            fa = pos >= lo + 1 && !RealTraits<Real>::lt(w, pivot);
-            fb = pos <= hi - 2 && !RealTraits<Real>::lt(pivot, w);
+            const auto w = S::key(p[pos]);
+            fa = pos >= lo + 1 && !S::lt(w, pivot);
+            fb = pos <= hi - 2 && !S::lt(pivot, w);
         }
         const unsigned ba = __ballot_sync(0xffffffffu, fa);
         const unsigned bb = __ballot_sync(0xffffffffu, fb);
@@ -413,21 +432,39 @@ __device__ void sort_edges_warp(const Arena<Real>& a, int m, bool try_distinct) 
     __syncwarp();
 }
 
-// The same sort by every warp of the CTA (`nthreads` threads, all of which
-// must call; the named barrier `bar` spans them): the partition tasks go in
-// rounds, each warp taking every nw-th task of the round, and the lane
-// segments are shared by all threads.  Segments are disjoint and each one's
-// partition depends only on its own bounds and depth code, so the result
-// equals the one-warp form's.  ctr: four ints of shared memory.
-template <typename Real>
-__device__ __forceinline__ void sort_edges_cta(const Arena<Real>& a, int m, int nthreads, int bar, int* ctr) {
+// NumPy's insertion sort of a segment of at most 16 elements by a half-warp:
+// insertion is stable, so an element's place is the count of smaller elements
+// plus that of equal ones before it.
+template <typename Pair>
+__device__ __forceinline__ void insertion_sort_half_warp(Pair* p, int lo, int hi) {
+    using S = SortTraits<Pair>;
+    const int sub = threadIdx.x & 15;
+    const unsigned half = 0xffffu << (threadIdx.x & 16);
+    const int size = hi - lo + 1;
+    Pair mine = p[lo + (sub < size ? sub : 0)];
+    const auto key = S::key(mine);
+    int place = 0;
+    for (int j = 0; j < size; ++j) {
+        const auto other = __shfl_sync(half, key, j, 16);
+        place += S::lt(other, key) || (j < sub && !S::lt(key, other));
+    }
+    __syncwarp(half);
+    if (sub < size) p[lo + place] = mine;
+}
+
+// The same sort of p[0..m) by every warp of the CTA (`nthreads` threads, all of
+// which must call; the named barrier `bar` spans them): the partition tasks go
+// in rounds, each warp taking every nw-th task of the round; segments of at
+// most 16 elements are shared by the half-warps, depth-exhausted ones by the
+// threads.  Segments are disjoint and each one's partition depends only on its
+// own bounds and depth code, so the result equals the one-warp form's.  ctr:
+// four ints of shared memory; scratch: s2..s9 of the arena.
+template <typename Pair, typename Real>
+__device__ __forceinline__ void sort_pairs_cta(Pair* p, const Arena<Real>& a, int m, int nthreads, int bar, int* ctr) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = nthreads >> 5;
-    SortPair<Real>* p = reinterpret_cast<SortPair<Real>*>(a.r1);
-    for (int i = tid; i < m; i += nthreads) { p[i].w = a.r0[i]; p[i].idx = i; }
     int16_t *task_lo = a.s5, *task_hi = a.s6, *task_depth = a.s7;  // two halves: this round, next round
     int16_t *leaf_lo = a.s8, *leaf_hi = a.s9, *leaf_code = a.s2;
     const int half = Arena<Real>::round_cap(m + 1) / 2;
-    const int lane_max = 33;
     if (tid == 0) {
         int depth = 0;
         for (int c = m; c > 1; c >>= 1) depth += 2;  // 2*floor(log2(m)), _kernels.py:429-431
@@ -446,8 +483,8 @@ __device__ __forceinline__ void sort_edges_cta(const Arena<Real>& a, int m, int 
             const int lo = task_lo[cur + t], hi = task_hi[cur + t], code = task_depth[cur + t];
             const int depth = code >> 1;  // arithmetic shift keeps negative depths
             const bool checked = code & 1;
-            if ((checked && depth < 0) || hi - lo + 1 < lane_max) {
-                if (lane == 0) {
+            if ((checked && depth < 0) || hi - lo <= 15) {
+                if (lane == 0 && hi > lo) {
                     const int k = atomicAdd(ctr + 3, 1);
                     leaf_lo[k] = (int16_t)lo; leaf_hi[k] = (int16_t)hi; leaf_code[k] = (int16_t)code;
                 }
@@ -470,8 +507,24 @@ __device__ __forceinline__ void sort_edges_cta(const Arena<Real>& a, int m, int 
         count = *pushes;
     }
     const int leaves = ctr[3];
-    for (int t = tid; t < leaves; t += nthreads) introsort_lane(p, leaf_lo[t], leaf_hi[t], leaf_code[t]);
+    for (int t = tid >> 4; t < leaves; t += nthreads >> 4) {
+        const int lo = leaf_lo[t], hi = leaf_hi[t], code = leaf_code[t];
+        if ((code & 1) && (code >> 1) < 0) {  // exhausted depth: heapsort (reference :442-443)
+            if ((tid & 15) == 0) heap_sort_pairs(p, lo, hi);
+        } else {
+            insertion_sort_half_warp(p, lo, hi);
+        }
+    }
     asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(nthreads) : "memory");
+}
+
+// sort_edges_warp's result by the whole CTA.
+template <typename Real>
+__device__ __forceinline__ void sort_edges_cta(const Arena<Real>& a, int m, int nthreads, int bar, int* ctr) {
+    const int tid = threadIdx.x;
+    SortPair<Real>* p = reinterpret_cast<SortPair<Real>*>(a.r1);
+    for (int i = tid; i < m; i += nthreads) { p[i].w = a.r0[i]; p[i].idx = i; }
+    sort_pairs_cta(p, a, m, nthreads, bar, ctr);
     for (int i = tid; i < m; i += nthreads) {
         a.s2[i] = (int16_t)p[i].idx;
         a.r0[i] = p[i].w;
