@@ -108,8 +108,13 @@ struct SparseArgs {
     int unit_core;
     int32_t* flags;              // [B+1] 1 = the window takes the general path; [B] = any window does
     int n_flags;                 // B
-    float* y;                    // [T, D] float64 input rounded to float32 around each window's first point
-    uint32_t* range;             // [B] float bits of max |x - x0| (float64)
+    int approx;                  // distances are bounded float32 ones (else exact: float32 windows of few dims)
+    int gram;                    // bounded squared distances from tensor-core products (else differences)
+    float* y;                    // differences: [T, D] input rounded to float32 around each window's first point
+    uint16_t* split;             // products: [T, dims / 32, 64] centred input as bfloat16 pairs, 32 high then 32 low parts
+    int dims;                    // D rounded up to 32
+    float* norm;                 // products: [T] squared norms of the centred points
+    uint32_t* range;             // [B] float bits of max |x - x0| (products: of the largest norm)
     void* dist;                  // distance blocks (float32 values, see sparse_block)
     const int64_t* dist_offsets;
     uint16_t* knn_idx;           // [T, list] nearest neighbours by (distance, index), self included

@@ -99,10 +99,11 @@ struct hdb_plan {
     std::vector<WindowClass> classes;
     std::vector<SparseGroup> groups;        // windows on the sparse path
     int list = 0, keep = 0;                 // neighbour list stride and length
+    bool gram = false, approx = false;      // bounded distances, from tensor-core products
     int light_cap = 0, star_cap = 0;        // light and star edges per point
     std::vector<int64_t> table_offsets;     // per window (entries) of the component tables
     size_t t_table = 0, t_flags = 0, t_range = 0, t_light_count = 0, t_star_count = 0;
-    size_t w_y = 0, w_knn_idx = 0, w_knn_d = 0, w_core_up = 0, w_core_down = 0, w_part = 0, w_parts = 0, w_edges = 0, w_table = 0, w_level_comp = 0, w_level_max_v = 0,
+    size_t w_y = 0, w_split = 0, w_norm = 0, w_knn_idx = 0, w_knn_d = 0, w_core_up = 0, w_core_down = 0, w_part = 0, w_parts = 0, w_edges = 0, w_table = 0, w_level_comp = 0, w_level_max_v = 0,
            w_level_end_v = 0, w_perm = 0, w_pos = 0, w_level_max = 0, w_level_end = 0, w_levels = 0, w_light_uv = 0, w_light_w = 0,
            w_star_uv = 0, w_star_mask = 0, w_edge_rank = 0, w_adj = 0;
     std::vector<int32_t> tiles;             // (window, ti, tj), grouped by class
@@ -158,6 +159,7 @@ constexpr int kTile128MinN = 384;  // float32 matrix classes from this size use 
 
 // Windows of fewer points stay on the general path (their dense loop is short).
 constexpr int kSparseMinN = 16;
+constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
 constexpr unsigned kGeneralGrid = 152 * 8;  // CTAs of a general-path launch that may find nothing to do
@@ -329,7 +331,16 @@ int build_plan(hdb_plan* p) {
     // class, which does the windows it flags.
     std::vector<char> sparse(p->B, 0);
     int sparse_nmax = 0;
-    p->list = hdb::sparse_list(p->precision, p->ms);
+    // Tensor-core products: always for wide float64 points; for float32 they
+    // replace exact distances at the price of three more launches and of exact
+    // distances for the few pairs that matter, which pays from about this many
+    // coordinate pairs (one window 4001 x 32: 1.58 ms without, 1.73 with; 512 ragged
+    // windows of 32 dims: 8.46 without, 8.00 with).
+    double coordinate_pairs = 0;
+    for (int w : order) coordinate_pairs += (double)size_of(w) * size_of(w) * p->D;
+    p->gram = hdb::sparse_gram(p->D) && (p->precision == HDB_F64 || coordinate_pairs >= kGramMinWork);
+    p->approx = p->gram || p->precision == HDB_F64;
+    p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
     if (p->list && !(p->flags & kNoSparseFlags)) {
         for (int w : order)
             sparse[w] = size_of(w) >= kSparseMinN && chosen[w]->cluster == 1 &&
@@ -420,7 +431,7 @@ int build_plan(hdb_plan* p) {
         if (c.fv->dp != 0) continue;
         // Float32 classes of larger windows take the 128x128 tile kernel.
         c.tile = (p->precision == HDB_F32 && c.nmax >= kTile128MinN) ? 128 : 64;
-        const bool tiles = !(c.general && p->precision == HDB_F32);  // those come from the sparse path
+        const bool tiles = !(c.general && !p->approx);  // exact ones are the sparse path's own
         for (int w : c.windows) {
             const int n = size_of(w);
             const int64_t ld = (n + 3) & ~3;
@@ -441,7 +452,7 @@ int build_plan(hdb_plan* p) {
     if (!unit) {
         for (auto& c : p->classes) {
             const bool matrix = c.fv->dp == 0;
-            if (c.general && p->precision == HDB_F32) continue;  // the sparse path leaves exact core distances
+            if (c.general && !p->approx) continue;  // the sparse path leaves exact core distances
             CoreLaunch launch;
             launch.matrix = matrix;
             launch.cv = choose_core(k, p->precision, p->ms, p->D, matrix);
@@ -563,7 +574,6 @@ int build_plan(hdb_plan* p) {
     p->w_prep = ws = align_up(ws, 256);
     if (p->prepared) ws += (size_t)p->T * (size_t)p->D * rb;
     if (!p->groups.empty()) {
-        p->keep = unit ? 8 : std::min(p->list, std::max(p->ms + 3, 8));
         // About one to three of each per point in ordinary data; more send a window to the general path.
         p->light_cap = 12;
         p->star_cap = unit ? 0 : 8;
@@ -574,8 +584,13 @@ int build_plan(hdb_plan* p) {
             ws = at + bytes;
             return at;
         };
-        if (p->precision == HDB_F64) {
-            p->w_y = take(T * (size_t)p->D * sizeof(float));
+        if (p->approx) {
+            if (p->gram) {
+                p->w_split = take(T * 2 * align_up((size_t)p->D, 32) * sizeof(uint16_t));
+                p->w_norm = take(T * sizeof(float));
+            } else {
+                p->w_y = take(T * (size_t)p->D * sizeof(float));
+            }
             p->w_core_up = take(T * sizeof(float));
             p->w_core_down = take(T * sizeof(float));
         }
@@ -760,7 +775,12 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.unit_core = unit ? 1 : 0;
         a.flags = reinterpret_cast<int32_t*>(ws + p->t_flags);
         a.n_flags = p->B;
+        a.approx = p->approx ? 1 : 0;
+        a.gram = p->gram ? 1 : 0;
         a.y = reinterpret_cast<float*>(ws + p->w_y);
+        a.split = reinterpret_cast<uint16_t*>(ws + p->w_split);
+        a.dims = (int)align_up((size_t)p->D, 32);
+        a.norm = reinterpret_cast<float*>(ws + p->w_norm);
         a.range = reinterpret_cast<uint32_t*>(ws + p->t_range);
         a.dist = dist;
         a.dist_offsets = d_dist_off;
@@ -770,8 +790,8 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.keep = p->keep;
         a.core = core;
         a.core_nbr = core_nbr;
-        a.core_up = p->precision == HDB_F64 ? reinterpret_cast<float*>(ws + p->w_core_up) : static_cast<float*>(core);
-        a.core_down = p->precision == HDB_F64 ? reinterpret_cast<float*>(ws + p->w_core_down) : static_cast<float*>(core);
+        a.core_up = p->approx ? reinterpret_cast<float*>(ws + p->w_core_up) : static_cast<float*>(core);
+        a.core_down = p->approx ? reinterpret_cast<float*>(ws + p->w_core_down) : static_cast<float*>(core);
         a.part = reinterpret_cast<uint16_t*>(ws + p->w_part);
         a.parts = reinterpret_cast<int32_t*>(ws + p->w_parts);
         a.edges = reinterpret_cast<unsigned long long*>(ws + p->w_edges);
@@ -802,7 +822,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             if (spans) HDB_CUDA(spans->end(s));
             return HDB_OK;
         };
-        const bool wide = p->precision == HDB_F64;
+        const bool wide = p->approx;
         int rc = HDB_OK;
         if (wide) rc = stage(hdb::SparseStage::kNarrow, HDB_PHASE_PREPARE, stream);
         if (!rc) rc = stage(hdb::SparseStage::kTiles, HDB_PHASE_DISTANCE, stream);
@@ -841,8 +861,8 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             joined = n_groups + i;
         }
         const unsigned grid_limit = c.general ? kGeneralGrid : 0xffffffffu;
-        // float32: the sparse path left the exact distances and core distances.
-        const bool have_rows = c.general && p->precision == HDB_F32;
+        // Where the sparse path's distances are exact, they and the core distances are there already.
+        const bool have_rows = c.general && !p->approx;
         // 1. distance blocks of this class's matrix-variant windows (caller's stream)
         if (c.n_tiles && !have_rows) {
             hdb::DistanceArgs a{};

@@ -227,17 +227,14 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_k
 // round-to-nearest adds, a correctly rounded sqrt.
 constexpr int kDistTile128 = 128;
 
-template <typename Real>
-__global__ void __launch_bounds__(256, 2) hdb_distance128_kernel(const DistanceArgs args) {
-    static_assert(sizeof(Real) == 4, "the 128x128 tile kernel is float32 only");
+__device__ __forceinline__ void distance128_tile(const DistanceArgs& args, int tile) {
     using T = RealTraits<float>;
     constexpr int KC = 32;
     constexpr int TS = kDistTile128;
     __shared__ __align__(16) float s_i[KC][TS];
     __shared__ __align__(16) float s_j[KC][TS];
-    const int tile = blockIdx.x;
-    if (tile >= args.n_tiles) return;
     const int w = args.tiles[3 * tile], ti = args.tiles[3 * tile + 1], tj = args.tiles[3 * tile + 2];
+    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const int D = args.D;
@@ -336,6 +333,14 @@ __global__ void __launch_bounds__(256, 2) hdb_distance128_kernel(const DistanceA
         }
     }
     if (__syncthreads_or(overflow) && tid == 0) atomic_status(args.status, kOverflow);
+}
+
+// One CTA a tile, or a fixed grid over all tiles behind the sparse path.
+template <typename Real>
+__global__ void __launch_bounds__(256, 2) hdb_distance128_kernel(const DistanceArgs args) {
+    static_assert(sizeof(Real) == 4, "the 128x128 tile kernel is float32 only");
+    if (args.only && !args.only[args.n_only]) return;
+    for (int tile = blockIdx.x; tile < args.n_tiles; tile += gridDim.x) distance128_tile(args, tile);
 }
 
 // ---------------------------------------------------------------------------

@@ -35,6 +35,8 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
             return launch_rows<Real>(a, s, priority);
         case SparseStage::kTiles: {
             const unsigned t = blocks(a.nmax, 128);
+            if (a.gram)
+                return launch_ex(hdb_sparse_gram_kernel<Real>, W * (t * (t + 1) / 2), 256, 2 * kGramStage, s, priority, 1, a);
             return launch_ex(hdb_sparse_tiles_kernel<Real>, W * (t * (t + 1) / 2), 256, 0, s, priority, 1, a);
         }
         case SparseStage::kForest:
@@ -57,30 +59,33 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
         default:
             break;
     }
-    if constexpr (sizeof(Real) == 8) {
-        switch (stage) {
-            case SparseStage::kNarrow:
+    switch (stage) {
+        case SparseStage::kNarrow:
+            if (a.gram)
+                return launch_ex(hdb_sparse_split_kernel<Real>, W * blocks(a.nmax, kSplitRows), 256, 0, s, priority, 1, a);
+            if constexpr (sizeof(Real) == 8)
                 return launch_ex(hdb_sparse_narrow_kernel, W * blocks(a.nmax, kNarrowRows), 256, 0, s, priority, 1, a);
-            case SparseStage::kCore:
-                return launch_ex(hdb_sparse_core_kernel, W * blocks(a.nmax, 128), 128, 0, s, priority, 1, a);
-            case SparseStage::kWeights:
-                return launch_ex(hdb_sparse_weights_kernel, W * kWeightsPerWindow, 128, 0, s, priority, 1, a);
-            default:
-                break;
-        }
+            break;
+        case SparseStage::kCore:
+            return launch_ex(hdb_sparse_core_kernel<Real>, W * blocks(a.nmax, 128), 128, 0, s, priority, 1, a);
+        case SparseStage::kWeights:
+            return launch_ex(hdb_sparse_weights_kernel<Real>, W * kWeightsPerWindow, 128, 0, s, priority, 1, a);
+        default:
+            break;
     }
     return cudaErrorInvalidValue;
 }
 
 template <typename Real>
 cudaError_t prepare(int n, size_t budget, bool* fits) {
-    const size_t need[5] = {sparse_forest_smem(n), sparse_between_smem(n), sparse_tree_smem(n), light_smem(n),
+    const size_t need[6] = {2 * kGramStage, sparse_forest_smem(n), sparse_between_smem(n), sparse_tree_smem(n), light_smem(n),
                             SparsePrimLayout<Real>::bytes(n)};
-    const void* func[5] = {(const void*)hdb_sparse_forest_kernel<Real>, (const void*)hdb_sparse_between_kernel<Real>,
+    const void* func[6] = {(const void*)hdb_sparse_gram_kernel<Real>,
+                           (const void*)hdb_sparse_forest_kernel<Real>, (const void*)hdb_sparse_between_kernel<Real>,
                            (const void*)hdb_sparse_tree_kernel<Real>, (const void*)hdb_sparse_light_kernel<Real>,
                            (const void*)hdb_sparse_prim_kernel<Real>};
     *fits = true;
-    for (int i = 0; i < 5; ++i) {
+    for (int i = 0; i < 6; ++i) {
         cudaFuncAttributes attr;
         cudaError_t e = cudaFuncGetAttributes(&attr, func[i]);
         if (e != cudaSuccess) return e;
@@ -103,11 +108,18 @@ cudaError_t sparse_prepare(int precision, int n, size_t budget, bool* fits) {
     return precision == 0 ? prepare<float>(n, budget, fits) : prepare<double>(n, budget, fits);
 }
 
-int sparse_list(int precision, int ms) {
-    // Entries past position ms - 1 show where the star ends (and bound float64's uncertain range).
-    const int need = ms <= 2 ? 8 : (precision == 0 ? ms + 1 : ms + 2);
+bool sparse_gram(int D) { return D >= kGramMinDims && D <= kGramMaxDims; }
+
+int sparse_list(bool approx, bool gram, int ms, int* keep) {
+    // Entries past position ms - 1 show where the star ends and bound the
+    // uncertain range, which is wider for products.
+    const int want = ms <= 2 ? 8 : (gram ? ms + ms / 4 + 10 : (approx ? ms + 3 : ms + 1));
+    const int need = ms <= 2 ? 8 : (gram ? ms + 6 : (approx ? ms + 2 : ms + 1));
     for (int k : {8, 16, 32, 64})
-        if (need <= k) return k;
+        if (want <= k || (need <= k && k == 64)) {
+            *keep = ms <= 2 ? 8 : (want < k ? (want < 8 ? 8 : want) : k);
+            return k;
+        }
     return 0;
 }
 

@@ -24,11 +24,12 @@
 // they are in the neighbour lists, and one of them for each component that the
 // star touches below core_x is enough for the order (hdb_sparse_star_kernel).
 //
-// float64: the pass over all pairs and the neighbour lists use float32
-// distances with a proven bound (sparse_bound); every comparison that decides
-// something takes the safe side, and all weights, core distances and ties come
-// from exact float64 arithmetic on the few pairs that remain.  float32: the
-// distance blocks are the exact ones and the bounds are zero.
+// float64 windows and wide float32 ones: the pass over all pairs and the
+// neighbour lists use float32 distances with a proven bound (sparse_bound), for
+// wide points from tensor-core products; every comparison that decides something
+// takes the safe side, and all weights, core distances and ties come from exact
+// arithmetic in the window's own precision on the few pairs that remain.
+// float32 windows of few dims: the distance blocks are exact, the bounds zero.
 //
 // A window that does not fit (more light edges than the workspace holds, as
 // with many equal distances; neighbours that the bound cannot tell apart;
@@ -39,6 +40,7 @@
 #include "hdb_distance.cuh"
 #include "hdb_forward.cuh"
 #include "hdb_tree_cta.cuh"
+#include <cuda_bf16.h>
 
 namespace hdb {
 
@@ -67,20 +69,43 @@ __device__ __forceinline__ float* sparse_block(const SparseArgs& a, int w) {
 // Both are taken 5% larger (plus some units) than that, which covers second
 // order terms, the float64 arithmetic's own rounding and the evaluation of the
 // bound itself.
+//
+// Products (D >= kGramMinDims): the block holds a lower bound of the squared
+// distance, n_i + n_j - 2 z_i.z_j - eta (n_i + n_j) with the centred points z as
+// sums of two bfloat16 parts (see sparse_eta), and the true value lies at most
+// 2 eta (n_i + n_j) above it.  Core distances and all weights of the kernels
+// below are then squares as well; exact values stay plain distances.
 struct SparseBound {
-    float shift, scale;
-    __device__ __forceinline__ float up(float d) const {
-        return __fmaf_ru(d, __fadd_ru(1.0f, scale), shift);
-    }
-    __device__ __forceinline__ float down(float d) const {
-        return __fmaf_rd(d, __fadd_rd(1.0f, -scale), -shift);
-    }
+    float up_shift, up_scale, down_shift, down_scale;
+    __device__ __forceinline__ float up(float d) const { return __fmaf_ru(d, up_scale, up_shift); }
+    __device__ __forceinline__ float down(float d) const { return __fmaf_rd(d, down_scale, down_shift); }
 };
+
+// Bound of |s~ - d^2| / (n_i + n_j) for s~ = n_i + n_j - 2 g, all in float32:
+//   * z = hi + lo + e with |lo| <= 2^-9 |z|, |e| <= 2^-18 |z| (bfloat16 has 8
+//     significant bits); hi.hi + hi.lo + lo.hi leaves out lo.lo and the products
+//     with e: 3 * 2^-18 |z_i||z_j|;
+//   * each matrix instruction adds 16 exact products to its accumulator; 2^-20 of
+//     the running magnitude a step allows for every operand being cut off at 24
+//     bits below the largest (its rounding is not specified).  The accumulator
+//     starts anew every 32 coordinates, six steps, so these errors are six shares
+//     of the parts' |z_i||z_j|, whose sum is at most the whole's;
+//   * the parts' sum, the norms' sums, z's own rounding to float32 and the last
+//     operations: (D / 8 + 32) 2^-24.
+// 2 |z_i||z_j| <= n_i + n_j turns the products' shares into shares of n_i + n_j;
+// 10% on top covers second order terms.
+__device__ __forceinline__ float sparse_eta(int D) {
+    return 1.1f * (3.0f * 3.8146973e-6f + 6.0f * 9.5367432e-7f + (float)(D / 8 + 32) * 5.9604645e-8f);
+}
+
 template <typename Real>
 __device__ __forceinline__ SparseBound sparse_bound(const SparseArgs& a, int w) {
-    if constexpr (sizeof(Real) == 4) return SparseBound{0.0f, 0.0f};
+    if (!a.approx) return SparseBound{0.0f, 1.0f, 0.0f, 1.0f};
     const float R = __uint_as_float(a.range[w]);
-    return SparseBound{1.05f * sqrtf((float)a.D) * 1.1920929e-7f * R, 1.05f * (0.5f * (float)a.D + 8.0f) * 5.9604645e-8f};
+    if (a.gram) return SparseBound{4.2f * sparse_eta(a.D) * R, 1.0000005f, 0.0f, 1.0f};
+    const float shift = 1.05f * sqrtf((float)a.D) * 1.1920929e-7f * R;
+    const float scale = 1.05f * (0.5f * (float)a.D + 8.0f) * 5.9604645e-8f;
+    return SparseBound{shift, __fadd_ru(1.0f, scale), -shift, __fadd_rd(1.0f, -scale)};
 }
 
 // Exact distance of two rows in the reference's order (k-ordered sum).
@@ -140,6 +165,227 @@ __global__ void __launch_bounds__(256) hdb_sparse_narrow_kernel(const SparseArgs
     const float R = __uint_as_float(top);
     if (bad || !(R <= 1.0995e12f)) sparse_flag(a, w);  // also tests NaN
     if ((threadIdx.x & 31) == 0) atomicMax(a.range + w, top);
+}
+
+// The same for products: points centred on the mean of kCentrePoints of the
+// window's points (any centre is exact enough; a near one keeps the norms, and
+// with them the bound, small), as bfloat16 pairs, and their squared norms.  One
+// warp a row.
+constexpr int kGramMinDims = 32;
+constexpr int kGramMaxDims = 2048;   // the centre in shared memory
+constexpr int kCentrePoints = 16;
+constexpr int kSplitRows = 32;
+
+template <typename Real>
+__global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs a) {
+    __shared__ Real s_centre[kGramMaxDims];
+    const int per = (a.nmax + kSplitRows - 1) / kSplitRows;
+    const int item = blockIdx.x / per, r0 = (blockIdx.x - item * per) * kSplitRows;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (r0 >= n) return;
+    const int D = a.D, dims = a.dims;
+    const Real* __restrict__ X = static_cast<const Real*>(a.X) + base * D;
+    for (int k = threadIdx.x; k < D; k += 256) {
+        Real sum = Real(0);
+#pragma unroll
+        for (int j = 0; j < kCentrePoints; ++j) sum += X[(int64_t)(j * n / kCentrePoints) * D + k];
+        s_centre[k] = sum * Real(1.0 / kCentrePoints);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int r = warp; r < kSplitRows; r += 8) {
+        const int i = r0 + r;
+        if (i >= n) break;
+        const Real* __restrict__ x = X + (int64_t)i * D;
+        uint16_t* __restrict__ out = a.split + (base + i) * 2 * dims;
+        float norm = 0.0f;
+        bool bad = false;
+        for (int k = lane; k < dims; k += 32) {
+            float z = 0.0f;
+            if (k < D) {
+                const Real v = x[k];
+                bad |= !isfinite(v);
+                z = (float)(v - s_centre[k]);
+            }
+            const __nv_bfloat16 hi = __float2bfloat16_rn(z);
+            const __nv_bfloat16 lo = __float2bfloat16_rn(__fsub_rn(z, __bfloat162float(hi)));
+            const int at = (k >> 5) * 64 + (k & 31);
+            out[at] = __bfloat16_as_ushort(hi);
+            out[at + 32] = __bfloat16_as_ushort(lo);
+            norm = __fmaf_rn(z, z, norm);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
+        bad = __any_sync(0xffffffffu, bad) || !(norm <= 1.2e24f);  // 2^80; also tests NaN
+        if (lane == 0) {
+            a.norm[base + i] = norm;
+            if (bad) sparse_flag(a, w);
+            else atomicMax(a.range + w, __float_as_uint(norm));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Lower bounds of the squared distances from tensor-core products: 128x128 tiles
+// of the upper triangle, 8 warps of 32x64 pairs, three bfloat16 matrix products
+// (high.high, high.low, low.high) accumulated in float32.  A row's 32
+// coordinates are one 128-byte line of high and low parts; two stages of
+// asynchronous copies, 16-byte chunks swizzled by row for ldmatrix.  Off-diagonal
+// values are written to both halves from one accumulator, so the block is
+// symmetric.  Bound by the block's own write (4 n^2 bytes) for small D.
+// ---------------------------------------------------------------------------
+constexpr int kGramStage = 2 * 128 * 128;  // bytes of a stage: two operands of 128 rows x 128 bytes
+
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t at) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArgs a) {
+    constexpr int TS = 128;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ float s_norm[2][TS];
+    const int tmax = (a.nmax + TS - 1) / TS;
+    const int per = tmax * (tmax + 1) / 2;
+    const int item = blockIdx.x / per;
+    const int t = blockIdx.x - item * per;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    int tj = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+    while (tj * (tj + 1) / 2 > t) --tj;
+    while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
+    const int ti = t - tj * (tj + 1) / 2;
+    if (tj * TS >= n || a.flags[w]) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int i0 = ti * TS, j0 = tj * TS;
+    const int chunks = a.dims >> 5;
+    const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
+    const uint16_t* __restrict__ S = a.split + base * 2 * a.dims;
+    for (int r = tid; r < 2 * TS; r += 256) {
+        const int g = (r < TS ? i0 + r : j0 + r - TS);
+        s_norm[r >> 7][r & (TS - 1)] = g < n ? a.norm[base + g] : 0.0f;
+    }
+    auto load = [&](int c, int stage) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int e = tid + 256 * q;          // 2 operands x 128 rows x 8 chunks
+            const int op = e >> 10, r = (e >> 3) & 127, ch = e & 7;
+            const int g = (op == 0 ? i0 : j0) + r;
+            const uint32_t dst = sbase + stage * kGramStage + op * (TS * 128) + r * 128 + ((ch ^ (r & 7)) << 4);
+            const uint16_t* src = S + (int64_t)min(g, n - 1) * 2 * a.dims + c * 64 + ch * 8;
+            const int bytes = g < n ? 16 : 0;     // rows past the window are zeros
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+        }
+        asm volatile("cp.async.commit_group;");
+    };
+    float acc[2][8][4];
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+#pragma unroll
+            for (int r = 0; r < 4; ++r) acc[p][q][r] = 0.0f;
+    const int wm = (warp & 3) * 32, wn = (warp >> 2) * 64;
+    load(0, 0);
+    for (int c = 0; c < chunks; ++c) {
+        if (c + 1 < chunks) {
+            load(c + 1, (c + 1) & 1);
+            asm volatile("cp.async.wait_group 1;");
+        } else {
+            asm volatile("cp.async.wait_group 0;");
+        }
+        __syncthreads();
+        const uint32_t A = sbase + (c & 1) * kGramStage, B = A + TS * 128;
+        uint32_t hi[2][2][4], lo[2][2][4];  // [16 coordinates][16 rows]
+#pragma unroll
+        for (int k = 0; k < 2; ++k)
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                const int r = wm + 16 * p + (lane & 15);
+                const int ch = 2 * k + (lane >> 4);
+                ldmatrix4(hi[k][p], A + r * 128 + ((ch ^ (r & 7)) << 4));
+                ldmatrix4(lo[k][p], A + r * 128 + (((ch + 4) ^ (r & 7)) << 4));
+            }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = wn + 16 * q + (lane & 7) + ((lane >> 4) << 3);
+            float part[2][2][4];
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) part[p][h][e] = 0.0f;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int ch = 2 * k + ((lane >> 3) & 1);
+                uint32_t bh[4], bl[4];
+                ldmatrix4(bh, B + r * 128 + ((ch ^ (r & 7)) << 4));
+                ldmatrix4(bl, B + r * 128 + (((ch + 4) ^ (r & 7)) << 4));
+#pragma unroll
+                for (int p = 0; p < 2; ++p)
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        mma_bf16(part[p][h], hi[k][p], bl[2 * h], bl[2 * h + 1]);
+                        mma_bf16(part[p][h], lo[k][p], bh[2 * h], bh[2 * h + 1]);
+                        mma_bf16(part[p][h], hi[k][p], bh[2 * h], bh[2 * h + 1]);
+                    }
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p)
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) acc[p][2 * q + h][e] += part[p][h][e];
+        }
+        __syncthreads();
+    }
+    const float eta = sparse_eta(a.D);
+    float* __restrict__ Dw = sparse_block<Real>(a, w);
+    const int64_t ld = dist_ld(n);
+    const bool diagonal = ti == tj;
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = wm + 16 * p + 8 * h + (lane >> 2), gi = i0 + r;
+            if (gi >= n) continue;
+            const float ni = s_norm[0][r];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int col = wn + 8 * q + 2 * (lane & 3), gj = j0 + col;
+                float v[2];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const float sum = ni + s_norm[1][col + b];
+                    v[b] = fmaxf(__fmaf_rn(-eta, sum, __fmaf_rn(-2.0f, acc[p][q][2 * h + b], sum)), 0.0f);
+                }
+                if (!diagonal) {
+                    // (gj < n and even imply that column gj + 1 lies inside the row's stride.)
+                    if (gj < n) *reinterpret_cast<float2*>(Dw + gi * ld + gj) = make_float2(v[0], v[1]);
+#pragma unroll
+                    for (int b = 0; b < 2; ++b)
+                        if (gj + b < n) Dw[(int64_t)(gj + b) * ld + gi] = v[b];
+                } else {
+#pragma unroll
+                    for (int b = 0; b < 2; ++b) {
+                        if (gj + b >= n || gi > gj + b) continue;
+                        const float x = gi == gj + b ? 0.0f : v[b];
+                        Dw[gi * ld + gj + b] = x;
+                        Dw[(int64_t)(gj + b) * ld + gi] = x;
+                    }
+                }
+            }
+        }
 }
 
 // ---------------------------------------------------------------------------
@@ -264,9 +510,9 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseAr
 // ---------------------------------------------------------------------------
 // Nearest-neighbour lists of every row, one warp a row, as hdb_core_rows_kernel
 // builds them (the K smallest (distance, index), ascending, position p in lane
-// p % 32).  float32 with core distances: position ms - 1 is the core distance.
-// float64: the rank ms - 1 is certain except among the entries whose bounds
-// overlap the entry at position ms - 1; their positions [c, e) go to core_nbr
+// p % 32).  Exact distances: position ms - 1 is the core distance.  Bounded
+// ones: the rank ms - 1 is certain except among the entries whose bounds
+// overlap that entry's; their positions [c, e) go to core_nbr
 // for hdb_sparse_core_kernel.  A list that ends inside that range, or a
 // distance that is not finite, flags the window.
 // ---------------------------------------------------------------------------
@@ -282,7 +528,7 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(co
     const int64_t base = a.offsets[w];
     const int n = (int)(a.offsets[w + 1] - base);
     // float32 core distances also serve the general path of a flagged window.
-    if (r0 >= n || (sizeof(Real) == 8 && a.flags[w])) return;
+    if (r0 >= n || (a.approx && a.flags[w])) return;
     const float* __restrict__ Dw = sparse_block<Real>(a, w);
     const int64_t ld = dist_ld(n);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -375,7 +621,7 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(co
         bool unsure = wild;
         if (!a.unit_core) {
             const int pos = a.ms - 1;
-            if constexpr (sizeof(Real) == 4) {
+            if (!a.approx) {
 #pragma unroll
                 for (int h = 0; h < E; ++h)
                     if (pos == lane + 32 * h) {
@@ -385,15 +631,30 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(co
                 // Points as far as the core distance may follow the list's end.
                 if (at(last) <= at(pos) && keep < n) unsure = true;
             } else {
-                const float mid = __uint_as_float(at(pos));
-                const float least = bound.down(mid), most = bound.up(mid);
-                int c = 0, e = 0;
+                // The value of rank ms - 1 is at least the lower bound at that
+                // position and at most the largest upper bound up to it.
+                const float least = bound.down(__uint_as_float(at(pos)));
+                const int inside = min(keep, n);
+                float up[E], most = 0.0f;
+                const float slack = 2.1f * sparse_eta(a.D);
+                const float norm_i = a.gram ? a.norm[row_at] : 0.0f;
 #pragma unroll
                 for (int h = 0; h < E; ++h) {
+                    const int p = lane + 32 * h;
                     const float d = __uint_as_float(lk[h]);
-                    const bool in = lane + 32 * h < min(keep, n);
-                    c += __popc(__ballot_sync(0xffffffffu, in && bound.up(d) < least));
-                    e += __popc(__ballot_sync(0xffffffffu, in && bound.down(d) <= most));
+                    up[h] = bound.up(d);
+                    if (a.gram && p < inside) up[h] = __fmaf_ru(slack, norm_i + a.norm[base + li[h]], d);
+                    if (p <= pos) most = fmaxf(most, up[h]);
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+                int c = inside, e = 0;
+#pragma unroll
+                for (int h = E - 1; h >= 0; --h) {
+                    const int p = lane + 32 * h;
+                    const unsigned open = __ballot_sync(0xffffffffu, p < inside && !(up[h] < least));
+                    if (open) c = 32 * h + __ffs(open) - 1;
+                    e += __popc(__ballot_sync(0xffffffffu, p < inside && bound.down(__uint_as_float(lk[h])) <= most));
                 }
                 if (e >= keep && keep < n) unsure = true;  // the range may go on beyond the list
                 if (lane == 0) a.core_nbr[row_at] = c | (e << 8);
@@ -403,50 +664,77 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(co
     }
 }
 
-// float64 core distances: the exact distances of each row's uncertain range
-// (nearly always one entry), the right one by (distance, index).
+// Core distances from bounded ones: the exact distances of each row's uncertain
+// range (mostly one entry), the right one by (distance, index).  A warp takes 32
+// rows and spreads all their entries over its lanes.
+constexpr int kCoreEntries = 256;  // uncertain entries of 32 rows
+
+template <typename Real>
 __global__ void __launch_bounds__(128) hdb_sparse_core_kernel(const SparseArgs a) {
+    __shared__ Real s_d[4][kCoreEntries];
+    __shared__ uint16_t s_entry[4][kCoreEntries];  // row << 8 | list position
     const int per = (a.nmax + 127) / 128;
-    const int item = blockIdx.x / per, i = (blockIdx.x - item * per) * 128 + threadIdx.x;
+    const int item = blockIdx.x / per, i0 = (blockIdx.x - item * per) * 128;
     const int w = a.queue[item];
     const int64_t base = a.offsets[w];
     const int n = (int)(a.offsets[w + 1] - base);
-    if (i >= n || a.flags[w]) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int first = i0 + 32 * warp, i = first + lane;
+    if (first >= n || a.flags[w]) return;  // warp-uniform
     const int D = a.D;
-    const double* __restrict__ X = static_cast<const double*>(a.X) + base * D;
-    const double* __restrict__ xi = X + (int64_t)i * D;
+    const Real* __restrict__ X = static_cast<const Real*>(a.X) + base * D;
     const int64_t row = base + i;
-    const uint16_t* __restrict__ list = a.knn_idx + row * a.list;
-    const int range = a.core_nbr[row];
+    const int range = i < n ? a.core_nbr[row] : 0;
     const int c = range & 0xff, e = range >> 8;
-    double value = 0;
-    int index = -1;
-    if (e - c == 1) {
-        index = list[c];
-        value = sparse_exact<double>(xi, X + (int64_t)index * D, D);
-    } else {
-        // The (ms - 1 - c)-th smallest of the range: repeated minimum above the last one taken.
-        double d_last = -1.0;
-        int j_last = -1;
-        for (int t = c; t <= a.ms - 1; ++t) {
-            double d_best = 0;
-            int j_best = -1;
-            for (int s = c; s < e; ++s) {
-                const int j = list[s];
-                const double d = sparse_exact<double>(xi, X + (int64_t)j * D, D);
-                const bool above = d > d_last || (d == d_last && j > j_last);
-                if (above && (j_best < 0 || d < d_best || (d == d_best && j < j_best))) { d_best = d; j_best = j; }
-            }
-            d_last = d_best;
-            j_last = j_best;
-        }
-        value = d_last;
-        index = j_last;
+    const int count = e - c;
+    int at = count;  // inclusive, then exclusive prefix
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += y;
     }
-    static_cast<double*>(a.core)[row] = value;
+    const int total = __shfl_sync(0xffffffffu, at, 31);
+    at -= count;
+    if (total > kCoreEntries) {  // the bound separates too little here
+        if (lane == 0) sparse_flag(a, w);
+        return;
+    }
+    for (int s = 0; s < count; ++s) s_entry[warp][at + s] = (uint16_t)((lane << 8) | (c + s));
+    __syncwarp();
+    for (int t = lane; t < total; t += 32) {
+        const int entry = s_entry[warp][t];
+        const int u = first + (entry >> 8);
+        const int v = a.knn_idx[(base + u) * a.list + (entry & 0xff)];
+        s_d[warp][t] = sparse_exact<Real>(X + (int64_t)u * D, X + (int64_t)v * D, D);
+    }
+    __syncwarp();
+    if (i >= n) return;
+    // The (ms - 1 - c)-th smallest of the range: repeated minimum above the last one taken.
+    const uint16_t* __restrict__ list = a.knn_idx + row * a.list;
+    Real value = Real(-1);
+    int index = -1;
+    for (int t = c; t <= a.ms - 1; ++t) {
+        Real best = Real(0);
+        int j_best = -1;
+        for (int s = 0; s < count; ++s) {
+            const Real d = s_d[warp][at + s];
+            const int j = list[c + s];
+            const bool above = d > value || (d == value && j > index);
+            if (above && (j_best < 0 || d < best || (d == best && j < j_best))) { best = d; j_best = j; }
+        }
+        value = best;
+        index = j_best;
+    }
+    static_cast<Real*>(a.core)[row] = value;
     a.core_nbr[row] = index;
-    a.core_up[row] = __double2float_ru(value);
-    a.core_down[row] = __double2float_rd(value);
+    // In the block's terms: squares where it holds squares.
+    if constexpr (sizeof(Real) == 4) {
+        a.core_up[row] = __fmul_ru(value, value);
+        a.core_down[row] = __fmul_rd(value, value);
+    } else {
+        a.core_up[row] = __double2float_ru(a.gram ? __dmul_ru(value, value) : value);
+        a.core_down[row] = __double2float_rd(a.gram ? __dmul_rd(value, value) : value);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -523,10 +811,10 @@ __global__ void __launch_bounds__(512) hdb_sparse_forest_kernel(const SparseArgs
     uint16_t* up = comp + cap;
     uint8_t* at = reinterpret_cast<uint8_t*>(up + cap);
     const SparseBound bound = sparse_bound<Real>(a, w);
-    if constexpr (sizeof(Real) == 8) {
+    if (a.approx) {
         // A range below 2^-40 (other than identical points) is outside the bound's domain.
         const float R = __uint_as_float(a.range[w]);
-        if (R != 0.0f && R < 9.1e-13f) {
+        if (R != 0.0f && R < (a.gram ? 8.3e-25f : 9.1e-13f)) {
             if (tid == 0) sparse_flag(a, w);
             return;
         }
@@ -912,7 +1200,7 @@ __global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs 
                     sparse_flag(a, w);
                 } else {
                     light_uv[at] = (uint32_t)u | ((uint32_t)v << 16);
-                    if constexpr (sizeof(Real) == 4) light_w[at] = d;  // above both cores
+                    if (!a.approx) light_w[at] = (Real)d;  // above both cores
                 }
             }
         }
@@ -1006,24 +1294,25 @@ __global__ void __launch_bounds__(256) hdb_sparse_star_kernel(const SparseArgs a
     }
 }
 
-// Exact weights of the light edges (float64).
+// Exact weights of the light edges (bounded distances).
 constexpr int kWeightsPerWindow = 8;  // CTAs of 128 threads sharing a window's edges
 
+template <typename Real>
 __global__ void __launch_bounds__(128) hdb_sparse_weights_kernel(const SparseArgs a) {
-    using T = RealTraits<double>;
+    using T = RealTraits<Real>;
     const int item = blockIdx.x / kWeightsPerWindow, part = blockIdx.x - item * kWeightsPerWindow;
     const int w = a.queue[item];
     if (a.flags[w]) return;
     const int64_t base = a.offsets[w];
     const int D = a.D;
     const int count = a.light_count[w];
-    const double* __restrict__ X = static_cast<const double*>(a.X) + base * D;
-    const double* core = static_cast<const double*>(a.core);
-    double* light_w = static_cast<double*>(a.light_w) + base * a.light_cap;
+    const Real* __restrict__ X = static_cast<const Real*>(a.X) + base * D;
+    const Real* core = static_cast<const Real*>(a.core);
+    Real* light_w = static_cast<Real*>(a.light_w) + base * a.light_cap;
     for (int e = part * 128 + threadIdx.x; e < count; e += 128 * kWeightsPerWindow) {
         const uint32_t uv = a.light_uv[base * a.light_cap + e];
         const int u = uv & 0xffff, v = uv >> 16;
-        double d = sparse_exact<double>(X + (int64_t)u * D, X + (int64_t)v * D, D);
+        Real d = sparse_exact<Real>(X + (int64_t)u * D, X + (int64_t)v * D, D);
         if (!a.unit_core) d = T::vmax(T::vmax(core[base + u], core[base + v]), d);
         light_w[e] = d;
     }

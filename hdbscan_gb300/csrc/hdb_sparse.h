@@ -9,8 +9,8 @@ namespace hdb {
 enum class SparseStage { kNarrow, kTiles, kRows, kCore, kForest, kBetween, kTree, kLight, kStar, kWeights, kPrim };
 
 // Launches `stage` for the windows of `a`; `f` is the forward's argument block
-// (kPrim only).  precision: 0 float32, 1 float64 (kNarrow, kCore and
-// kWeights exist for float64 only).
+// (kPrim only).  precision: 0 float32, 1 float64 (kNarrow, kCore and kWeights
+// belong to bounded distances, SparseArgs::approx).
 cudaError_t sparse_launch(int precision, SparseStage stage, const SparseArgs& a, const ForwardArgs* f,
                           cudaStream_t stream, int priority);
 
@@ -18,7 +18,11 @@ cudaError_t sparse_launch(int precision, SparseStage stage, const SparseArgs& a,
 // in *fits when a window of that size does not fit in `budget` bytes.
 cudaError_t sparse_prepare(int precision, int n, size_t budget, bool* fits);
 
-// Row stride of the neighbour lists for min_samples ms (0: not supported).
-int sparse_list(int precision, int ms);
+// Whether windows of D dims take tensor-core products.
+bool sparse_gram(int D);
+
+// Row stride of the neighbour lists for min_samples ms (0: not supported) and
+// the entries used of them.
+int sparse_list(bool approx, bool gram, int ms, int* keep);
 
 }  // namespace hdb

@@ -147,3 +147,21 @@ def test_long_lists(cuda, ms, precision):
     rng = np.random.default_rng(ms)
     d = 7 if precision == "float64" else 70
     _check([_mixture(rng, n, d) for n in (ms, ms + 1, 200, 900)], 10, ms, 0.0, precision)
+
+
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_many_flagged_windows(cuda, precision):
+    # More distance tiles and rows on the general path than one pass of its fixed grids holds.
+    rng = np.random.default_rng(99)
+    # (Every point 50 times: no list can reach past its copies.)
+    windows = [np.repeat(rng.normal(size=(22 + i % 5, 36)), 50, axis=0) for i in range(40)]
+    windows += [_mixture(rng, 700, 36) for _ in range(3)]
+    dtype = np.float32 if precision == "float32" else np.float64
+    host, offsets, describe, flags = _run([x.astype(dtype) for x in windows], 5, 6, 0.0, precision)
+    assert flags[:40].all() and not flags[40:].any()
+    for w in (0, 7, 23, 39, 40, 42):
+        o = oracle.cluster(windows[w].astype(dtype), 5, 6, 0.0, precision)
+        lo, hi = offsets[w], offsets[w + 1]
+        np.testing.assert_array_equal(host["edges_uv"][lo - w:hi - w - 1], o["edges_uv"])
+        np.testing.assert_array_equal(host["core"][lo:hi].view(np.uint8), o["core"].view(np.uint8))
+        np.testing.assert_array_equal(host["labels"][lo:hi], o["labels"])
