@@ -113,6 +113,7 @@ struct SparseArgs {
     float* y;                    // differences: [T, D] input rounded to float32 around each window's first point
     uint16_t* split;             // products: [T, dims / 32, 64] centred input as bfloat16 pairs, 32 high then 32 low parts
     int dims;                    // D rounded up to 32
+    float* minima;               // products: minimum of every 16 entries of the blocks' rows
     float* norm;                 // products: [T] squared norms of the centred points
     uint32_t* range;             // [B] float bits of max |x - x0| (products: of the largest norm)
     void* dist;                  // distance blocks (float32 values, see sparse_block)
@@ -132,10 +133,8 @@ struct SparseArgs {
     const int64_t* table_offsets;  // [B]
     uint16_t* level_comp;        // [kSparseLevels, T] component (its representative vertex) after each merge round
     float* level_max_v;          // [kSparseLevels, T] by vertex: largest tree edge on the way up
-    uint16_t* level_end_v;       // [kSparseLevels, T] by vertex: end of the component's leaf interval
-    uint16_t* perm;              // [T] leaf order -> vertex
-    float* level_max;            // the same in leaf order
-    uint16_t* level_end;
+    uint32_t* level_span;        // [kSparseLevels, T] by vertex: its component's leaf interval, begin | end << 16
+    uint16_t* perm;              // [T] vertices in component order
     int32_t* levels;             // [B] merge rounds
     uint16_t* pos;               // [T] vertex -> leaf position
     int32_t* light_count;        // [B] light edges other than star edges

@@ -104,7 +104,7 @@ struct hdb_plan {
     std::vector<int64_t> table_offsets;     // per window (entries) of the component tables
     size_t t_table = 0, t_flags = 0, t_range = 0, t_light_count = 0, t_star_count = 0;
     size_t w_y = 0, w_split = 0, w_norm = 0, w_knn_idx = 0, w_knn_d = 0, w_core_up = 0, w_core_down = 0, w_part = 0, w_parts = 0, w_edges = 0, w_table = 0, w_level_comp = 0, w_level_max_v = 0,
-           w_level_end_v = 0, w_perm = 0, w_pos = 0, w_level_max = 0, w_level_end = 0, w_levels = 0, w_light_uv = 0, w_light_w = 0,
+           w_level_span = 0, w_perm = 0, w_pos = 0, w_minima = 0, w_levels = 0, w_light_uv = 0, w_light_w = 0,
            w_star_uv = 0, w_star_mask = 0, w_edge_rank = 0, w_adj = 0;
     std::vector<int32_t> tiles;             // (window, ti, tj), grouped by class
     std::vector<int64_t> dist_offsets;      // per window (elements), -1 if not materialized
@@ -588,6 +588,7 @@ int build_plan(hdb_plan* p) {
             if (p->gram) {
                 p->w_split = take(T * 2 * align_up((size_t)p->D, 32) * sizeof(uint16_t));
                 p->w_norm = take(T * sizeof(float));
+                p->w_minima = take((size_t)p->dist_elems / 8 * sizeof(float) + 256);
             } else {
                 p->w_y = take(T * (size_t)p->D * sizeof(float));
             }
@@ -602,10 +603,8 @@ int build_plan(hdb_plan* p) {
         p->w_table = take((size_t)p->table_offsets[p->B] * sizeof(unsigned long long));
         p->w_level_comp = take(T * L * sizeof(uint16_t));
         p->w_level_max_v = take(T * L * sizeof(float));
-        p->w_level_end_v = take(T * L * sizeof(uint16_t));
+        p->w_level_span = take(T * L * sizeof(uint32_t));
         p->w_perm = take(T * sizeof(uint16_t));
-        p->w_level_max = take(T * L * sizeof(float));
-        p->w_level_end = take(T * L * sizeof(uint16_t));
         p->w_levels = take((size_t)p->B * sizeof(int32_t));
         p->w_pos = take(T * sizeof(uint16_t));
         p->w_light_uv = take(T * (size_t)p->light_cap * sizeof(uint32_t));
@@ -799,10 +798,9 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.table_offsets = reinterpret_cast<const int64_t*>(ws + p->t_table);
         a.level_comp = reinterpret_cast<uint16_t*>(ws + p->w_level_comp);
         a.level_max_v = reinterpret_cast<float*>(ws + p->w_level_max_v);
-        a.level_end_v = reinterpret_cast<uint16_t*>(ws + p->w_level_end_v);
+        a.level_span = reinterpret_cast<uint32_t*>(ws + p->w_level_span);
         a.perm = reinterpret_cast<uint16_t*>(ws + p->w_perm);
-        a.level_max = reinterpret_cast<float*>(ws + p->w_level_max);
-        a.level_end = reinterpret_cast<uint16_t*>(ws + p->w_level_end);
+        a.minima = reinterpret_cast<float*>(ws + p->w_minima);
         a.levels = reinterpret_cast<int32_t*>(ws + p->w_levels);
         a.pos = reinterpret_cast<uint16_t*>(ws + p->w_pos);
         a.light_count = reinterpret_cast<int32_t*>(ws + p->t_light_count);

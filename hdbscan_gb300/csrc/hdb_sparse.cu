@@ -11,14 +11,13 @@ namespace {
 // Threads of the one-CTA-a-window kernels.
 int window_threads(int nmax) { return nmax <= 128 ? 64 : (nmax <= 512 ? 128 : (nmax <= 1024 ? 256 : 512)); }
 
-size_t light_smem(int nmax) { return (size_t)((nmax + 3) & ~3) * sizeof(float); }
-
 unsigned blocks(int n, int per) { return (unsigned)((n + per - 1) / per); }
 
 template <typename Real>
 cudaError_t launch_rows(const SparseArgs& a, cudaStream_t s, int priority) {
     const unsigned grid = (unsigned)a.n_windows * blocks(a.nmax, kSparseRowsCta);
     const unsigned threads = 32 * kCoreRowsWarps;
+    if (a.gram && a.list <= 32) return launch_ex(hdb_sparse_gram_rows_kernel<Real>, grid, threads, 0, s, priority, 1, a);
     switch (a.list) {
         case 8: return launch_ex(hdb_sparse_rows_kernel<Real, 8>, grid, threads, 0, s, priority, 1, a);
         case 16: return launch_ex(hdb_sparse_rows_kernel<Real, 16>, grid, threads, 0, s, priority, 1, a);
@@ -49,8 +48,7 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
             return launch_ex(hdb_sparse_tree_kernel<Real>, W, (unsigned)window_threads(a.nmax), sparse_tree_smem(a.nmax),
                              s, priority, 1, a);
         case SparseStage::kLight:
-            return launch_ex(hdb_sparse_light_kernel<Real>, W * blocks(a.nmax, kLightRows), 256, light_smem(a.nmax), s,
-                             priority, 1, a);
+            return launch_ex(hdb_sparse_light_kernel<Real>, W * blocks(a.nmax, kLightRows), 256, 0, s, priority, 1, a);
         case SparseStage::kStar:
             return launch_ex(hdb_sparse_star_kernel<Real>, W * blocks(a.nmax, kSparseRowsCta), 256, 0, s, priority, 1, a);
         case SparseStage::kPrim:
@@ -78,14 +76,14 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
 
 template <typename Real>
 cudaError_t prepare(int n, size_t budget, bool* fits) {
-    const size_t need[6] = {2 * kGramStage, sparse_forest_smem(n), sparse_between_smem(n), sparse_tree_smem(n), light_smem(n),
+    const size_t need[5] = {2 * kGramStage, sparse_forest_smem(n), sparse_between_smem(n), sparse_tree_smem(n),
                             SparsePrimLayout<Real>::bytes(n)};
-    const void* func[6] = {(const void*)hdb_sparse_gram_kernel<Real>,
+    const void* func[5] = {(const void*)hdb_sparse_gram_kernel<Real>,
                            (const void*)hdb_sparse_forest_kernel<Real>, (const void*)hdb_sparse_between_kernel<Real>,
-                           (const void*)hdb_sparse_tree_kernel<Real>, (const void*)hdb_sparse_light_kernel<Real>,
+                           (const void*)hdb_sparse_tree_kernel<Real>,
                            (const void*)hdb_sparse_prim_kernel<Real>};
     *fits = true;
-    for (int i = 0; i < 6; ++i) {
+    for (int i = 0; i < 5; ++i) {
         cudaFuncAttributes attr;
         cudaError_t e = cudaFuncGetAttributes(&attr, func[i]);
         if (e != cudaSuccess) return e;

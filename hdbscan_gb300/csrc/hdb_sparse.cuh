@@ -351,24 +351,76 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArg
     }
     const float eta = sparse_eta(a.D);
     float* __restrict__ Dw = sparse_block<Real>(a, w);
+    float* __restrict__ minima = a.minima + a.dist_offsets[w] / 8;
+    const int groups = (n + 15) >> 4;
     const int64_t ld = dist_ld(n);
     const bool diagonal = ti == tj;
+    const float inf = __int_as_float(0x7f800000);
+    // Accumulators become bounds in place; entries outside the window are infinite.
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = wm + 16 * p + 8 * h + (lane >> 2), gi = i0 + r;
+            const float ni = s_norm[0][r];
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int col = wn + 8 * q + 2 * (lane & 3) + b, gj = j0 + col;
+                    const float sum = ni + s_norm[1][col];
+                    float v = fmaxf(__fmaf_rn(-eta, sum, __fmaf_rn(-2.0f, acc[p][q][2 * h + b], sum)), 0.0f);
+                    if (diagonal && gi == gj) v = 0.0f;
+                    acc[p][q][2 * h + b] = gi < n && gj < n ? v : inf;
+                }
+        }
+    // Minima of 16 columns of each row: four values here, four lanes of the quad.
+    // (In a diagonal tile both halves are in the accumulators; their minima may
+    // differ from the stored upper half's by the products' asymmetry, so they are
+    // taken from the stored values below.)
+    if (!diagonal) {
+#pragma unroll
+        for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int gi = i0 + wm + 16 * p + 8 * h + (lane >> 2);
+#pragma unroll
+                for (int q = 0; q < 8; q += 2) {
+                    float v = fminf(fminf(acc[p][q][2 * h], acc[p][q][2 * h + 1]),
+                                    fminf(acc[p][q + 1][2 * h], acc[p][q + 1][2 * h + 1]));
+                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 1));
+                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 2));
+                    const int g = (j0 + wn + 8 * q) >> 4;
+                    if ((lane & 3) == 0 && gi < n && g < groups) minima[(int64_t)gi * groups + g] = v;
+                }
+            }
+        // Of 16 rows of each column, for the mirrored half: two values here, eight lanes.
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+            const int g = (i0 + wm + 16 * p) >> 4;
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    float v = fminf(acc[p][q][b], acc[p][q][2 + b]);
+                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 4));
+                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 8));
+                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 16));
+                    const int gj = j0 + wn + 8 * q + 2 * (lane & 3) + b;
+                    if (lane < 4 && gj < n && g < groups) minima[(int64_t)gj * groups + g] = v;
+                }
+        }
+    }
 #pragma unroll
     for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = wm + 16 * p + 8 * h + (lane >> 2), gi = i0 + r;
             if (gi >= n) continue;
-            const float ni = s_norm[0][r];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 const int col = wn + 8 * q + 2 * (lane & 3), gj = j0 + col;
-                float v[2];
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const float sum = ni + s_norm[1][col + b];
-                    v[b] = fmaxf(__fmaf_rn(-eta, sum, __fmaf_rn(-2.0f, acc[p][q][2 * h + b], sum)), 0.0f);
-                }
+                const float v[2] = {acc[p][q][2 * h], acc[p][q][2 * h + 1]};
                 if (!diagonal) {
                     // (gj < n and even imply that column gj + 1 lies inside the row's stride.)
                     if (gj < n) *reinterpret_cast<float2*>(Dw + gi * ld + gj) = make_float2(v[0], v[1]);
@@ -379,13 +431,23 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArg
 #pragma unroll
                     for (int b = 0; b < 2; ++b) {
                         if (gj + b >= n || gi > gj + b) continue;
-                        const float x = gi == gj + b ? 0.0f : v[b];
-                        Dw[gi * ld + gj + b] = x;
-                        Dw[(int64_t)(gj + b) * ld + gi] = x;
+                        Dw[gi * ld + gj + b] = v[b];
+                        Dw[(int64_t)(gj + b) * ld + gi] = v[b];
                     }
                 }
             }
         }
+    if (diagonal) {
+        __syncthreads();  // the CTA's own stores
+        const int first = i0 >> 4, count = min(TS / 16, groups - first);
+        for (int e = tid; e < TS * count; e += 256) {
+            const int r = e / count, g = first + e - r * count, gi = i0 + r;
+            if (gi >= n) continue;
+            float v = inf;
+            for (int c = 16 * g; c < min(16 * g + 16, n); ++c) v = fminf(v, Dw[gi * ld + c]);
+            minima[(int64_t)gi * groups + g] = v;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -516,6 +578,75 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_tiles_kernel(const SparseAr
 // for hdb_sparse_core_kernel.  A list that ends inside that range, or a
 // distance that is not finite, flags the window.
 // ---------------------------------------------------------------------------
+// The end of a row: its list, and its core distance or the list positions where
+// that is to be looked for.
+template <typename Real, int E>
+__device__ __forceinline__ void finish_row(const SparseArgs& a, const SparseBound& bound, int w, int64_t base, int n, int i,
+                                           const uint32_t (&lk)[E], const int (&li)[E], bool wild) {
+    const int lane = threadIdx.x & 31;
+    const int keep = a.keep, last = keep - 1;
+    auto at = [&](int p) {
+        const uint32_t lo = __shfl_sync(0xffffffffu, lk[0], p & 31);
+        if constexpr (E > 1) {
+            const uint32_t hi = __shfl_sync(0xffffffffu, lk[1], p & 31);
+            return p < 32 ? lo : hi;
+        }
+        return lo;
+    };
+    const int64_t row_at = base + i;
+#pragma unroll
+    for (int h = 0; h < E; ++h) {
+        const int p = lane + 32 * h;
+        if (p < keep) {
+            a.knn_idx[row_at * a.list + p] = (uint16_t)(p < n ? li[h] : i);
+            a.knn_d[row_at * a.list + p] = __uint_as_float(p < n ? lk[h] : 0x7f800000u);
+        }
+    }
+    bool unsure = wild;
+    if (!a.unit_core) {
+        const int pos = a.ms - 1;
+        if (!a.approx) {
+#pragma unroll
+            for (int h = 0; h < E; ++h)
+                if (pos == lane + 32 * h) {
+                    static_cast<float*>(a.core)[row_at] = __uint_as_float(lk[h]);
+                    a.core_nbr[row_at] = li[h];
+                }
+            // Points as far as the core distance may follow the list's end.
+            if (at(last) <= at(pos) && keep < n) unsure = true;
+        } else {
+            // The value of rank ms - 1 is at least the lower bound at that
+            // position and at most the largest upper bound up to it.
+            const float least = bound.down(__uint_as_float(at(pos)));
+            const int inside = min(keep, n);
+            float up[E], most = 0.0f;
+            const float slack = 2.1f * sparse_eta(a.D);
+            const float norm_i = a.gram ? a.norm[row_at] : 0.0f;
+#pragma unroll
+            for (int h = 0; h < E; ++h) {
+                const int p = lane + 32 * h;
+                const float d = __uint_as_float(lk[h]);
+                up[h] = bound.up(d);
+                if (a.gram && p < inside) up[h] = __fmaf_ru(slack, norm_i + a.norm[base + li[h]], d);
+                if (p <= pos) most = fmaxf(most, up[h]);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+            int c = inside, e = 0;
+#pragma unroll
+            for (int h = E - 1; h >= 0; --h) {
+                const int p = lane + 32 * h;
+                const unsigned open = __ballot_sync(0xffffffffu, p < inside && !(up[h] < least));
+                if (open) c = 32 * h + __ffs(open) - 1;
+                e += __popc(__ballot_sync(0xffffffffu, p < inside && bound.down(__uint_as_float(lk[h])) <= most));
+            }
+            if (e >= keep && keep < n) unsure = true;  // the range may go on beyond the list
+            if (lane == 0) a.core_nbr[row_at] = c | (e << 8);
+        }
+    }
+    if (unsure && lane == 0) sparse_flag(a, w);
+}
+
 template <typename Real, int K>
 __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(const SparseArgs a) {
     static_assert(K <= 64, "at most two list entries per lane");
@@ -609,58 +740,146 @@ __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_rows_kernel(co
             }
         }
         const bool wild = __any_sync(0xffffffffu, biggest >= 0x7f800000u);
-        const int64_t row_at = base + i;
+        finish_row<Real, E>(a, bound, w, base, n, i, lk, li, wild);
+    }
+}
+
+// One compare-exchange stage of (key, index) over the lanes, distance j.
+__device__ __forceinline__ void pair_stage(uint32_t& k, int& i, int j, bool keep_min) {
+    const uint32_t pk = __shfl_xor_sync(0xffffffffu, k, j);
+    const int pi = __shfl_xor_sync(0xffffffffu, i, j);
+    const bool partner_less = pk < k || (pk == k && pi < i);
+    const bool take = keep_min ? partner_less : !partner_less;
+    k = take ? pk : k;
+    i = take ? pi : i;
+}
+
+// The keep-th smallest (keep <= 32) of the 64 values x0, x1 of the lanes.
+__device__ __forceinline__ uint32_t smallest_of_64(uint32_t x0, uint32_t x1, int keep) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int h = 0; h < E; ++h) {
-            const int p = lane + 32 * h;
-            if (p < keep) {
-                a.knn_idx[row_at * a.list + p] = (uint16_t)(p < n ? li[h] : i);
-                a.knn_d[row_at * a.list + p] = __uint_as_float(p < n ? lk[h] : 0x7f800000u);
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const bool keep_min = ((lane & k) == 0) == ((lane & j) == 0);
+            const uint32_t p0 = __shfl_xor_sync(0xffffffffu, x0, j), p1 = __shfl_xor_sync(0xffffffffu, x1, j);
+            x0 = keep_min ? min(x0, p0) : max(x0, p0);
+            // The second half descends: its first 32 meet the first half's last.
+            x1 = keep_min ? max(x1, p1) : min(x1, p1);
+        }
+    }
+    // x0 ascending, x1 descending: the lane-wise minima are the 32 smallest, a bitonic sequence.
+    x0 = min(x0, x1);
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) {
+        const uint32_t p0 = __shfl_xor_sync(0xffffffffu, x0, j);
+        x0 = (lane & j) == 0 ? min(x0, p0) : max(x0, p0);
+    }
+    return __shfl_sync(0xffffffffu, x0, keep - 1);
+}
+
+// Merges `count` (<= 32) gathered entries into the ascending list (k, i).
+__device__ __forceinline__ void merge_batch(uint32_t& k, int& i, const uint2* batch, int count) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    const uint2 e = lane < count ? batch[lane] : make_uint2(0xffffffffu, 0x7fffffffu);
+    uint32_t bk = e.x;
+    int bi = (int)e.y;
+#pragma unroll
+    for (int s = 2; s <= 32; s <<= 1)
+#pragma unroll
+        for (int j = s >> 1; j > 0; j >>= 1)  // descending
+            pair_stage(bk, bi, j, ((lane & s) == 0) != ((lane & j) == 0));
+    const bool less = bk < k || (bk == k && bi < i);
+    k = less ? bk : k;
+    i = less ? bi : i;
+#pragma unroll
+    for (int j = 16; j > 0; j >>= 1) pair_stage(k, i, j, (lane & j) == 0);
+    __syncwarp();
+}
+
+// Product blocks come with the minimum of every 16 entries of a row (written by
+// hdb_sparse_gram_kernel), so a row is read in two steps: its minima, whose
+// keep-th smallest (of 64 partial ones, two a lane) bounds the list's end, and
+// the groups that reach below it, little more than keep of them.  Entries below
+// the bound gather in shared memory and join the list 32 at a time (sort,
+// bitonic merge).
+constexpr int kGroup = 16;
+
+// The window's group minima, [n][ceil(n / 16)], after the distance blocks.
+template <typename Real>
+__device__ __forceinline__ float* sparse_minima(const SparseArgs& a, int w) {
+    return a.minima + a.dist_offsets[w] / 8;
+}
+
+template <typename Real>
+__global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_sparse_gram_rows_kernel(const SparseArgs a) {
+    constexpr uint32_t kNone = 0xffffffffu;
+    constexpr int kGroups = 4096 / kGroup;
+    __shared__ uint2 s_batch[kCoreRowsWarps][64];
+    __shared__ uint8_t s_group[kCoreRowsWarps][kGroups];
+    const int per = (a.nmax + kSparseRowsCta - 1) / kSparseRowsCta;
+    const int item = blockIdx.x / per, r0 = (blockIdx.x - item * per) * kSparseRowsCta;
+    const int w = a.queue[item];
+    const int64_t base = a.offsets[w];
+    const int n = (int)(a.offsets[w + 1] - base);
+    if (r0 >= n || a.flags[w]) return;
+    const float* __restrict__ Dw = sparse_block<Real>(a, w);
+    const float* __restrict__ minima = sparse_minima<Real>(a, w);
+    const int64_t ld = dist_ld(n);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int keep = a.keep, last = keep - 1, groups = (n + kGroup - 1) / kGroup;
+    const SparseBound bound = sparse_bound<Real>(a, w);
+    uint2* batch = s_batch[warp];
+    uint8_t* group = s_group[warp];
+    for (int r = warp; r < kSparseRowsCta; r += kCoreRowsWarps) {
+        const int i = r0 + r;
+        if (i >= n) break;  // warp-uniform
+        const float* __restrict__ row = Dw + (int64_t)i * ld;
+        const float* __restrict__ least = minima + (int64_t)i * groups;
+        uint32_t g[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) g[q] = lane + 32 * q < groups ? __float_as_uint(__ldcg(least + lane + 32 * q)) : kNone;
+        const uint32_t m0 = min(min(g[0], g[2]), min(g[4], g[6])), m1 = min(min(g[1], g[3]), min(g[5], g[7]));
+        uint32_t limit = smallest_of_64(m0, m1, keep);  // entries up to it pass
+        int found = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const unsigned bal = __ballot_sync(0xffffffffu, g[q] <= limit && g[q] != kNone);
+            if ((bal >> lane) & 1u) group[found + __popc(bal & lanemask_lt())] = (uint8_t)(lane + 32 * q);
+            found += __popc(bal);
+        }
+        __syncwarp();
+        uint32_t lk[1] = {kNone};
+        int li[1] = {0x7fffffff};
+        int waiting = 0;
+        for (int t = 0; t < found; t += 8) {
+            uint32_t v[4];
+            int col[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int e = t + 2 * q + (lane >> 4);
+                col[q] = e < found ? (int)group[e] * kGroup + (lane & (kGroup - 1)) : n;
+                v[q] = col[q] < n ? __float_as_uint(__ldcg(row + col[q])) : kNone;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool pass = v[q] <= limit && v[q] != kNone;
+                const unsigned bal = __ballot_sync(0xffffffffu, pass);
+                if (pass) batch[waiting + __popc(bal & lanemask_lt())] = make_uint2(v[q], (uint32_t)col[q]);
+                waiting += __popc(bal);
+                if (waiting >= 32) {
+                    merge_batch(lk[0], li[0], batch, 32);
+                    waiting -= 32;
+                    const uint2 rest = batch[32 + lane];
+                    __syncwarp();
+                    if (lane < waiting) batch[lane] = rest;
+                    limit = min(limit, __shfl_sync(0xffffffffu, lk[0], last));
+                }
             }
         }
-        bool unsure = wild;
-        if (!a.unit_core) {
-            const int pos = a.ms - 1;
-            if (!a.approx) {
-#pragma unroll
-                for (int h = 0; h < E; ++h)
-                    if (pos == lane + 32 * h) {
-                        static_cast<float*>(a.core)[row_at] = __uint_as_float(lk[h]);
-                        a.core_nbr[row_at] = li[h];
-                    }
-                // Points as far as the core distance may follow the list's end.
-                if (at(last) <= at(pos) && keep < n) unsure = true;
-            } else {
-                // The value of rank ms - 1 is at least the lower bound at that
-                // position and at most the largest upper bound up to it.
-                const float least = bound.down(__uint_as_float(at(pos)));
-                const int inside = min(keep, n);
-                float up[E], most = 0.0f;
-                const float slack = 2.1f * sparse_eta(a.D);
-                const float norm_i = a.gram ? a.norm[row_at] : 0.0f;
-#pragma unroll
-                for (int h = 0; h < E; ++h) {
-                    const int p = lane + 32 * h;
-                    const float d = __uint_as_float(lk[h]);
-                    up[h] = bound.up(d);
-                    if (a.gram && p < inside) up[h] = __fmaf_ru(slack, norm_i + a.norm[base + li[h]], d);
-                    if (p <= pos) most = fmaxf(most, up[h]);
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
-                int c = inside, e = 0;
-#pragma unroll
-                for (int h = E - 1; h >= 0; --h) {
-                    const int p = lane + 32 * h;
-                    const unsigned open = __ballot_sync(0xffffffffu, p < inside && !(up[h] < least));
-                    if (open) c = 32 * h + __ffs(open) - 1;
-                    e += __popc(__ballot_sync(0xffffffffu, p < inside && bound.down(__uint_as_float(lk[h])) <= most));
-                }
-                if (e >= keep && keep < n) unsure = true;  // the range may go on beyond the list
-                if (lane == 0) a.core_nbr[row_at] = c | (e << 8);
-            }
-        }
-        if (unsure && lane == 0) sparse_flag(a, w);
+        if (waiting > 0) merge_batch(lk[0], li[0], batch, waiting);
+        finish_row<Real, 1>(a, bound, w, base, n, i, lk, li, false);
     }
 }
 
@@ -769,7 +988,7 @@ __host__ __device__ inline size_t sparse_forest_smem(int n) {
     return (size_t)sparse_round(n) * (8 + 4 + 4 + 4 + 2 + 2 + 1) + 64;
 }
 __host__ __device__ inline size_t sparse_between_smem(int n) {
-    return (size_t)sparse_round(n) * (2 + 4) + (size_t)sparse_parts_cap(n) * 8 + 64;
+    return (size_t)sparse_round(n) * (2 + 4) + (size_t)sparse_parts_cap(n) * 8 * 8 + 64;
 }
 __host__ __device__ inline size_t sparse_tree_smem(int n) {
     return (size_t)sparse_round(n) * (8 + 8 + 4 + 2 + 2) + 64;
@@ -924,14 +1143,16 @@ __global__ void __launch_bounds__(512) hdb_sparse_forest_kernel(const SparseArgs
     if (tid == 0) a.parts[w] = parts;
 }
 
-// The least edge between each two components: every row against all columns of
-// higher-numbered components.  A CTA takes kBetweenRows rows in component order
-// and keeps the table row of the current component in shared memory.
-constexpr int kBetweenRows = 32;
+// The least edge between each two components, from the upper triangle of the
+// block: every row u against its columns v > u, into table row part[u].  A warp
+// takes a run of rows in component order and keeps the table row of the current
+// component in shared memory.
+constexpr int kBetweenRows = 32;  // rows per CTA: runs of four a warp
 
 template <typename Real>
 __global__ void __launch_bounds__(256) hdb_sparse_between_kernel(const SparseArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int kRun = kBetweenRows / 8;
     const int per = (a.nmax + kBetweenRows - 1) / kBetweenRows;
     const int item = blockIdx.x / per, p0 = (blockIdx.x - item * per) * kBetweenRows;
     const int w = a.queue[item];
@@ -940,54 +1161,54 @@ __global__ void __launch_bounds__(256) hdb_sparse_between_kernel(const SparseArg
     if (p0 >= n || a.flags[w]) return;
     const int parts = a.parts[w];
     if (parts <= 1) return;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int cap = sparse_round(n);
-    unsigned long long* least = reinterpret_cast<unsigned long long*>(smem);
-    float* core = reinterpret_cast<float*>(least + sparse_parts_cap(n));
+    float* core = reinterpret_cast<float*>(smem);
     uint16_t* part = reinterpret_cast<uint16_t*>(core + cap);
+    unsigned long long* least = reinterpret_cast<unsigned long long*>(part + cap) + (size_t)warp * parts;
     const uint32_t* least_w = reinterpret_cast<const uint32_t*>(least) + 1;  // high words: weights
-    const float* core_g = a.core_up;
     for (int u = tid; u < n; u += 256) {
-        core[u] = a.unit_core ? 0.0f : core_g[base + u];
+        core[u] = a.unit_core ? 0.0f : a.core_up[base + u];
         part[u] = a.part[base + u];
     }
+    __syncthreads();
     const float* __restrict__ Dw = sparse_block<Real>(a, w);
     const int64_t ld = dist_ld(n);
     const SparseBound bound = sparse_bound<Real>(a, w);
     unsigned long long* table = a.table + a.table_offsets[w];
-    const int pend = min(p0 + kBetweenRows, n);
     int mine = -1;
     auto flush = [&]() {
-        __syncthreads();
+        __syncwarp();
         if (mine >= 0)
-            for (int c = mine + 1 + tid; c < parts; c += 256)
+            for (int c = lane; c < parts; c += 32)
                 if (least[c] < table[(int64_t)mine * parts + c]) atomicMin(&table[(int64_t)mine * parts + c], least[c]);
+        __syncwarp();
     };
-    __syncthreads();
-    for (int p = p0; p < pend; ++p) {
+    for (int p = p0 + kRun * warp; p < min(p0 + kRun * (warp + 1), n); ++p) {
         const int u = a.perm[base + p];
         const int cu = part[u];
-        if (cu == parts - 1) continue;
         if (cu != mine) {
             flush();
             mine = cu;
-            __syncthreads();
-            for (int c = mine + 1 + tid; c < parts; c += 256) least[c] = table[(int64_t)mine * parts + c];
-            __syncthreads();
+            for (int c = lane; c < parts; c += 32) least[c] = table[(int64_t)mine * parts + c];
+            __syncwarp();
         }
         const float* __restrict__ row = Dw + (int64_t)u * ld;
         const float core_u = core[u];
         constexpr int U = 8;
-        for (int v0 = tid; v0 < n; v0 += 256 * U) {
+        for (int v0 = (u + 1) & ~31; v0 < n; v0 += 32 * U) {
             float d[U];
 #pragma unroll
-            for (int q = 0; q < U; ++q) d[q] = v0 + 256 * q < n ? __ldcg(row + v0 + 256 * q) : 0.0f;
+            for (int q = 0; q < U; ++q) {
+                const int v = v0 + 32 * q + lane;
+                d[q] = v < n ? __ldcg(row + v) : 0.0f;
+            }
 #pragma unroll
             for (int q = 0; q < U; ++q) {
-                const int v = v0 + 256 * q;
-                if (v >= n) break;
+                const int v = v0 + 32 * q + lane;
+                if (v >= n || v <= u) continue;
                 const int cv = part[v];
-                if (cv <= cu) continue;
+                if (cv == cu) continue;
                 const float wgt = fmaxf(fmaxf(core_u, core[v]), bound.up(d[q]));
                 if (__float_as_uint(wgt) > least_w[2 * cv]) continue;
                 atomicMin(&least[cv], sparse_key(wgt, u, v));
@@ -1031,10 +1252,10 @@ __global__ void __launch_bounds__(512) hdb_sparse_tree_kernel(const SparseArgs a
         __syncthreads();
         for (int i = tid; i < parts * parts; i += nt) {
             const int r = i / parts, c = i - r * parts;
-            if (c <= r) continue;
             const int cr = owner[r], cc = owner[c];
             if (cr == cc) continue;
             const unsigned long long key = table[i];
+            if (key == kNoChoice) continue;
             if (key < choice[cr]) atomicMin(&choice[cr], key);
             if (key < choice[cc]) atomicMin(&choice[cc], key);
         }
@@ -1118,80 +1339,79 @@ __global__ void __launch_bounds__(512) hdb_sparse_tree_kernel(const SparseArgs a
             for (int r = tid; r < n; r += nt)
                 if (child[r] == r) cursor[r] = place[r];
             for (int u = tid; u < n; u += nt)
-                a.level_end_v[(int64_t)(l - 2) * a.T + base + u] = (uint16_t)(place[child[u]] + size[child[u]]);
+                a.level_span[(int64_t)(l - 2) * a.T + base + u] = place[child[u]] | ((place[child[u]] + size[child[u]]) << 16);
             __syncthreads();
         }
     }
     for (int u = tid; u < n; u += nt) {
-        const uint32_t p = place[u];
-        a.perm[base + p] = (uint16_t)u;
-        a.pos[base + u] = (uint16_t)p;
-        for (int l = 0; l < level; ++l) {
-            a.level_max[(int64_t)l * a.T + base + p] = a.level_max_v[(int64_t)l * a.T + base + u];
-            a.level_end[(int64_t)l * a.T + base + p] =
-                l + 1 < level ? a.level_end_v[(int64_t)l * a.T + base + u] : (uint16_t)n;
-        }
+        a.pos[base + u] = (uint16_t)place[u];
+        a.level_span[(int64_t)(level - 1) * a.T + base + u] = (uint32_t)n << 16;
     }
     if (tid == 0) a.levels[w] = level;
 }
 
 // ---------------------------------------------------------------------------
-// Light edges: all pairs (p < q in leaf order) whose distance is at most the
-// path maximum max(top_l(p), top_l(q)), l the first round that joins them.  Core
-// distances need no test: both ends' maxima are at least their own cores.
-// Pairs whose weight is certainly a core distance are star edges and left to
-// hdb_sparse_star_kernel.  One CTA per kLightRows rows; a row is staged in
-// shared memory and read in leaf order.
+// Light edges: all pairs (u < v) whose distance is at most the path maximum
+// max(top_l(u), top_l(v)), l the first round that joins them.  Core distances
+// need no test: both ends' maxima are at least their own cores.  Pairs whose
+// weight is certainly a core distance are star edges and left to
+// hdb_sparse_star_kernel.  A warp streams the upper triangle's part of a row in
+// vertex order; pairs within the maxima at the root (mostly those inside one
+// cluster) gather in shared memory and are settled 32 at a time.  A warp takes
+// rows r and n - 1 - r, which together are one row long.  Bound by the block's read (2 n^2 bytes).
 // ---------------------------------------------------------------------------
 template <typename Real>
 __global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs a) {
-    extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ int s_end[kSparseLevels];
-    __shared__ float s_top[kSparseLevels];
-    float* row = reinterpret_cast<float*>(smem);
+    __shared__ uint32_t s_span[8][kSparseLevels];
+    __shared__ float s_top[8][kSparseLevels];
+    __shared__ uint2 s_pair[8][64];  // (distance, column) of pairs that may be light
     const int per = (a.nmax + kLightRows - 1) / kLightRows;
-    const int item = blockIdx.x / per, p0 = (blockIdx.x - item * per) * kLightRows;
+    const int item = blockIdx.x / per, j = blockIdx.x - item * per;
     const int w = a.queue[item];
     const int64_t base = a.offsets[w];
     const int n = (int)(a.offsets[w + 1] - base);
-    if (p0 >= n || a.flags[w]) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int r = j * (kLightRows / 2) + warp;
+    if (2 * r > n - 1 || a.flags[w]) return;  // warp-uniform
     const int levels = a.levels[w];
     const float* __restrict__ Dw = sparse_block<Real>(a, w);
     const int64_t ld = dist_ld(n);
     const SparseBound bound = sparse_bound<Real>(a, w);
-    const uint16_t* __restrict__ perm = a.perm + base;
-    const int tid = threadIdx.x, lane = tid & 31;
+    const uint16_t* __restrict__ pos = a.pos + base;
+    const float* __restrict__ top_root = a.level_max_v + (int64_t)(levels - 1) * a.T + base;
     const int limit = n * a.light_cap;
     uint32_t* light_uv = a.light_uv + base * a.light_cap;
     Real* light_w = static_cast<Real*>(a.light_w) + base * a.light_cap;
-    const int pend = min(p0 + kLightRows, n - 1);
-    for (int p = p0; p < pend; ++p) {
-        const int u = perm[p];
-        const float* __restrict__ src = Dw + (int64_t)u * ld;
-        __syncthreads();
-        for (int j = 4 * tid; j < n; j += 4 * 256)
-            *reinterpret_cast<float4*>(row + j) = __ldcg(reinterpret_cast<const float4*>(src + j));
-        if (tid < levels) {
-            s_end[tid] = a.level_end[(int64_t)tid * a.T + base + p];
-            s_top[tid] = a.level_max[(int64_t)tid * a.T + base + p];
+    uint32_t* span = s_span[warp];
+    float* top = s_top[warp];
+    uint2* pair = s_pair[warp];
+    for (int side = 0; side < 2; ++side) {
+        const int u = side == 0 ? r : n - 1 - r;
+        if (side == 1 && u == r) break;
+        __syncwarp();
+        if (lane < levels) {
+            span[lane] = a.level_span[(int64_t)lane * a.T + base + u];
+            top[lane] = a.level_max_v[(int64_t)lane * a.T + base + u];
         }
-        __syncthreads();
+        __syncwarp();
         const float core_u = a.unit_core ? -1.0f : a.core_down[base + u];
-        int l = 0;
-        for (int q0 = p + 1; q0 < n; q0 += 256) {
-            const int q = q0 + tid;
-            bool light = false;
-            int v = 0;
-            float d = 0.0f;
-            if (q < n) {
-                while (l + 1 < levels && q >= s_end[l]) ++l;
-                v = perm[q];
-                d = row[v];
-                light = bound.down(d) <= fmaxf(s_top[l], a.level_max[(int64_t)l * a.T + base + q]);
+        const float top_u = top[levels - 1];
+        const float* __restrict__ row = Dw + (int64_t)u * ld;
+        int waiting = 0;
+        auto settle = [&](int count) {  // the first `count` waiting pairs, one a lane
+            bool light = lane < count;
+            const uint2 e = pair[lane];
+            const float d = __uint_as_float(e.x);
+            const int v = (int)e.y;
+            if (light) {
+                const uint32_t p = pos[v];
+                int l = levels - 1;
+                while (l > 0 && p >= (span[l - 1] & 0xffffu) && p < (span[l - 1] >> 16)) --l;
+                light = bound.down(d) <= fmaxf(top[l], a.level_max_v[(int64_t)l * a.T + base + v]);
                 if (light && !a.unit_core) light = !(bound.up(d) <= fmaxf(core_u, a.core_down[base + v]));
             }
             const unsigned bal = __ballot_sync(0xffffffffu, light);
-            if (!bal) continue;
+            if (!bal) return;
             int at = 0;
             if (lane == 0) at = atomicAdd(a.light_count + w, __popc(bal));
             at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & lanemask_lt());
@@ -1203,7 +1423,36 @@ __global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs 
                     if (!a.approx) light_w[at] = (Real)d;  // above both cores
                 }
             }
+        };
+        constexpr int U = 8;
+        for (int v0 = (u + 1) & ~31; v0 < n; v0 += 32 * U) {
+            float d[U], t[U];
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const int v = v0 + 32 * q + lane;
+                const bool in = v > u && v < n;
+                d[q] = in ? __ldcs(row + v) : __int_as_float(0x7f800000);
+                t[q] = in ? top_root[v] : 0.0f;
+            }
+#pragma unroll
+            for (int q = 0; q < U; ++q) {
+                const bool may = bound.down(d[q]) <= fmaxf(top_u, t[q]);
+                const unsigned bal = __ballot_sync(0xffffffffu, may);
+                if (!bal) continue;
+                if (may) pair[waiting + __popc(bal & lanemask_lt())] = make_uint2(__float_as_uint(d[q]), v0 + 32 * q + lane);
+                waiting += __popc(bal);
+                __syncwarp();
+                if (waiting >= 32) {
+                    settle(32);
+                    waiting -= 32;
+                    const uint2 rest = pair[32 + lane];
+                    __syncwarp();
+                    if (lane < waiting) pair[lane] = rest;
+                    __syncwarp();
+                }
+            }
         }
+        settle(waiting);
     }
 }
 
@@ -1265,10 +1514,11 @@ __global__ void __launch_bounds__(256) hdb_sparse_star_kernel(const SparseArgs a
             const bool valid = key != 0xffffffffu;
             bool joined = false;  // to the entry before, below core_x
             if (valid && lane > 0) {
-                const int p = (int)(before >> 12), q = (int)(key >> 12);
-                int l = 0;
-                while (l + 1 < levels && q >= a.level_end[(int64_t)l * a.T + base + p]) ++l;
-                joined = fmaxf(a.level_max[(int64_t)l * a.T + base + p], a.level_max[(int64_t)l * a.T + base + q]) < down_x;
+                const int64_t p = base + (before & 0xfffu), q = base + (key & 0xfffu);
+                const uint32_t place = key >> 12;
+                int l = 0;  // first round that joins them (the entry before lies to the left)
+                while (l + 1 < levels && place >= (a.level_span[(int64_t)l * a.T + p] >> 16)) ++l;
+                joined = fmaxf(a.level_max_v[(int64_t)l * a.T + p], a.level_max_v[(int64_t)l * a.T + q]) < down_x;
             }
             // Lowest vertex of each run of joined entries.
             uint32_t low = key & 0xfffu;
