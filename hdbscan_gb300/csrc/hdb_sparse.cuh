@@ -1715,7 +1715,6 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
     using T = RealTraits<Real>;
     using Key = typename T::Bits;
     constexpr bool kWide = sizeof(Real) == 8;
-    constexpr Key kNoKey = (Key)~(Key)0;
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint32_t s_scan[33];
     __shared__ int s_ctr[4];
@@ -1804,13 +1803,11 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
         if (tid == 0) sparse_flag(a, w);
         return;
     }
-    Key* sorted = reinterpret_cast<Key*>(ar.r1);  // over r1 and r2 while sorting
-    int P = 1;
-    while (P < n - 1) P <<= 1;
+    Key* sorted = reinterpret_cast<Key*>(ar.r1);
     __syncthreads();
-    for (int i = tid; i < P; i += nt) sorted[i] = i < n - 1 ? T::key(ar.r0[i]) : kNoKey;
+    for (int i = tid; i < n - 1; i += nt) sorted[i] = T::key(ar.r0[i]);
     __syncthreads();
-    bitonic_cta<Key>(sorted, P);
+    bitonic_cta<Key>(sorted, n - 1);
     bool twin = false;
     for (int i = tid; i + 1 < n - 1; i += nt) twin |= key_eq(sorted[i], sorted[i + 1]);
     const bool distinct = !__syncthreads_or(twin);
@@ -1941,7 +1938,7 @@ __global__ void __launch_bounds__(512) hdb_sparse_prim_kernel(const SparseArgs a
         return;
     }
     if (f.stage_ns && tid == 0) f.stage_ns[8 * w + 2] = global_ns();
-    tree_window_cta<Real>(f, smem, w, n, distinct, s_scan, s_ctr, kBarHelp);
+    tree_window_cta<Real>(f, smem, w, n, distinct ? EdgeOrder::kSorted : EdgeOrder::kRanks, s_scan, s_ctr, kBarHelp);
 }
 
 }  // namespace hdb

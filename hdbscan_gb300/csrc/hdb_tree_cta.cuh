@@ -25,15 +25,21 @@ namespace hdb {
 
 constexpr int kTieRunMax = 128;  // larger groups of equal weights go to the one-warp union-find
 
-// Ascending bitonic sort of k[0..P) (P a power of two) by the CTA.
+// Ascending bitonic sort of k[0..n) by the CTA.  Every comparator puts the
+// smaller word at the lower index (each merge starts by mirroring its second
+// half), so entries past n count as largest and stay where they are.
 template <typename Key>
-__device__ __forceinline__ void bitonic_cta(Key* k, int P) {
+__device__ __forceinline__ void bitonic_cta(Key* k, int n) {
+    int P = 1;
+    while (P < n) P <<= 1;
     for (int size = 2; size <= P; size <<= 1) {
         for (int j = size >> 1; j > 0; j >>= 1) {
+            const bool mirror = j == size >> 1;
             for (int i = threadIdx.x; i < P / 2; i += blockDim.x) {
-                const int lo = 2 * i - (i & (j - 1)), hi = lo + j;
+                const int lo = 2 * i - (i & (j - 1)), hi = mirror ? lo ^ (size - 1) : lo + j;
+                if (hi >= n) continue;
                 const Key x = k[lo], y = k[hi];
-                if (key_lt(y, x) == ((lo & size) == 0)) { k[lo] = y; k[hi] = x; }
+                if (key_lt(y, x)) { k[lo] = y; k[hi] = x; }
             }
             __syncthreads();
         }
@@ -367,11 +373,7 @@ __device__ int condense_cta(const Arena<Real>& a, int n, int mcs, int32_t* cl_si
     __syncthreads();
     const int splits = (int)s_scan[32];
     const int clusters = 1 + 2 * splits;
-    int P = 1;
-    while (P < splits) P <<= 1;
-    for (int i = splits + tid; i < P; i += nt) keys[i] = 0xffffffffu;
-    __syncthreads();
-    bitonic_cta<uint32_t>(keys, P);
+    bitonic_cta<uint32_t>(keys, splits);
     auto rank_of = [&](int t) {
         const uint32_t key = ((uint32_t)dep[t] << 12) | off[t];
         int lo = 0, hi = splits;
@@ -518,12 +520,46 @@ __device__ int condense_cta(const Arena<Real>& a, int n, int mcs, int32_t* cl_si
     return n + clusters;
 }
 
-// The hierarchy of one window by the whole CTA (all threads call).  r1 holds the
-// sorted keys; s2 the sorted order when no two weights are equal (distinct),
-// else the rank of each edge in Prim order (first sorted position of its weight).
+// What tree_window_cta finds in the arena beside the Prim edges (r0, s0, s1).
+enum class EdgeOrder {
+    kNone,    // nothing
+    kRanks,   // r1: sorted keys, s2: rank of each edge (first sorted position of its weight)
+    kSorted,  // r1: sorted keys, s2: sorted order; no two weights are equal
+};
+
+// Sorted order of r0[0..m) into s2, sorted weights into r0.  With float32 and few
+// ties (min_samples <= 2) a bitonic sort of (key, index) words serves first; it
+// stands when no two weights are equal.  True in that case.
+template <typename Real>
+__device__ __forceinline__ bool order_edges_cta(const Arena<Real>& a, int m, bool try_distinct, int bar, int* s_ctr) {
+    using T = RealTraits<Real>;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    if constexpr (sizeof(Real) == 4) {
+        if (try_distinct) {
+            unsigned long long* word = reinterpret_cast<unsigned long long*>(a.r1);  // over r1 and r2
+            for (int i = tid; i < m; i += nt) word[i] = ((unsigned long long)T::key(a.r0[i]) << 32) | (uint32_t)i;
+            __syncthreads();
+            bitonic_cta(word, m);
+            bool twin = false;
+            for (int i = tid; i + 1 < m; i += nt) twin |= (uint32_t)(word[i] >> 32) == (uint32_t)(word[i + 1] >> 32);
+            if (!__syncthreads_or(twin)) {
+                for (int i = tid; i < m; i += nt) {
+                    a.s2[i] = (int16_t)(uint32_t)word[i];
+                    a.r0[i] = T::from_key((uint32_t)(word[i] >> 32));
+                }
+                __syncthreads();
+                return true;
+            }
+        }
+    }
+    sort_edges_cta<Real>(a, m, nt, bar, s_ctr);
+    return false;
+}
+
+// The hierarchy of one window by the whole CTA (all threads call).
 // s_scan: 33 words, s_ctr: 4 words of shared memory.
 template <typename Real>
-__device__ __noinline__ void tree_window_cta(const ForwardArgs& args, unsigned char* base_ptr, int w, int n, bool distinct,
+__device__ __noinline__ void tree_window_cta(const ForwardArgs& args, unsigned char* base_ptr, int w, int n, EdgeOrder known,
                                              uint32_t* s_scan, int* s_ctr, int bar) {
     using T = RealTraits<Real>;
     const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -545,19 +581,22 @@ __device__ __noinline__ void tree_window_cta(const ForwardArgs& args, unsigned c
             args.edges_uv[2 * (ebase + i) + 1] = a.s1[i];
             static_cast<Real*>(args.edge_w)[ebase + i] = a.r0[i];
         }
-        __syncthreads();
     }
-    if (distinct) {
-        __syncthreads();
-    } else {
-        RankPair* p = reinterpret_cast<RankPair*>(a.r2);
-        for (int i = tid; i < m; i += nt) p[i].v = ((uint32_t)(uint16_t)a.s2[i] << 16) | (uint32_t)i;
-        sort_pairs_cta(p, a, m, nt, bar, s_ctr);
-        for (int i = tid; i < m; i += nt) a.s2[i] = (int16_t)(p[i].v & 0xffffu);
-    }
-    const typename T::Bits* sorted = reinterpret_cast<const typename T::Bits*>(a.r1);
-    for (int t = tid; t < m; t += nt) a.r0[t] = T::from_key(sorted[t]);
+    bool distinct = known == EdgeOrder::kSorted;
     __syncthreads();
+    if (known == EdgeOrder::kNone) {
+        distinct = order_edges_cta<Real>(a, m, args.unit_core != 0, bar, s_ctr);
+    } else {
+        if (known == EdgeOrder::kRanks) {
+            RankPair* p = reinterpret_cast<RankPair*>(a.r2);
+            for (int i = tid; i < m; i += nt) p[i].v = ((uint32_t)(uint16_t)a.s2[i] << 16) | (uint32_t)i;
+            sort_pairs_cta(p, a, m, nt, bar, s_ctr);
+            for (int i = tid; i < m; i += nt) a.s2[i] = (int16_t)(p[i].v & 0xffffu);
+        }
+        const typename T::Bits* sorted = reinterpret_cast<const typename T::Bits*>(a.r1);
+        for (int t = tid; t < m; t += nt) a.r0[t] = T::from_key(sorted[t]);
+        __syncthreads();
+    }
     stamp(4);
     if (args.order)
         for (int i = tid; i < m; i += nt) args.order[ebase + i] = a.s2[i];
