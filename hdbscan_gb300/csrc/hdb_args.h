@@ -72,8 +72,10 @@ struct DistanceArgs {
     void* dist;                  // packed blocks
     const int64_t* dist_offsets; // [B]
     int32_t* status;
-    const int32_t* only;         // as ForwardArgs::only
+    const int32_t* only;         // as ForwardArgs::only, with its windows (no table then)
     int n_only;
+    const int32_t* queue;
+    int n_windows;
 };
 
 struct CoreArgs {
@@ -89,8 +91,10 @@ struct CoreArgs {
     void* core;                  // [T]
     int32_t* core_nbr;           // [T] or null
     int32_t* status;
-    const int32_t* only;         // as ForwardArgs::only
+    const int32_t* only;         // as ForwardArgs::only, with its windows (no table then)
     int n_only;
+    const int32_t* queue;
+    int n_windows;
 };
 
 // Sparse path (hdb_sparse.cuh): one launch group covers the `n_windows` windows
@@ -160,7 +164,7 @@ constexpr int kBackwardWarps = 8;  // backward kernel: warps (32 linkage rows ea
 struct BackwardArgs {
     const void* X;               // [T, D]
     const int64_t* offsets;      // [B+1]
-    const int32_t* edge_window;  // [T-B] window of each packed edge row
+    int windows;                 // B
     int n_edges;                 // T - B
     int D;
     int unit_core;

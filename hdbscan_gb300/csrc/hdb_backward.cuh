@@ -53,7 +53,11 @@ __global__ void __launch_bounds__(32 * kBackwardWarps) hdb_backward_kernel(const
         const Real g = static_cast<const Real*>(args.grad)[r];
         const Real wgt = static_cast<const Real*>(args.link_w)[r];
         if (g != Real(0) && wgt > Real(0)) {
-            const int w = args.edge_window[r];
+            int w = 0;  // the last window whose rows start at or before r (offsets[w] - w)
+            for (int hi = args.windows; hi - w > 1;) {
+                const int mid = (w + hi) >> 1;
+                if (args.offsets[mid] - mid <= r) w = mid; else hi = mid;
+            }
             const int64_t base = args.offsets[w];
             const int64_t ebase = base - w;
             const int e = args.order[r];

@@ -110,7 +110,7 @@ struct hdb_plan {
     std::vector<int64_t> dist_offsets;      // per window (elements), -1 if not materialized
     int64_t dist_elems = 0;
     // Table layout (byte offsets within the workspace).
-    size_t t_offsets = 0, t_dist_off = 0, t_queue = 0, t_tickets = 0, t_tiles = 0, t_edge_window = 0;
+    size_t t_offsets = 0, t_dist_off = 0, t_queue = 0, t_tickets = 0, t_tiles = 0;
     size_t tables_bytes = 0;
     size_t w_core = 0, w_core_nbr = 0, w_dist = 0, w_prep = 0, ws_bytes = 0;
     int input_type = 0;     // hdb::InputType of X
@@ -162,7 +162,7 @@ constexpr int kSparseMinN = 16;
 constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
-constexpr unsigned kGeneralGrid = 152 * 8;  // CTAs of a general-path launch that may find nothing to do
+constexpr int kGeneralGrid = 152 * 4;  // CTAs of a general-path launch that may find nothing to do
 
 // Windows of one bin share their launches; shared memory, threads and grids
 // are sized by the largest.
@@ -431,7 +431,7 @@ int build_plan(hdb_plan* p) {
         if (c.fv->dp != 0) continue;
         // Float32 classes of larger windows take the 128x128 tile kernel.
         c.tile = (p->precision == HDB_F32 && c.nmax >= kTile128MinN) ? 128 : 64;
-        const bool tiles = !(c.general && !p->approx);  // exact ones are the sparse path's own
+        const bool tiles = !c.general;  // found on the device for flagged windows
         for (int w : c.windows) {
             const int n = size_of(w);
             const int64_t ld = (n + 3) & ~3;
@@ -461,13 +461,15 @@ int build_plan(hdb_plan* p) {
             select.select_rows = hdb::select_rows(c.nmax, real_bytes(p->precision));
             for (int w : c.windows) {
                 const int n = size_of(w);
-                if (launch.cv) {
+                if (c.general) {
+                    // (Rows of flagged windows are found on the device.)
+                } else if (launch.cv) {
                     for (int r = 0; r < n; r += launch.cv->rows) { launch.items.push_back(w); launch.items.push_back(r); }
                 } else {
                     for (int r = 0; r < n; r += select.select_rows) { select.items.push_back(w); select.items.push_back(r); }
                 }
             }
-            if (!launch.items.empty()) c.cores.push_back(launch);
+            if (!launch.items.empty() || c.general) c.cores.push_back(launch);
             if (!select.items.empty()) {
                 select.select_smem = (size_t)select.select_rows * (size_t)c.nmax * (size_t)real_bytes(p->precision);
                 c.cores.push_back(select);
@@ -552,11 +554,6 @@ int build_plan(hdb_plan* p) {
     p->t_tiles = put(image, cursor, p->tiles);
     for (auto& cls : p->classes)
         for (auto& c : cls.cores) c.items_off = put(image, cursor, c.items);
-    std::vector<int32_t> edge_window;
-    edge_window.reserve((size_t)(p->T - p->B));
-    for (int w = 0; w < p->B; ++w)
-        for (int i = 0; i < size_of(w) - 1; ++i) edge_window.push_back(w);
-    p->t_edge_window = put(image, cursor, edge_window);
     p->tables_bytes = align_up(std::max<size_t>(cursor, 256), 256);
     image.resize(p->tables_bytes, 0);
     HDB_CUDA(cudaMallocHost((void**)&p->h_tables, p->tables_bytes));
@@ -858,11 +855,10 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             if (rc) return rc;
             joined = n_groups + i;
         }
-        const unsigned grid_limit = c.general ? kGeneralGrid : 0xffffffffu;
         // Where the sparse path's distances are exact, they and the core distances are there already.
         const bool have_rows = c.general && !p->approx;
         // 1. distance blocks of this class's matrix-variant windows (caller's stream)
-        if (c.n_tiles && !have_rows) {
+        if (c.n_tiles || (c.general && !have_rows)) {
             hdb::DistanceArgs a{};
             a.X = X;
             a.offsets = d_offsets;
@@ -876,7 +872,9 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             if (spans) HDB_CUDA(spans->begin(HDB_PHASE_DISTANCE, stream));
             a.only = c.general ? only : nullptr;
             a.n_only = p->B;
-            HDB_CUDA(k.launch_distance(a, (int)std::min<unsigned>((unsigned)a.n_tiles, grid_limit), stream, c.priority));
+            a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
+            a.n_windows = (int)c.windows.size();
+            HDB_CUDA(k.launch_distance(a, c.general ? kGeneralGrid : a.n_tiles, stream, c.priority));
             if (spans) HDB_CUDA(spans->end(stream));
         }
         // 2. core distances of its windows (caller's stream)
@@ -898,7 +896,9 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             if (spans) HDB_CUDA(spans->begin(HDB_PHASE_CORE, stream));
             a.only = c.general ? only : nullptr;
             a.n_only = p->B;
-            if (cl.cv) HDB_CUDA(cl.cv->launch(a, (int)std::min<unsigned>((unsigned)a.n_items, grid_limit), stream, c.priority));
+            a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
+            a.n_windows = (int)c.windows.size();
+            if (cl.cv) HDB_CUDA(cl.cv->launch(a, c.general ? kGeneralGrid : a.n_items, stream, c.priority));
             else HDB_CUDA(k.launch_select(a, a.n_items, cl.select_smem, stream, c.priority));
             if (spans) HDB_CUDA(spans->end(stream));
         }
@@ -1290,7 +1290,7 @@ int hdb_plan_backward(hdb_plan_t* p, const void* X, const hdb_exports_t* ex, con
     hdb::BackwardArgs a{};
     a.X = X;
     a.offsets = reinterpret_cast<const int64_t*>(ws + p->t_offsets);
-    a.edge_window = reinterpret_cast<const int32_t*>(ws + p->t_edge_window);
+    a.windows = p->B;
     a.n_edges = (int)(p->T - p->B);
     a.D = p->D;
     a.unit_core = unit ? 1 : 0;

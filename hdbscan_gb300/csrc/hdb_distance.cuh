@@ -59,13 +59,11 @@ template <> struct DistVec<double> {
 // float64: 64 registers, 4 CTAs per SM (the integer-pipe arithmetic is
 // latency-bound at 3 CTAs; 5 would spill).
 template <typename Real>
-__device__ __forceinline__ void distance_tile(const DistanceArgs& args, int tile) {
+__device__ __forceinline__ void distance_tile(const DistanceArgs& args, int w, int ti, int tj) {
     using T = RealTraits<Real>;
     constexpr int KC = DistVec<Real>::KC;
     __shared__ __align__(16) Real s_i[KC][kDistTile];
     __shared__ __align__(16) Real s_j[KC][kDistTile];
-    const int w = args.tiles[3 * tile], ti = args.tiles[3 * tile + 1], tj = args.tiles[3 * tile + 2];
-    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const int D = args.D;
@@ -210,12 +208,29 @@ __device__ __forceinline__ void distance_tile(const DistanceArgs& args, int tile
     if (__syncthreads_or(overflow) && tid == 0) atomic_status(args.status, kOverflow);
 }
 
-// One CTA a tile, or (behind the sparse path, where most launches find no
-// flagged window) a fixed grid over all tiles.
+// One CTA a tile of the table, or (behind the sparse path, where most launches
+// find no flagged window) a fixed grid over the tiles of the flagged windows.
+template <typename Tile>
+__device__ __forceinline__ void for_tiles(const DistanceArgs& args, int edge, Tile tile) {
+    if (!args.only) {
+        const int t = blockIdx.x;
+        if (t < args.n_tiles) tile(args.tiles[3 * t], args.tiles[3 * t + 1], args.tiles[3 * t + 2]);
+        return;
+    }
+    if (!args.only[args.n_only]) return;
+    for (int item = 0; item < args.n_windows; ++item) {
+        const int w = args.queue[item];
+        if (!args.only[w]) continue;
+        const int n = (int)(args.offsets[w + 1] - args.offsets[w]);
+        const int side = (n + edge - 1) / edge;
+        for (int t = blockIdx.x; t < side * side; t += gridDim.x)
+            if (t / side <= t % side) tile(w, t / side, t % side);
+    }
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_kernel(const DistanceArgs args) {
-    if (args.only && !args.only[args.n_only]) return;
-    for (int tile = blockIdx.x; tile < args.n_tiles; tile += gridDim.x) distance_tile<Real>(args, tile);
+    for_tiles(args, kDistTile, [&](int w, int ti, int tj) { distance_tile<Real>(args, w, ti, tj); });
 }
 
 // Float32 blocks of larger windows: 128x128 tiles, 256 threads, 8x8 pairs per
@@ -227,14 +242,12 @@ __global__ void __launch_bounds__(256, sizeof(Real) == 8 ? 4 : 1) hdb_distance_k
 // round-to-nearest adds, a correctly rounded sqrt.
 constexpr int kDistTile128 = 128;
 
-__device__ __forceinline__ void distance128_tile(const DistanceArgs& args, int tile) {
+__device__ __forceinline__ void distance128_tile(const DistanceArgs& args, int w, int ti, int tj) {
     using T = RealTraits<float>;
     constexpr int KC = 32;
     constexpr int TS = kDistTile128;
     __shared__ __align__(16) float s_i[KC][TS];
     __shared__ __align__(16) float s_j[KC][TS];
-    const int w = args.tiles[3 * tile], ti = args.tiles[3 * tile + 1], tj = args.tiles[3 * tile + 2];
-    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const int D = args.D;
@@ -335,12 +348,10 @@ __device__ __forceinline__ void distance128_tile(const DistanceArgs& args, int t
     if (__syncthreads_or(overflow) && tid == 0) atomic_status(args.status, kOverflow);
 }
 
-// One CTA a tile, or a fixed grid over all tiles behind the sparse path.
 template <typename Real>
 __global__ void __launch_bounds__(256, 2) hdb_distance128_kernel(const DistanceArgs args) {
     static_assert(sizeof(Real) == 4, "the 128x128 tile kernel is float32 only");
-    if (args.only && !args.only[args.n_only]) return;
-    for (int tile = blockIdx.x; tile < args.n_tiles; tile += gridDim.x) distance128_tile(args, tile);
+    for_tiles(args, kDistTile128, [&](int w, int ti, int tj) { distance128_tile(args, w, ti, tj); });
 }
 
 // ---------------------------------------------------------------------------
@@ -501,15 +512,13 @@ __device__ __forceinline__ Key key_select(bool c, Key a, Key b) {
 }
 
 template <typename Real, int K>
-__device__ __forceinline__ void core_rows_item(const CoreArgs& args, int item) {
+__device__ __forceinline__ void core_rows_item(const CoreArgs& args, int w, int r0) {
     static_assert(K <= 64, "at most two list entries per lane");
     using T = RealTraits<Real>;
     using Key = typename T::Bits;
     constexpr int E = (K + 31) / 32;     // list entries per lane
     constexpr Key kNone = (Key)~(Key)0;  // above every distance key (and +inf's)
     constexpr int U = 8;                 // row chunks per group of loads
-    const int w = args.items[2 * item], r0 = args.items[2 * item + 1];
-    if (args.only && !args.only[w]) return;
     const int64_t base = args.offsets[w];
     const int n = (int)(args.offsets[w + 1] - base);
     const Real* __restrict__ Dw = static_cast<const Real*>(args.dist) + args.dist_offsets[w];
@@ -592,11 +601,22 @@ __device__ __forceinline__ void core_rows_item(const CoreArgs& args, int item) {
     }
 }
 
-// One CTA an item, or a fixed grid over all items behind the sparse path.
+// One CTA an item of the table, or a fixed grid over the flagged windows' rows.
 template <typename Real, int K>
 __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_core_rows_kernel(const CoreArgs args) {
-    if (args.only && !args.only[args.n_only]) return;
-    for (int item = blockIdx.x; item < args.n_items; item += gridDim.x) core_rows_item<Real, K>(args, item);
+    if (!args.only) {
+        if ((int)blockIdx.x < args.n_items)
+            core_rows_item<Real, K>(args, args.items[2 * blockIdx.x], args.items[2 * blockIdx.x + 1]);
+        return;
+    }
+    if (!args.only[args.n_only]) return;
+    for (int item = 0; item < args.n_windows; ++item) {
+        const int w = args.queue[item];
+        if (!args.only[w]) continue;
+        const int n = (int)(args.offsets[w + 1] - args.offsets[w]);
+        for (int r0 = kCoreMatrixRows * blockIdx.x; r0 < n; r0 += kCoreMatrixRows * gridDim.x)
+            core_rows_item<Real, K>(args, w, r0);
+    }
 }
 
 // Any ms: a CTA of 8 warps takes args.rows (1 to 8) rows of a window, computes
