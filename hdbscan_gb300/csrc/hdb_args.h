@@ -62,6 +62,13 @@ struct ForwardArgs {
     int n_only;
 };
 
+// Small-window kernel (hdb_small.cuh): core distances, beside ForwardArgs.
+struct SmallArgs {
+    int ms;
+    void* core;          // [T] Real
+    int32_t* core_nbr;   // [T]
+};
+
 struct DistanceArgs {
     const void* X;
     const int64_t* offsets;

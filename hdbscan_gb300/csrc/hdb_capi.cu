@@ -26,6 +26,7 @@
 #include "../../include/hdbscan_gb300.h"
 #include "hdb_args.h"
 #include "hdb_registry.h"
+#include "hdb_small.h"
 #include "hdb_sparse.h"
 
 namespace {
@@ -54,8 +55,10 @@ struct CoreLaunch {
     int select_rows = 1;                    // rows per item
 };
 
-// Windows of the sparse path that are launched together (hdb_sparse.cuh).
+// Windows of the sparse path (hdb_sparse.cuh) or of the small-window kernel
+// (hdb_small.cuh) that are launched together.
 struct SparseGroup {
+    bool small = false;
     std::vector<int> windows;  // descending n
     int nmax = 0;
     size_t queue_off = 0;
@@ -97,7 +100,8 @@ struct hdb_plan {
     std::vector<int64_t> offsets;
     const hdb::PrecisionKernels* k = nullptr;
     std::vector<WindowClass> classes;
-    std::vector<SparseGroup> groups;        // windows on the sparse path
+    std::vector<SparseGroup> groups;        // windows on the sparse path, then small ones
+    size_t n_sparse = 0;                    // groups of the former
     int list = 0, keep = 0;                 // neighbour list stride and length
     bool gram = false, approx = false;      // bounded distances, from tensor-core products
     int light_cap = 0, star_cap = 0;        // light and star edges per point
@@ -157,8 +161,13 @@ constexpr size_t kChunks = 4;     // pipeline depth for large matrix-variant cla
 constexpr size_t kMinChunk = 8;   // windows per chunk at least
 constexpr int kTile128MinN = 384;  // float32 matrix classes from this size use 128x128 distance tiles
 
-// Windows of fewer points stay on the general path (their dense loop is short).
-constexpr int kSparseMinN = 16;
+// Windows of fewer points stay on the general path.  In float32 the dense loop has
+// its distances ready in a matrix, and the ten launches of the sparse passes pay from
+// about 400 points (device time in the sparse form and in the general one, 64..256 dims: one window of 256 points 219 and 175 us, of 400 289
+// and 270, of 512 315 and 320; 16 windows of 320 points 259 and 252, of 400 300 and
+// 315, of 512 383 and 421).  In float64 the general form recomputes every distance at
+// two operations a clock on an SM.
+constexpr int kSparseMinN[2] = {384, 16};
 constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
@@ -310,9 +319,13 @@ int build_plan(hdb_plan* p) {
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return size_of(a) > size_of(b); });
     std::vector<const hdb::ForwardVariant*> chosen(p->B, nullptr);
     int ctas = 0;  // CTAs the batch occupies at once: one per window, CS per clustered window
+    // Small windows: one kernel does them whole.
+    std::vector<char> small(p->B, 0);
+    const bool special = !(p->flags & kNoSparseFlags);
     for (int w : order) {
         chosen[w] = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix);
         if (!chosen[w]) return fail(HDB_E_INVALID, "no kernel variant for a window of " + std::to_string(size_of(w)) + " points");
+        small[w] = special && chosen[w]->cluster == 1 && hdb::small_window(p->precision, size_of(w), p->D, unit, p->B);
         ctas += chosen[w]->cluster;
     }
     // A cluster shortens one window's Prim but holds CS SMs; once the batch
@@ -320,7 +333,7 @@ int build_plan(hdb_plan* p) {
     // each, until the batch fits the SMs again.
     for (auto it = order.rbegin(); it != order.rend() && ctas > p->sms; ++it) {
         const int w = *it;
-        if (chosen[w]->cluster <= 1) continue;
+        if (small[w] || chosen[w]->cluster <= 1) continue;
         const hdb::ForwardVariant* single = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix, false);
         if (!single) continue;
         ctas -= chosen[w]->cluster - 1;
@@ -341,9 +354,9 @@ int build_plan(hdb_plan* p) {
     p->gram = hdb::sparse_gram(p->D) && (p->precision == HDB_F64 || coordinate_pairs >= kGramMinWork);
     p->approx = p->gram || p->precision == HDB_F64;
     p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
-    if (p->list && !(p->flags & kNoSparseFlags)) {
+    if (p->list && special) {
         for (int w : order)
-            sparse[w] = size_of(w) >= kSparseMinN && chosen[w]->cluster == 1 &&
+            sparse[w] = !small[w] && size_of(w) >= kSparseMinN[p->precision != 0] && chosen[w]->cluster == 1 &&
                         (p->precision == HDB_F64 || chosen[w]->dp == 0);
         for (int w : order)
             if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
@@ -356,6 +369,7 @@ int build_plan(hdb_plan* p) {
     }
     for (int w : order) {
         const int n = size_of(w);
+        if (small[w]) continue;
         if (sparse[w]) {
             // Descending sizes: a group ends where the next size bin begins.
             if (p->groups.empty() || sparse_bin(n) != sparse_bin(p->groups.back().nmax)) p->groups.emplace_back();
@@ -418,6 +432,20 @@ int build_plan(hdb_plan* p) {
             }
         }
         p->groups.swap(groups);
+        p->n_sparse = p->groups.size();
+        int bin = -1;
+        for (int w : order) {
+            if (!small[w]) continue;
+            const int b = size_of(w) <= 32 ? 0 : (size_of(w) <= 64 ? 1 : 2);
+            if (b != bin) {
+                p->groups.emplace_back();
+                p->groups.back().small = true;
+                p->groups.back().nmax = size_of(w);
+                HDB_CUDA(hdb::small_prepare(p->precision, size_of(w)));
+                bin = b;
+            }
+            p->groups.back().windows.push_back(w);
+        }
     }
     std::stable_sort(p->classes.begin(), p->classes.end(), [](const WindowClass& a, const WindowClass& b) {
         return a.general != b.general ? b.general : a.nmax > b.nmax;
@@ -535,11 +563,11 @@ int build_plan(hdb_plan* p) {
         queue.insert(queue.end(), g.windows.begin(), g.windows.end());
     }
     p->t_queue = put(image, cursor, queue);
-    if (!p->groups.empty()) {
+    if (p->n_sparse) {
         const std::vector<int32_t> zeros((size_t)p->B + 1, 0);
         p->table_offsets.assign(p->B + 1, 0);
-        for (auto& g : p->groups)
-            for (int w : g.windows) {
+        for (size_t i = 0; i < p->n_sparse; ++i)
+            for (int w : p->groups[i].windows) {
                 const int64_t c = hdb::sparse_parts_cap(size_of(w));
                 p->table_offsets[w] = p->table_offsets[p->B];
                 p->table_offsets[p->B] += c * c;
@@ -570,7 +598,7 @@ int build_plan(hdb_plan* p) {
     ws += (size_t)p->dist_elems * rb;
     p->w_prep = ws = align_up(ws, 256);
     if (p->prepared) ws += (size_t)p->T * (size_t)p->D * rb;
-    if (!p->groups.empty()) {
+    if (p->n_sparse) {
         // About one to three of each per point in ordinary data; more send a window to the general path.
         p->light_cap = 12;
         p->star_cap = unit ? 0 : 8;
@@ -617,7 +645,7 @@ int build_plan(hdb_plan* p) {
 
     // ---- streams for concurrent classes ------------------------------------
     const size_t forks = p->classes.size() + p->groups.size();
-    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && forks > (p->groups.empty() ? 1 : 2);
+    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && forks > (p->n_sparse ? 2 : 1);
     if (fork) {
         int least = 0, greatest = 0;  // numerically: greatest <= least
         HDB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
@@ -721,7 +749,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         return fail(HDB_E_INVALID, "cl_parent needs cl_birth, cl_stability, cl_selected, point_parent, n_clusters");
 
     const bool fork = !p->aux.empty() && !spans;
-    const int32_t* only = p->groups.empty() ? nullptr : reinterpret_cast<const int32_t*>(ws + p->t_flags);
+    const int32_t* only = !p->n_sparse ? nullptr : reinterpret_cast<const int32_t*>(ws + p->t_flags);
     auto forward_args = [&]() {
         hdb::ForwardArgs a{};
         a.X = X;
@@ -759,6 +787,22 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
     // rest of each group on its own ---------------------------------------------
     for (size_t i = 0; i < p->groups.size(); ++i) {
         const SparseGroup& g = p->groups[i];
+        if (g.small) {  // whole windows, on a stream of their own
+            cudaStream_t s = stream;
+            if (fork) {
+                s = p->aux[i];
+                HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
+                HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * i], 0));
+            }
+            hdb::ForwardArgs fa = forward_args();
+            fa.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + g.queue_off;
+            const hdb::SmallArgs sa{p->ms, core, core_nbr};
+            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_FORWARD, s));
+            HDB_CUDA(hdb::small_launch(p->precision, fa, sa, (int)g.windows.size(), g.nmax, s, g.priority));
+            if (spans) HDB_CUDA(spans->end(s));
+            if (fork) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], s));
+            continue;
+        }
         hdb::SparseArgs a{};
         a.X = X;
         a.offsets = d_offsets;
@@ -931,7 +975,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         if (spans) HDB_CUDA(spans->end(s));
         if (forked) HDB_CUDA(cudaEventRecord(p->events[2 * f + 1], s));
     }
-    return join(joined, n_groups + p->classes.size() - (p->groups.empty() ? 0 : 1));
+    return join(joined, n_groups + p->classes.size() - (p->n_sparse ? 1 : 0));
 }
 
 // ---- plan cache of the dense seam -----------------------------------------
@@ -1132,7 +1176,7 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
                     ",\"dims\":" + std::to_string(p->D) + ",\"workspace_bytes\":" + std::to_string(p->ws_bytes) +
                     ",\"distance_tiles\":" + std::to_string(p->tiles.size() / 3) +
                     // int32 [windows] in the workspace after a forward: 1 = the window left the sparse path.
-                    ",\"general_flags_offset\":" + std::to_string(p->groups.empty() ? -1 : (int64_t)p->t_flags) +
+                    ",\"general_flags_offset\":" + std::to_string(!p->n_sparse ? -1 : (int64_t)p->t_flags) +
                     ",\"classes\":[";
     bool first_class = true;
     auto points = [&](const std::vector<int>& windows, int power) {
@@ -1144,8 +1188,8 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
         return std::to_string(total);
     };
     for (const auto& g : p->groups) {
-        s += (first_class ? "" : ",") + std::string("{\"variant\":\"sparse\",\"cluster\":1,\"list\":") +
-             std::to_string(p->list) + ",\"light_edges_per_point\":" + std::to_string(p->light_cap) + ",\"priority\":" +
+        s += (first_class ? "" : ",") + std::string("{\"variant\":\"") + (g.small ? "small" : "sparse") +
+             "\",\"cluster\":1,\"list\":" + std::to_string(g.small ? 0 : p->list) + ",\"priority\":" +
              std::to_string(g.priority) + ",\"windows\":" + std::to_string(g.windows.size()) + ",\"points\":" +
              points(g.windows, 1) + ",\"sum_n2\":" + points(g.windows, 2) + ",\"nmax\":" + std::to_string(g.nmax) + "}";
         first_class = false;
