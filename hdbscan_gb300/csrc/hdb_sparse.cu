@@ -48,7 +48,8 @@ cudaError_t launch_stage(SparseStage stage, const SparseArgs& a, const ForwardAr
             return launch_ex(hdb_sparse_tree_kernel<Real>, W, (unsigned)window_threads(a.nmax), sparse_tree_smem(a.nmax),
                              s, priority, 1, a);
         case SparseStage::kLight:
-            return launch_ex(hdb_sparse_light_kernel<Real>, W * blocks(a.nmax, kLightRows), 256, 0, s, priority, 1, a);
+            return launch_ex(hdb_sparse_light_kernel<Real>, W * blocks(a.nmax, kLightRows), 256,
+                             (size_t)sparse_round(a.nmax) * sizeof(float), s, priority, 1, a);
         case SparseStage::kStar:
             return launch_ex(hdb_sparse_star_kernel<Real>, W * blocks(a.nmax, kSparseRowsCta), 256, 0, s, priority, 1, a);
         case SparseStage::kPrim:

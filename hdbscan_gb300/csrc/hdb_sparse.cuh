@@ -234,7 +234,13 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
 // coordinates are one 128-byte line of high and low parts; two stages of
 // asynchronous copies, 16-byte chunks swizzled by row for ldmatrix.  Off-diagonal
 // values are written to both halves from one accumulator, so the block is
-// symmetric.  Bound by the block's own write (4 n^2 bytes) for small D.
+// symmetric.  A finished tile goes out by way of shared memory, in whole lines, with
+// the minima of 16 columns of each row and of 16 rows of each column: half of the
+// instructions and store wavefronts of stores from the accumulators.  Floor: the
+// block's own write (4 n^2 bytes) for small D; held back by two CTAs an SM (128
+// registers a thread).  16 windows of 2048 points x 64 dims (268 MB): 112 us from
+// the accumulators, 109 this way; ragged batch of 64..4096 points x 32 dims, whole
+// call: 6.09 and 5.97 ms.
 // ---------------------------------------------------------------------------
 constexpr int kGramStage = 2 * 128 * 128;  // bytes of a stage: two operands of 128 rows x 128 bytes
 
@@ -248,11 +254,18 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
+// Place of a finished tile's entry in shared memory: 16-byte chunks of a row are
+// permuted by the row, such that stores of accumulator pairs (8 rows x 4), reads of
+// rows and reads of 32 rows' chunks have no bank conflicts.
+__device__ __forceinline__ int gram_at(int r, int c) {
+    return (r << 7) + ((((c >> 2) ^ ((r << 1 | ((r >> 2) & 1)) & 7)) << 2) | (c & 3));
+}
+
 template <typename Real>
 __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArgs a) {
     constexpr int TS = 128;
     extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ float s_norm[2][TS];
+    __shared__ __align__(8) float s_norm[2][TS];  // times 1 - eta
     const int tmax = (a.nmax + TS - 1) / TS;
     const int per = tmax * (tmax + 1) / 2;
     const int item = blockIdx.x / per;
@@ -269,21 +282,23 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArg
     const int i0 = ti * TS, j0 = tj * TS;
     const int chunks = a.dims >> 5;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint16_t* __restrict__ S = a.split + base * 2 * a.dims;
+    const float inf = __int_as_float(0x7f800000);
     for (int r = tid; r < 2 * TS; r += 256) {
         const int g = (r < TS ? i0 + r : j0 + r - TS);
-        s_norm[r >> 7][r & (TS - 1)] = g < n ? a.norm[base + g] : 0.0f;
+        s_norm[r >> 7][r & (TS - 1)] = (g < n ? a.norm[base + g] : inf) * (1.0f - sparse_eta(a.D));
     }
+    const int row_bytes = 4 * a.dims;
+    const int lr = tid >> 3;                      // 2 operands x 128 rows x 8 chunks of 16 bytes
+    const uint32_t dst0 = sbase + lr * 128 + (((tid & 7) ^ (lr & 7)) << 4);
+    const char* src0 = reinterpret_cast<const char*>(a.split + base * 2 * a.dims) + (tid & 7) * 16;
     auto load = [&](int c, int stage) {
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int e = tid + 256 * q;          // 2 operands x 128 rows x 8 chunks
-            const int op = e >> 10, r = (e >> 3) & 127, ch = e & 7;
-            const int g = (op == 0 ? i0 : j0) + r;
-            const uint32_t dst = sbase + stage * kGramStage + op * (TS * 128) + r * 128 + ((ch ^ (r & 7)) << 4);
-            const uint16_t* src = S + (int64_t)min(g, n - 1) * 2 * a.dims + c * 64 + ch * 8;
+            const int g = (q < 4 ? i0 : j0) + lr + 32 * (q & 3);
+            const char* src = src0 + (int64_t)min(g, n - 1) * row_bytes + c * 128;
             const int bytes = g < n ? 16 : 0;     // rows past the window are zeros
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes));
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst0 + stage * kGramStage + q * 4096),
+                         "l"(src), "r"(bytes));
         }
         asm volatile("cp.async.commit_group;");
     };
@@ -349,103 +364,91 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArg
         }
         __syncthreads();
     }
-    const float eta = sparse_eta(a.D);
     float* __restrict__ Dw = sparse_block<Real>(a, w);
     float* __restrict__ minima = a.minima + a.dist_offsets[w] / 8;
     const int groups = (n + 15) >> 4;
     const int64_t ld = dist_ld(n);
     const bool diagonal = ti == tj;
-    const float inf = __int_as_float(0x7f800000);
-    // Accumulators become bounds in place; entries outside the window are infinite.
+    // Accumulators become bounds in place (the norms carry 1 - eta); points past the
+    // window have infinite norms, so their entries are infinite.
 #pragma unroll
     for (int p = 0; p < 2; ++p)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int r = wm + 16 * p + 8 * h + (lane >> 2), gi = i0 + r;
-            const float ni = s_norm[0][r];
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    const int col = wn + 8 * q + 2 * (lane & 3) + b, gj = j0 + col;
-                    const float sum = ni + s_norm[1][col];
-                    float v = fmaxf(__fmaf_rn(-eta, sum, __fmaf_rn(-2.0f, acc[p][q][2 * h + b], sum)), 0.0f);
-                    if (diagonal && gi == gj) v = 0.0f;
-                    acc[p][q][2 * h + b] = gi < n && gj < n ? v : inf;
-                }
-        }
-    // Minima of 16 columns of each row: four values here, four lanes of the quad.
-    // (In a diagonal tile both halves are in the accumulators; their minima may
-    // differ from the stored upper half's by the products' asymmetry, so they are
-    // taken from the stored values below.)
-    if (!diagonal) {
-#pragma unroll
-        for (int p = 0; p < 2; ++p)
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int gi = i0 + wm + 16 * p + 8 * h + (lane >> 2);
-#pragma unroll
-                for (int q = 0; q < 8; q += 2) {
-                    float v = fminf(fminf(acc[p][q][2 * h], acc[p][q][2 * h + 1]),
-                                    fminf(acc[p][q + 1][2 * h], acc[p][q + 1][2 * h + 1]));
-                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 1));
-                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 2));
-                    const int g = (j0 + wn + 8 * q) >> 4;
-                    if ((lane & 3) == 0 && gi < n && g < groups) minima[(int64_t)gi * groups + g] = v;
-                }
-            }
-        // Of 16 rows of each column, for the mirrored half: two values here, eight lanes.
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            const int g = (i0 + wm + 16 * p) >> 4;
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-#pragma unroll
-                for (int b = 0; b < 2; ++b) {
-                    float v = fminf(acc[p][q][b], acc[p][q][2 + b]);
-                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 4));
-                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 8));
-                    v = fminf(v, __shfl_xor_sync(0xffffffffu, v, 16));
-                    const int gj = j0 + wn + 8 * q + 2 * (lane & 3) + b;
-                    if (lane < 4 && gj < n && g < groups) minima[(int64_t)gj * groups + g] = v;
-                }
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = wm + 16 * p + 8 * h + (lane >> 2), gi = i0 + r;
-            if (gi >= n) continue;
+            const float ni = s_norm[0][wm + 16 * p + 8 * h + (lane >> 2)];
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
-                const int col = wn + 8 * q + 2 * (lane & 3), gj = j0 + col;
-                const float v[2] = {acc[p][q][2 * h], acc[p][q][2 * h + 1]};
+                const float2 nj = *reinterpret_cast<const float2*>(&s_norm[1][wn + 8 * q + 2 * (lane & 3)]);
+                acc[p][q][2 * h] = fmaxf(__fmaf_rn(-2.0f, acc[p][q][2 * h], ni + nj.x), 0.0f);
+                acc[p][q][2 * h + 1] = fmaxf(__fmaf_rn(-2.0f, acc[p][q][2 * h + 1], ni + nj.y), 0.0f);
+            }
+        }
+    // The tile in shared memory, over the stages (the loop's last barrier ended their
+    // use).  In a diagonal tile both halves are in the accumulators; the products'
+    // asymmetry could make them differ, so the upper one is taken for both.
+    float* tile = reinterpret_cast<float*>(smem);
+#pragma unroll
+    for (int p = 0; p < 2; ++p)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = wm + 16 * p + 8 * h + (lane >> 2);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const int col = wn + 8 * q + 2 * (lane & 3);
+                const float v0 = acc[p][q][2 * h], v1 = acc[p][q][2 * h + 1];
                 if (!diagonal) {
-                    // (gj < n and even imply that column gj + 1 lies inside the row's stride.)
-                    if (gj < n) *reinterpret_cast<float2*>(Dw + gi * ld + gj) = make_float2(v[0], v[1]);
-#pragma unroll
-                    for (int b = 0; b < 2; ++b)
-                        if (gj + b < n) Dw[(int64_t)(gj + b) * ld + gi] = v[b];
+                    *reinterpret_cast<float2*>(tile + gram_at(r, col)) = make_float2(v0, v1);
                 } else {
-#pragma unroll
-                    for (int b = 0; b < 2; ++b) {
-                        if (gj + b >= n || gi > gj + b) continue;
-                        Dw[gi * ld + gj + b] = v[b];
-                        Dw[(int64_t)(gj + b) * ld + gi] = v[b];
-                    }
+                    if (r <= col) tile[gram_at(r, col)] = tile[gram_at(col, r)] = v0;
+                    if (r <= col + 1) tile[gram_at(r, col + 1)] = tile[gram_at(col + 1, r)] = v1;
                 }
             }
         }
-    if (diagonal) {
-        __syncthreads();  // the CTA's own stores
-        const int first = i0 >> 4, count = min(TS / 16, groups - first);
-        for (int e = tid; e < TS * count; e += 256) {
-            const int r = e / count, g = first + e - r * count, gi = i0 + r;
-            if (gi >= n) continue;
-            float v = inf;
-            for (int c = 16 * g; c < min(16 * g + 16, n); ++c) v = fminf(v, Dw[gi * ld + c]);
-            minima[(int64_t)gi * groups + g] = v;
+    __syncthreads();
+    // Rows: 512 bytes a warp and store, with the minima of 16 columns (four lanes).
+    // (Entries past the window, up to three in a row's padding, are infinite.)
+    {
+        const int gi = i0 + warp * (TS / 8), gj = j0 + 4 * lane, g = gj >> 4;
+        float* out = Dw + gi * ld + gj;
+        float* least = minima + (int64_t)gi * groups + g;
+        const bool store = gj < n, store_min = (lane & 3) == 0 && g < groups;
+#pragma unroll 8
+        for (int k = 0; k < TS / 8; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(tile + gram_at(warp * (TS / 8) + k, 4 * lane));
+            float m = fminf(fminf(v.x, v.y), fminf(v.z, v.w));
+            m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+            m = fminf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+            if (gi + k < n) {
+                if (store) *reinterpret_cast<float4*>(out + k * ld) = v;
+                if (store_min) least[k * groups] = m;
+            }
+        }
+    }
+    if (diagonal) return;
+    // Columns: a lane reads four of one row; a warp's stores are 32 rows of one column.
+    // (Rows lie above the diagonal, so inside the window.)
+    for (int q = warp * 4; q < warp * 4 + 4; ++q) {
+        const int gj = j0 + 4 * q;
+        float* out = Dw + (int64_t)gj * ld + i0 + lane;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 v = *reinterpret_cast<const float4*>(tile + gram_at(32 * k + lane, 4 * q));
+            if (gj < n) out[32 * k] = v.x;
+            if (gj + 1 < n) out[32 * k + ld] = v.y;
+            if (gj + 2 < n) out[32 * k + 2 * ld] = v.z;
+            if (gj + 3 < n) out[32 * k + 3 * ld] = v.w;
+        }
+    }
+    // The columns' minima of 16 rows: a thread takes half a column.
+    const int col = tid & (TS - 1), half = tid >> 7;
+    if (j0 + col < n) {
+        float* least = minima + (int64_t)(j0 + col) * groups + (i0 >> 4) + 4 * half;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            float m = inf;
+#pragma unroll
+            for (int r = 0; r < 16; ++r) m = fminf(m, tile[gram_at(64 * half + 16 * g + r, col)]);
+            least[g] = m;
         }
     }
 }
@@ -1146,7 +1149,9 @@ __global__ void __launch_bounds__(512) hdb_sparse_forest_kernel(const SparseArgs
 // The least edge between each two components, from the upper triangle of the
 // block: every row u against its columns v > u, into table row part[u].  A warp
 // takes a run of rows in component order and keeps the table row of the current
-// component in shared memory.
+// component in shared memory.  Bound by the latency of the block's read (2 n^2
+// bytes): 16 bytes a lane and load, four in flight, 63 us for 16 windows of 2048
+// points; 4 bytes, eight in flight, 76; two of 16 with more CTAs an SM 75.
 constexpr int kBetweenRows = 32;  // rows per CTA: runs of four a warp
 
 template <typename Real>
@@ -1170,6 +1175,10 @@ __global__ void __launch_bounds__(256) hdb_sparse_between_kernel(const SparseArg
     for (int u = tid; u < n; u += 256) {
         core[u] = a.unit_core ? 0.0f : a.core_up[base + u];
         part[u] = a.part[base + u];
+    }
+    for (int u = n + tid; u < cap; u += 256) {  // (rows are read by fours)
+        core[u] = 0.0f;
+        part[u] = 0;
     }
     __syncthreads();
     const float* __restrict__ Dw = sparse_block<Real>(a, w);
@@ -1195,23 +1204,34 @@ __global__ void __launch_bounds__(256) hdb_sparse_between_kernel(const SparseArg
         }
         const float* __restrict__ row = Dw + (int64_t)u * ld;
         const float core_u = core[u];
-        constexpr int U = 8;
-        for (int v0 = (u + 1) & ~31; v0 < n; v0 += 32 * U) {
-            float d[U];
+        constexpr int U = 4;
+        for (int v0 = ((u + 1) & ~31) + 4 * lane; v0 < n; v0 += 128 * U) {
+            float4 d4[U];
 #pragma unroll
             for (int q = 0; q < U; ++q) {
-                const int v = v0 + 32 * q + lane;
-                d[q] = v < n ? __ldcg(row + v) : 0.0f;
+                const int v = v0 + 128 * q;
+                d4[q] = v < n ? __ldcg(reinterpret_cast<const float4*>(row + v)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             }
 #pragma unroll
             for (int q = 0; q < U; ++q) {
-                const int v = v0 + 32 * q + lane;
-                if (v >= n || v <= u) continue;
-                const int cv = part[v];
-                if (cv == cu) continue;
-                const float wgt = fmaxf(fmaxf(core_u, core[v]), bound.up(d[q]));
-                if (__float_as_uint(wgt) > least_w[2 * cv]) continue;
-                atomicMin(&least[cv], sparse_key(wgt, u, v));
+                const int v = v0 + 128 * q;
+                if (v >= n) break;
+                const float4 core4 = *reinterpret_cast<const float4*>(core + v);
+                const ushort4 part4 = *reinterpret_cast<const ushort4*>(part + v);
+                const float d[4] = {d4[q].x, d4[q].y, d4[q].z, d4[q].w};
+                const float cores[4] = {core4.x, core4.y, core4.z, core4.w};
+                const int cv[4] = {part4.x, part4.y, part4.z, part4.w};
+                float wgt[4];
+                unsigned hit = 0;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    wgt[b] = fmaxf(fmaxf(core_u, cores[b]), bound.up(d[b]));
+                    if (cv[b] != cu && __float_as_uint(wgt[b]) <= least_w[2 * cv[b]]) hit |= 1u << b;
+                }
+                if (!hit) continue;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    if ((hit >> b & 1) && v + b > u && v + b < n) atomicMin(&least[cv[b]], sparse_key(wgt[b], u, v + b));
             }
         }
     }
@@ -1358,36 +1378,44 @@ __global__ void __launch_bounds__(512) hdb_sparse_tree_kernel(const SparseArgs a
 // hdb_sparse_star_kernel.  A warp streams the upper triangle's part of a row in
 // vertex order; pairs within the maxima at the root (mostly those inside one
 // cluster) gather in shared memory and are settled 32 at a time.  A warp takes
-// rows r and n - 1 - r, which together are one row long.  Bound by the block's read (2 n^2 bytes).
+// rows r and n - 1 - r, which together are one row long.  Bound by the instructions a pair takes and the latency
+// of the block's read (2 n^2 bytes): with four columns a lane and load, and the
+// maxima at the root in shared memory, 16 windows of 2048 points take 87 us (one
+// column a lane and load: 102; 134 MB at the copy rate: 20).
 // ---------------------------------------------------------------------------
 template <typename Real>
-__global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs a) {
+__global__ void __launch_bounds__(256, 5) hdb_sparse_light_kernel(const SparseArgs a) {
     __shared__ uint32_t s_span[8][kSparseLevels];
     __shared__ float s_top[8][kSparseLevels];
     __shared__ uint2 s_pair[8][64];  // (distance, column) of pairs that may be light
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* top_root = reinterpret_cast<float*>(smem);  // of every vertex; read by fours
     const int per = (a.nmax + kLightRows - 1) / kLightRows;
     const int item = blockIdx.x / per, j = blockIdx.x - item * per;
     const int w = a.queue[item];
     const int64_t base = a.offsets[w];
     const int n = (int)(a.offsets[w + 1] - base);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int r = j * (kLightRows / 2) + warp;
-    if (2 * r > n - 1 || a.flags[w]) return;  // warp-uniform
+    if (j * kLightRows > n - 1) return;
+    if (__syncthreads_or(threadIdx.x == 0 && a.flags[w])) return;  // (may be set meanwhile)
     const int levels = a.levels[w];
     const float* __restrict__ Dw = sparse_block<Real>(a, w);
     const int64_t ld = dist_ld(n);
     const SparseBound bound = sparse_bound<Real>(a, w);
     const uint16_t* __restrict__ pos = a.pos + base;
-    const float* __restrict__ top_root = a.level_max_v + (int64_t)(levels - 1) * a.T + base;
+    for (int v = threadIdx.x; v < sparse_round(n); v += 256)
+        top_root[v] = v < n ? a.level_max_v[(int64_t)(levels - 1) * a.T + base + v] : 0.0f;
+    __syncthreads();
     const int limit = n * a.light_cap;
     uint32_t* light_uv = a.light_uv + base * a.light_cap;
     Real* light_w = static_cast<Real*>(a.light_w) + base * a.light_cap;
     uint32_t* span = s_span[warp];
     float* top = s_top[warp];
     uint2* pair = s_pair[warp];
-    for (int side = 0; side < 2; ++side) {
-        const int u = side == 0 ? r : n - 1 - r;
-        if (side == 1 && u == r) break;
+    for (int turn = 0; turn < kLightRows / 8; ++turn) {
+        const int r = j * (kLightRows / 2) + (turn >> 1) * 8 + warp;
+        const int u = (turn & 1) == 0 ? r : n - 1 - r;
+        if (2 * r > n - 1 || ((turn & 1) && u == r)) break;
         __syncwarp();
         if (lane < levels) {
             span[lane] = a.level_span[(int64_t)lane * a.T + base + u];
@@ -1424,31 +1452,43 @@ __global__ void __launch_bounds__(256) hdb_sparse_light_kernel(const SparseArgs 
                 }
             }
         };
-        constexpr int U = 8;
-        for (int v0 = (u + 1) & ~31; v0 < n; v0 += 32 * U) {
-            float d[U], t[U];
+        constexpr int U = 2;
+        const float inf = __int_as_float(0x7f800000);
+        for (int v0 = (u + 1) & ~31; v0 < n; v0 += 128 * U) {
+            float4 d4[U];
 #pragma unroll
             for (int q = 0; q < U; ++q) {
-                const int v = v0 + 32 * q + lane;
-                const bool in = v > u && v < n;
-                d[q] = in ? __ldcs(row + v) : __int_as_float(0x7f800000);
-                t[q] = in ? top_root[v] : 0.0f;
+                const int v = v0 + 128 * q + 4 * lane;
+                d4[q] = v < n ? __ldcs(reinterpret_cast<const float4*>(row + v)) : make_float4(inf, inf, inf, inf);
             }
 #pragma unroll
             for (int q = 0; q < U; ++q) {
-                const bool may = bound.down(d[q]) <= fmaxf(top_u, t[q]);
-                const unsigned bal = __ballot_sync(0xffffffffu, may);
-                if (!bal) continue;
-                if (may) pair[waiting + __popc(bal & lanemask_lt())] = make_uint2(__float_as_uint(d[q]), v0 + 32 * q + lane);
-                waiting += __popc(bal);
-                __syncwarp();
-                if (waiting >= 32) {
-                    settle(32);
-                    waiting -= 32;
-                    const uint2 rest = pair[32 + lane];
+                const int v = v0 + 128 * q + 4 * lane;
+                const float4 t = v < n ? *reinterpret_cast<const float4*>(top_root + v) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                const float d[4] = {d4[q].x, d4[q].y, d4[q].z, d4[q].w};
+                unsigned may = 0;
+                if (bound.down(d[0]) <= fmaxf(top_u, t.x)) may |= 1;
+                if (bound.down(d[1]) <= fmaxf(top_u, t.y)) may |= 2;
+                if (bound.down(d[2]) <= fmaxf(top_u, t.z)) may |= 4;
+                if (bound.down(d[3]) <= fmaxf(top_u, t.w)) may |= 8;
+                may &= (15u << min(max(u + 1 - v, 0), 4)) & (15u >> min(max(v + 4 - n, 0), 4));  // u < v + b < n
+                if (!__any_sync(0xffffffffu, may)) continue;
+#pragma unroll
+                for (int b = 0; b < 4; ++b) {
+                    const unsigned bal = __ballot_sync(0xffffffffu, may >> b & 1);
+                    if (!bal) continue;
+                    if (may >> b & 1)
+                        pair[waiting + __popc(bal & lanemask_lt())] = make_uint2(__float_as_uint(d[b]), v + b);
+                    waiting += __popc(bal);
                     __syncwarp();
-                    if (lane < waiting) pair[lane] = rest;
-                    __syncwarp();
+                    if (waiting >= 32) {
+                        settle(32);
+                        waiting -= 32;
+                        const uint2 rest = pair[32 + lane];
+                        __syncwarp();
+                        if (lane < waiting) pair[lane] = rest;
+                        __syncwarp();
+                    }
                 }
             }
         }
