@@ -228,16 +228,19 @@ def phase_report(phase_ms, phase_launches, describe, D, itemsize, peak, core_dis
     """Distance and core phases as achieved GB/s of algorithmic bytes (against the HBM peak), the
     distance phase also as pair-coordinates per second (its arithmetic rate), the forward as device
     ms.  Algorithmic bytes (sums over the windows of each kind):
-      distance: read X (n*D*s) + write the n x n block (n^2*s), matrix-variant windows;
-      core:     matrix windows read their block (n^2*s) + write core and neighbour (n*(s+4));
-                recompute windows read X (n*D*s) + the same writes (these are SIMT-bound)."""
-    matrix = [c for c in describe["classes"] if c["variant"] == "matrix"]
-    recompute = [c for c in describe["classes"] if c["variant"] != "matrix"]
+      distance: read X (n*D*s) + write the n x n block (n^2*s, 4 n^2 in sparse windows), matrix
+                and sparse windows;
+      core:     those windows read their block + write core and neighbour (n*(s+4));
+                recompute windows read X (n*D*s) + the same writes (these are SIMT-bound).
+    Windows of the small-window kernel have no phase but the forward."""
+    matrix = [c for c in describe["classes"] if c["variant"] in ("matrix", "sparse")]
+    recompute = [c for c in describe["classes"] if c["variant"] == "recompute"]
     points_m = sum(c["points"] for c in matrix)
     n2_m = sum(c["sum_n2"] for c in matrix)
+    block_bytes = sum(c["sum_n2"] * (4 if c["variant"] == "sparse" else itemsize) for c in matrix)
     points_r = sum(c["points"] for c in recompute)
     out = {}
-    dist_bytes = (n2_m + points_m * D) * itemsize
+    dist_bytes = block_bytes + points_m * D * itemsize
     if phase_launches["distance"]:
         gbs = dist_bytes / (phase_ms["distance"] / 1e3) / 1e9
         pair_coords = (n2_m - points_m) // 2 * D  # distinct pairs i < j times coordinates
@@ -245,9 +248,10 @@ def phase_report(phase_ms, phase_launches, describe, D, itemsize, peak, core_dis
                            "achieved_gbs": gbs, "frac_of_measured_hbm": gbs / peak,
                            "pair_coordinates": pair_coords,
                            "pair_coordinates_per_s": pair_coords / (phase_ms["distance"] / 1e3),
-                           "note": "arithmetic-bound: FP64 and ALU pipes (float64), FMA-pipe issue (float32)"}
+                           "note": "matrix windows: arithmetic-bound (FP64 and ALU pipes, FMA-pipe issue); "
+                                   "sparse windows: bounds by tensor-core products or float32 differences"}
     if core_distances and phase_launches["core"]:
-        core_bytes = n2_m * itemsize + (points_m + points_r) * (itemsize + 4) + points_r * D * itemsize
+        core_bytes = block_bytes + (points_m + points_r) * (itemsize + 4) + points_r * D * itemsize
         gbs = core_bytes / (phase_ms["core"] / 1e3) / 1e9
         out["core"] = {"ms": phase_ms["core"], "launches": phase_launches["core"], "bytes": core_bytes,
                        "achieved_gbs": gbs, "frac_of_measured_hbm": gbs / peak}
@@ -618,9 +622,10 @@ def main():
     sizes = np.diff(offsets)
     describe = json.loads(plan.describe())
     # Algorithmic bytes per launch: read X (N*D*s) + write labels (4N) per window,
-    # plus the N^2*s distance block read by windows of the matrix variant.
+    # plus the N^2*s distance block read by windows of the matrix variant (4 N^2 in the sparse form).
     algo_bytes = float(np.sum(sizes * D * itemsize + sizes * 4))
-    algo_bytes += float(sum(c["sum_n2"] for c in describe["classes"] if c["variant"] == "matrix") * itemsize)
+    algo_bytes += float(sum(c["sum_n2"] * {"matrix": itemsize, "sparse": 4}.get(c["variant"], 0)
+                            for c in describe["classes"]))
     achieved = algo_bytes / (kernel_ms_mean / 1e3) / 1e9
     traffic = None
     traffic_path = ROOT / "profiles" / f"traffic_{args.config}.json"

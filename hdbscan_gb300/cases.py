@@ -9,14 +9,15 @@ run as well).
 
   tile64     64 windows x 256 points x 64 dims float32, ms=5: hdb_distance_kernel<float>
              (64x64 tiles; small float32 windows of wide points take the matrix variant)
-  tile128    16 windows x 2048 x 64 float32, ms=5: hdb_distance128_kernel, hdb_core_rows_kernel,
-             hdb_forward_kernel<float, 512, 4, 0, 1> (matrix Prim)
-  tile128d32 16 windows x 2048 x 32 float32, ms=10: the same kernels at the ragged workload's
-             dimension and list length (hdb_core_rows_kernel<float, 16>)
-  tile64f64  2 windows x 3072 x 128 float64, ms=16: hdb_distance_kernel<double>, hdb_core_rows_kernel<double>
+  tile128    16 windows x 2048 x 64 float32, ms=5: the sparse passes with tensor-core bounds
+             (hdb_sparse_gram_kernel, hdb_sparse_gram_rows_kernel, ..., hdb_sparse_prim_kernel)
+  tile128d32 16 windows x 2048 x 32 float32, ms=10: the sparse passes with exact float32
+             distances (hdb_sparse_tiles_kernel, hdb_sparse_rows_kernel)
+  tile64f64  2 windows x 3072 x 128 float64, ms=16: the sparse passes of float64 windows
   points     64 windows x 1000 x 32 float32, ms=10: hdb_core_points_kernel (register windows)
   select     16 windows x 512 x 8 float32, ms=80: hdb_core_select_kernel (lists longer than 64)
-  key        8 windows x 2048 x 16 float64, ms=40: hdb_core_matrix_key_kernel (float64 lists of 64)
+  key        8 windows x 2048 x 16 float64, ms=40: the sparse passes with lists of 64 on float32
+             bounds of float64 distances
   prepare    64 windows x 1024 x 16 bfloat16 input, L2-normalised: hdb_prepare_kernel
   backward   8 windows x 2048 x 64 float32, ms=5, forward + hdb_backward_kernel
   c2         64 windows x 1024 x 16 float32 of the uniform-batch workload: hdb_forward_kernel<float, 512, 2, 16, 1>

@@ -90,8 +90,9 @@ extern "C" {
  * HDB_STATUS_INTERNAL and writes no labels.  It exercises the give-up path of
  * the cluster waits without any transfer in flight. */
 #define HDB_FLAG_TEST_STALL 256u
-/* Keep every window on the general path (dense Prim loop): the autotuner's
- * measurements and comparisons of the two paths.  Results are the same. */
+/* Keep every window on the general path (distances, cores, dense Prim loop): no
+ * sparse passes and no small-window kernel.  For the autotuner's measurements and
+ * comparisons of the paths.  Results are the same. */
 #define HDB_FLAG_NO_SPARSE 512u
 
 typedef struct hdb_plan hdb_plan_t;
