@@ -168,6 +168,19 @@ constexpr int kTile128MinN = 384;  // float32 matrix classes from this size use 
 // 315, of 512 383 and 421).  In float64 the general form recomputes every distance at
 // two operations a clock on an SM.
 constexpr int kSparseMinN[2] = {384, 16};
+// float32 windows whose general form keeps coordinates in registers (no block):
+// `many` such windows of 512 points or more in the batch.  A dense step then
+// computes its distances on one SM, 0.5 to 1.8 us, but all SMs work at once, while
+// the sparse passes cost about 5 ps a pair of points in all and write the block.
+// Device time, sparse and general form, min_samples 5: one window of 1024 x 16 444
+// and 731 us, of 4000 x 16 1301 and 10148; 24 of 1024 x 4 614 and 944, of 4000 x 4
+// 2962 and 10136; 80 of 1024 x 16 964 and 891; 152 of 2048 x 32 3745 and 6160.  With
+// unit cores 24 of 1024 x 16 586 and 553, of 1536 x 4 769 and 1080.
+bool sparse_pays(int n, int D, bool unit, size_t many) {
+    if (D > 16 && n >= 1536) return many <= 152;
+    return many <= 24 && n >= (D > 16 ? 512 : (unit ? 1536 : 1024));
+}
+
 constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
@@ -355,9 +368,11 @@ int build_plan(hdb_plan* p) {
     p->approx = p->gram || p->precision == HDB_F64;
     p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
     if (p->list && special) {
+        size_t many = 0;
+        for (int w : order) many += chosen[w]->dp != 0 && chosen[w]->cluster == 1 && size_of(w) >= 512;
         for (int w : order)
             sparse[w] = !small[w] && size_of(w) >= kSparseMinN[p->precision != 0] && chosen[w]->cluster == 1 &&
-                        (p->precision == HDB_F64 || chosen[w]->dp == 0);
+                        (p->precision == HDB_F64 || chosen[w]->dp == 0 || sparse_pays(size_of(w), p->D, unit, many));
         for (int w : order)
             if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
         bool fits = true;

@@ -165,3 +165,16 @@ def test_many_flagged_windows(cuda, precision):
         np.testing.assert_array_equal(host["edges_uv"][lo - w:hi - w - 1], o["edges_uv"])
         np.testing.assert_array_equal(host["core"][lo:hi].view(np.uint8), o["core"].view(np.uint8))
         np.testing.assert_array_equal(host["labels"][lo:hi], o["labels"])
+
+
+@pytest.mark.parametrize("n, dims, ms, count, sparse", [
+    (1023, 16, 3, 1, False), (1024, 16, 3, 1, True), (1024, 16, 3, 24, True), (1024, 16, 3, 25, False),
+    (1535, 4, 2, 2, False), (1536, 4, 2, 2, True), (511, 17, 4, 2, False), (512, 17, 4, 2, True),
+    (1536, 32, 3, 25, True), (2049, 2, 5, 1, True), (3000, 8, 2, 1, True)])
+def test_few_windows_of_few_dims(cuda, n, dims, ms, count, sparse):
+    # float32 windows whose coordinates the general form keeps in registers.
+    rng = np.random.default_rng(n + dims)
+    windows = [(_mixture, _lattice)[w % 2](rng, n, dims) for w in range(count)]
+    describe, _ = _check(windows, 5, ms, 0.0, "float32")
+    if sparse or all(c["variant"] != "matrix" for c in describe["classes"]):
+        assert any(c["variant"] == "sparse" for c in describe["classes"]) == sparse
