@@ -175,6 +175,11 @@ constexpr int kGramMinDims = 32;
 constexpr int kGramMaxDims = 2048;   // the centre in shared memory
 constexpr int kCentrePoints = 16;
 constexpr int kSplitRows = 32;
+// All shares of sparse_eta are relative to the norms, so products below float32's
+// normal range must not count: with points of at least this squared norm (2^-90),
+// up to 3 * 2048 products of less than 2^-126 are under 2^-22 of it even when each is
+// lost.  A point at the centre itself has a norm of zero and exact products.
+constexpr float kGramLeastNorm = 8.077936e-28f;
 
 template <typename Real>
 __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs a) {
@@ -188,10 +193,15 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
     const int D = a.D, dims = a.dims;
     const Real* __restrict__ X = static_cast<const Real*>(a.X) + base * D;
     for (int k = threadIdx.x; k < D; k += 256) {
-        Real sum = Real(0);
+        // Summed in pairs: of sixteen copies of a point the mean is that point.
+        Real sum[kCentrePoints];
 #pragma unroll
-        for (int j = 0; j < kCentrePoints; ++j) sum += X[(int64_t)(j * n / kCentrePoints) * D + k];
-        s_centre[k] = sum * Real(1.0 / kCentrePoints);
+        for (int j = 0; j < kCentrePoints; ++j) sum[j] = X[(int64_t)(j * n / kCentrePoints) * D + k];
+#pragma unroll
+        for (int h = kCentrePoints / 2; h > 0; h >>= 1)
+#pragma unroll
+            for (int j = 0; j < h; ++j) sum[j] += sum[j + h];
+        s_centre[k] = sum[0] * Real(1.0 / kCentrePoints);
     }
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -201,12 +211,13 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
         const Real* __restrict__ x = X + (int64_t)i * D;
         uint16_t* __restrict__ out = a.split + (base + i) * 2 * dims;
         float norm = 0.0f;
-        bool bad = false;
+        bool bad = false, off = false;
         for (int k = lane; k < dims; k += 32) {
             float z = 0.0f;
             if (k < D) {
                 const Real v = x[k];
                 bad |= !isfinite(v);
+                off |= v != s_centre[k];
                 z = (float)(v - s_centre[k]);
             }
             const __nv_bfloat16 hi = __float2bfloat16_rn(z);
@@ -218,7 +229,8 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
-        bad = __any_sync(0xffffffffu, bad) || !(norm <= 1.2e24f);  // 2^80; also tests NaN
+        off = __any_sync(0xffffffffu, off);
+        bad = __any_sync(0xffffffffu, bad) || !(norm <= 1.2e24f) || (off && norm < kGramLeastNorm);  // 2^80; also tests NaN
         if (lane == 0) {
             a.norm[base + i] = norm;
             if (bad) sparse_flag(a, w);
