@@ -73,8 +73,11 @@ __device__ __forceinline__ float* sparse_block(const SparseArgs& a, int w) {
 // Products (D >= kGramMinDims): the block holds a lower bound of the squared
 // distance, n_i + n_j - 2 z_i.z_j - eta (n_i + n_j) with the centred points z as
 // sums of two bfloat16 parts (see sparse_eta), and the true value lies at most
-// 2 eta (n_i + n_j) above it.  Core distances and all weights of the kernels
-// below are then squares as well; exact values stay plain distances.
+// 2 eta (n_i + n_j) above it.  What decides ranks and weights is not the true
+// value but the window's own arithmetic on it (sparse_exact), which adds its
+// share of the square itself (sparse_chain), on both sides.  Core distances and all
+// weights of the kernels below are then squares as well; exact values stay plain
+// distances.
 struct SparseBound {
     float up_shift, up_scale, down_shift, down_scale;
     __device__ __forceinline__ float up(float d) const { return __fmaf_ru(d, up_scale, up_shift); }
@@ -98,11 +101,26 @@ __device__ __forceinline__ float sparse_eta(int D) {
     return 1.1f * (3.0f * 3.8146973e-6f + 6.0f * 9.5367432e-7f + (float)(D / 8 + 32) * 5.9604645e-8f);
 }
 
+// Largest relative difference between the square of sparse_exact's value and the
+// true square.  float32: two roundings of a coordinate's difference and one of its
+// square in each term, one of each of the D - 1 sums, two of the root (squared), and
+// the squares of core distances taken up and down: D + 8 units of 2^-24; 5% covers
+// second order terms.  float64: D + 8 units of 2^-53, below a float32 unit at all
+// D that take products; sparse_eta's 10% covers it.
+template <typename Real>
+__device__ __forceinline__ float sparse_chain(int D) {
+    return sizeof(Real) == 4 ? 1.05f * (float)(D + 8) * 5.9604645e-8f : 0.0f;
+}
+
 template <typename Real>
 __device__ __forceinline__ SparseBound sparse_bound(const SparseArgs& a, int w) {
     if (!a.approx) return SparseBound{0.0f, 1.0f, 0.0f, 1.0f};
     const float R = __uint_as_float(a.range[w]);
-    if (a.gram) return SparseBound{4.2f * sparse_eta(a.D) * R, 1.0000005f, 0.0f, 1.0f};
+    if (a.gram) {
+        // (4.2 instead of 4: the sums' and the chain's share of the shift itself.)
+        const float chain = sparse_chain<Real>(a.D);
+        return SparseBound{4.2f * sparse_eta(a.D) * R, __fadd_ru(1.0000005f, chain), 0.0f, __fadd_rd(1.0f, -chain)};
+    }
     const float shift = 1.05f * sqrtf((float)a.D) * 1.1920929e-7f * R;
     const float scale = 1.05f * (0.5f * (float)a.D + 8.0f) * 5.9604645e-8f;
     return SparseBound{shift, __fadd_ru(1.0f, scale), -shift, __fadd_rd(1.0f, -scale)};
@@ -642,7 +660,7 @@ __device__ __forceinline__ void finish_row(const SparseArgs& a, const SparseBoun
                 const int p = lane + 32 * h;
                 const float d = __uint_as_float(lk[h]);
                 up[h] = bound.up(d);
-                if (a.gram && p < inside) up[h] = __fmaf_ru(slack, norm_i + a.norm[base + li[h]], d);
+                if (a.gram && p < inside) up[h] = __fmaf_ru(d, bound.up_scale, slack * (norm_i + a.norm[base + li[h]]));
                 if (p <= pos) most = fmaxf(most, up[h]);
             }
 #pragma unroll

@@ -12,6 +12,31 @@ from tests.test_gpu_sparse import _check
 pytestmark = pytest.mark.gpu
 
 
+def rounding_window(n=2048, d=1024):
+    """float32 sums of squares that round far apart: one point's neighbours lie at a squared distance of 4 and a
+    little.  Eight of them add that little in one coordinate (kept), one adds half a unit of 4's last place in every
+    coordinate (each rounded away): the farthest of the nine, by (d - 1) / 2 units, is the nearest in float32."""
+    rng = np.random.default_rng(7)
+    x = np.zeros((n, d))
+    # The rest: groups of about 16, each away from all others, with nothing undecided inside.
+    unit = rng.normal(0, 1 / np.sqrt(d), (n + n // 16, d - 1))
+    x[:, 1:] = 2 * unit[n + rng.integers(0, n // 16, n)] + rng.uniform(0.1, 1, (n, 1)) * unit[:n]
+    x[:, 0] = 1.0
+    samples = np.arange(16) * n // 16  # where the path takes its centre: their mean is zero
+    far = rng.normal(0, 1, (8, d - 1))
+    far *= 3 / np.linalg.norm(far, axis=1, keepdims=True)
+    x[samples[:8], 1:], x[samples[8:], 1:] = far, -far
+    x[samples, 0] = np.where(np.arange(16) % 2 == 0, 1.0, -1.0)
+    free = np.setdiff1d(np.arange(n), samples)
+    place = rng.choice(free, 10, replace=False)
+    x[place] = 0.0
+    x[place[0], 0] = -1.0  # the point whose neighbours these are
+    x[place[1:], 0] = 1.0
+    x[place[1:9], 1] = np.sqrt(2.0 ** -21 * 2 * np.arange(1, 9))
+    x[place[9], 1:] = 2.0 ** -11
+    return x.astype(np.float32)
+
+
 def tiny_window(n=3000, d=32):
     """A float64 cluster so small that the squares of its points' coordinates have no place in float32, in a window of ordinary
     range whose centre lies in that cluster."""
@@ -21,6 +46,10 @@ def tiny_window(n=3000, d=32):
     others = rng.choice(np.setdiff1d(np.arange(n), samples), 24, replace=False)
     x[np.concatenate([samples, others])] = rng.normal(0, 1, (40, d)) * 2e-22 / np.sqrt(d)
     return x
+
+
+def test_rounding_of_the_exact_sum(cuda):
+    _check([rounding_window()], 5, 5, 0.0, "float32")
 
 
 def test_squares_below_float32(cuda):
