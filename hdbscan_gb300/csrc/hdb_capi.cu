@@ -367,7 +367,7 @@ int build_plan(hdb_plan* p) {
     p->gram = hdb::sparse_gram(p->D) && (p->precision == HDB_F64 || coordinate_pairs >= kGramMinWork);
     p->approx = p->gram || p->precision == HDB_F64;
     p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
-    if (p->list && special) {
+    if (p->list && special && hdb::sparse_dims(p->approx, p->D)) {
         size_t many = 0;
         for (int w : order) many += chosen[w]->dp != 0 && chosen[w]->cluster == 1 && size_of(w) >= 512;
         for (int w : order)

@@ -109,6 +109,8 @@ cudaError_t sparse_prepare(int precision, int n, size_t budget, bool* fits) {
 
 bool sparse_gram(int D) { return D >= kGramMinDims && D <= kGramMaxDims; }
 
+bool sparse_dims(bool approx, int D) { return !approx || D <= kNarrowMaxDims; }
+
 int sparse_list(bool approx, bool gram, int ms, int* keep) {
     // Entries past position ms - 1 show where the star ends and bound the
     // uncertain range, which is wider for products.

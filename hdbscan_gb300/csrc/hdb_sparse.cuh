@@ -156,6 +156,10 @@ __device__ __forceinline__ Real sparse_exact(const Real* __restrict__ xa, const 
 // the window.
 // ---------------------------------------------------------------------------
 constexpr int kNarrowRows = 64;
+// The bound's relative part is of first order in D * 2^-24 (5% on top covers the rest
+// up to about 2 million dims), and a CTA's share of the input is counted in 32 bits
+// (up to 2^25 dims): wider points keep the general path, far below both.
+constexpr int kNarrowMaxDims = 1 << 16;
 
 __global__ void __launch_bounds__(256) hdb_sparse_narrow_kernel(const SparseArgs a) {
     const int per = (a.nmax + kNarrowRows - 1) / kNarrowRows;

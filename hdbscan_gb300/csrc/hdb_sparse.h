@@ -21,6 +21,9 @@ cudaError_t sparse_prepare(int precision, int n, size_t budget, bool* fits);
 // Whether windows of D dims take tensor-core products.
 bool sparse_gram(int D);
 
+// Whether the bound of the distances holds for windows of D dims.
+bool sparse_dims(bool approx, int D);
+
 // Row stride of the neighbour lists for min_samples ms (0: not supported) and
 // the entries used of them.
 int sparse_list(bool approx, bool gram, int ms, int* keep);

@@ -54,3 +54,10 @@ def test_rounding_of_the_exact_sum(cuda):
 
 def test_squares_below_float32(cuda):
     _check([tiny_window()], 5, 5, 0.0, "float64")
+
+
+@pytest.mark.parametrize("d, sparse", [(1 << 16, True), ((1 << 16) + 1, False)])
+def test_most_dims_of_narrowed_points(cuda, d, sparse):
+    rng = np.random.default_rng(d)
+    describe, _ = _check([rng.normal(size=(40, d))], 4, 3, 0.0, "float64")
+    assert any(c["variant"] == "sparse" for c in describe["classes"]) == sparse
