@@ -23,6 +23,7 @@ HDB_FLAG_INPUT_F16 = 64
 HDB_FLAG_L2_NORMALIZE = 128
 HDB_FLAG_TEST_STALL = 256
 HDB_FLAG_NO_SPARSE = 512
+HDB_FLAG_FORCE_PRODUCTS = 1024
 STATUS_OVERFLOW = 1
 STATUS_NONFINITE = 2
 STATUS_INTERNAL = 4

@@ -364,7 +364,8 @@ int build_plan(hdb_plan* p) {
     // windows of 32 dims: 8.46 without, 8.00 with).
     double coordinate_pairs = 0;
     for (int w : order) coordinate_pairs += (double)size_of(w) * size_of(w) * p->D;
-    p->gram = hdb::sparse_gram(p->D) && (p->precision == HDB_F64 || coordinate_pairs >= kGramMinWork);
+    p->gram = hdb::sparse_gram(p->D) && (p->precision == HDB_F64 || coordinate_pairs >= kGramMinWork ||
+                                         (p->flags & HDB_FLAG_FORCE_PRODUCTS));
     p->approx = p->gram || p->precision == HDB_F64;
     p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
     if (p->list && special && hdb::sparse_dims(p->approx, p->D)) {
@@ -1192,6 +1193,7 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
                     ",\"distance_tiles\":" + std::to_string(p->tiles.size() / 3) +
                     // int32 [windows] in the workspace after a forward: 1 = the window left the sparse path.
                     ",\"general_flags_offset\":" + std::to_string(!p->n_sparse ? -1 : (int64_t)p->t_flags) +
+                    ",\"products\":" + (p->n_sparse && p->gram ? "true" : "false") +
                     ",\"classes\":[";
     bool first_class = true;
     auto points = [&](const std::vector<int>& windows, int power) {

@@ -94,6 +94,9 @@ extern "C" {
  * sparse passes and no small-window kernel.  For the autotuner's measurements and
  * comparisons of the paths.  Results are the same. */
 #define HDB_FLAG_NO_SPARSE 512u
+/* Test switch: float32 batches of any size take tensor-core products where their
+ * points have the dims for them (float64 ones always do).  Results are the same. */
+#define HDB_FLAG_FORCE_PRODUCTS 1024u
 
 typedef struct hdb_plan hdb_plan_t;
 
