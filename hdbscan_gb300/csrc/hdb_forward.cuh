@@ -50,6 +50,10 @@ constexpr int kBarEmpty = 5;  // 5, 6: tree -> Prim release of arena 0 / 1
 constexpr int kBarHelp = 7;   // whole CTA: the last window's sort
 // A CTA's last window is done by every warp from this many edges.
 constexpr int kHelpMinEdges = 48;
+// Not in the float32 matrix variant of 8 slots a thread: with that code in the kernel its
+// Prim loop with core distances loses its overlapped row reads (one window of 4001
+// points 10.5 ms, 5.4 without; 16 of them 19.7 and 7.3).
+template <typename Real, int SV, int DP> constexpr bool kWholeCtaTail = sizeof(Real) == 8 || DP > 0 || SV <= 4;
 
 __device__ __forceinline__ void bar_sync(int id, int count) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
@@ -478,10 +482,12 @@ __global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid
             bar_sync(kBarFull + b, PT + 32);
             const WindowMeta meta = s_meta[b];
             if (meta.w < 0) return;
-            if (meta.help) {  // no release: the Prim warps consumed every earlier one and exit too
-                tree_window_cta<Real>(args, smem + (size_t)b * args.arena_stride, meta.w, meta.n, EdgeOrder::kNone,
-                                      reinterpret_cast<uint32_t*>(s_scan), s_ctr, kBarHelp);
-                return;
+            if constexpr (kWholeCtaTail<Real, SV, DP>) {
+                if (meta.help) {  // no release: the Prim warps consumed every earlier one and exit too
+                    tree_window_cta<Real>(args, smem + (size_t)b * args.arena_stride, meta.w, meta.n, EdgeOrder::kNone,
+                                          reinterpret_cast<uint32_t*>(s_scan), s_ctr, kBarHelp);
+                    return;
+                }
             }
             if (!meta.skip) tree_window<Real>(args, smem + (size_t)b * args.arena_stride, meta.w, meta.n);
             __syncwarp();
@@ -581,17 +587,20 @@ __global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid
             for (int j = tid; j < n; j += PT) args.labels[base + j] = -1;
             skip = 1;
         }
-        const int help = s_item >= args.queue_len && !skip && n - 1 >= kHelpMinEdges;
+        int help = 0;
+        if constexpr (kWholeCtaTail<Real, SV, DP>) help = s_item >= args.queue_len && !skip && n - 1 >= kHelpMinEdges;
         if (tid == 0) { s_meta[b].w = w; s_meta[b].n = n; s_meta[b].skip = skip; s_meta[b].help = help; }
         __threadfence_block();
         bar_arrive(kBarFull + b, PT + 32);
-        if (help) {
-            // Take the tree warp's release of the previous window (nothing may
-            // stay pending at exit), then do this one with it.
-            if (nb == 2 && k >= 1) bar_sync(kBarEmpty + (b ^ 1), PT + 32);
-            tree_window_cta<Real>(args, smem + (size_t)b * args.arena_stride, w, n, EdgeOrder::kNone,
-                                  reinterpret_cast<uint32_t*>(s_scan), s_ctr, kBarHelp);
-            return;
+        if constexpr (kWholeCtaTail<Real, SV, DP>) {
+            if (help) {
+                // Take the tree warp's release of the previous window (nothing may
+                // stay pending at exit), then do this one with it.
+                if (nb == 2 && k >= 1) bar_sync(kBarEmpty + (b ^ 1), PT + 32);
+                tree_window_cta<Real>(args, smem + (size_t)b * args.arena_stride, w, n, EdgeOrder::kNone,
+                                      reinterpret_cast<uint32_t*>(s_scan), s_ctr, kBarHelp);
+                return;
+            }
         }
     }
 }
