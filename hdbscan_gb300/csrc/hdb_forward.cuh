@@ -448,8 +448,24 @@ struct WindowMeta {
 // MINB CTAs share an SM (register budget from the launch bounds): with two,
 // one window's barrier and reduction latency hides behind another's distance
 // arithmetic.
+//
+// The whole-CTA tail needs more registers than the Prim loop of the small variants, and
+// a batch of many windows lives from the CTAs an SM holds (four at most: each takes
+// eight barriers) and, in matrix variants, from the room for the next chunk's distance
+// tiles beside them.  So they keep the registers that the loop needs, given here as
+// CTAs an SM, and the tail spills a little (600 windows of 130 x 4 float32: 136 us with
+// the tail's registers, 115 with the loop's; 2000 of 200 x 64: 1600 and 1520; 2000 of
+// 300 x 64: 3309 and 2974).
+template <typename Real> constexpr int forward_ctas(int pt, int sv, int dp, int minb) {
+    const bool wide = sizeof(Real) == 8;
+    if (minb > 1 || sv != 2) return minb;
+    if (dp == 0) return pt == 32 ? (wide ? 14 : 16) : (pt == 64 ? (wide ? 8 : 9) : (pt == 128 ? 5 : (pt == 256 && !wide ? 3 : 1)));
+    if (dp == 8 && !wide) return pt == 64 ? 7 : (pt == 128 ? 4 : 1);
+    return 1;
+}
+
 template <typename Real, int PT, int SV, int DP, int MINB>
-__global__ void __launch_bounds__(PT + 32, MINB) hdb_forward_kernel(const __grid_constant__ ForwardArgs args) {
+__global__ void __launch_bounds__(PT + 32, forward_ctas<Real>(PT, SV, DP, MINB)) hdb_forward_kernel(const __grid_constant__ ForwardArgs args) {
     using T = RealTraits<Real>;
     using Key = typename T::Bits;
     constexpr int PW = PT / 32;
