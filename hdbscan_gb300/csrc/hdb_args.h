@@ -11,6 +11,18 @@ enum Status : int32_t {
     kInternal = 4,     // device-side bounds check tripped (a bug, never expected)
 };
 
+// The general path behind the sparse one does the windows of `queue` whose flag is in
+// `mask` (bit f for flag f): 1 = left it by the core distances, 2 = later.  flags[n]
+// and flags[n + 1] tell whether any window has either.  flags null = no such rule, all
+// windows of the launch.
+struct FlaggedWindows {
+    const int32_t* flags;
+    int n;
+    int mask;
+    const int32_t* queue;
+    int n_windows;
+};
+
 struct ForwardArgs {
     const void* X;             // packed [T, D] Real
     const int64_t* offsets;    // [B+1] device
@@ -56,10 +68,7 @@ struct ForwardArgs {
     // broadcast, so every CTA's first wait runs out (nothing is in flight then).
     int64_t wait_limit_ns;
     int stall_first_ticket;
-    // General path behind the sparse one: only windows with a non-zero flag are
-    // done (null = all; only[n_only] = 0: none is).
-    const int32_t* only;
-    int n_only;
+    FlaggedWindows flagged;
 };
 
 // Small-window kernel (hdb_small.cuh): core distances, beside ForwardArgs.
@@ -79,10 +88,7 @@ struct DistanceArgs {
     void* dist;                  // packed blocks
     const int64_t* dist_offsets; // [B]
     int32_t* status;
-    const int32_t* only;         // as ForwardArgs::only, with its windows (no table then)
-    int n_only;
-    const int32_t* queue;
-    int n_windows;
+    FlaggedWindows flagged;      // if set, the work is found in its windows instead of the table
 };
 
 struct CoreArgs {
@@ -98,10 +104,7 @@ struct CoreArgs {
     void* core;                  // [T]
     int32_t* core_nbr;           // [T] or null
     int32_t* status;
-    const int32_t* only;         // as ForwardArgs::only, with its windows (no table then)
-    int n_only;
-    const int32_t* queue;
-    int n_windows;
+    FlaggedWindows flagged;      // if set, the work is found in its windows instead of the table
 };
 
 // Sparse path (hdb_sparse.cuh): one launch group covers the `n_windows` windows
@@ -117,8 +120,9 @@ struct SparseArgs {
     int D;
     int ms;
     int unit_core;
-    int32_t* flags;              // [B+1] 1 = the window takes the general path; [B] = any window does
+    int32_t* flags;              // [B+2] see FlaggedWindows
     int n_flags;                 // B
+    int stage;                   // flag value of the pass: 1 up to the core distances, 2 from the trees on
     int approx;                  // distances are bounded float32 ones (else exact: float32 windows of few dims)
     int gram;                    // bounded squared distances from tensor-core products (else differences)
     float* y;                    // differences: [T, D] input rounded to float32 around each window's first point

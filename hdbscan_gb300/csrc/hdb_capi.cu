@@ -67,7 +67,7 @@ struct SparseGroup {
 
 struct WindowClass {
     const hdb::ForwardVariant* fv = nullptr;
-    bool general = false;      // does the sparse path's flagged windows, after all else
+    int part = -1;             // general part (of flagged windows) that the class belongs to, -1: none
     int x_in_smem = 0;
     int n_arenas = 1;
     hdb::ForwardLayout layout{};
@@ -82,6 +82,22 @@ struct WindowClass {
     size_t n_tiles = 0;
     int tile = 64;             // distance tile edge
     std::vector<CoreLaunch> cores;
+};
+
+// The way back for windows that leave the sparse path, in the form they had without it:
+// their distances and core distances, found on the device, then the classes of
+// their own variants.  One part a group for the windows that have left by their core
+// distances, beside the group's further passes, and the last part for those of all
+// groups that leave later (or, in a plan without the former, at any time).
+struct GeneralPart {
+    int group = -1;            // -1: the last part
+    std::vector<int> windows;
+    int nmax = 0;
+    size_t queue_off = 0;
+    bool distances = false;    // the blocks hold bounds, or those of another precision
+    int tile = 64;
+    const hdb::CoreVariant* cv = nullptr;  // core distances from the blocks (null: not needed)
+    int priority = 0;
 };
 
 }  // namespace
@@ -102,6 +118,7 @@ struct hdb_plan {
     std::vector<WindowClass> classes;
     std::vector<SparseGroup> groups;        // windows on the sparse path, then small ones
     size_t n_sparse = 0;                    // groups of the former
+    std::vector<GeneralPart> parts;
     int list = 0, keep = 0;                 // neighbour list stride and length
     bool gram = false, approx = false;      // bounded distances, from tensor-core products
     int light_cap = 0, star_cap = 0;        // light and star edges per point
@@ -121,8 +138,10 @@ struct hdb_plan {
     int normalize = 0;      // L2-normalise every point first
     bool prepared = false;  // X passes through the producer stage into the workspace
     unsigned char* h_tables = nullptr;      // pinned
-    std::vector<cudaStream_t> aux;          // one per class (empty: everything on the caller's stream)
-    std::vector<cudaEvent_t> events;        // [2i] class i inputs ready, [2i+1] class i done
+    // Streams of the groups, the classes and the general parts but the last, in this
+    // order (null: the caller's stream), and two events each: inputs ready, done.
+    std::vector<cudaStream_t> aux;
+    std::vector<cudaEvent_t> events;
     cudaEvent_t uploaded = nullptr;         // after the latest (uncaptured) upload of h_tables
     cudaGraphExec_t graph = nullptr;
     // Serializes the host-side enqueue of forward, capture and backward calls:
@@ -184,7 +203,7 @@ bool sparse_pays(int n, int D, bool unit, size_t many) {
 constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
-constexpr int kGeneralGrid = 152 * 4;  // CTAs of a general-path launch that may find nothing to do
+constexpr int kGeneralCtas = 4;  // CTAs an SM of a general launch that may find nothing to do
 
 // Windows of one bin share their launches; shared memory, threads and grids
 // are sized by the largest.
@@ -353,8 +372,8 @@ int build_plan(hdb_plan* p) {
         chosen[w] = single;
     }
     // The sparse path: float64 windows and float32 windows of the matrix
-    // variant that the table gives one CTA.  All of them share one general
-    // class, which does the windows it flags.
+    // variant that the table gives one CTA.  Those that it flags are done as chosen
+    // above.
     std::vector<char> sparse(p->B, 0);
     int sparse_nmax = 0;
     // Tensor-core products: always for wide float64 points; for float32 they
@@ -383,6 +402,31 @@ int build_plan(hdb_plan* p) {
             sparse_nmax = 0;
         }
     }
+    // The class of `w`, a new one for the first of its variant and layout.
+    auto add_to_class = [&](int w, int part) -> int {
+        const int n = size_of(w);
+        const hdb::ForwardVariant* fv = chosen[w];
+        size_t budget = 0;
+        int rc = smem_budget(fv, optin, per_sm_smem, &budget);
+        if (rc) return rc;
+        hdb::ForwardLayout layout{};
+        if (!fv->layout(n, unit, budget, &layout))
+            return fail(HDB_E_INVALID, "window of " + std::to_string(n) + " points exceeds shared memory");
+        WindowClass* cls = nullptr;
+        for (auto& c : p->classes)
+            if (c.fv == fv && c.x_in_smem == layout.x_in_smem && c.n_arenas == layout.n_arenas && c.part == part) { cls = &c; break; }
+        if (!cls) {
+            p->classes.emplace_back();
+            cls = &p->classes.back();
+            cls->fv = fv;
+            cls->x_in_smem = layout.x_in_smem;
+            cls->n_arenas = layout.n_arenas;
+            cls->part = part;
+        }
+        cls->windows.push_back(w);
+        cls->nmax = std::max(cls->nmax, n);
+        return HDB_OK;
+    };
     for (int w : order) {
         const int n = size_of(w);
         if (small[w]) continue;
@@ -391,30 +435,10 @@ int build_plan(hdb_plan* p) {
             if (p->groups.empty() || sparse_bin(n) != sparse_bin(p->groups.back().nmax)) p->groups.emplace_back();
             p->groups.back().windows.push_back(w);
             p->groups.back().nmax = std::max(p->groups.back().nmax, n);
-            chosen[w] = choose_variant(k, p->precision, sparse_nmax, p->D, unit, true);
-            if (!chosen[w]) return fail(HDB_E_INVALID, "no matrix variant for a window of " + std::to_string(n) + " points");
+            continue;
         }
-        const hdb::ForwardVariant* fv = chosen[w];
-        size_t budget = 0;
-        int rc = smem_budget(fv, optin, per_sm_smem, &budget);
+        const int rc = add_to_class(w, -1);
         if (rc) return rc;
-        hdb::ForwardLayout layout{};
-        if (!fv->layout(sparse[w] ? sparse_nmax : n, unit, budget, &layout))
-            return fail(HDB_E_INVALID, "window of " + std::to_string(n) + " points exceeds shared memory");
-        WindowClass* cls = nullptr;
-        for (auto& c : p->classes)
-            if (c.fv == fv && c.x_in_smem == layout.x_in_smem && c.n_arenas == layout.n_arenas &&
-                c.general == (sparse[w] != 0)) { cls = &c; break; }
-        if (!cls) {
-            p->classes.emplace_back();
-            cls = &p->classes.back();
-            cls->fv = fv;
-            cls->x_in_smem = layout.x_in_smem;
-            cls->n_arenas = layout.n_arenas;
-            cls->general = sparse[w] != 0;
-        }
-        cls->windows.push_back(w);
-        cls->nmax = std::max(cls->nmax, n);
     }
     // Matrix-variant classes with many windows are cut into chunks of the
     // size-sorted queue: each chunk's Prim loops start once its own distance
@@ -423,7 +447,7 @@ int build_plan(hdb_plan* p) {
         std::vector<WindowClass> chunked;
         for (auto& c : p->classes) {
             const size_t W = c.windows.size();
-            const size_t parts = (c.fv->dp == 0 && !c.general && W >= 2 * kMinChunk) ? std::min<size_t>(kChunks, W / kMinChunk) : 1;
+            const size_t parts = (c.fv->dp == 0 && W >= 2 * kMinChunk) ? std::min<size_t>(kChunks, W / kMinChunk) : 1;
             for (size_t part = 0; part < parts; ++part) {
                 WindowClass piece = c;
                 const size_t lo = W * part / parts, hi = W * (part + 1) / parts;
@@ -463,25 +487,58 @@ int build_plan(hdb_plan* p) {
             p->groups.back().windows.push_back(w);
         }
     }
-    std::stable_sort(p->classes.begin(), p->classes.end(), [](const WindowClass& a, const WindowClass& b) {
-        return a.general != b.general ? b.general : a.nmax > b.nmax;
-    });
+    std::stable_sort(p->classes.begin(), p->classes.end(),
+                     [](const WindowClass& a, const WindowClass& b) { return a.nmax > b.nmax; });
+
+    // ---- general parts ------------------------------------------------------
+    if (p->n_sparse) {
+        std::vector<int> all;
+        for (size_t g = 0; g < p->n_sparse; ++g) all.insert(all.end(), p->groups[g].windows.begin(), p->groups[g].windows.end());
+        auto add_part = [&](int group, const std::vector<int>& windows) -> int {
+            GeneralPart part;
+            part.group = group;
+            part.windows = windows;
+            bool matrix = false;
+            for (int w : windows) {
+                part.nmax = std::max(part.nmax, size_of(w));
+                matrix |= chosen[w]->dp == 0;
+                const int rc = add_to_class(w, (int)p->parts.size());
+                if (rc) return rc;
+            }
+            // (Without bounds the sparse path leaves exact distances and core distances.)
+            if (p->approx) {
+                part.distances = matrix || !unit;
+                part.tile = (p->precision == HDB_F32 && part.nmax >= kTile128MinN) ? 128 : 64;
+                if (!unit) part.cv = choose_core(k, p->precision, p->ms, p->D, true);
+            }
+            p->parts.push_back(std::move(part));
+            return HDB_OK;
+        };
+        const bool early = all.size() > 1 && !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS);
+        for (size_t g = 0; early && g < p->n_sparse; ++g) {
+            const int rc = add_part((int)g, p->groups[g].windows);
+            if (rc) return rc;
+        }
+        const int rc = add_part(-1, all);
+        if (rc) return rc;
+    }
 
     // ---- distance blocks and tiles for matrix-variant windows --------------
     p->dist_offsets.assign(p->B, -1);
     p->dist_elems = 0;
+    auto add_block = [&](int w) {
+        const int64_t n = size_of(w), ld = (n + 3) & ~3;
+        p->dist_offsets[w] = p->dist_elems;
+        p->dist_elems += align_up((size_t)(n * ld), 64);
+    };
     for (auto& c : p->classes) {
         c.tiles_first = p->tiles.size() / 3;
-        if (c.fv->dp != 0) continue;
+        if (c.fv->dp != 0 || c.part >= 0) continue;
         // Float32 classes of larger windows take the 128x128 tile kernel.
         c.tile = (p->precision == HDB_F32 && c.nmax >= kTile128MinN) ? 128 : 64;
-        const bool tiles = !c.general;  // found on the device for flagged windows
         for (int w : c.windows) {
-            const int n = size_of(w);
-            const int64_t ld = (n + 3) & ~3;
-            p->dist_offsets[w] = p->dist_elems;
-            p->dist_elems += align_up((size_t)(n * ld), 64);
-            const int t = tiles ? (n + c.tile - 1) / c.tile : 0;
+            add_block(w);
+            const int t = (size_of(w) + c.tile - 1) / c.tile;
             for (int ti = 0; ti < t; ++ti)
                 for (int tj = ti; tj < t; ++tj) {
                     p->tiles.push_back(w);
@@ -491,12 +548,14 @@ int build_plan(hdb_plan* p) {
         }
         c.n_tiles = p->tiles.size() / 3 - c.tiles_first;
     }
+    for (size_t g = 0; g < p->n_sparse; ++g)
+        for (int w : p->groups[g].windows) add_block(w);
 
     // ---- core distances -----------------------------------------------------
     if (!unit) {
         for (auto& c : p->classes) {
             const bool matrix = c.fv->dp == 0;
-            if (c.general && !p->approx) continue;  // the sparse path leaves exact core distances
+            if (c.part >= 0) continue;
             CoreLaunch launch;
             launch.matrix = matrix;
             launch.cv = choose_core(k, p->precision, p->ms, p->D, matrix);
@@ -505,15 +564,13 @@ int build_plan(hdb_plan* p) {
             select.select_rows = hdb::select_rows(c.nmax, real_bytes(p->precision));
             for (int w : c.windows) {
                 const int n = size_of(w);
-                if (c.general) {
-                    // (Rows of flagged windows are found on the device.)
-                } else if (launch.cv) {
+                if (launch.cv) {
                     for (int r = 0; r < n; r += launch.cv->rows) { launch.items.push_back(w); launch.items.push_back(r); }
                 } else {
                     for (int r = 0; r < n; r += select.select_rows) { select.items.push_back(w); select.items.push_back(r); }
                 }
             }
-            if (!launch.items.empty() || c.general) c.cores.push_back(launch);
+            if (!launch.items.empty()) c.cores.push_back(launch);
             if (!select.items.empty()) {
                 select.select_smem = (size_t)select.select_rows * (size_t)c.nmax * (size_t)real_bytes(p->precision);
                 c.cores.push_back(select);
@@ -578,9 +635,13 @@ int build_plan(hdb_plan* p) {
         g.queue_off = queue.size();
         queue.insert(queue.end(), g.windows.begin(), g.windows.end());
     }
+    for (auto& g : p->parts) {
+        g.queue_off = queue.size();
+        queue.insert(queue.end(), g.windows.begin(), g.windows.end());
+    }
     p->t_queue = put(image, cursor, queue);
     if (p->n_sparse) {
-        const std::vector<int32_t> zeros((size_t)p->B + 1, 0);
+        const std::vector<int32_t> zeros((size_t)p->B + 2, 0);
         p->table_offsets.assign(p->B + 1, 0);
         for (size_t i = 0; i < p->n_sparse; ++i)
             for (int w : p->groups[i].windows) {
@@ -660,24 +721,35 @@ int build_plan(hdb_plan* p) {
     HDB_CUDA(cudaEventCreateWithFlags(&p->uploaded, cudaEventDisableTiming));
 
     // ---- streams for concurrent classes ------------------------------------
-    const size_t forks = p->classes.size() + p->groups.size();
-    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && forks > (p->n_sparse ? 2 : 1);
-    if (fork) {
+    // (A plan with one thing to do beside its last part does it on the caller's stream.)
+    const size_t G = p->groups.size(), C = p->classes.size();
+    const size_t lanes = G + C + p->parts.size();
+    size_t regular = 0;
+    for (auto& c : p->classes) regular += c.part < 0;
+    const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && G + regular > 1;
+    if (fork || p->parts.size() > 1) {
         int least = 0, greatest = 0;  // numerically: greatest <= least
         HDB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        for (size_t i = 0; i < forks; ++i) {
-            cudaStream_t s;
-            const size_t g = i < p->groups.size() ? i : i - p->groups.size();
-            const int priority = std::min(least, greatest + (int)g);
-            if (i < p->groups.size()) p->groups[i].priority = priority;
-            else p->classes[g].priority = priority;
-            HDB_CUDA(cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking, priority));
-            p->aux.push_back(s);
-        }
-        for (size_t i = 0; i < 2 * forks; ++i) {
-            cudaEvent_t e;
-            HDB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-            p->events.push_back(e);
+        auto priority = [&](size_t i) { return std::min(least, greatest + (int)i); };
+        p->aux.assign(lanes, nullptr);
+        p->events.assign(2 * lanes, nullptr);
+        for (size_t i = 0; i < lanes; ++i) {
+            int level = 0;
+            if (i < G) {
+                if (!fork) continue;
+                level = p->groups[i].priority = priority(i);
+            } else if (i < G + C) {
+                if (!fork || p->classes[i - G].part >= 0) continue;
+                level = p->classes[i - G].priority = priority(i - G);
+            } else {
+                GeneralPart& part = p->parts[i - G - C];
+                if (part.group < 0) continue;
+                level = part.priority = priority((size_t)part.group);
+                for (auto& c : p->classes)
+                    if (c.part == (int)(i - G - C)) c.priority = level;
+            }
+            HDB_CUDA(cudaStreamCreateWithPriority(&p->aux[i], cudaStreamNonBlocking, level));
+            for (int e = 0; e < 2; ++e) HDB_CUDA(cudaEventCreateWithFlags(&p->events[2 * i + e], cudaEventDisableTiming));
         }
     }
     return HDB_OK;
@@ -764,8 +836,26 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
     if (ex->cl_parent && (!ex->cl_birth || !ex->cl_stability || !ex->cl_selected || !ex->point_parent || !ex->n_clusters))
         return fail(HDB_E_INVALID, "cl_parent needs cl_birth, cl_stability, cl_selected, point_parent, n_clusters");
 
-    const bool fork = !p->aux.empty() && !spans;
-    const int32_t* only = !p->n_sparse ? nullptr : reinterpret_cast<const int32_t*>(ws + p->t_flags);
+    // A lane's own stream, behind the caller's work so far (profiling: the caller's).
+    const size_t n_groups = p->groups.size(), n_classes = p->classes.size();
+    auto has_lane = [&](size_t i) { return !spans && !p->aux.empty() && p->aux[i]; };
+    auto begin_lane = [&](size_t i, cudaStream_t* s) -> int {
+        *s = stream;
+        if (!has_lane(i)) return HDB_OK;
+        *s = p->aux[i];
+        HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
+        HDB_CUDA(cudaStreamWaitEvent(*s, p->events[2 * i], 0));
+        return HDB_OK;
+    };
+    auto end_lane = [&](size_t i) -> int {
+        if (has_lane(i)) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], p->aux[i]));
+        return HDB_OK;
+    };
+    auto join = [&](size_t first, size_t last) -> int {
+        for (size_t i = first; i < last; ++i)
+            if (has_lane(i)) HDB_CUDA(cudaStreamWaitEvent(stream, p->events[2 * i + 1], 0));
+        return HDB_OK;
+    };
     auto forward_args = [&]() {
         hdb::ForwardArgs a{};
         a.X = X;
@@ -799,24 +889,87 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.allow_single = (p->flags & HDB_FLAG_ALLOW_SINGLE) ? 1 : 0;
         return a;
     };
+    // The persistent forward of a class over its queue.
+    auto launch_class = [&](const WindowClass& c, cudaStream_t s, const hdb::FlaggedWindows& flagged) -> int {
+        hdb::ForwardArgs a = forward_args();
+        a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
+        a.queue_len = (int)c.windows.size();
+        a.ticket = reinterpret_cast<int32_t*>(ws + p->t_tickets) + c.ticket;
+        a.x_in_smem = c.x_in_smem;
+        a.n_arenas = c.layout.n_arenas;
+        a.arena_stride = (int)c.layout.arena_stride;
+        a.x_off = (int)c.layout.x_off;
+        a.core_off = (int)c.layout.core_off;
+        a.flagged = flagged;
+        if (p->flags & HDB_FLAG_TEST_STALL) {
+            a.stall_first_ticket = 1;
+            a.wait_limit_ns = 1000000;  // 1 ms
+        }
+        if (spans) HDB_CUDA(spans->begin(HDB_PHASE_FORWARD, s));
+        HDB_CUDA(c.fv->launch(a, c.grid, c.smem, s, c.priority));
+        if (spans) HDB_CUDA(spans->end(s));
+        return HDB_OK;
+    };
+    // A general part: the flagged windows of its queue.
+    auto launch_part = [&](size_t i, cudaStream_t s, int mask) -> int {
+        const GeneralPart& part = p->parts[i];
+        const hdb::FlaggedWindows flagged{reinterpret_cast<const int32_t*>(ws + p->t_flags), p->B, mask,
+                                          reinterpret_cast<const int32_t*>(ws + p->t_queue) + part.queue_off,
+                                          (int)part.windows.size()};
+        const int grid = kGeneralCtas * p->sms;
+        if (part.distances) {
+            hdb::DistanceArgs a{};
+            a.X = X;
+            a.offsets = d_offsets;
+            a.tile = part.tile;
+            a.D = p->D;
+            a.dist = dist;
+            a.dist_offsets = d_dist_off;
+            a.status = status;
+            a.flagged = flagged;
+            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_DISTANCE, s));
+            HDB_CUDA(k.launch_distance(a, grid, s, part.priority));
+            if (spans) HDB_CUDA(spans->end(s));
+        }
+        if (part.cv) {
+            hdb::CoreArgs a{};
+            a.X = X;
+            a.offsets = d_offsets;
+            a.D = p->D;
+            a.ms = p->ms;
+            a.dist = dist;
+            a.dist_offsets = d_dist_off;
+            a.core = core;
+            a.core_nbr = core_nbr;
+            a.status = status;
+            a.flagged = flagged;
+            if (spans) HDB_CUDA(spans->begin(HDB_PHASE_CORE, s));
+            HDB_CUDA(part.cv->launch(a, grid, s, part.priority));
+            if (spans) HDB_CUDA(spans->end(s));
+        }
+        for (const auto& c : p->classes)
+            if (c.part == (int)i) {
+                const int rc = launch_class(c, s, flagged);
+                if (rc) return rc;
+            }
+        return HDB_OK;
+    };
     // ---- sparse path: distances, lists and cores on the caller's stream, the
     // rest of each group on its own ---------------------------------------------
     for (size_t i = 0; i < p->groups.size(); ++i) {
         const SparseGroup& g = p->groups[i];
         if (g.small) {  // whole windows, on a stream of their own
-            cudaStream_t s = stream;
-            if (fork) {
-                s = p->aux[i];
-                HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
-                HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * i], 0));
-            }
+            cudaStream_t s;
+            int rc = begin_lane(i, &s);
+            if (rc) return rc;
             hdb::ForwardArgs fa = forward_args();
             fa.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + g.queue_off;
             const hdb::SmallArgs sa{p->ms, core, core_nbr};
             if (spans) HDB_CUDA(spans->begin(HDB_PHASE_FORWARD, s));
             HDB_CUDA(hdb::small_launch(p->precision, fa, sa, (int)g.windows.size(), g.nmax, s, g.priority));
             if (spans) HDB_CUDA(spans->end(s));
-            if (fork) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], s));
+            rc = end_lane(i);
+            if (rc) return rc;
             continue;
         }
         hdb::SparseArgs a{};
@@ -831,6 +984,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.unit_core = unit ? 1 : 0;
         a.flags = reinterpret_cast<int32_t*>(ws + p->t_flags);
         a.n_flags = p->B;
+        a.stage = 1;
         a.approx = p->approx ? 1 : 0;
         a.gram = p->gram ? 1 : 0;
         a.y = reinterpret_cast<float*>(ws + p->w_y);
@@ -884,12 +1038,19 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         if (!rc) rc = stage(hdb::SparseStage::kRows, HDB_PHASE_CORE, stream);
         if (!rc && wide && !unit) rc = stage(hdb::SparseStage::kCore, HDB_PHASE_CORE, stream);
         if (rc) return rc;
-        cudaStream_t s = stream;
-        if (fork) {
-            s = p->aux[i];
-            HDB_CUDA(cudaEventRecord(p->events[2 * i], stream));
-            HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * i], 0));
+        // Windows that have left so far: beside the other passes.
+        if (p->parts.size() > 1 && !spans) {
+            const size_t lane = n_groups + n_classes + i;
+            cudaStream_t s;
+            rc = begin_lane(lane, &s);
+            if (!rc) rc = launch_part(i, s, 1 << 1);
+            if (!rc) rc = end_lane(lane);
+            if (rc) return rc;
         }
+        a.stage = 2;
+        cudaStream_t s;
+        rc = begin_lane(i, &s);
+        if (rc) return rc;
         rc = stage(hdb::SparseStage::kForest, HDB_PHASE_FORWARD, s);
         if (!rc) rc = stage(hdb::SparseStage::kBetween, HDB_PHASE_FORWARD, s);
         if (!rc) rc = stage(hdb::SparseStage::kTree, HDB_PHASE_FORWARD, s);
@@ -897,28 +1058,14 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         if (!rc && !unit) rc = stage(hdb::SparseStage::kStar, HDB_PHASE_FORWARD, s);
         if (!rc && wide) rc = stage(hdb::SparseStage::kWeights, HDB_PHASE_FORWARD, s);
         if (!rc) rc = stage(hdb::SparseStage::kPrim, HDB_PHASE_FORWARD, s);
+        if (!rc) rc = end_lane(i);
         if (rc) return rc;
-        if (fork) HDB_CUDA(cudaEventRecord(p->events[2 * i + 1], s));
     }
-    auto join = [&](size_t first, size_t last) -> int {
-        if (fork)
-            for (size_t i = first; i < last; ++i) HDB_CUDA(cudaStreamWaitEvent(stream, p->events[2 * i + 1], 0));
-        return HDB_OK;
-    };
-    const size_t n_groups = p->groups.size();
-    size_t joined = 0;
-    for (size_t i = 0; i < p->classes.size(); ++i) {
+    for (size_t i = 0; i < n_classes; ++i) {
         const WindowClass& c = p->classes[i];
-        // The general class (the last one) starts when everything else is done.
-        if (c.general) {
-            int rc = join(0, n_groups + i);
-            if (rc) return rc;
-            joined = n_groups + i;
-        }
-        // Where the sparse path's distances are exact, they and the core distances are there already.
-        const bool have_rows = c.general && !p->approx;
+        if (c.part >= 0) continue;
         // 1. distance blocks of this class's matrix-variant windows (caller's stream)
-        if (c.n_tiles || (c.general && !have_rows)) {
+        if (c.n_tiles) {
             hdb::DistanceArgs a{};
             a.X = X;
             a.offsets = d_offsets;
@@ -930,16 +1077,11 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             a.dist_offsets = d_dist_off;
             a.status = status;
             if (spans) HDB_CUDA(spans->begin(HDB_PHASE_DISTANCE, stream));
-            a.only = c.general ? only : nullptr;
-            a.n_only = p->B;
-            a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
-            a.n_windows = (int)c.windows.size();
-            HDB_CUDA(k.launch_distance(a, c.general ? kGeneralGrid : a.n_tiles, stream, c.priority));
+            HDB_CUDA(k.launch_distance(a, a.n_tiles, stream, c.priority));
             if (spans) HDB_CUDA(spans->end(stream));
         }
         // 2. core distances of its windows (caller's stream)
         for (const auto& cl : c.cores) {
-            if (have_rows) break;
             hdb::CoreArgs a{};
             a.X = X;
             a.offsets = d_offsets;
@@ -954,44 +1096,22 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
             a.core_nbr = core_nbr;
             a.status = status;
             if (spans) HDB_CUDA(spans->begin(HDB_PHASE_CORE, stream));
-            a.only = c.general ? only : nullptr;
-            a.n_only = p->B;
-            a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
-            a.n_windows = (int)c.windows.size();
-            if (cl.cv) HDB_CUDA(cl.cv->launch(a, c.general ? kGeneralGrid : a.n_items, stream, c.priority));
+            if (cl.cv) HDB_CUDA(cl.cv->launch(a, a.n_items, stream, c.priority));
             else HDB_CUDA(k.launch_select(a, a.n_items, cl.select_smem, stream, c.priority));
             if (spans) HDB_CUDA(spans->end(stream));
         }
-        cudaStream_t s = stream;
-        const size_t f = n_groups + i;
-        const bool forked = fork && !c.general;
-        if (forked) {
-            s = p->aux[f];
-            HDB_CUDA(cudaEventRecord(p->events[2 * f], stream));
-            HDB_CUDA(cudaStreamWaitEvent(s, p->events[2 * f], 0));
-        }
-        // 3. the persistent forward over its queue
-        hdb::ForwardArgs a = forward_args();
-        a.queue = reinterpret_cast<const int32_t*>(ws + p->t_queue) + c.queue_off;
-        a.queue_len = (int)c.windows.size();
-        a.ticket = reinterpret_cast<int32_t*>(ws + p->t_tickets) + c.ticket;
-        a.x_in_smem = c.x_in_smem;
-        a.n_arenas = c.layout.n_arenas;
-        a.arena_stride = (int)c.layout.arena_stride;
-        a.x_off = (int)c.layout.x_off;
-        a.core_off = (int)c.layout.core_off;
-        a.only = c.general ? only : nullptr;
-        a.n_only = p->B;
-        if (p->flags & HDB_FLAG_TEST_STALL) {
-            a.stall_first_ticket = 1;
-            a.wait_limit_ns = 1000000;  // 1 ms
-        }
-        if (spans) HDB_CUDA(spans->begin(HDB_PHASE_FORWARD, s));
-        HDB_CUDA(c.fv->launch(a, c.grid, c.smem, s, c.priority));
-        if (spans) HDB_CUDA(spans->end(s));
-        if (forked) HDB_CUDA(cudaEventRecord(p->events[2 * f + 1], s));
+        // 3. the persistent forward
+        cudaStream_t s;
+        int rc = begin_lane(n_groups + i, &s);
+        if (!rc) rc = launch_class(c, s, hdb::FlaggedWindows{});
+        if (!rc) rc = end_lane(n_groups + i);
+        if (rc) return rc;
     }
-    return join(joined, n_groups + p->classes.size() - (p->n_sparse ? 1 : 0));
+    // Flagged windows that no other part has done, when all groups are through.
+    int rc = join(0, n_groups);
+    if (!rc && p->n_sparse) rc = launch_part(p->parts.size() - 1, stream, p->parts.size() > 1 && !spans ? 1 << 2 : 1 << 1 | 1 << 2);
+    if (!rc) rc = join(n_groups, n_groups + n_classes + p->parts.size());
+    return rc;
 }
 
 // ---- plan cache of the dense seam -----------------------------------------
@@ -1176,8 +1296,10 @@ int hdb_plan_destroy(hdb_plan_t* p) {
         cudaEventDestroy(p->uploaded);
     }
     if (p->graph) cudaGraphExecDestroy(p->graph);
-    for (auto s : p->aux) cudaStreamDestroy(s);
-    for (auto e : p->events) cudaEventDestroy(e);
+    for (auto s : p->aux)
+        if (s) cudaStreamDestroy(s);
+    for (auto e : p->events)
+        if (e) cudaEventDestroy(e);
     if (p->h_tables) cudaFreeHost(p->h_tables);
     delete p;
     return HDB_OK;
@@ -1191,7 +1313,7 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
                     "\",\"windows\":" + std::to_string(p->B) + ",\"points\":" + std::to_string(p->T) +
                     ",\"dims\":" + std::to_string(p->D) + ",\"workspace_bytes\":" + std::to_string(p->ws_bytes) +
                     ",\"distance_tiles\":" + std::to_string(p->tiles.size() / 3) +
-                    // int32 [windows] in the workspace after a forward: 1 = the window left the sparse path.
+                    // int32 [windows] in the workspace after a forward: not 0 = the window left the sparse path.
                     ",\"general_flags_offset\":" + std::to_string(!p->n_sparse ? -1 : (int64_t)p->t_flags) +
                     ",\"products\":" + (p->n_sparse && p->gram ? "true" : "false") +
                     ",\"classes\":[";
@@ -1213,7 +1335,7 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
     }
     for (size_t i = 0; i < p->classes.size(); ++i) {
         const auto& c = p->classes[i];
-        if (c.general) continue;
+        if (c.part >= 0) continue;
         s += (first_class ? "" : ",") + std::string("{\"threads\":") + std::to_string(c.fv->threads) +
              ",\"vertices_per_thread\":" + std::to_string(c.fv->v) + ",\"register_dims\":" +
              std::to_string(c.fv->dp) + ",\"cluster\":" + std::to_string(c.fv->cluster) +
@@ -1232,7 +1354,7 @@ int hdb_plan_describe(const hdb_plan_t* p, char* buffer, size_t size) {
     bool first = true;
     for (const auto& cls : p->classes)
         for (const auto& c : cls.cores) {
-            if (cls.general) continue;
+            if (cls.part >= 0) continue;
             s += (first ? "" : ",") + std::string("{\"kernel\":\"") +
                  (c.cv ? (c.matrix ? "core_matrix" : "core_points") : "core_select") + "\",\"k\":" +
                  std::to_string(c.cv ? c.cv->k : 0) + ",\"register_dims\":" + std::to_string(c.cv ? c.cv->dp : 0) +

@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(PT + 32, 1) hdb_cluster_forward_kernel(const _
     int homes = 0;
     for (int k = 0; k < (1 << 30); ++k) {
         if (rank == 0 && tid == 0 && !(args.stall_first_ticket && k == 0)) {
-            const int item = s_abort ? args.queue_len : atomicAdd(args.ticket, 1);
+            const int item = s_abort ? args.queue_len : next_ticket(args);
 #pragma unroll
             for (uint32_t r = 0; r < (uint32_t)CS; ++r) {
                 st_cluster_u32(map_rank(smem_u32(&s_item[k & 1]), r), (uint32_t)item);

@@ -125,4 +125,9 @@ __device__ __forceinline__ void atomic_status(int32_t* status, int32_t code) {
     if (status && code) atomicOr(status, code);
 }
 
+__device__ __forceinline__ bool any_flagged(const FlaggedWindows& f) {
+    return ((f.mask & 2) && f.flags[f.n]) || ((f.mask & 4) && f.flags[f.n + 1]);
+}
+__device__ __forceinline__ bool is_flagged(const FlaggedWindows& f, int w) { return (f.mask >> f.flags[w]) & 1; }
+
 }  // namespace hdb

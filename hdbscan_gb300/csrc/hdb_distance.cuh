@@ -208,24 +208,72 @@ __device__ __forceinline__ void distance_tile(const DistanceArgs& args, int w, i
     if (__syncthreads_or(overflow) && tid == 0) atomic_status(args.status, kOverflow);
 }
 
-// One CTA a tile of the table, or (behind the sparse path, where most launches
-// find no flagged window) a fixed grid over the tiles of the flagged windows.
+// A fixed grid over the work items of the flagged windows, items(n) of a window of n
+// points: their numbers run through all of these windows, so that many small ones
+// keep every CTA busy as well as a few large ones do.  (256 windows at a time: a count
+// each, their running sum, then a search for every item.)
+template <typename Items, typename Do>
+__device__ __forceinline__ void for_flagged(const FlaggedWindows& f, const int64_t* __restrict__ offsets, Items items,
+                                            Do work) {
+    constexpr int kBatch = 256;
+    __shared__ int s_window[kBatch], s_first[kBatch], s_sum[kBatch / 32];
+    if (!any_flagged(f)) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // kBatch threads
+    unsigned before = 0;  // items of earlier batches, modulo the grid
+    for (int i0 = 0; i0 < f.n_windows; i0 += kBatch) {
+        int w = -1, count = 0;
+        if (i0 + tid < f.n_windows) {
+            w = f.queue[i0 + tid];
+            if (is_flagged(f, w)) count = items((int)(offsets[w + 1] - offsets[w]));
+        }
+        int sum = count;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, sum, o);
+            if (lane >= o) sum += y;
+        }
+        __syncthreads();  // the last batch's entries are read no more
+        if (lane == 31) s_sum[warp] = sum;
+        __syncthreads();
+        int total = 0;
+#pragma unroll
+        for (int j = 0; j < kBatch / 32; ++j) {
+            if (j < warp) sum += s_sum[j];
+            total += s_sum[j];
+        }
+        s_window[tid] = w;
+        s_first[tid] = sum - count;
+        __syncthreads();
+        unsigned t = blockIdx.x + (blockIdx.x < before ? gridDim.x : 0u) - before;
+        for (; t < (unsigned)total; t += gridDim.x) {
+            int lo = 0;  // the last window whose items start at or before t
+#pragma unroll
+            for (int step = kBatch / 2; step > 0; step >>= 1)
+                if (s_first[lo + step] <= (int)t) lo += step;
+            work(s_window[lo], (int)t - s_first[lo]);
+        }
+        before = (before + (unsigned)total) % gridDim.x;
+    }
+}
+
+// One CTA a tile of the table, or a fixed grid over the flagged windows' tiles.
 template <typename Tile>
 __device__ __forceinline__ void for_tiles(const DistanceArgs& args, int edge, Tile tile) {
-    if (!args.only) {
+    if (!args.flagged.flags) {
         const int t = blockIdx.x;
         if (t < args.n_tiles) tile(args.tiles[3 * t], args.tiles[3 * t + 1], args.tiles[3 * t + 2]);
         return;
     }
-    if (!args.only[args.n_only]) return;
-    for (int item = 0; item < args.n_windows; ++item) {
-        const int w = args.queue[item];
-        if (!args.only[w]) continue;
-        const int n = (int)(args.offsets[w + 1] - args.offsets[w]);
+    auto tiles = [&](int n) {
         const int side = (n + edge - 1) / edge;
-        for (int t = blockIdx.x; t < side * side; t += gridDim.x)
-            if (t / side <= t % side) tile(w, t / side, t % side);
-    }
+        return side * (side + 1) / 2;
+    };
+    for_flagged(args.flagged, args.offsets, tiles, [&](int w, int t) {
+        int tj = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+        while (tj * (tj + 1) / 2 > t) --tj;
+        while ((tj + 1) * (tj + 2) / 2 <= t) ++tj;
+        tile(w, t - tj * (tj + 1) / 2, tj);
+    });
 }
 
 template <typename Real>
@@ -604,19 +652,14 @@ __device__ __forceinline__ void core_rows_item(const CoreArgs& args, int w, int 
 // One CTA an item of the table, or a fixed grid over the flagged windows' rows.
 template <typename Real, int K>
 __global__ void __launch_bounds__(32 * kCoreRowsWarps) hdb_core_rows_kernel(const CoreArgs args) {
-    if (!args.only) {
+    static_assert(32 * kCoreRowsWarps == 256, "threads of for_flagged");
+    if (!args.flagged.flags) {
         if ((int)blockIdx.x < args.n_items)
             core_rows_item<Real, K>(args, args.items[2 * blockIdx.x], args.items[2 * blockIdx.x + 1]);
         return;
     }
-    if (!args.only[args.n_only]) return;
-    for (int item = 0; item < args.n_windows; ++item) {
-        const int w = args.queue[item];
-        if (!args.only[w]) continue;
-        const int n = (int)(args.offsets[w + 1] - args.offsets[w]);
-        for (int r0 = kCoreMatrixRows * blockIdx.x; r0 < n; r0 += kCoreMatrixRows * gridDim.x)
-            core_rows_item<Real, K>(args, w, r0);
-    }
+    for_flagged(args.flagged, args.offsets, [](int n) { return (n + kCoreMatrixRows - 1) / kCoreMatrixRows; },
+                [&](int w, int t) { core_rows_item<Real, K>(args, w, kCoreMatrixRows * t); });
 }
 
 // Any ms: a CTA of 8 warps takes args.rows (1 to 8) rows of a window, computes

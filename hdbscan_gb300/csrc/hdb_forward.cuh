@@ -427,12 +427,12 @@ __device__ __noinline__ void tree_window(const ForwardArgs& args, unsigned char*
 // Next window of the queue for this CTA (queue_len = none left).  Behind the
 // sparse path only flagged windows are taken.
 __device__ __forceinline__ int next_ticket(const ForwardArgs& args) {
-    if (!args.only) return atomicAdd(args.ticket, 1);
-    if (!args.only[args.n_only]) return args.queue_len;
+    if (!args.flagged.flags) return atomicAdd(args.ticket, 1);
+    if (!any_flagged(args.flagged)) return args.queue_len;
     int item;
     do {
         item = atomicAdd(args.ticket, 1);
-    } while (item < args.queue_len && !args.only[args.queue[item]]);
+    } while (item < args.queue_len && !is_flagged(args.flagged, args.queue[item]));
     return item;
 }
 

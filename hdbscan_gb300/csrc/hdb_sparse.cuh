@@ -48,8 +48,8 @@ constexpr int kSparseRowsCta = 32;   // rows per CTA of the neighbour kernel
 constexpr int kLightRows = 16;       // rows per CTA of the light-edge kernel
 
 __device__ __forceinline__ void sparse_flag(const SparseArgs& a, int w) {
-    a.flags[w] = 1;
-    a.flags[a.n_flags] = 1;
+    a.flags[w] = a.stage;
+    a.flags[a.n_flags + a.stage - 1] = 1;
 }
 
 // The window's float32 distance block: its own block (float32), or the first

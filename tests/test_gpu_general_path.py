@@ -1,0 +1,140 @@
+"""Windows that leave the sparse path: the same outputs as without it, in about the same time, in the variants that
+they have without it."""
+
+import json
+
+import numpy as np
+import pytest
+
+from tests.test_gpu_sparse import _mixture
+
+pytestmark = pytest.mark.gpu
+
+
+def _plan(sizes, dims, ms, precision, flags=0, mcs=5):
+    from hdbscan_gb300._cuda import Plan
+
+    offsets = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    return Plan(offsets, dims, min_cluster_size=mcs, min_samples=ms, precision=precision, test_flags=flags)
+
+
+def _forward(plan, X):
+    """All outputs of a forward, and the flags of its windows."""
+    import torch
+
+    workspace = plan.workspace()
+    buffers = plan.export_buffers(hierarchy=True, gradients=True, probabilities=True)
+    for value in buffers.values():
+        value.zero_()
+    labels, status = plan.forward(X, workspace=workspace, exports=buffers)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    at = json.loads(plan.describe())["general_flags_offset"]
+    flags = None if at < 0 else workspace[at:at + 4 * plan.windows].view(torch.int32).cpu().numpy()
+    return dict(buffers, labels=labels), flags
+
+
+def _assert_same(a, b):
+    import torch
+
+    for name in a:
+        assert torch.equal(a[name].contiguous().view(torch.uint8), b[name].contiguous().view(torch.uint8)), name
+
+
+def _milliseconds(plan, X):
+    import torch
+
+    workspace = plan.workspace()
+    times = []
+    for _ in range(7):
+        start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        start.record()
+        plan.forward(X, workspace=workspace)
+        end.record()
+        end.synchronize()
+        times.append(start.elapsed_time(end))
+    return float(np.median(times[2:]))
+
+
+def _repeated(rng, n, dims, copies):
+    x = _mixture(rng, -(-n // copies), dims)
+    return np.tile(x, (copies, 1))[rng.permutation(len(x) * copies)[:n]]
+
+
+def _tied(dims, copies, n_max=None):
+    """`copies` of every unit vector: all distances but zero are equal."""
+    return np.repeat(np.eye(dims), copies, axis=0)[:n_max]
+
+
+@pytest.mark.parametrize("count", [1, 2, 7, 300])
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_windows_that_leave_early_and_late(cuda, precision, count):
+    # 10 copies of a point outnumber the neighbour lists (flag 1); of equal distances between groups of 6 there are
+    # more than the light edges held (flag 2).  300: more windows than one pass over the flags takes.
+    import torch
+
+    from hdbscan_gb300 import _lib
+
+    rng = np.random.default_rng(count)
+    dims = 80 if count < 300 else 66
+    kinds = [(2, _tied(dims, 6)), (1, _tied(dims, 10, 6 * dims)), (0, _mixture(rng, 6 * dims, dims))]
+    order = [(w * w + w // 3) % 3 for w in range(count)]
+    windows = [kinds[i][1][rng.permutation(6 * dims)] for i in order]
+    X = torch.as_tensor(np.concatenate(windows)).to(getattr(torch, precision)).cuda()
+    sizes = [len(x) for x in windows]
+    got, flags = _forward(_plan(sizes, dims, 5, precision), X)
+    want, _ = _forward(_plan(sizes, dims, 5, precision, _lib.HDB_FLAG_NO_SPARSE), X)
+    np.testing.assert_array_equal(flags, [kinds[i][0] for i in order])
+    _assert_same(got, want)
+
+
+@pytest.mark.parametrize("ms", [4, 16])
+def test_many_small_windows(cuda, ms):
+    import torch
+
+    from hdbscan_gb300 import _lib
+
+    rng = np.random.default_rng(5)
+    sizes = rng.integers(33, 201, 1100)
+    X = torch.as_tensor(np.concatenate([_repeated(rng, n, 6, 2 + 10 * (w % 3 > 0) + ms)
+                                        for w, n in enumerate(sizes)])).cuda()
+    sparse, general = _plan(sizes, 6, ms, "float64"), _plan(sizes, 6, ms, "float64", _lib.HDB_FLAG_NO_SPARSE)
+    got, flags = _forward(sparse, X)
+    want, _ = _forward(general, X)
+    assert (flags != 0).mean() > 0.5
+    _assert_same(got, want)
+    # (All on the CTAs that one window's tiles and rows keep busy: 20 times as long.)
+    assert _milliseconds(sparse, X) < 3 * _milliseconds(general, X)
+
+
+@pytest.mark.parametrize("precision, sizes, dims", [
+    ("float32", [999] * 48, 384), ("float32", [2048] * 32, 64), ("float64", [1024] * 32, 8), ("float64", [2048] * 24, 64),
+    ("float64", [4000, 2500, 1300, 700, 300], 32)])
+def test_repeated_rows(cuda, precision, sizes, dims):
+    import torch
+
+    from hdbscan_gb300 import _lib
+
+    rng = np.random.default_rng(dims)
+    X = torch.as_tensor(np.concatenate([_repeated(rng, n, dims, 20) for n in sizes])).to(getattr(torch, precision)).cuda()
+    sparse, general = _plan(sizes, dims, 5, precision), _plan(sizes, dims, 5, precision, _lib.HDB_FLAG_NO_SPARSE)
+    got, flags = _forward(sparse, X)
+    want, _ = _forward(general, X)
+    assert flags.all()
+    _assert_same(got, want)
+    assert _milliseconds(sparse, X) < 1.6 * _milliseconds(general, X)
+
+
+def test_capture_with_flagged_windows(cuda):
+    import torch
+
+    rng = np.random.default_rng(9)
+    windows = [_tied(80, 6), _tied(80, 10, 480), _mixture(rng, 480, 80)]
+    X = torch.as_tensor(np.concatenate(windows)).cuda()
+    plan = _plan([len(x) for x in windows], 80, 5, "float64")
+    labels = plan.forward(X)[0].clone()
+    plan.capture(X)
+    for _ in range(3):
+        replayed, status = plan.replay()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and torch.equal(labels, replayed)
