@@ -53,6 +53,7 @@ def _declare(handle):
         "hdb_version": (ctypes.c_int, []),
         "hdb_last_error": (ctypes.c_char_p, []),
         "hdb_set_tuning": (ctypes.c_int, [_P, ctypes.c_int]),
+        "hdb_set_general_tuning": (ctypes.c_int, [_P, ctypes.c_int]),
         "hdb_get_tuning": (ctypes.c_int, [_P, ctypes.c_int]),
         "hdb_list_variants": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int]),
         "hdb_plan_create": (ctypes.c_int, [ctypes.POINTER(_P), ctypes.c_int, ctypes.c_int, _P, ctypes.c_int,
@@ -82,7 +83,7 @@ def _declare(handle):
 
 
 # Every symbol include/hdbscan_gb300.h declares.
-SYMBOLS = ("hdb_version", "hdb_last_error", "hdb_set_tuning", "hdb_get_tuning", "hdb_list_variants",
+SYMBOLS = ("hdb_version", "hdb_last_error", "hdb_set_tuning", "hdb_set_general_tuning", "hdb_get_tuning", "hdb_list_variants",
            "hdb_plan_create", "hdb_plan_destroy", "hdb_plan_workspace_bytes",
            "hdb_plan_describe", "hdb_plan_forward", "hdb_plan_profile", "hdb_plan_capture", "hdb_plan_replay",
            "hdb_plan_backward",

@@ -6,7 +6,8 @@ to fill every SM, times each compiled variant that can hold such a window
 (`hdb_list_variants`: Prim threads x slots per thread, register dimensions or
 the materialized-matrix variant, CTAs per window) and keeps the fastest.  The result is
 written to autotune_table.json next to this file; the package applies it
-through `hdb_set_tuning` when the library loads.  Replaces the fixed launch
+through `hdb_set_general_tuning` when the library loads (the measurements leave
+the sparse path out, so a cluster rule does not keep a window off it).  Replaces the fixed launch
 choice of the reference (hdbscan_gpu/_cuda.py:82-88).
 
 Run on the target GPU:  python -m hdbscan_gb300.autotune [--quick]
@@ -57,7 +58,7 @@ def apply_table(lib, path: Path | None = None) -> int:
         return 0
     rules = [r["rule"] for r in json.loads(path.read_text())["rules"]]
     arr = _rules_array(rules)
-    rc = lib.hdb_set_tuning(arr.ctypes.data_as(ctypes.c_void_p), len(rules))
+    rc = lib.hdb_set_general_tuning(arr.ctypes.data_as(ctypes.c_void_p), len(rules))
     if rc != 0:
         raise RuntimeError(f"invalid autotune table {path}: {lib.hdb_last_error().decode()}")
     return len(rules)

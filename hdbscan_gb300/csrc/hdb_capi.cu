@@ -229,6 +229,7 @@ struct TuningRule {
     int dims;       // register dimensions; 0 = matrix variant
     int cluster;    // CTAs per window (thread-block cluster size); 1 = single CTA
     int per_sm;     // CTAs per SM of a single-CTA variant (1 or 2)
+    bool binding = true;  // a cluster keeps its windows off the sparse path
 };
 constexpr int kRuleFields = 9;
 
@@ -257,9 +258,11 @@ const hdb::ForwardVariant* find_variant(const hdb::PrecisionKernels& k, int thre
 }
 
 const hdb::ForwardVariant* choose_variant(const hdb::PrecisionKernels& k, int precision, int n, int D,
-                                          bool unit, bool force_matrix, bool allow_cluster = true) {
+                                          bool unit, bool force_matrix, bool allow_cluster = true,
+                                          bool* binding = nullptr) {
     int threads, v;
     class_shape(n, &threads, &v);
+    if (binding) *binding = true;
     if (force_matrix) return find_variant(k, threads, v, 0);
     {
         std::lock_guard<std::mutex> lock(g_tuning_mutex);
@@ -269,7 +272,10 @@ const hdb::ForwardVariant* choose_variant(const hdb::PrecisionKernels& k, int pr
                 (!allow_cluster && r.cluster > 1))
                 continue;
             const hdb::ForwardVariant* f = find_variant(k, r.threads, r.slots, r.dims, r.cluster, r.per_sm);
-            if (f) return f;
+            if (f) {
+                if (binding) *binding = r.binding;
+                return f;
+            }
         }
     }
     // Defaults.  float32 windows above 1024 points with D <= 32 spread their
@@ -352,10 +358,12 @@ int build_plan(hdb_plan* p) {
     std::vector<const hdb::ForwardVariant*> chosen(p->B, nullptr);
     int ctas = 0;  // CTAs the batch occupies at once: one per window, CS per clustered window
     // Small windows: one kernel does them whole.
-    std::vector<char> small(p->B, 0);
+    std::vector<char> small(p->B, 0), binding(p->B, 0);
     const bool special = !(p->flags & kNoSparseFlags);
     for (int w : order) {
-        chosen[w] = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix);
+        bool rule = false;
+        chosen[w] = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix, true, &rule);
+        binding[w] = rule;
         if (!chosen[w]) return fail(HDB_E_INVALID, "no kernel variant for a window of " + std::to_string(size_of(w)) + " points");
         small[w] = special && chosen[w]->cluster == 1 && hdb::small_window(p->precision, size_of(w), p->D, unit, p->B);
         ctas += chosen[w]->cluster;
@@ -372,8 +380,9 @@ int build_plan(hdb_plan* p) {
         chosen[w] = single;
     }
     // The sparse path: float64 windows and float32 windows of the matrix
-    // variant that the table gives one CTA.  Those that it flags are done as chosen
-    // above.
+    // variant (on one CTA: a cluster is one window's way to more SMs, and the sparse
+    // passes have all of them), unless a rule that says so keeps them on a cluster.
+    // Those that it flags are done as chosen above.
     std::vector<char> sparse(p->B, 0);
     int sparse_nmax = 0;
     // Tensor-core products: always for wide float64 points; for float32 they
@@ -388,11 +397,18 @@ int build_plan(hdb_plan* p) {
     p->approx = p->gram || p->precision == HDB_F64;
     p->list = hdb::sparse_list(p->approx, p->gram, p->ms, &p->keep);
     if (p->list && special && hdb::sparse_dims(p->approx, p->D)) {
+        std::vector<int> dims(p->B);  // coordinates in registers, on one CTA
         size_t many = 0;
-        for (int w : order) many += chosen[w]->dp != 0 && chosen[w]->cluster == 1 && size_of(w) >= 512;
+        for (int w : order) {
+            const hdb::ForwardVariant* fv = chosen[w];
+            if (fv->cluster > 1 && !binding[w]) fv = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix, false);
+            dims[w] = fv ? fv->dp : 0;
+            many += dims[w] != 0 && fv && fv->cluster == 1 && size_of(w) >= 512;
+        }
         for (int w : order)
-            sparse[w] = !small[w] && size_of(w) >= kSparseMinN[p->precision != 0] && chosen[w]->cluster == 1 &&
-                        (p->precision == HDB_F64 || chosen[w]->dp == 0 || sparse_pays(size_of(w), p->D, unit, many));
+            sparse[w] = !small[w] && size_of(w) >= kSparseMinN[p->precision != 0] &&
+                        !(chosen[w]->cluster > 1 && binding[w]) &&
+                        (p->precision == HDB_F64 || dims[w] == 0 || sparse_pays(size_of(w), p->D, unit, many));
         for (int w : order)
             if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
         bool fits = true;
@@ -1187,12 +1203,12 @@ extern "C" {
 
 int hdb_version(void) { return HDB_VERSION; }
 
-int hdb_set_tuning(const int32_t* rules, int n_rules) {
+static int set_tuning(const int32_t* rules, int n_rules, bool binding) {
     if (n_rules < 0 || (n_rules > 0 && !rules)) return fail(HDB_E_INVALID, "tuning rules must be a [n, 9] int32 array");
     std::vector<TuningRule> table;
     for (int i = 0; i < n_rules; ++i) {
         const int32_t* r = rules + kRuleFields * i;
-        TuningRule t{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8]};
+        TuningRule t{r[0], r[1], r[2], r[3], r[4], r[5], r[6], r[7], r[8], binding};
         if (t.precision < -1 || t.precision > 1 || t.unit < -1 || t.unit > 1 || t.n_max < 2 || t.d_max < 1 ||
             t.threads < 32 || t.threads % 32 || t.threads > 992 || t.slots < 1 || t.dims < 0 || t.cluster < 1 ||
             t.cluster > 8 || t.per_sm < 1 || t.per_sm > 4)
@@ -1203,6 +1219,9 @@ int hdb_set_tuning(const int32_t* rules, int n_rules) {
     g_tuning = std::move(table);
     return HDB_OK;
 }
+
+int hdb_set_tuning(const int32_t* rules, int n_rules) { return set_tuning(rules, n_rules, true); }
+int hdb_set_general_tuning(const int32_t* rules, int n_rules) { return set_tuning(rules, n_rules, false); }
 
 int hdb_list_variants(int precision, int32_t* out, int capacity) {
     if (precision != HDB_F32 && precision != HDB_F64) return fail(HDB_E_INVALID, "precision must be 'float32' or 'float64'");

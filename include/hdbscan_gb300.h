@@ -146,6 +146,9 @@ const char* hdb_last_error(void);
  * n_rules = 0 restores the defaults.  Replaces the fixed launch choice of
  * hdbscan_gpu/_cuda.py:82-88 (block width, register Prim, shared arena). */
 int hdb_set_tuning(const int32_t* rules, int n_rules);
+/* The same for rules that were measured on the general path alone: a cluster
+ * does not keep a window off the sparse path, and serves it where that ends. */
+int hdb_set_general_tuning(const int32_t* rules, int n_rules);
 
 /* Copies up to `capacity` rules of the current table; returns their count. */
 int hdb_get_tuning(int32_t* rules, int capacity);

@@ -138,3 +138,15 @@ def test_capture_with_flagged_windows(cuda):
         replayed, status = plan.replay()
     torch.cuda.synchronize()
     assert int(status.item()) == 0 and torch.equal(labels, replayed)
+
+
+@pytest.mark.parametrize("precision, n, dims, ms, cluster", [
+    ("float64", 4001, 16, 100, 4), ("float64", 2000, 64, 100, 2), ("float64", 4001, 16, 10, 4), ("float32", 2000, 32, 2, 2)])
+def test_cluster_rules_of_the_table(cuda, precision, n, dims, ms, cluster):
+    # A cluster serves one large window on the general path; the sparse path takes the window all the same.
+    from hdbscan_gb300 import _lib
+
+    classes = json.loads(_plan([n], dims, ms, precision, _lib.HDB_FLAG_NO_SPARSE).describe())["classes"]
+    assert [c["cluster"] for c in classes] == [cluster]
+    classes = json.loads(_plan([n], dims, ms, precision).describe())["classes"]
+    assert [c["variant"] for c in classes] == ["matrix" if ms > 64 else "sparse"]
