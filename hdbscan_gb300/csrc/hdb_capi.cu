@@ -203,6 +203,11 @@ bool sparse_pays(int n, int D, bool unit, size_t many) {
 constexpr double kGramMinWork = 4e9;  // float32: coordinate pairs of a batch from which products pay
 constexpr unsigned kNoSparseFlags =
     HDB_FLAG_FORCE_MATRIX | HDB_FLAG_ONE_PERSISTENT | HDB_FLAG_TEST_STALL | HDB_FLAG_NO_SPARSE;
+// Bytes that the sparse path may add to the workspace: its arrays, which cover all points
+// of the batch, and the blocks of windows that have none without it.  A sixteenth of
+// the device's memory; a batch that needs more (5000 float64 windows of 1500 points 90
+// GB of blocks, 20000 also 30 GB of arrays) has its largest windows on it, or none.
+constexpr size_t kSparseMaxBytes = (size_t)16 << 30;
 constexpr int kGeneralCtas = 4;  // CTAs an SM of a general launch that may find nothing to do
 
 // Windows of one bin share their launches; shared memory, threads and grids
@@ -341,6 +346,52 @@ size_t put(std::vector<unsigned char>& image, size_t& cursor, const std::vector<
     return at;
 }
 
+// Places the sparse path's arrays in the workspace from `ws` on; returns their end.
+size_t sparse_layout(hdb_plan* p, size_t ws, size_t table_entries, size_t dist_elems) {
+    // About one to three of each per point in ordinary data; more send a window to the general path.
+    p->light_cap = 12;
+    const bool unit = p->ms <= 2;
+    const size_t rb = (size_t)real_bytes(p->precision);
+    p->star_cap = unit ? 0 : 8;
+    const size_t per_point = (size_t)(p->light_cap + p->star_cap);
+    const size_t T = (size_t)p->T, L = hdb::kSparseLevels;
+    auto take = [&](size_t bytes) {
+        const size_t at = align_up(ws, 256);
+        ws = at + bytes;
+        return at;
+    };
+    if (p->approx) {
+        if (p->gram) {
+            p->w_split = take(T * 2 * align_up((size_t)p->D, 32) * sizeof(uint16_t));
+            p->w_norm = take(T * sizeof(float));
+            p->w_minima = take(dist_elems / 8 * sizeof(float) + 256);
+        } else {
+            p->w_y = take(T * (size_t)p->D * sizeof(float));
+        }
+        p->w_core_up = take(T * sizeof(float));
+        p->w_core_down = take(T * sizeof(float));
+    }
+    p->w_knn_idx = take(T * (size_t)p->list * sizeof(uint16_t));
+    p->w_knn_d = take(T * (size_t)p->list * sizeof(float));
+    p->w_part = take(T * sizeof(uint16_t));
+    p->w_parts = take((size_t)p->B * sizeof(int32_t));
+    p->w_edges = take(T * sizeof(unsigned long long));
+    p->w_table = take(table_entries * sizeof(unsigned long long));
+    p->w_level_comp = take(T * L * sizeof(uint16_t));
+    p->w_level_max_v = take(T * L * sizeof(float));
+    p->w_level_span = take(T * L * sizeof(uint32_t));
+    p->w_perm = take(T * sizeof(uint16_t));
+    p->w_levels = take((size_t)p->B * sizeof(int32_t));
+    p->w_pos = take(T * sizeof(uint16_t));
+    p->w_light_uv = take(T * (size_t)p->light_cap * sizeof(uint32_t));
+    p->w_light_w = take(T * (size_t)p->light_cap * rb);
+    p->w_star_uv = take(T * (size_t)p->star_cap * sizeof(uint32_t));
+    p->w_star_mask = take(unit ? 0 : T * sizeof(unsigned long long));
+    p->w_edge_rank = take(T * per_point * sizeof(uint16_t));
+    p->w_adj = take(2 * T * per_point * sizeof(uint32_t));
+    return ws;
+}
+
 int build_plan(hdb_plan* p) {
     const hdb::PrecisionKernels& k = *p->k;
     const bool unit = p->ms <= 2;
@@ -409,8 +460,19 @@ int build_plan(hdb_plan* p) {
             sparse[w] = !small[w] && size_of(w) >= kSparseMinN[p->precision != 0] &&
                         !(chosen[w]->cluster > 1 && binding[w]) &&
                         (p->precision == HDB_F64 || dims[w] == 0 || sparse_pays(size_of(w), p->D, unit, many));
+        size_t table_entries = 0;
         for (int w : order)
-            if (sparse[w]) sparse_nmax = std::max(sparse_nmax, size_of(w));
+            if (sparse[w]) table_entries += (size_t)hdb::sparse_parts_cap(size_of(w)) * hdb::sparse_parts_cap(size_of(w));
+        const size_t arrays = sparse_layout(p, 0, table_entries, 0);
+        size_t bytes = arrays;
+        for (int w : order) {  // descending sizes
+            if (!sparse[w]) continue;
+            const size_t n = (size_t)size_of(w), block = n * ((n + 3) & ~(size_t)3);
+            if (chosen[w]->dp != 0) bytes += block * real_bytes(p->precision);
+            if (p->gram) bytes += block / 8 * sizeof(float);  // minima
+            if (bytes > kSparseMaxBytes) sparse[w] = 0;
+            else sparse_nmax = std::max(sparse_nmax, size_of(w));
+        }
         bool fits = true;
         if (sparse_nmax) HDB_CUDA(hdb::sparse_prepare(p->precision, sparse_nmax, (size_t)optin, &fits));
         if (!fits) {
@@ -691,47 +753,7 @@ int build_plan(hdb_plan* p) {
     ws += (size_t)p->dist_elems * rb;
     p->w_prep = ws = align_up(ws, 256);
     if (p->prepared) ws += (size_t)p->T * (size_t)p->D * rb;
-    if (p->n_sparse) {
-        // About one to three of each per point in ordinary data; more send a window to the general path.
-        p->light_cap = 12;
-        p->star_cap = unit ? 0 : 8;
-        const size_t per_point = (size_t)(p->light_cap + p->star_cap);
-        const size_t T = (size_t)p->T, L = hdb::kSparseLevels;
-        auto take = [&](size_t bytes) {
-            const size_t at = align_up(ws, 256);
-            ws = at + bytes;
-            return at;
-        };
-        if (p->approx) {
-            if (p->gram) {
-                p->w_split = take(T * 2 * align_up((size_t)p->D, 32) * sizeof(uint16_t));
-                p->w_norm = take(T * sizeof(float));
-                p->w_minima = take((size_t)p->dist_elems / 8 * sizeof(float) + 256);
-            } else {
-                p->w_y = take(T * (size_t)p->D * sizeof(float));
-            }
-            p->w_core_up = take(T * sizeof(float));
-            p->w_core_down = take(T * sizeof(float));
-        }
-        p->w_knn_idx = take(T * (size_t)p->list * sizeof(uint16_t));
-        p->w_knn_d = take(T * (size_t)p->list * sizeof(float));
-        p->w_part = take(T * sizeof(uint16_t));
-        p->w_parts = take((size_t)p->B * sizeof(int32_t));
-        p->w_edges = take(T * sizeof(unsigned long long));
-        p->w_table = take((size_t)p->table_offsets[p->B] * sizeof(unsigned long long));
-        p->w_level_comp = take(T * L * sizeof(uint16_t));
-        p->w_level_max_v = take(T * L * sizeof(float));
-        p->w_level_span = take(T * L * sizeof(uint32_t));
-        p->w_perm = take(T * sizeof(uint16_t));
-        p->w_levels = take((size_t)p->B * sizeof(int32_t));
-        p->w_pos = take(T * sizeof(uint16_t));
-        p->w_light_uv = take(T * (size_t)p->light_cap * sizeof(uint32_t));
-        p->w_light_w = take(T * (size_t)p->light_cap * rb);
-        p->w_star_uv = take(T * (size_t)p->star_cap * sizeof(uint32_t));
-        p->w_star_mask = take(unit ? 0 : T * sizeof(unsigned long long));
-        p->w_edge_rank = take(T * per_point * sizeof(uint16_t));
-        p->w_adj = take(2 * T * per_point * sizeof(uint32_t));
-    }
+    if (p->n_sparse) ws = sparse_layout(p, ws, (size_t)p->table_offsets[p->B], (size_t)p->dist_elems);
     p->ws_bytes = align_up(std::max<size_t>(ws, 256), 256);
 
     HDB_CUDA(cudaEventCreateWithFlags(&p->uploaded, cudaEventDisableTiming));

@@ -150,3 +150,23 @@ def test_cluster_rules_of_the_table(cuda, precision, n, dims, ms, cluster):
     assert [c["cluster"] for c in classes] == [cluster]
     classes = json.loads(_plan([n], dims, ms, precision).describe())["classes"]
     assert [c["variant"] for c in classes] == ["matrix" if ms > 64 else "sparse"]
+
+
+@pytest.mark.parametrize("precision, sizes, dims, ms, sparse", [
+    ("float64", [1500] * 5000, 6, 5, True),              # 90 GB of distance blocks: room for some windows
+    ("float64", [1500] * 20000, 6, 5, False),            # 30 GB of arrays over all points
+    ("float64", [200] * 200000, 6, 5, False),
+    ("float32", [4000] + [60] * 700000, 4, 5, False),
+    ("float64", [1024] * 64, 8, 5, True)])
+def test_workspace_of_large_batches(cuda, precision, sizes, dims, ms, sparse):
+    # The sparse path adds at most 16 GB (and its rounding) to what the batch takes without it.
+    from hdbscan_gb300 import _lib
+
+    # (Register variants, which have no blocks, as float64 windows of few dims had them.)
+    from tests.test_gpu_cluster import forced_variant
+
+    with forced_variant(precision, 512, 4, 8, 1):
+        plan = _plan(sizes, dims, ms, precision)
+        general = _plan(sizes, dims, ms, precision, _lib.HDB_FLAG_NO_SPARSE)
+    assert plan.workspace_bytes <= general.workspace_bytes + (17 << 30)
+    assert any(c["variant"] == "sparse" for c in json.loads(plan.describe())["classes"]) == sparse
