@@ -217,7 +217,8 @@ __device__ __forceinline__ void for_flagged(const FlaggedWindows& f, const int64
                                             Do work) {
     constexpr int kBatch = 256;
     __shared__ int s_window[kBatch], s_first[kBatch], s_sum[kBatch / 32];
-    if (!any_flagged(f)) return;
+    // (One thread reads for all: another group's passes may set the word meanwhile.)
+    if (!__syncthreads_or(threadIdx.x == 0 && any_flagged(f))) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;  // kBatch threads
     unsigned before = 0;  // items of earlier batches, modulo the grid
     for (int i0 = 0; i0 < f.n_windows; i0 += kBatch) {

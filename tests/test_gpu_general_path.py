@@ -125,6 +125,27 @@ def test_repeated_rows(cuda, precision, sizes, dims):
     assert _milliseconds(sparse, X) < 1.6 * _milliseconds(general, X)
 
 
+@pytest.mark.parametrize("precision", ["float32", "float64"])
+def test_groups_that_flag_while_others_return(cuda, precision):
+    # Windows of several groups: one group's way back starts while the next one's lists are still being looked at.
+    import torch
+
+    from hdbscan_gb300 import _lib
+
+    rng = np.random.default_rng(3)
+    sizes = [int(n) for n in rng.integers(400, 3000, 40)] + [int(n) for n in rng.integers(40, 400, 200)]
+    dims, ms = (40, 5) if precision == "float32" else (6, 4)
+    makers = [lambda n: _mixture(rng, n, dims), lambda n: _repeated(rng, n, dims, 3), lambda n: _repeated(rng, n, dims, 12)]
+    X = torch.as_tensor(np.concatenate([makers[int(rng.integers(0, 20)) // 18 + (w % 37 == 0)](n)
+                                        for w, n in enumerate(sizes)])).to(getattr(torch, precision)).cuda()
+    plan = _plan(sizes, dims, ms, precision)
+    want, _ = _forward(_plan(sizes, dims, ms, precision, _lib.HDB_FLAG_NO_SPARSE), X)
+    for _ in range(20):
+        got, flags = _forward(plan, X)
+        assert flags.any() and not flags.all()
+        _assert_same(got, want)
+
+
 def test_capture_with_flagged_windows(cuda):
     import torch
 
