@@ -135,8 +135,8 @@ def test_groups_that_flag_while_others_return(cuda, precision):
     rng = np.random.default_rng(3)
     sizes = [int(n) for n in rng.integers(400, 3000, 40)] + [int(n) for n in rng.integers(40, 400, 200)]
     dims, ms = (40, 5) if precision == "float32" else (6, 4)
-    makers = [lambda n: _mixture(rng, n, dims), lambda n: _repeated(rng, n, dims, 3), lambda n: _repeated(rng, n, dims, 12)]
-    X = torch.as_tensor(np.concatenate([makers[int(rng.integers(0, 20)) // 18 + (w % 37 == 0)](n)
+    makers = [lambda n: _mixture(rng, n, dims), lambda n: _repeated(rng, n, dims, 3), lambda n: _repeated(rng, n, dims, 20)]
+    X = torch.as_tensor(np.concatenate([makers[2 if w % 37 == 0 else w % 5 // 4](n)
                                         for w, n in enumerate(sizes)])).to(getattr(torch, precision)).cuda()
     plan = _plan(sizes, dims, ms, precision)
     want, _ = _forward(_plan(sizes, dims, ms, precision, _lib.HDB_FLAG_NO_SPARSE), X)
