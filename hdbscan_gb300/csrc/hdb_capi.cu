@@ -187,16 +187,16 @@ constexpr int kTile128MinN = 384;  // float32 matrix classes from this size use 
 // 315, of 512 383 and 421).  In float64 the general form recomputes every distance at
 // two operations a clock on an SM.
 constexpr int kSparseMinN[2] = {384, 16};
-// float32 windows whose general form keeps coordinates in registers (no block):
-// `many` such windows of 512 points or more in the batch.  A dense step then
-// computes its distances on one SM, 0.5 to 1.8 us, but all SMs work at once, while
-// the sparse passes cost about 5 ps a pair of points in all and write the block.
-// Device time, sparse and general form, min_samples 5: one window of 1024 x 16 444
-// and 731 us, of 4000 x 16 1301 and 10148; 24 of 1024 x 4 614 and 944, of 4000 x 4
-// 2962 and 10136; 80 of 1024 x 16 964 and 891; 152 of 2048 x 32 3745 and 6160.  With
-// unit cores 24 of 1024 x 16 586 and 553, of 1536 x 4 769 and 1080.
+// float32 windows whose general form keeps coordinates in registers (no block; at most
+// 1024 points above 16 dims): `many` such windows of 512 points or more in the batch.
+// A dense step then computes its distances on one SM, 0.5 to 3 us, but all SMs work at
+// once, while the sparse passes cost about 5 ps a pair of points in all and write the
+// block.  Device time, sparse and general form, min_samples 5: one window of 1024 x 16
+// 444 and 731 us; 24 of 1024 x 4 614 and 944, of 4000 x 4 2962 and 10136; 80 of
+// 1024 x 16 964 and 891.  With unit cores 24 of 1024 x 16 586 and 553, of 1536 x 4 769
+// and 1080.  (The count is not the cost: more than 24 windows of 4000 points would
+// still be faster in the sparse form.)
 bool sparse_pays(int n, int D, bool unit, size_t many) {
-    if (D > 16 && n >= 1536) return many <= 152;
     return many <= 24 && n >= (D > 16 ? 512 : (unit ? 1536 : 1024));
 }
 
@@ -416,7 +416,7 @@ int build_plan(hdb_plan* p) {
         chosen[w] = choose_variant(k, p->precision, size_of(w), p->D, unit, force_matrix, true, &rule);
         binding[w] = rule;
         if (!chosen[w]) return fail(HDB_E_INVALID, "no kernel variant for a window of " + std::to_string(size_of(w)) + " points");
-        small[w] = special && chosen[w]->cluster == 1 && hdb::small_window(p->precision, size_of(w), p->D, unit, p->B);
+        small[w] = special && chosen[w]->cluster == 1 && hdb::small_window(p->precision, size_of(w), p->D, unit, p->B, p->sms);
         ctas += chosen[w]->cluster;
     }
     // A cluster shortens one window's Prim but holds CS SMs; once the batch

@@ -28,7 +28,7 @@ cudaError_t small_launch(int precision, const ForwardArgs& f, const SmallArgs& s
 
 cudaError_t small_prepare(int precision, int nmax) { return precision == 0 ? prepare<float>(nmax) : prepare<double>(nmax); }
 
-bool small_window(int precision, int n, int D, bool unit_core, int windows) {
+bool small_window(int precision, int n, int D, bool unit_core, int windows, int sms) {
     // One CTA computes all distances, which bounds n^2 D.  float32, device time of a
     // batch here and in the general form: 128 points x 64 dims 91 and 112 us (one
     // window), 189 and 323 us (600); x 256 dims 247 and 144 us (one).  float64 runs
@@ -41,7 +41,7 @@ bool small_window(int precision, int n, int D, bool unit_core, int windows) {
     // Above 96 points two CTAs fill an SM's shared memory; past one wave of them
     // the register form, with no cores to compute, is faster (600 windows of
     // 128 x 4: 132 and 99 us).
-    return !(n > 96 && unit_core && D <= 16 && windows > 2 * 152);
+    return !(n > 96 && unit_core && D <= 16 && windows > 2 * sms);
 }
 
 }  // namespace hdb

@@ -6,9 +6,9 @@
 
 namespace hdb {
 
-// Whether windows of n points and D dims, among `windows` of a batch, belong to
-// the kernel (unit_core: min_samples <= 2).
-bool small_window(int precision, int n, int D, bool unit_core, int windows);
+// Whether windows of n points and D dims, among `windows` of a batch on `sms` SMs,
+// belong to the kernel (unit_core: min_samples <= 2).
+bool small_window(int precision, int n, int D, bool unit_core, int windows, int sms);
 
 // Raises the dynamic shared-memory limit for windows of up to nmax points.
 cudaError_t small_prepare(int precision, int nmax);

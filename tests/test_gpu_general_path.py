@@ -191,3 +191,15 @@ def test_workspace_of_large_batches(cuda, precision, sizes, dims, ms, sparse):
         general = _plan(sizes, dims, ms, precision, _lib.HDB_FLAG_NO_SPARSE)
     assert plan.workspace_bytes <= general.workspace_bytes + (17 << 30)
     assert any(c["variant"] == "sparse" for c in json.loads(plan.describe())["classes"]) == sparse
+
+
+@pytest.mark.parametrize("n, dims, ms, count, sparse", [
+    (1023, 8, 3, 1, False), (1024, 8, 3, 24, True), (1024, 8, 3, 25, False), (1535, 8, 2, 2, False),
+    (1536, 8, 2, 2, True), (4000, 8, 3, 24, True)])
+def test_register_windows_on_the_sparse_path(cuda, n, dims, ms, count, sparse):
+    # The rule by itself: the variant is given, whatever the table says of these sizes.
+    from tests.test_gpu_cluster import forced_variant
+
+    with forced_variant("float32", 512, 8, 8, 1, small=True):
+        classes = json.loads(_plan([n] * count, dims, ms, "float32").describe())["classes"]
+    assert [c["variant"] for c in classes][0] == ("sparse" if sparse else "recompute")
