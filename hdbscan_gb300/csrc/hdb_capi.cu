@@ -86,11 +86,12 @@ struct WindowClass {
 
 // The way back for windows that leave the sparse path, in the form they had without it:
 // their distances and core distances, found on the device, then the classes of
-// their own variants.  One part a group for the windows that have left by their core
-// distances, beside the group's further passes, and the last part for those of all
-// groups that leave later (or, in a plan without the former, at any time).
+// their own variants.  One part a group (one for all groups of small windows) for those
+// that have left by their core distances, beside the groups' further passes, and the
+// last part for those of all groups that leave later (or, in a plan without the
+// former, at any time).
 struct GeneralPart {
-    int group = -1;            // -1: the last part
+    int group = -1;            // starts behind this group's core distances; -1: the last part
     std::vector<int> windows;
     int nmax = 0;
     size_t queue_off = 0;
@@ -138,8 +139,9 @@ struct hdb_plan {
     int normalize = 0;      // L2-normalise every point first
     bool prepared = false;  // X passes through the producer stage into the workspace
     unsigned char* h_tables = nullptr;      // pinned
-    // Streams of the groups, the classes and the general parts but the last, in this
-    // order (null: the caller's stream), and two events each: inputs ready, done.
+    // Streams of the groups, of the classes and kPartStreams for the general parts but
+    // the last, in this order (null: the caller's stream), and two events each: inputs
+    // ready, done.
     std::vector<cudaStream_t> aux;
     std::vector<cudaEvent_t> events;
     cudaEvent_t uploaded = nullptr;         // after the latest (uncaptured) upload of h_tables
@@ -208,6 +210,9 @@ constexpr unsigned kNoSparseFlags =
 // the device's memory; a batch that needs more (5000 float64 windows of 1500 points 90
 // GB of blocks, 20000 also 30 GB of arrays) has its largest windows on it, or none.
 constexpr size_t kSparseMaxBytes = (size_t)16 << 30;
+// General parts take turns on so many streams: the chunks of a group run side by side
+// (on two, 32 windows of 1024 x 8 float64 whose rows repeat took 3.4 ms instead of 2.4).
+constexpr size_t kPartStreams = kChunks;
 constexpr int kGeneralCtas = 4;  // CTAs an SM of a general launch that may find nothing to do
 
 // Windows of one bin share their launches; shared memory, threads and grids
@@ -481,14 +486,13 @@ int build_plan(hdb_plan* p) {
         }
     }
     // The class of `w`, a new one for the first of its variant and layout.
-    auto add_to_class = [&](int w, int part) -> int {
+    auto add_to_class = [&](int w, int part, const hdb::ForwardVariant* fv, int layout_n) -> int {
         const int n = size_of(w);
-        const hdb::ForwardVariant* fv = chosen[w];
         size_t budget = 0;
         int rc = smem_budget(fv, optin, per_sm_smem, &budget);
         if (rc) return rc;
         hdb::ForwardLayout layout{};
-        if (!fv->layout(n, unit, budget, &layout))
+        if (!fv->layout(layout_n, unit, budget, &layout))
             return fail(HDB_E_INVALID, "window of " + std::to_string(n) + " points exceeds shared memory");
         WindowClass* cls = nullptr;
         for (auto& c : p->classes)
@@ -515,7 +519,7 @@ int build_plan(hdb_plan* p) {
             p->groups.back().nmax = std::max(p->groups.back().nmax, n);
             continue;
         }
-        const int rc = add_to_class(w, -1);
+        const int rc = add_to_class(w, -1, chosen[w], n);
         if (rc) return rc;
     }
     // Matrix-variant classes with many windows are cut into chunks of the
@@ -576,11 +580,16 @@ int build_plan(hdb_plan* p) {
             GeneralPart part;
             part.group = group;
             part.windows = windows;
-            bool matrix = false;
+            for (int w : windows) part.nmax = std::max(part.nmax, size_of(w));
+            // Few windows leave late: where others have gone before, one class will do.
+            const hdb::ForwardVariant* one = nullptr;
+            if (group < 0 && !p->parts.empty())
+                for (int w : windows)
+                    if (chosen[w] != chosen[windows[0]]) one = choose_variant(k, p->precision, part.nmax, p->D, unit, true);
+            bool matrix = one != nullptr;
             for (int w : windows) {
-                part.nmax = std::max(part.nmax, size_of(w));
                 matrix |= chosen[w]->dp == 0;
-                const int rc = add_to_class(w, (int)p->parts.size());
+                const int rc = add_to_class(w, (int)p->parts.size(), one ? one : chosen[w], one ? part.nmax : size_of(w));
                 if (rc) return rc;
             }
             // (Without bounds the sparse path leaves exact distances and core distances.)
@@ -593,9 +602,13 @@ int build_plan(hdb_plan* p) {
             return HDB_OK;
         };
         const bool early = all.size() > 1 && !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS);
+        std::vector<int> windows;
         for (size_t g = 0; early && g < p->n_sparse; ++g) {
-            const int rc = add_part((int)g, p->groups[g].windows);
+            windows.insert(windows.end(), p->groups[g].windows.begin(), p->groups[g].windows.end());
+            if (p->groups[g].nmax <= 512 && g + 1 < p->n_sparse) continue;
+            const int rc = add_part((int)g, windows);
             if (rc) return rc;
+            windows.clear();
         }
         const int rc = add_part(-1, all);
         if (rc) return rc;
@@ -761,7 +774,7 @@ int build_plan(hdb_plan* p) {
     // ---- streams for concurrent classes ------------------------------------
     // (A plan with one thing to do beside its last part does it on the caller's stream.)
     const size_t G = p->groups.size(), C = p->classes.size();
-    const size_t lanes = G + C + p->parts.size();
+    const size_t lanes = G + C + (p->parts.empty() ? 0 : std::min(kPartStreams, p->parts.size() - 1));
     size_t regular = 0;
     for (auto& c : p->classes) regular += c.part < 0;
     const bool fork = !(p->flags & HDB_FLAG_NO_GRAPH_STREAMS) && G + regular > 1;
@@ -769,6 +782,11 @@ int build_plan(hdb_plan* p) {
         int least = 0, greatest = 0;  // numerically: greatest <= least
         HDB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
         auto priority = [&](size_t i) { return std::min(least, greatest + (int)i); };
+        for (size_t i = 0; i < p->parts.size(); ++i) {
+            if (p->parts[i].group >= 0) p->parts[i].priority = priority((size_t)p->parts[i].group);
+            for (auto& c : p->classes)
+                if (c.part == (int)i) c.priority = p->parts[i].priority;
+        }
         p->aux.assign(lanes, nullptr);
         p->events.assign(2 * lanes, nullptr);
         for (size_t i = 0; i < lanes; ++i) {
@@ -780,11 +798,7 @@ int build_plan(hdb_plan* p) {
                 if (!fork || p->classes[i - G].part >= 0) continue;
                 level = p->classes[i - G].priority = priority(i - G);
             } else {
-                GeneralPart& part = p->parts[i - G - C];
-                if (part.group < 0) continue;
-                level = part.priority = priority((size_t)part.group);
-                for (auto& c : p->classes)
-                    if (c.part == (int)(i - G - C)) c.priority = level;
+                level = greatest;
             }
             HDB_CUDA(cudaStreamCreateWithPriority(&p->aux[i], cudaStreamNonBlocking, level));
             for (int e = 0; e < 2; ++e) HDB_CUDA(cudaEventCreateWithFlags(&p->events[2 * i + e], cudaEventDisableTiming));
@@ -1077,11 +1091,12 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         if (!rc && wide && !unit) rc = stage(hdb::SparseStage::kCore, HDB_PHASE_CORE, stream);
         if (rc) return rc;
         // Windows that have left so far: beside the other passes.
-        if (p->parts.size() > 1 && !spans) {
-            const size_t lane = n_groups + n_classes + i;
+        for (size_t j = 0; !spans && j + 1 < p->parts.size(); ++j) {
+            if (p->parts[j].group != (int)i) continue;
+            const size_t lane = n_groups + n_classes + j % kPartStreams;
             cudaStream_t s;
             rc = begin_lane(lane, &s);
-            if (!rc) rc = launch_part(i, s, 1 << 1);
+            if (!rc) rc = launch_part(j, s, 1 << 1);
             if (!rc) rc = end_lane(lane);
             if (rc) return rc;
         }
@@ -1148,7 +1163,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
     // Flagged windows that no other part has done, when all groups are through.
     int rc = join(0, n_groups);
     if (!rc && p->n_sparse) rc = launch_part(p->parts.size() - 1, stream, p->parts.size() > 1 && !spans ? 1 << 2 : 1 << 1 | 1 << 2);
-    if (!rc) rc = join(n_groups, n_groups + n_classes + p->parts.size());
+    if (!rc) rc = join(n_groups, p->aux.size());
     return rc;
 }
 
