@@ -130,6 +130,7 @@ struct SparseArgs {
     int dims;                    // D rounded up to 32
     float* minima;               // products: minimum of every 16 entries of the blocks' rows
     float* norm;                 // products: [T] squared norms of the centred points
+    uint32_t* split_share;       // products: [2 B] float bits of the largest |lo|^2 / norm, then |rest|^2 / norm
     uint32_t* range;             // [B] float bits of max |x - x0| (products: of the largest norm)
     void* dist;                  // distance blocks (float32 values, see sparse_block)
     const int64_t* dist_offsets;

@@ -124,7 +124,7 @@ struct hdb_plan {
     bool gram = false, approx = false;      // bounded distances, from tensor-core products
     int light_cap = 0, star_cap = 0;        // light and star edges per point
     std::vector<int64_t> table_offsets;     // per window (entries) of the component tables
-    size_t t_table = 0, t_flags = 0, t_range = 0, t_light_count = 0, t_star_count = 0;
+    size_t t_table = 0, t_flags = 0, t_share = 0, t_range = 0, t_light_count = 0, t_star_count = 0;
     size_t w_y = 0, w_split = 0, w_norm = 0, w_knn_idx = 0, w_knn_d = 0, w_core_up = 0, w_core_down = 0, w_part = 0, w_parts = 0, w_edges = 0, w_table = 0, w_level_comp = 0, w_level_max_v = 0,
            w_level_span = 0, w_perm = 0, w_pos = 0, w_minima = 0, w_levels = 0, w_light_uv = 0, w_light_w = 0,
            w_star_uv = 0, w_star_mask = 0, w_edge_rank = 0, w_adj = 0;
@@ -742,6 +742,7 @@ int build_plan(hdb_plan* p) {
             }
         p->t_table = put(image, cursor, p->table_offsets);
         p->t_flags = put(image, cursor, zeros);
+        p->t_share = put(image, cursor, std::vector<int32_t>(p->gram ? 2 * (size_t)p->B : 0, 0));
         p->t_range = put(image, cursor, zeros);
         p->t_light_count = put(image, cursor, zeros);
         p->t_star_count = put(image, cursor, zeros);
@@ -1043,6 +1044,7 @@ int run_forward(hdb_plan* p, const void* X, int32_t* labels, void* ws_v, int32_t
         a.split = reinterpret_cast<uint16_t*>(ws + p->w_split);
         a.dims = (int)align_up((size_t)p->D, 32);
         a.norm = reinterpret_cast<float*>(ws + p->w_norm);
+        a.split_share = reinterpret_cast<uint32_t*>(ws + p->t_share);
         a.range = reinterpret_cast<uint32_t*>(ws + p->t_range);
         a.dist = dist;
         a.dist_offsets = d_dist_off;

@@ -80,14 +80,17 @@ __device__ __forceinline__ float* sparse_block(const SparseArgs& a, int w) {
 // distances.
 struct SparseBound {
     float up_shift, up_scale, down_shift, down_scale;
+    float eta;  // products
     __device__ __forceinline__ float up(float d) const { return __fmaf_ru(d, up_scale, up_shift); }
     __device__ __forceinline__ float down(float d) const { return __fmaf_rd(d, down_scale, down_shift); }
 };
 
 // Bound of |s~ - d^2| / (n_i + n_j) for s~ = n_i + n_j - 2 g, all in float32:
-//   * z = hi + lo + e with |lo| <= 2^-9 |z|, |e| <= 2^-18 |z| (bfloat16 has 8
-//     significant bits); hi.hi + hi.lo + lo.hi leaves out lo.lo and the products
-//     with e: 3 * 2^-18 |z_i||z_j|;
+//   * z = hi + lo + e; hi.hi + hi.lo + lo.hi leaves out lo.lo and the products with e:
+//     (l^2 + 2 e) |z_i||z_j| with l = |lo| / |z| and e = |e| / |z|.  bfloat16 has 8
+//     significant bits, so l <= 2^-8 and e <= 2^-17 (3.1e-5 in all); over the
+//     coordinates of a point they average to a third of that, and the window's largest
+//     of each, measured as the points are split, are taken;
 //   * each matrix instruction adds 16 exact products to its accumulator; 2^-20 of
 //     the running magnitude a step allows for every operand being cut off at 24
 //     bits below the largest (its rounding is not specified).  The accumulator
@@ -97,8 +100,9 @@ struct SparseBound {
 //     operations: (D / 8 + 32) 2^-24.
 // 2 |z_i||z_j| <= n_i + n_j turns the products' shares into shares of n_i + n_j;
 // 10% on top covers second order terms.
-__device__ __forceinline__ float sparse_eta(int D) {
-    return 1.1f * (3.0f * 3.8146973e-6f + 6.0f * 9.5367432e-7f + (float)(D / 8 + 32) * 5.9604645e-8f);
+__device__ __forceinline__ float sparse_eta(const SparseArgs& a, int w) {
+    const float split = __uint_as_float(a.split_share[w]) + 2.0f * sqrtf(__uint_as_float(a.split_share[a.n_flags + w]));
+    return 1.1f * (split + 6.0f * 9.5367432e-7f + (float)(a.D / 8 + 32) * 5.9604645e-8f);
 }
 
 // Largest relative difference between the square of sparse_exact's value and the
@@ -114,16 +118,16 @@ __device__ __forceinline__ float sparse_chain(int D) {
 
 template <typename Real>
 __device__ __forceinline__ SparseBound sparse_bound(const SparseArgs& a, int w) {
-    if (!a.approx) return SparseBound{0.0f, 1.0f, 0.0f, 1.0f};
+    if (!a.approx) return SparseBound{0.0f, 1.0f, 0.0f, 1.0f, 0.0f};
     const float R = __uint_as_float(a.range[w]);
     if (a.gram) {
         // (4.2 instead of 4: the sums' and the chain's share of the shift itself.)
-        const float chain = sparse_chain<Real>(a.D);
-        return SparseBound{4.2f * sparse_eta(a.D) * R, __fadd_ru(1.0000005f, chain), 0.0f, __fadd_rd(1.0f, -chain)};
+        const float chain = sparse_chain<Real>(a.D), eta = sparse_eta(a, w);
+        return SparseBound{4.2f * eta * R, __fadd_ru(1.0000005f, chain), 0.0f, __fadd_rd(1.0f, -chain), eta};
     }
     const float shift = 1.05f * sqrtf((float)a.D) * 1.1920929e-7f * R;
     const float scale = 1.05f * (0.5f * (float)a.D + 8.0f) * 5.9604645e-8f;
-    return SparseBound{shift, __fadd_ru(1.0f, scale), -shift, __fadd_rd(1.0f, -scale)};
+    return SparseBound{shift, __fadd_ru(1.0f, scale), -shift, __fadd_rd(1.0f, -scale), 0.0f};
 }
 
 // Exact distance of two rows in the reference's order (k-ordered sum).
@@ -232,7 +236,7 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
         if (i >= n) break;
         const Real* __restrict__ x = X + (int64_t)i * D;
         uint16_t* __restrict__ out = a.split + (base + i) * 2 * dims;
-        float norm = 0.0f;
+        float norm = 0.0f, low = 0.0f, rest = 0.0f;  // squared
         bool bad = false, off = false;
         for (int k = lane; k < dims; k += 32) {
             float z = 0.0f;
@@ -243,20 +247,35 @@ __global__ void __launch_bounds__(256) hdb_sparse_split_kernel(const SparseArgs 
                 z = (float)(v - s_centre[k]);
             }
             const __nv_bfloat16 hi = __float2bfloat16_rn(z);
-            const __nv_bfloat16 lo = __float2bfloat16_rn(__fsub_rn(z, __bfloat162float(hi)));
+            const float below = __fsub_rn(z, __bfloat162float(hi));  // exact, as is what is left of it
+            const __nv_bfloat16 lo = __float2bfloat16_rn(below);
+            const float left = __fsub_rn(below, __bfloat162float(lo));
             const int at = (k >> 5) * 64 + (k & 31);
             out[at] = __bfloat16_as_ushort(hi);
             out[at + 32] = __bfloat16_as_ushort(lo);
             norm = __fmaf_rn(z, z, norm);
+            low = __fmaf_rn(__bfloat162float(lo), __bfloat162float(lo), low);
+            rest = __fmaf_rn(left, left, rest);
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) norm += __shfl_xor_sync(0xffffffffu, norm, o);
+        for (int o = 16; o > 0; o >>= 1) {
+            norm += __shfl_xor_sync(0xffffffffu, norm, o);
+            low += __shfl_xor_sync(0xffffffffu, low, o);
+            rest += __shfl_xor_sync(0xffffffffu, rest, o);
+        }
         off = __any_sync(0xffffffffu, off);
         bad = __any_sync(0xffffffffu, bad) || !(norm <= 1.2e24f) || (off && norm < kGramLeastNorm);  // 2^80; also tests NaN
         if (lane == 0) {
             a.norm[base + i] = norm;
-            if (bad) sparse_flag(a, w);
-            else atomicMax(a.range + w, __float_as_uint(norm));
+            if (bad) {
+                sparse_flag(a, w);
+            } else {
+                atomicMax(a.range + w, __float_as_uint(norm));
+                if (norm > 0.0f) {
+                    atomicMax(a.split_share + w, __float_as_uint(low / norm));
+                    atomicMax(a.split_share + a.n_flags + w, __float_as_uint(rest / norm));
+                }
+            }
         }
     }
 }
@@ -317,9 +336,10 @@ __global__ void __launch_bounds__(256, 2) hdb_sparse_gram_kernel(const SparseArg
     const int chunks = a.dims >> 5;
     const uint32_t sbase = (uint32_t)__cvta_generic_to_shared(smem);
     const float inf = __int_as_float(0x7f800000);
+    const float less = 1.0f - sparse_eta(a, w);
     for (int r = tid; r < 2 * TS; r += 256) {
         const int g = (r < TS ? i0 + r : j0 + r - TS);
-        s_norm[r >> 7][r & (TS - 1)] = (g < n ? a.norm[base + g] : inf) * (1.0f - sparse_eta(a.D));
+        s_norm[r >> 7][r & (TS - 1)] = (g < n ? a.norm[base + g] : inf) * less;
     }
     const int row_bytes = 4 * a.dims;
     const int lr = tid >> 3;                      // 2 operands x 128 rows x 8 chunks of 16 bytes
@@ -657,7 +677,7 @@ __device__ __forceinline__ void finish_row(const SparseArgs& a, const SparseBoun
             const float least = bound.down(__uint_as_float(at(pos)));
             const int inside = min(keep, n);
             float up[E], most = 0.0f;
-            const float slack = 2.1f * sparse_eta(a.D);
+            const float slack = 2.1f * bound.eta;
             const float norm_i = a.gram ? a.norm[row_at] : 0.0f;
 #pragma unroll
             for (int h = 0; h < E; ++h) {

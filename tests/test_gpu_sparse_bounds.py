@@ -4,6 +4,8 @@ Each set makes one share of the error as large as it gets; a bound without that 
 and no fallback.
 """
 
+import json
+
 import numpy as np
 import pytest
 
@@ -61,3 +63,34 @@ def test_most_dims_of_narrowed_points(cuda, d, sparse):
     rng = np.random.default_rng(d)
     describe, _ = _check([rng.normal(size=(40, d))], 4, 3, 0.0, "float64")
     assert any(c["variant"] == "sparse" for c in describe["classes"]) == sparse
+
+
+def one_coordinate(windows, n, d, seed):
+    """Points on an axis: what bfloat16 pairs leave of them is one coordinate's rounding, which nothing averages."""
+    rng = np.random.default_rng(seed)
+    x = np.zeros((windows, n, d))
+    x[:, :, 0] = np.cumsum(1.0 + 0.3 * rng.random((windows, n)), axis=1)
+    return rng.permuted(x, axis=1)
+
+
+@pytest.mark.parametrize("precision, d, ms", [("float64", 32, 28)] + [
+    (p, d, ms) for p in ("float32", "float64") for d, ms in ((37, 28), (64, 10), (64, 22))])
+def test_rounding_of_bfloat16_pairs(cuda, precision, d, ms):
+    import torch
+
+    from hdbscan_gb300 import _lib
+    from hdbscan_gb300._cuda import Plan
+
+    windows, n = 300, 900
+    X = torch.as_tensor(one_coordinate(windows, n, d, d + ms).reshape(-1, d)).to(getattr(torch, precision)).cuda()
+    outputs = []
+    for flags in (_lib.HDB_FLAG_FORCE_PRODUCTS, _lib.HDB_FLAG_NO_SPARSE):
+        plan = Plan(np.arange(windows + 1) * n, d, min_cluster_size=5, min_samples=ms, precision=precision, test_flags=flags)
+        assert json.loads(plan.describe())["products"] == (flags == _lib.HDB_FLAG_FORCE_PRODUCTS)
+        buffers = plan.export_buffers(hierarchy=False, gradients=True)
+        labels, status = plan.forward(X, exports=buffers)
+        assert int(status.item()) == 0
+        outputs.append(dict(buffers, labels=labels))
+    for name in outputs[0]:
+        got, want = (o[name].contiguous().view(torch.uint8) for o in outputs)
+        assert torch.equal(got, want), name
